@@ -1,6 +1,7 @@
 """Compiles the CUDA sources into ``boostr_b200/libb200q.so`` for sm_100a with nvcc.
 
-No GPU is needed to build.  ``python -m boostr_b200.build`` (or ``build()``) recompiles
+and the Python entry points (``host_ops.cpp``) into ``boostr_b200/_hostops.so`` against torch's
+headers.  No GPU is needed to build.  ``python -m boostr_b200.build`` (or ``build()``) recompiles
 only the translation units whose sources changed.
 """
 from __future__ import annotations
@@ -10,11 +11,14 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJDIR = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libb200q.so")
+HOST_LIB = os.path.join(HERE, "_hostops.so")
+HOST_SOURCE = os.path.join(CSRC, "host_ops.cpp")
 SOURCES = ["api.cu", "dequant.cu", "gemv.cu", "gemv_m1.cu", "gemv_m1_f32.cu", "kquant_generic.cu", "prefill.cu", "smallm_i8.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -51,6 +55,25 @@ def _compile(src: str, verbose: bool) -> str:
     return obj
 
 
+def _build_host() -> None:
+    header = os.path.join(HERE, "..", "include", "b200q.h")
+    if os.path.exists(HOST_LIB) and os.path.getmtime(HOST_LIB) >= max(os.path.getmtime(HOST_SOURCE), os.path.getmtime(header)):
+        return
+    import torch
+    from torch.utils.cpp_extension import include_paths
+
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    incs = [*include_paths(), os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           *[f"-I{i}" for i in incs], HOST_SOURCE, "-o", HOST_LIB, f"-L{tlib}", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
+           "-ltorch_python", f"-L{HERE}", "-l:libb200q.so", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("g++ failed on host_ops.cpp")
+
+
 def build(verbose: bool = False, force: bool = False) -> str:
     os.makedirs(OBJDIR, exist_ok=True)
     if force:
@@ -64,6 +87,7 @@ def build(verbose: bool = False, force: bool = False) -> str:
         if r.returncode:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    _build_host()
     return LIB
 
 

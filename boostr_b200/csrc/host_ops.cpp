@@ -1,0 +1,376 @@
+// Python entry points of the quantized operators, as a CPython extension (boostr_b200/_hostops.so).
+//
+// A decode-sized product keeps the GPU busy for 2-15 us, and the Python form of a call (argument checks on torch tensors,
+// ctypes conversions, device and stream context managers, the scratch look-up) took 12-16 us of host time, so eager calls
+// were bound by it: Q4_0 4096 x 4096 at M = 1 ran at 16.1 us a call around a 4.9 us kernel.  Here a call is one
+// METH_FASTCALL function: it reads the tensors' fields, allocates the output from torch's caching allocator, takes the
+// scratch buffer of (device, stream) and enters the C ABI (include/b200q.h); nothing is kept from one call for the next.
+//
+// Only well-formed calls are served: anything unusual (a tensor subclass, a non-contiguous or misaligned activation, a
+// shape or type the operators reject) returns NotImplemented and the Python form of the operator takes the call, which
+// also raises the error texts.  A non-zero status of the C ABI is returned as an int and raised by the caller.
+#include <Python.h>
+
+#include <ATen/core/Tensor.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <algorithm>
+#include <map>
+#include <memory>
+#include <mutex>
+#include <optional>
+#include <utility>
+#include <vector>
+
+#include "../../include/b200q.h"
+
+namespace {
+
+// What the C ABI needs of a QuantTensor; held by its Python object as a capsule.
+struct WeightRef {
+    at::Tensor storage;
+    int format = 0;
+    bool matrix = false;   // a 2-D [n, k] weight
+    size_t n = 0, k = 0;
+    std::vector<int64_t> shape;
+    size_t numel = 0;
+};
+constexpr const char* CAPSULE = "boostr_b200.WeightRef";
+PyObject* s_ref = nullptr;  // interned "_ref"
+
+WeightRef* ref_of_capsule(PyObject* o) {
+    if (!PyCapsule_CheckExact(o)) return nullptr;
+    return static_cast<WeightRef*>(PyCapsule_GetPointer(o, CAPSULE));
+}
+// The WeightRef of a QuantTensor; nullptr (no Python error) when the object has none.
+WeightRef* ref_of(PyObject* qt) {
+    PyObject* c = PyObject_GetAttr(qt, s_ref);
+    if (!c) {
+        PyErr_Clear();
+        return nullptr;
+    }
+    WeightRef* r = ref_of_capsule(c);
+    if (!r) PyErr_Clear();
+    Py_DECREF(c);  // the QuantTensor keeps it alive for the duration of the call
+    return r;
+}
+
+// Scratch buffers: one per (device, stream), grown on demand.  Calls on one stream run in order, so they may share a
+// buffer; the entry's mutex keeps the launches of two threads on one stream from interleaving inside a call, and the
+// call's own reference keeps a buffer that another thread replaces alive until its launches are enqueued.
+struct Scratch {
+    std::mutex m;
+    at::Tensor buf;
+};
+std::mutex g_scratch_mutex;
+// never destroyed: its tensors must not outlive the CUDA context at exit
+auto& g_scratch = *new std::map<std::pair<int, cudaStream_t>, std::unique_ptr<Scratch>>;
+Scratch& scratch_of(int device, cudaStream_t st) {
+    std::lock_guard<std::mutex> g(g_scratch_mutex);
+    auto& e = g_scratch[{device, st}];
+    if (!e) e = std::make_unique<Scratch>();
+    return *e;
+}
+
+at::Tensor empty(c10::IntArrayRef shape, at::ScalarType t, c10::Device dev) {
+    return at::Tensor(at::detail::empty_cuda(shape, t, dev, std::nullopt));
+}
+
+int dtype_code(at::ScalarType t) {
+    switch (t) {
+    case at::kFloat: return B200Q_F32;
+    case at::kBFloat16: return B200Q_BF16;
+    case at::kHalf: return B200Q_F16;
+    case at::kDouble: return B200Q_F64;
+    default: return -1;
+    }
+}
+at::ScalarType scalar_type(long code) {
+    return code == B200Q_F32 ? at::kFloat : code == B200Q_BF16 ? at::kBFloat16 : code == B200Q_F16 ? at::kHalf : at::kDouble;
+}
+
+// A contiguous, 16-byte aligned F32 / BF16 CUDA activation [..., k]; false: not one.
+struct Act {
+    const at::Tensor* t = nullptr;
+    size_t m = 0, k = 0;
+    int dt = 0;
+    c10::Device dev{c10::DeviceType::CUDA, 0};
+};
+bool act_of(PyObject* o, Act& a) {
+    if (!THPVariable_CheckExact(o)) return false;
+    const at::Tensor& t = THPVariable_Unpack(o);
+    if (!t.defined() || !t.is_cuda() || t.layout() != at::kStrided || t.dim() < 1 || !t.is_contiguous()) return false;
+    a.dt = dtype_code(t.scalar_type());
+    if (a.dt != B200Q_F32 && a.dt != B200Q_BF16) return false;
+    a.k = (size_t)t.size(-1);
+    if (a.k == 0 || t.numel() == 0 || (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15)) return false;
+    a.m = (size_t)t.numel() / a.k;
+    a.t = &t;
+    a.dev = t.device();
+    return true;
+}
+bool weight_fits(const WeightRef* w, const Act& a) { return w && w->matrix && w->k == a.k && w->storage.device() == a.dev; }
+
+// The output: `given` (validated) or a new tensor [..., n]; false: `given` does not fit.
+bool out_of(PyObject* given, const Act& a, size_t n, at::ScalarType t, at::Tensor& out) {
+    const auto sz = a.t->sizes();
+    if (given == Py_None) {
+        c10::SmallVector<int64_t, 6> shape(sz.begin(), sz.end());
+        shape.back() = (int64_t)n;
+        out = empty(shape, t, a.dev);
+        return true;
+    }
+    if (!THPVariable_CheckExact(given)) return false;
+    out = THPVariable_Unpack(given);
+    if (!out.is_cuda() || out.device() != a.dev || out.scalar_type() != t || !out.is_contiguous() || out.dim() != a.t->dim() ||
+        out.size(-1) != (int64_t)n)
+        return false;
+    for (int64_t i = 0; i + 1 < out.dim(); ++i)
+        if (out.size(i) != sz[i]) return false;
+    return true;
+}
+
+// Makes `dev` current for the scope when it is not (a no-op in a one-GPU process).
+struct DeviceScope {
+    std::optional<c10::cuda::CUDAGuard> guard;
+    explicit DeviceScope(c10::Device d) {
+        if (c10::cuda::current_device() != d.index()) guard.emplace(d);
+    }
+};
+
+// Runs call(scratch pointer, scratch bytes, stream) without the GIL, with at least `need` bytes of scratch.
+template <typename F>
+int with_scratch(c10::Device dev, size_t need, F&& call) {
+    const cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    if (!need) {
+        int rc;
+        Py_BEGIN_ALLOW_THREADS
+        rc = call(static_cast<void*>(nullptr), (size_t)0, st);
+        Py_END_ALLOW_THREADS
+        return rc;
+    }
+    Scratch& s = scratch_of(dev.index(), st);
+    int rc = B200Q_OK;
+    bool oom = false;
+    Py_BEGIN_ALLOW_THREADS
+    {
+        std::lock_guard<std::mutex> g(s.m);
+        if (!s.buf.defined() || (size_t)s.buf.numel() < need) {
+            s.buf = at::Tensor();  // back to the allocator first: a grown buffer may reuse its memory
+            try {
+                s.buf = empty({(int64_t)std::max<size_t>(need, (size_t)1 << 20)}, at::kByte, dev);
+            } catch (...) {
+                oom = true;
+            }
+        }
+        if (!oom) rc = call(s.buf.data_ptr(), (size_t)s.buf.numel(), st);
+    }
+    Py_END_ALLOW_THREADS
+    return oom ? -1 : rc;  // -1: no scratch; the Python form retries and raises torch's own error
+}
+
+PyObject* not_served() { Py_RETURN_NOTIMPLEMENTED; }
+PyObject* result(int rc, const at::Tensor& out) {
+    if (rc == -1) return not_served();
+    if (rc != B200Q_OK) return PyLong_FromLong(rc);
+    return THPVariable_Wrap(out);
+}
+template <typename F>
+PyObject* guarded(F&& f) {  // no C++ exception may cross into the interpreter
+    try {
+        return f();
+    } catch (...) {
+        PyErr_Clear();
+        return not_served();  // the Python form runs the same call and raises what torch raises
+    }
+}
+
+// make_ref(storage, format id, shape) -> capsule
+PyObject* make_ref(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 3 || !THPVariable_Check(args[0]) || !PyTuple_Check(args[2])) {
+        PyErr_SetString(PyExc_TypeError, "make_ref(storage, format, shape)");
+        return nullptr;
+    }
+    auto r = std::make_unique<WeightRef>();
+    r->storage = THPVariable_Unpack(args[0]);
+    r->format = (int)PyLong_AsLong(args[1]);
+    r->numel = 1;
+    for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(args[2]); ++i) {
+        r->shape.push_back((int64_t)PyLong_AsLongLong(PyTuple_GET_ITEM(args[2], i)));
+        r->numel *= (size_t)r->shape.back();
+    }
+    if (PyErr_Occurred()) return nullptr;
+    if (r->shape.size() == 2 && r->storage.is_cuda()) {
+        r->matrix = true;
+        r->n = (size_t)r->shape[0];
+        r->k = (size_t)r->shape[1];
+    }
+    return PyCapsule_New(r.release(), CAPSULE, [](PyObject* c) { delete static_cast<WeightRef*>(PyCapsule_GetPointer(c, CAPSULE)); });
+}
+
+// quant_matmul(act, weight, out dtype code, out or None)
+PyObject* quant_matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        Act a;
+        if (nargs != 4 || !act_of(args[0], a)) return not_served();
+        WeightRef* w = ref_of(args[1]);
+        if (!weight_fits(w, a)) return not_served();
+        const long odt = PyLong_AsLong(args[2]);
+        DeviceScope dev(a.dev);
+        at::Tensor out;
+        if (!out_of(args[3], a, w->n, scalar_type(odt), out)) return not_served();
+        const size_t need = b200q_workspace_bytes(B200Q_OP_QUANT_MATMUL, w->format, a.m, a.k, w->n);
+        const int rc = with_scratch(a.dev, need, [&](void* ws, size_t bytes, cudaStream_t st) {
+            return b200q_quant_matmul(w->format, a.t->data_ptr(), a.dt, w->storage.data_ptr(), out.data_ptr(), (int)odt, a.m, a.k, w->n, ws,
+                                      bytes, st);
+        });
+        return result(rc, out);
+    });
+}
+
+// quant_matmul_batch(act, norm weight or None, eps, weights, out dtype code, outs or None) -> list
+PyObject* quant_matmul_batch(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        Act a;
+        if (nargs != 6 || !act_of(args[0], a)) return not_served();
+        PyObject* seq = args[3];
+        if (!PyList_CheckExact(seq) && !PyTuple_CheckExact(seq)) return not_served();
+        const Py_ssize_t nw = PySequence_Fast_GET_SIZE(seq);
+        if (nw < 1 || nw > 16) return not_served();
+        PyObject* given = args[5];
+        if (given != Py_None && ((!PyList_CheckExact(given) && !PyTuple_CheckExact(given)) || PySequence_Fast_GET_SIZE(given) != nw)) return not_served();
+        const long odt = PyLong_AsLong(args[4]);
+        DeviceScope dev(a.dev);
+        int fmts[16];
+        const void* wp[16];
+        size_t ns[16];
+        void* op[16];
+        at::Tensor outs[16];
+        size_t need = 0;
+        for (Py_ssize_t i = 0; i < nw; ++i) {
+            WeightRef* w = ref_of(PySequence_Fast_GET_ITEM(seq, i));
+            if (!weight_fits(w, a)) return not_served();
+            fmts[i] = w->format;
+            wp[i] = w->storage.data_ptr();
+            ns[i] = w->n;
+            need = std::max(need, b200q_workspace_bytes(B200Q_OP_QUANT_MATMUL, w->format, a.m, a.k, w->n));
+        }
+        const float* norm = nullptr;
+        float eps = 0.f;
+        if (args[1] != Py_None) {
+            if (!THPVariable_CheckExact(args[1])) return not_served();
+            const at::Tensor& t = THPVariable_Unpack(args[1]);
+            if (!t.is_cuda() || t.device() != a.dev || t.scalar_type() != at::kFloat || (size_t)t.numel() != a.k || !t.is_contiguous()) return not_served();
+            norm = t.data_ptr<float>();
+            eps = (float)PyFloat_AsDouble(args[2]);
+            need += (a.m * a.k * 4 + 255) / 256 * 256;
+        }
+        if (PyErr_Occurred()) {
+            PyErr_Clear();
+            return not_served();
+        }
+        for (Py_ssize_t i = 0; i < nw; ++i) {
+            if (!out_of(given == Py_None ? Py_None : PySequence_Fast_GET_ITEM(given, i), a, ns[i], scalar_type(odt), outs[i])) return not_served();
+            op[i] = outs[i].data_ptr();
+        }
+        const int rc = with_scratch(a.dev, need, [&](void* ws, size_t bytes, cudaStream_t st) {
+            if (norm)
+                return b200q_rmsnorm_quant_matmul_batch((int)nw, fmts, wp, ns, op, a.t->data_ptr(), norm, eps, a.dt, (int)odt, a.m, a.k, ws, bytes, st);
+            return b200q_quant_matmul_batch((int)nw, fmts, wp, ns, op, a.t->data_ptr(), a.dt, (int)odt, a.m, a.k, ws, bytes, st);
+        });
+        if (rc == -1) return not_served();
+        if (rc != B200Q_OK) return PyLong_FromLong(rc);
+        PyObject* list = PyList_New(nw);
+        if (!list) return nullptr;
+        for (Py_ssize_t i = 0; i < nw; ++i) {
+            PyObject* o = given == Py_None ? THPVariable_Wrap(outs[i]) : Py_NewRef(PySequence_Fast_GET_ITEM(given, i));
+            if (!o) {
+                Py_DECREF(list);
+                return nullptr;
+            }
+            PyList_SET_ITEM(list, i, o);
+        }
+        return list;
+    });
+}
+
+// quant_swiglu(act, gate, up, out dtype code, out or None)
+PyObject* quant_swiglu(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        Act a;
+        if (nargs != 5 || !act_of(args[0], a)) return not_served();
+        WeightRef *g = ref_of(args[1]), *u = ref_of(args[2]);
+        if (!weight_fits(g, a) || !weight_fits(u, a) || g->format != u->format || g->n != u->n) return not_served();
+        const long odt = PyLong_AsLong(args[3]);
+        DeviceScope dev(a.dev);
+        at::Tensor out;
+        if (!out_of(args[4], a, g->n, scalar_type(odt), out)) return not_served();
+        const size_t need = b200q_workspace_bytes(B200Q_OP_QUANT_SWIGLU, g->format, a.m, a.k, g->n);
+        const int rc = with_scratch(a.dev, need, [&](void* ws, size_t bytes, cudaStream_t st) {
+            return b200q_quant_swiglu(g->format, a.t->data_ptr(), a.dt, g->storage.data_ptr(), u->storage.data_ptr(), out.data_ptr(), (int)odt, a.m,
+                                      a.k, g->n, ws, bytes, st);
+        });
+        return result(rc, out);
+    });
+}
+
+// quant_mlp(act, gate, up, down, out dtype code, out or None)
+PyObject* quant_mlp(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        Act a;
+        if (nargs != 6 || !act_of(args[0], a)) return not_served();
+        WeightRef *g = ref_of(args[1]), *u = ref_of(args[2]), *d = ref_of(args[3]);
+        if (!weight_fits(g, a) || !weight_fits(u, a) || g->format != u->format || g->n != u->n || !d || !d->matrix || d->k != g->n ||
+            d->storage.device() != a.dev)
+            return not_served();
+        const long odt = PyLong_AsLong(args[4]);
+        DeviceScope dev(a.dev);
+        at::Tensor out;
+        if (!out_of(args[5], a, d->n, scalar_type(odt), out)) return not_served();
+        const size_t need = b200q_mlp_workspace_bytes(g->format, d->format, a.m, a.k, g->n, d->n);
+        const int rc = with_scratch(a.dev, need, [&](void* ws, size_t bytes, cudaStream_t st) {
+            return b200q_quant_mlp(g->format, g->storage.data_ptr(), u->storage.data_ptr(), d->format, d->storage.data_ptr(), a.t->data_ptr(), a.dt,
+                                   out.data_ptr(), (int)odt, a.m, a.k, g->n, d->n, ws, bytes, st);
+        });
+        return result(rc, out);
+    });
+}
+
+// dequantize(weight, out dtype code)
+PyObject* dequantize(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        if (nargs != 2) return not_served();
+        WeightRef* w = ref_of(args[0]);
+        if (!w || !w->storage.is_cuda()) return not_served();
+        const long odt = PyLong_AsLong(args[1]);
+        const c10::Device d = w->storage.device();
+        DeviceScope dev(d);
+        at::Tensor out = empty(w->shape, scalar_type(odt), d);
+        const size_t nblocks = w->numel / b200q_block_size(w->format);
+        const int rc = with_scratch(d, 0, [&](void*, size_t, cudaStream_t st) {
+            return b200q_dequantize(w->format, w->storage.data_ptr(), nblocks, out.data_ptr(), (int)odt, st);
+        });
+        return result(rc, out);
+    });
+}
+
+PyMethodDef methods[] = {
+    {"make_ref", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(make_ref)), METH_FASTCALL, nullptr},
+    {"quant_matmul", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(quant_matmul)), METH_FASTCALL, nullptr},
+    {"quant_matmul_batch", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(quant_matmul_batch)), METH_FASTCALL, nullptr},
+    {"quant_swiglu", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(quant_swiglu)), METH_FASTCALL, nullptr},
+    {"quant_mlp", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(quant_mlp)), METH_FASTCALL, nullptr},
+    {"dequantize", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(dequantize)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_hostops", nullptr, -1, methods};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__hostops(void) {
+    s_ref = PyUnicode_InternFromString("_ref");
+    return PyModule_Create(&module);
+}

@@ -7,6 +7,9 @@ and the same error texts as the reference's CUDA implementation
 (src/quant/cuda/quant_matmul/impl_ops.rs:112-172, src/quant/cuda/dequant.rs:74-146).  The
 calls enqueue on torch's current stream and do not synchronise.  torch supplies device
 memory and the stream handle only; all arithmetic happens in ``libb200q.so``.
+
+Well-formed calls go through the compiled entry points of ``_hostops`` (``csrc/host_ops.cpp``); whatever those do not
+serve comes back as ``NotImplemented`` and takes the Python form below, which also words the errors.
 """
 from __future__ import annotations
 
@@ -17,12 +20,21 @@ import torch
 
 from . import _cabi
 from .format import QuantError
-from .tensor import QuantTensor
+from .tensor import QuantTensor, hostops
 
 _DT = {torch.float32: _cabi.DT_F32, torch.bfloat16: _cabi.DT_BF16, torch.float16: _cabi.DT_F16,
        torch.float64: _cabi.DT_F64}
 
 _workspaces: dict = {}
+
+
+def _served(r) -> bool:
+    """Whether a compiled entry point took the call; raises when the library reported an error."""
+    if r is NotImplemented:
+        return False
+    if r.__class__ is int:
+        _cabi.check(r)
+    return True
 
 
 def _stream() -> int:
@@ -45,6 +57,10 @@ def workspace(nbytes: int, device) -> torch.Tensor:
 
 
 def dequantize(qt: QuantTensor, target_dtype: torch.dtype = torch.float32) -> torch.Tensor:
+    if target_dtype in _DT:
+        r = hostops().dequantize(qt, _DT[target_dtype])
+        if _served(r):
+            return r
     if target_dtype not in _DT:
         raise QuantError(f"dequantize target must be float, got {target_dtype}")
     _require_cuda(qt.storage, "QuantTensor")
@@ -89,6 +105,10 @@ def quant_matmul(activation: torch.Tensor, weight: QuantTensor, out_dtype: torch
 
     ``out`` lets the caller supply the result buffer (as boostr's CUDA backend allocates the
     output before the launch); with it the call allocates nothing, which CUDA-graph capture needs."""
+    if out_dtype in _DT and allow_bf16_activation:
+        r = hostops().quant_matmul(activation, weight, _DT[out_dtype], out)
+        if _served(r):
+            return r
     act, m, k, n = _check_act("quant_matmul", activation, weight, allow_bf16_activation)
     out = _out_buffer(out, (*activation.shape[:-1], n), out_dtype, act.device)
     if m == 0:
@@ -161,6 +181,10 @@ def quant_matmul_batch(activation: torch.Tensor, weights: Sequence[QuantTensor],
     """One activation against several weights sharing K (q/k/v, gate/up)."""
     if not weights:
         return []
+    if out_dtype in _DT:
+        r = hostops().quant_matmul_batch(activation, None, 0.0, weights, _DT[out_dtype], outs)
+        if _served(r):
+            return r
     acts = [_check_act("quant_matmul", activation, w, True) for w in weights]
     act, m, k, _ = acts[0]
     outs = [_out_buffer(None if outs is None else outs[i], (*activation.shape[:-1], a[3]), out_dtype, act.device)
@@ -190,6 +214,10 @@ def rmsnorm_quant_matmul_batch(activation: torch.Tensor, norm_weight: torch.Tens
     the normalisation happens inside the decode kernel."""
     if not weights:
         return []
+    if out_dtype in _DT:
+        r = hostops().quant_matmul_batch(activation, norm_weight, eps, weights, _DT[out_dtype], outs)
+        if _served(r):
+            return r
     acts = [_check_act("rmsnorm_quant_matmul", activation, w, True) for w in weights]
     act, m, k, _ = acts[0]
     if norm_weight.dtype != torch.float32 or norm_weight.numel() != k or not norm_weight.is_cuda or not norm_weight.is_contiguous():
@@ -216,6 +244,10 @@ def rmsnorm_quant_matmul_batch(activation: torch.Tensor, norm_weight: torch.Tens
 def quant_swiglu(activation: torch.Tensor, gate_weight: QuantTensor, up_weight: QuantTensor,
                  out_dtype: torch.dtype = torch.float32, out: torch.Tensor = None) -> torch.Tensor:
     """silu(activation x gate^T) * (activation x up^T); gate and up share N, K and format."""
+    if out_dtype in _DT:
+        r = hostops().quant_swiglu(activation, gate_weight, up_weight, _DT[out_dtype], out)
+        if _served(r):
+            return r
     if gate_weight.format != up_weight.format or tuple(gate_weight.shape) != tuple(up_weight.shape):
         raise QuantError("quant_swiglu: gate and up weights must have the same format and shape")
     act, m, k, n = _check_act("quant_swiglu", activation, gate_weight, True)
@@ -252,6 +284,10 @@ def quant_mlp(activation: torch.Tensor, gate_weight: QuantTensor, up_weight: Qua
               out_dtype: torch.dtype = torch.float32, out: torch.Tensor = None) -> torch.Tensor:
     """down(silu(activation x gate^T) * (activation x up^T)): the feed-forward block of a quantized layer
     (src/model/llama/model/blocks_mlp.rs:38-46) as one call; the hidden state stays in scratch."""
+    if out_dtype in _DT:
+        r = hostops().quant_mlp(activation, gate_weight, up_weight, down_weight, _DT[out_dtype], out)
+        if _served(r):
+            return r
     if gate_weight.format != up_weight.format or tuple(gate_weight.shape) != tuple(up_weight.shape):
         raise QuantError("quant_mlp: gate and up weights must have the same format and shape")
     act, m, k, n_ff = _check_act("quant_mlp", activation, gate_weight, True)

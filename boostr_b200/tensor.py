@@ -12,12 +12,29 @@ import torch
 
 from .format import QuantError, QuantFormat
 
+_hostops = None
+
+
+def hostops():
+    """The compiled Python entry points (``csrc/host_ops.cpp``)."""
+    global _hostops
+    if _hostops is None:
+        try:
+            from . import _hostops as mod
+        except ImportError as e:
+            raise ImportError("boostr_b200/_hostops.so cannot be loaded: build it with `python -m boostr_b200.build` "
+                              "(needs nvcc and g++; no GPU required)") from e
+        _hostops = mod
+    return _hostops
+
 
 class QuantTensor:
     def __init__(self, storage: torch.Tensor, fmt: QuantFormat, shape: Sequence[int]):
         self._storage = storage
         self._format = fmt
         self._shape = tuple(int(x) for x in shape)
+        # what the compiled entry points need of this tensor, read once
+        self._ref = hostops().make_ref(storage, fmt.format_id, self._shape)
 
     @classmethod
     def from_bytes(cls, data, fmt, shape: Sequence[int], device="cuda") -> "QuantTensor":
