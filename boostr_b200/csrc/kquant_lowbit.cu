@@ -1,0 +1,814 @@
+// Quantized matmul for Q2_K and Q3_K, every number of activation rows, with the bits of boostr's CPU path
+// (src/quant/cpu/kernels/quant_matmul.rs:107-135): each activation row is quantised to Q8_K
+// (src/quant/cpu/kernels/simd/quantize_act_q8k.rs:26-98), a 256-block contributes
+// (d * d8) * isum - (dmin * d8) * summs with exact integer sums (src/quant/cpu/kernels/simd/fused_q2k_q8k_dot.rs:152-214,
+// fused_q3k_q8k_dot.rs:33-205 in the form x86-64 runs; Q3_K has no min term) and the blocks are added in K order without
+// FMA contraction.
+//
+// What both kernels build on: the PRODUCT of a code and its 16-wide sub-block's scale fits a signed byte (Q2_K: 0..3 times
+// 0..15; Q3_K: -(-4..3) times -32..31 lies in [-128, 124]; the sign is given back by the f32 factor), so the scales go
+// into the operand, a whole 256-block is one K = 256 integer product and only one sum per (row, activation row, block)
+// has to be scaled.  The min term is a second integer product of the mins with the activation's sums of 16 codes, which
+// travel as two bytes, sum = lo + 16 hi.
+//
+//   * kq_act_prep_kernel: codes [M][K], min operand [M][K / 256][lo 16 | hi 16], scales d8 [K / 256][M]: 292 bytes per run;
+//   * kq_tc_kernel<FMT>: tcgen05.mma.kind::i8, tiles of 128 weight rows x up to 128 activation rows;
+//   * kq_small_kernel<FMT, NT>: mma.sync, slabs of 16 weight rows x 8 NT activation rows, for few activation rows.
+#include <cuda.h>
+
+#include <cstdio>
+#include <type_traits>
+
+#include "common.cuh"
+#include "tcgen05_i8.cuh"
+#include "tmap.cuh"
+
+namespace b200q {
+
+namespace {
+
+constexpr uint32_t RUN_BYTES = 292;  // of scratch per (activation row, 256-block): 256 codes, 32 bytes of sums, f32 d8
+
+// Words of a packed block in shared memory.  Blocks are only 4-byte (Q2_K) or 2-byte (Q3_K) aligned in a row: a copy takes
+// the NW words from the 4-byte boundary at or below the block; PITCH is odd, so one word of 32 rows lies in 32 banks.
+__host__ __device__ constexpr uint32_t kq_nw(int fmt) { return fmt == FMT_Q2_K ? 21 : 28; }
+__host__ __device__ constexpr uint32_t kq_pitch(int fmt) { return fmt == FMT_Q2_K ? 21 : 29; }
+
+// One warp per (activation row, 256-block): Q8_K codes (d = amax / 127, id = 127 / amax, round half to even), the sums of
+// 16 codes as lo + 16 hi with lo in [-8, 7] (a sum is at most 2048 in size, so hi fits a signed byte), the scale.
+template <typename InT>
+__global__ void __launch_bounds__(256) kq_act_prep_kernel(const InT* __restrict__ act, uint8_t* __restrict__ codes, uint8_t* __restrict__ mins,
+                                                          float* __restrict__ d8, size_t M, uint32_t nblk) {
+    const int lane = threadIdx.x & 31;
+    grid_dep_launch();
+    grid_dep_wait();  // the activations may be the previous kernel's output; the image may still be read by it
+    const size_t nruns = M * nblk;
+    for (size_t run = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); run < nruns; run += (size_t)gridDim.x * 8) {
+        float v[8];
+        const size_t base = run * 256 + 8 * lane;
+        if constexpr (sizeof(InT) == 4) {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(act + base)), b = __ldg(reinterpret_cast<const float4*>(act + base) + 1);
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        } else {
+            const uint4 r = __ldg(reinterpret_cast<const uint4*>(act + base));
+            v[0] = __uint_as_float(r.x << 16); v[1] = __uint_as_float(r.x & 0xFFFF0000u);
+            v[2] = __uint_as_float(r.y << 16); v[3] = __uint_as_float(r.y & 0xFFFF0000u);
+            v[4] = __uint_as_float(r.z << 16); v[5] = __uint_as_float(r.z & 0xFFFF0000u);
+            v[6] = __uint_as_float(r.w << 16); v[7] = __uint_as_float(r.w & 0xFFFF0000u);
+        }
+        float amax = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+        const float id = amax != 0.f ? __fdiv_rn(127.0f, amax) : 0.f;
+        int c[8], s = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            c[i] = max(-128, min(127, __float2int_rn(__fmul_rn(v[i], id))));  // round half to even, as the AVX2 quantiser
+            s += c[i];
+        }
+        uint32_t w0 = 0, w1 = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            w0 |= (uint32_t)(c[i] & 0xFF) << (8 * i);
+            w1 |= (uint32_t)(c[4 + i] & 0xFF) << (8 * i);
+        }
+        *reinterpret_cast<uint2*>(codes + base) = make_uint2(w0, w1);
+        s += __shfl_xor_sync(0xFFFFFFFFu, s, 1);  // 16 codes = two lanes
+        if ((lane & 1) == 0) {
+            const int hi = (s + 8) >> 4;
+            mins[run * 32 + (lane >> 1)] = (uint8_t)(s - 16 * hi);
+            mins[run * 32 + 16 + (lane >> 1)] = (uint8_t)hi;
+        }
+        const size_t m = run / nblk, b = run % nblk;
+        if (lane == 0) d8[b * M + m] = __fdiv_rn(amax, 127.0f);
+    }
+}
+
+// ------------------------------------------------------------------------------------------ scaled codes of a block
+// Q2_K (src/quant/cpu/kernels/dequant_k_quants/q2k_q3k.rs:13-58): 16 bytes scale | min << 4, 64 code bytes, f16 d, f16 dmin;
+// element 128 n + 32 g + 16 h + l takes bits 2g..2g+1 of code byte 32 n + 16 h + l and the scale of sub-block 8 n + 2 g + h.
+// Four codes (bytes 0..3) times one scale below 16 cannot carry into the next byte.
+template <int G>
+__device__ __forceinline__ uint32_t q2k_scaled(uint32_t w, uint32_t sc) {
+    return ((w >> (2 * G)) & 0x03030303u) * sc;
+}
+// Q3_K (q2k_q3k.rs:64-144): 32 bytes of high bits, 64 code bytes as Q2_K, 12 bytes of 6-bit scales (plus 32), f16 d; the high
+// bit 4 n + g of byte 16 h + l, clear, subtracts 4.  With c = 0..7 and the stored scale u = s + 32, the byte wanted is
+// -s (c - 4) = c (32 - u) + 4 u - 128; c (32 - u) + 4 u lies in 0..252, so the four bytes of a word come out of ONE
+// multiply-add exactly and the 128 is a sign-bit flip.  `hw`: high bits shifted right by 4 n.
+template <int G>
+__device__ __forceinline__ uint32_t q3k_scaled(uint32_t w, uint32_t hw, uint32_t neg_s, uint32_t u4) {
+    const uint32_t high = (G < 2 ? hw << (2 - G) : hw >> (G - 2)) & 0x04040404u;
+    const uint32_t c = ((w >> (2 * G)) & 0x03030303u) | high;
+    return (c * neg_s + u4) ^ 0x80808080u;
+}
+__device__ __forceinline__ uint32_t byte_of(uint32_t x, uint32_t i) { return __byte_perm(x, 0u, 0x4440u | i); }
+
+// ---------------------------------------------------------------------------------------------------- f32x2 arithmetic
+__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// A product that is added to something next.  The assembler fuses a packed multiply (and an FMA with a constant zero) with
+// the packed add behind it, one rounding where the CPU makes two; an FMA with a -0 that it cannot see (a kernel parameter)
+// gives the same value as the product and stays apart.
+__device__ __forceinline__ uint64_t mul2_apart(uint64_t a, uint64_t b, uint64_t neg_zero) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(neg_zero));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t splat2(float x) { return pack2(__float_as_uint(x), __float_as_uint(x)); }
+// Integers below 2^22 in size to f32, exactly: added to the bit pattern of 1.5 * 2^23 they sit in its mantissa.  The sums
+// here are at most 128 * 128 * 256 = 2^22, which this still takes exactly.
+__device__ __forceinline__ uint64_t int2_to_f32(uint32_t a, uint32_t b) {
+    return add2(pack2(a + 0x4B400000u, b + 0x4B400000u), splat2(-12582912.0f));
+}
+
+__device__ __forceinline__ void store_as(void* out, int dt, size_t idx, float v) {
+    if (dt == DT_F32) static_cast<float*>(out)[idx] = v;
+    else if (dt == DT_BF16) static_cast<__nv_bfloat16*>(out)[idx] = __float2bfloat16_rn(v);
+    else static_cast<__half*>(out)[idx] = __float2half_rn(v);
+}
+
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, uint32_t nbytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(nbytes) : "memory");
+}
+// Word `lane` of the block at `blk` (row in range) to dst + 4 lane; the last word is clipped at the tensor's end.
+template <int FMT>
+__device__ __forceinline__ void copy_block_word(uint32_t dst, const uint8_t* blk, const uint8_t* wend, uint32_t lane, bool in, const uint8_t* any) {
+    if (lane >= kq_nw(FMT)) return;
+    const uint8_t* src = blk - (FMT == FMT_Q3_K ? (reinterpret_cast<uintptr_t>(blk) & 2) : 0) + 4 * lane;
+    const uint32_t n = !in ? 0u : (FMT == FMT_Q2_K || src + 4 <= wend) ? 4u : src + 2 <= wend ? 2u : 0u;
+    cp_async4(dst + 4 * lane, in && n ? src : any, n);
+}
+
+// =================================================================================================== tensor-core kernel
+// One CTA per SM, persistent over (128 weight rows, mt activation rows) tiles, all of K each (the sums grow in K order, so
+// no tile is cut).  Per 256-block: two copy warps bring the 128 packed blocks (cp.async: any row alignment), one of two sets
+// of four decode warps writes the scaled codes as two 128-byte-swizzled K-major operand tiles, the activation codes come by
+// TMA, one thread issues 8 MMAs (+ 2 for the mins) into one of two accumulators, and sixteen drain warps (thread = weight
+// row x every fourth group of 8 activation rows) scale the sums in packed f32 and add them to their registers.
+// What bounds it: instruction issue - per (128 rows x 256 K) about 300 instructions a row of decode, and 6 (Q2_K) or 3
+// (Q3_K) a sum of drain - ahead of the tensor pipe.
+struct KqTcParams {
+    const uint8_t* w;
+    void* out;
+    const float* d8;  // [nblk][M]
+    uint32_t M, N, nblk;
+    uint32_t mt;              // activation rows of a tile: a multiple of 16, at most 128
+    uint32_t nct, nunits;     // column tiles; row tiles x column tiles
+    uint32_t row_bytes;
+    uint32_t idesc;
+    int out_dtype;
+    uint64_t neg_zero;        // two f32 -0 (mul2_apart)
+    unsigned int* status;
+};
+
+constexpr int KT_DEC = 8, KT_DRAIN = 16, KT_COPY = 2;
+constexpr int KT_W_COPY = KT_DEC + KT_DRAIN, KT_W_ACT = KT_W_COPY + KT_COPY, KT_W_MMA = KT_W_ACT + 1;
+constexpr int KT_THREADS = (KT_W_MMA + 1) * 32;
+// Every ring has an even depth: the decode sets take the blocks in turn, so a slot belongs to one set, which sees every
+// phase of the slot's barriers (a parity wait cannot tell phase k from k - 2).
+constexpr uint32_t KT_NS = 2, KT_NR = 4, KT_NQ = 4;
+constexpr uint32_t KT_ATOM = 128 * 128;
+constexpr uint32_t KT_REC = 512 + 512;  // the rows' d | dmin, the activation rows' d8
+constexpr int KO_FULL = 0, KO_EMPTY = 16, KO_RAW_FULL = 32, KO_RAW_EMPTY = 64, KO_ACC_FULL = 96, KO_ACC_EMPTY = 112, KO_REC_FULL = 128,
+              KO_REC_EMPTY = 160, KO_TMEM = 192, KO_DEAD = 196, KO_RECS = 1024, KO_STAGES = KO_RECS + KT_NQ * KT_REC;
+// a stage: two operand tiles of scaled codes | tile of mins (Q2_K) | two tiles of activation codes | sums of 16 (Q2_K)
+__host__ __device__ constexpr uint32_t kt_stage(int fmt) { return 4 * KT_ATOM + (fmt == FMT_Q2_K ? KT_ATOM + 128 * 32 : 0); }
+__host__ __device__ constexpr uint32_t kt_raw(int fmt) { return 128 * 4 * kq_pitch(fmt); }
+__host__ __device__ constexpr size_t kt_smem(int fmt) { return 1024 + KO_STAGES + KT_NS * kt_stage(fmt) + KT_NR * kt_raw(fmt); }
+static_assert(KO_STAGES % 1024 == 0 && kt_stage(FMT_Q2_K) % 1024 == 0 && kt_smem(FMT_Q2_K) <= 232448 && kt_smem(FMT_Q3_K) <= 232448, "shared memory");
+
+// rows of 32 bytes with 32-byte swizzle (8-row groups 256 bytes apart)
+__device__ __forceinline__ uint64_t desc_sw32(uint32_t lo) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"((256u >> 4) | (1u << 14) | (6u << 29)));
+    return d;
+}
+
+template <int FMT>
+__global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant__ CUtensorMap tmap_min,
+                                                              const KqTcParams p) {
+    constexpr bool MIN = FMT == FMT_Q2_K;
+    constexpr uint32_t BB = fmt_block_bytes(FMT), PITCH = kq_pitch(FMT), RAW = kt_raw(FMT), STAGE = kt_stage(FMT);
+    constexpr uint32_t OFF_AM = 2 * KT_ATOM, OFF_B = OFF_AM + (MIN ? KT_ATOM : 0), OFF_BM = OFF_B + 2 * KT_ATOM;
+    constexpr uint32_t ACC_COLS = MIN ? 256 : 128, TMEM_COLS = 2 * ACC_COLS;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);  // the launch reserves 1 KB of slack
+    const uint32_t sbase = smem_u32(smem), st_base = sbase + KO_STAGES;
+    constexpr uint32_t OFF_RAW = KO_STAGES + KT_NS * STAGE;
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    volatile uint32_t* dead = reinterpret_cast<volatile uint32_t*>(smem + KO_DEAD);
+    if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < KT_NS; ++s) {
+            mbar_init(sbase + KO_FULL + 8 * s, 5);   // four decode warps + the activation copies (with their byte count)
+            mbar_init(sbase + KO_EMPTY + 8 * s, 1);  // the commit behind the block's MMAs
+        }
+        for (uint32_t s = 0; s < KT_NR; ++s) {
+            mbar_init(sbase + KO_RAW_FULL + 8 * s, KT_COPY * 32);  // every copying thread, once its copies have landed
+            mbar_init(sbase + KO_RAW_EMPTY + 8 * s, 4);
+        }
+        for (uint32_t s = 0; s < 2; ++s) {
+            mbar_init(sbase + KO_ACC_FULL + 8 * s, 1);
+            mbar_init(sbase + KO_ACC_EMPTY + 8 * s, KT_DRAIN);
+        }
+        for (uint32_t s = 0; s < KT_NQ; ++s) {
+            mbar_init(sbase + KO_REC_FULL + 8 * s, 4 + 32);  // four decode warps + the lanes that copy d8
+            mbar_init(sbase + KO_REC_EMPTY + 8 * s, KT_DRAIN);
+        }
+        *dead = 0;
+        mbar_fence_init();
+    }
+    if (warp == KT_W_MMA) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + KO_TMEM), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_before();
+    __syncthreads();
+    tc_after();
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(smem + KO_TMEM);
+    grid_dep_launch();
+    // A wait of a whole warp: all lanes leave together; on a timeout the CTA is marked dead and every role ends.
+    auto wait = [&](uint32_t off, uint32_t parity, unsigned int code) {
+        const bool ok = __all_sync(0xFFFFFFFFu, i8_wait(sbase + off, parity, dead));
+        if (!ok && lane == 0) i8_fail(dead, p.status, code);
+        return ok;
+    };
+    // blocks of this CTA: its units (blockIdx.x, + gridDim.x, ...) one after the other, nblk blocks each
+    const uint32_t units = (p.nunits - blockIdx.x + gridDim.x - 1) / gridDim.x, total = units * p.nblk;
+
+    if (warp >= KT_W_COPY && warp < KT_W_ACT) {
+        // ------------------------------------------------------------ packed blocks (do not depend on the previous kernel)
+        const uint32_t r0 = (uint32_t)(warp - KT_W_COPY) * (128 / KT_COPY);
+        const uint8_t* wend = p.w + (size_t)p.N * p.row_bytes;
+        uint32_t unit = blockIdx.x, b = 0;
+        for (uint32_t i = 0; i < total; ++i) {
+            const uint32_t rs = i % KT_NR;
+            if (!wait(KO_RAW_EMPTY + 8 * rs, ((i / KT_NR) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) break;
+            const uint32_t n0 = unit / p.nct * 128 + r0;
+            const uint8_t* blk = p.w + (size_t)n0 * p.row_bytes + (size_t)b * BB;
+            uint32_t dst = sbase + OFF_RAW + rs * RAW + r0 * PITCH * 4;
+#pragma unroll 8
+            for (uint32_t q = 0; q < 128 / KT_COPY; ++q) {  // rows past N are zero-filled
+                copy_block_word<FMT>(dst, blk, wend, lane, n0 + q < p.N, p.w);
+                blk += p.row_bytes;
+                dst += PITCH * 4;
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(sbase + KO_RAW_FULL + 8 * rs) : "memory");
+            if (++b == p.nblk) { b = 0; unit += gridDim.x; }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else if (warp == KT_W_ACT) {
+        // ------------------------------------------------------------ activation codes, sums and scales (previous kernel's output)
+        grid_dep_wait();
+        uint32_t unit = blockIdx.x, b = 0;
+        for (uint32_t i = 0; i < total; ++i) {
+            const uint32_t s = i % KT_NS, q = i % KT_NQ, m0 = unit % p.nct * p.mt;
+            if (!wait(KO_EMPTY + 8 * s, ((i / KT_NS) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) break;
+            if (lane == 0) {
+                const uint32_t st = st_base + s * STAGE, bar = sbase + KO_FULL + 8 * s;
+                mbar_expect_tx(bar, 256 * p.mt + (MIN ? 32 * p.mt : 0));
+                tma2d(st + OFF_B, &tmap_act, (int)(b * 256), (int)m0, bar);
+                tma2d(st + OFF_B + KT_ATOM, &tmap_act, (int)(b * 256 + 128), (int)m0, bar);
+                if constexpr (MIN) tma2d(st + OFF_BM, &tmap_min, (int)(b * 32), (int)m0, bar);
+            }
+            __syncwarp();
+            if (!wait(KO_REC_EMPTY + 8 * q, ((i / KT_NQ) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) break;
+            const uint32_t dst = sbase + KO_RECS + q * KT_REC + 512;
+            const float* src = p.d8 + (size_t)b * p.M + m0;
+            for (uint32_t m = lane; m < p.mt; m += 32) cp_async4(dst + 4 * m, m0 + m < p.M ? src + m : p.d8, m0 + m < p.M ? 4u : 0u);
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(sbase + KO_REC_FULL + 8 * q) : "memory");
+            if (++b == p.nblk) { b = 0; unit += gridDim.x; }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (*dead) {  // TMA copies in flight land within microseconds: the CTA's shared memory stays until then
+            const uint64_t t0 = global_timer_ns();
+            while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
+        }
+    } else if (warp == KT_W_MMA) {
+        // ------------------------------------------------------------ MMA issue
+        for (uint32_t i = 0; i < total; ++i) {
+            const uint32_t s = i % KT_NS, buf = i & 1;
+            if (!wait(KO_FULL + 8 * s, (i / KT_NS) & 1, STATUS_TIMEOUT_FULL)) break;
+            if (!wait(KO_ACC_EMPTY + 8 * buf, ((i >> 1) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) break;
+            tc_after();
+            if (elect_one_lane()) {
+                const uint32_t st = st_base + s * STAGE, a_lo = desc_lo(st), b_lo = desc_lo(st + OFF_B), d = tmem + buf * ACC_COLS;
+#pragma unroll
+                for (uint32_t k = 0; k < 8; ++k)
+                    tc_mma_i8(d, desc_sw128(a_lo + (k >> 2) * (KT_ATOM >> 4) + 2 * (k & 3)), desc_sw128(b_lo + (k >> 2) * (KT_ATOM >> 4) + 2 * (k & 3)), p.idesc,
+                              k > 0);
+                if constexpr (MIN) {  // sum of 16 = lo + 16 hi: [m | 8 m] . [lo | hi] + [0 | 8 m] . [lo | hi]
+                    const uint32_t am = desc_lo(st + OFF_AM), bm = desc_lo(st + OFF_BM);
+                    tc_mma_i8(d + 128, desc_sw128(am), desc_sw32(bm), p.idesc, false);
+                    tc_mma_i8(d + 128, desc_sw128(am + 2), desc_sw32(bm), p.idesc, true);
+                }
+                tc_commit_to(sbase + KO_EMPTY + 8 * s);       // the stage may be overwritten once these MMAs have read it
+                tc_commit_to(sbase + KO_ACC_FULL + 8 * buf);  // and the sums are complete
+            }
+            __syncwarp();
+        }
+    } else if (warp < KT_DEC) {
+        // ------------------------------------------------------------ decode: one thread per weight row
+        const uint32_t r = threadIdx.x & 127, set = threadIdx.x >> 7, x7 = r & 7;
+        for (uint32_t i = set; i < total; i += 2) {
+            const uint32_t rs = i % KT_NR, s = i % KT_NS, q = i % KT_NQ;
+            if (!wait(KO_RAW_FULL + 8 * rs, (i / KT_NR) & 1, STATUS_TIMEOUT_FULL)) break;
+            const uint32_t* raw = reinterpret_cast<const uint32_t*>(smem + OFF_RAW + rs * RAW) + r * PITCH;
+            uint32_t* rec = reinterpret_cast<uint32_t*>(smem + KO_RECS + q * KT_REC) + r;
+            uint8_t* a0 = smem + KO_STAGES + s * STAGE + (r >> 3) * 1024 + x7 * 128;
+            auto put = [&](uint32_t tile, uint32_t c, uint4 v) { *reinterpret_cast<uint4*>(a0 + tile * KT_ATOM + ((c ^ x7) << 4)) = v; };
+            if (!wait(KO_EMPTY + 8 * s, ((i / KT_NS) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) break;
+            uint32_t dm;
+            // sub-block 8 n + 2 g + h = 16-byte chunk 2 g + h of operand tile n
+            if constexpr (FMT == FMT_Q2_K) {
+                uint32_t scw[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) scw[k] = raw[k];
+                dm = raw[20];
+                uint4 mn = make_uint4((scw[0] >> 4) & 0x0F0F0F0Fu, (scw[1] >> 4) & 0x0F0F0F0Fu, (scw[2] >> 4) & 0x0F0F0F0Fu, (scw[3] >> 4) & 0x0F0F0F0Fu);
+                const uint4 mn8 = make_uint4(mn.x << 3, mn.y << 3, mn.z << 3, mn.w << 3);
+                put(2, 0, mn);
+                put(2, 1, mn8);
+                put(2, 2, make_uint4(0, 0, 0, 0));
+                put(2, 3, mn8);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) scw[k] &= 0x0F0F0F0Fu;
+#pragma unroll
+                for (int nh = 0; nh < 4; ++nh) {
+                    const int n = nh >> 1, h = nh & 1;
+                    const uint32_t w0 = raw[4 + 4 * nh], w1 = raw[5 + 4 * nh], w2 = raw[6 + 4 * nh], w3 = raw[7 + 4 * nh];
+                    auto one = [&](auto gc) {
+                        constexpr int G = decltype(gc)::value;
+                        const uint32_t sc = byte_of(scw[2 * n + (G >> 1)], 2 * (G & 1) + h);
+                        put(n, 2 * G + h, make_uint4(q2k_scaled<G>(w0, sc), q2k_scaled<G>(w1, sc), q2k_scaled<G>(w2, sc), q2k_scaled<G>(w3, sc)));
+                    };
+                    one(std::integral_constant<int, 0>{});
+                    one(std::integral_constant<int, 1>{});
+                    one(std::integral_constant<int, 2>{});
+                    one(std::integral_constant<int, 3>{});
+                }
+            } else {
+                // the row's block sits 0 or 2 bytes into its slot: the low bits of its global address
+                const uint32_t b = i % p.nblk, n0 = (blockIdx.x + i / p.nblk * gridDim.x) / p.nct * 128;
+                const uint32_t sh = 8 * (((n0 + r) * p.row_bytes + b * BB) & 2u);
+                auto word = [&](int k) { return __funnelshift_r(raw[k], raw[k + 1], sh); };
+                dm = (raw[27] >> sh) & 0xFFFFu;
+                const uint32_t l0 = word(24), l1 = word(25), hh = word(26);
+                const uint32_t scw[4] = {(l0 & 0x0F0F0F0Fu) | ((hh << 4) & 0x30303030u), (l1 & 0x0F0F0F0Fu) | ((hh << 2) & 0x30303030u),
+                                         ((l0 >> 4) & 0x0F0F0F0Fu) | (hh & 0x30303030u), ((l1 >> 4) & 0x0F0F0F0Fu) | ((hh >> 2) & 0x30303030u)};
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t hw[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) hw[k] = word(4 * h + k);
+#pragma unroll
+                    for (int n = 0; n < 2; ++n) {
+                        uint32_t w[4];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) w[k] = word(8 + 8 * n + 4 * h + k);
+                        auto one = [&](auto gc) {
+                            constexpr int G = decltype(gc)::value;
+                            const uint32_t u = byte_of(scw[2 * n + (G >> 1)], 2 * (G & 1) + h), ns = 32u - u, u4 = u * 0x04040404u;
+                            put(n, 2 * G + h, make_uint4(q3k_scaled<G>(w[0], hw[0] >> (4 * n), ns, u4), q3k_scaled<G>(w[1], hw[1] >> (4 * n), ns, u4),
+                                                         q3k_scaled<G>(w[2], hw[2] >> (4 * n), ns, u4), q3k_scaled<G>(w[3], hw[3] >> (4 * n), ns, u4)));
+                        };
+                        one(std::integral_constant<int, 0>{});
+                        one(std::integral_constant<int, 1>{});
+                        one(std::integral_constant<int, 2>{});
+                        one(std::integral_constant<int, 3>{});
+                    }
+                }
+            }
+            proxy_fence();  // the operand bytes are read by the tensor core (async proxy)
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(sbase + KO_FULL + 8 * s);
+                mbar_arrive(sbase + KO_RAW_EMPTY + 8 * rs);
+            }
+            if (!wait(KO_REC_EMPTY + 8 * q, ((i / KT_NQ) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) break;
+            *rec = dm;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(sbase + KO_REC_FULL + 8 * q);
+        }
+    } else {
+        // ------------------------------------------------------------ drain: integer sums -> scaled f32 terms, in K order
+        const uint32_t quarter = warp & 3, cg = (uint32_t)(warp - KT_DEC) >> 2, r = quarter * 32 + lane;
+        const uint32_t t_base = tmem + ((quarter * 32) << 16);
+        uint64_t sum[4][4];  // activation rows 8 (cg + 4 c) + 2 j, + 1
+        grid_dep_wait();     // the output may still be in use by the previous kernel
+        uint32_t unit = blockIdx.x, b = 0;
+        for (uint32_t i = 0; i < total; ++i) {
+            const uint32_t q = i % KT_NQ, buf = i & 1;
+            if (!wait(KO_REC_FULL + 8 * q, (i / KT_NQ) & 1, STATUS_TIMEOUT_FULL)) break;
+            const uint8_t* rec = smem + KO_RECS + q * KT_REC;
+            const uint32_t dm = reinterpret_cast<const uint32_t*>(rec)[r];
+            const float df = f16bits_to_f32(dm & 0xFFFF);
+            const uint64_t d = splat2(MIN ? df : -df), nm = MIN ? splat2(-f16bits_to_f32(dm >> 16)) : 0;
+            if (b == 0)
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) sum[c][j] = 0;
+            if (!wait(KO_ACC_FULL + 8 * buf, (i >> 1) & 1, STATUS_TIMEOUT_MMA)) break;
+            tc_after();
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const uint32_t col = 8 * (cg + 4 * c);
+                if (col < p.mt) {  // warp-uniform
+                    uint32_t v[8], u[8];
+                    tmem_ld8_async(t_base + buf * ACC_COLS + col, v);
+                    if constexpr (MIN) tmem_ld8_async(t_base + buf * ACC_COLS + 128 + col, u);
+                    const ulonglong2* d8 = reinterpret_cast<const ulonglong2*>(rec + 512 + 4 * col);
+                    const ulonglong2 d80 = d8[0], d81 = d8[1];
+                    const uint64_t dd[4] = {d80.x, d80.y, d81.x, d81.y};
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        uint64_t t = mul2_apart(mul2(d, dd[j]), int2_to_f32(v[2 * j], v[2 * j + 1]), p.neg_zero);
+                        if constexpr (MIN) t = add2(t, mul2_apart(mul2(nm, dd[j]), int2_to_f32(u[2 * j], u[2 * j + 1]), p.neg_zero));
+                        sum[c][j] = add2(sum[c][j], t);
+                    }
+                }
+            }
+            tc_before();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(sbase + KO_ACC_EMPTY + 8 * buf);
+                mbar_arrive(sbase + KO_REC_EMPTY + 8 * q);
+            }
+            if (++b < p.nblk) continue;
+            b = 0;
+            const uint32_t n = unit / p.nct * 128 + r, m0 = unit % p.nct * p.mt;
+            unit += gridDim.x;
+            if (n < p.N)
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const uint32_t m = 8 * (cg + 4 * c) + j;
+                        if (m < p.mt && m0 + m < p.M)
+                            store_as(p.out, p.out_dtype, (size_t)(m0 + m) * p.N + n, __uint_as_float((uint32_t)(sum[c][j >> 1] >> (32 * (j & 1)))));
+                    }
+        }
+    }
+    tc_before();
+    __syncthreads();
+    if (warp == KT_W_MMA) {
+        tc_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+    }
+}
+
+// ================================================================================================== few activation rows
+// CTA = 16 warps and a contiguous range of 16-row slabs; an item is one (slab, 256-block), the items of the CTA in order are
+// dealt to its warps in turn.  A warp brings its items through a private ring (cp.async, no barrier), multiplies the 16
+// rows with 8 NT activation rows (8 mma.sync per 8 activation rows; one more for the mins), scales the sums and leaves the
+// 16 x 8 NT terms in a table.  Once per R items the CTA meets and a few warps (in turn) add the terms of every slab in K
+// order.  Inside a block the operand's K order is free: lane t of a quad takes the 16 code bytes 16 t .. of its row, whose
+// four bit pairs belong to four sub-blocks, and the same elements of the activation row (16-byte loads of the code image).
+// What bounds it: instruction issue (about 250 (Q2_K) or 400 (Q3_K) instructions an item of 1.3 or 1.8 KB).
+struct KqSmallParams {
+    const uint8_t *w, *codes, *mins;
+    const float* d8;
+    void* out;
+    uint32_t M, N, nblk, row_bytes;
+    uint32_t m_first;  // activation row of the grid's first group
+    int out_dtype;
+};
+constexpr int KS_WARPS = 16;
+__host__ __device__ constexpr uint32_t ks_depth(int fmt) { return fmt == FMT_Q2_K ? 6 : 4; }      // items in flight per warp
+__host__ __device__ constexpr uint32_t ks_slot(int fmt) { return 16 * 4 * kq_pitch(fmt); }        // bytes of an item
+__host__ __device__ constexpr uint32_t ks_round(int nt) { return 64 / nt; }                       // items between two meetings
+constexpr uint32_t KS_COL = 20;  // floats from one activation row's 16 terms to the next: 8 lanes x 4 quads hit 32 banks
+__host__ __device__ constexpr uint32_t ks_table(int nt) { return ks_round(nt) * 8 * nt * KS_COL * 4; }
+__host__ __device__ constexpr size_t ks_smem(int fmt, int nt) { return KS_WARPS * ks_depth(fmt) * ks_slot(fmt) + 2 * ks_table(nt) + 128 * nt * 4; }
+static_assert(ks_smem(FMT_Q2_K, 1) <= 232448 && ks_smem(FMT_Q3_K, 4) <= 232448 && ks_smem(FMT_Q2_K, 4) <= 232448, "shared memory");
+
+// The operand words of one row of an item: v[g][k] = scaled codes of bit pair g, word k of the lane's 16 code bytes.
+__device__ __forceinline__ void q2k_row(const uint32_t* raw, uint32_t t, uint32_t (&v)[4][4]) {
+    const uint32_t n = t >> 1, h8 = 8 * (t & 1);
+    const uint32_t s0 = (raw[2 * n] >> h8) & 0x000F000Fu, s1 = (raw[2 * n + 1] >> h8) & 0x000F000Fu;
+    const uint32_t sc[4] = {s0 & 0xFFu, s0 >> 16, s1 & 0xFFu, s1 >> 16};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const uint32_t w = raw[4 + 4 * t + k];
+        v[0][k] = q2k_scaled<0>(w, sc[0]);
+        v[1][k] = q2k_scaled<1>(w, sc[1]);
+        v[2][k] = q2k_scaled<2>(w, sc[2]);
+        v[3][k] = q2k_scaled<3>(w, sc[3]);
+    }
+}
+__device__ __forceinline__ void q3k_row(const uint32_t* raw, uint32_t sh, uint32_t t, uint32_t (&v)[4][4]) {
+    const uint32_t n = t >> 1, h = t & 1;
+    auto word = [&](uint32_t k) { return __funnelshift_r(raw[k], raw[k + 1], sh); };
+    const uint32_t l0 = word(24) >> (4 * n), l1 = word(25) >> (4 * n), hh = word(26);
+    const uint32_t sa = (l0 & 0x0F0F0F0Fu) | ((n ? hh : hh << 4) & 0x30303030u), sb = (l1 & 0x0F0F0F0Fu) | ((n ? hh >> 2 : hh << 2) & 0x30303030u);
+    const uint32_t u[4] = {byte_of(sa, h), byte_of(sa, 2 + h), byte_of(sb, h), byte_of(sb, 2 + h)};
+    uint32_t ns[4], u4[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        ns[g] = 32u - u[g];
+        u4[g] = u[g] * 0x04040404u;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const uint32_t w = word(8 + 4 * t + k), hw = word(4 * h + k) >> (4 * n);
+        v[0][k] = q3k_scaled<0>(w, hw, ns[0], u4[0]);
+        v[1][k] = q3k_scaled<1>(w, hw, ns[1], u4[1]);
+        v[2][k] = q3k_scaled<2>(w, hw, ns[2], u4[2]);
+        v[3][k] = q3k_scaled<3>(w, hw, ns[3], u4[3]);
+    }
+}
+
+template <int FMT, int NT>
+__global__ void __launch_bounds__(KS_WARPS * 32, 1) kq_small_kernel(const KqSmallParams p) {
+    constexpr bool MIN = FMT == FMT_Q2_K;
+    constexpr uint32_t BB = fmt_block_bytes(FMT), PITCH = kq_pitch(FMT), DEPTH = ks_depth(FMT), SLOT = ks_slot(FMT), R = ks_round(NT);
+    constexpr uint32_t ITEM = 8 * NT * KS_COL;  // floats of an item's terms
+    extern __shared__ __align__(16) uint8_t smem[];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const uint32_t ring = smem_u32(smem) + warp * DEPTH * SLOT;
+    float* table = reinterpret_cast<float*>(smem + KS_WARPS * DEPTH * SLOT);
+    float* run = table + 2 * R * ITEM;  // running sums of the slab that the last round left unfinished
+    const uint32_t m_base = p.m_first + blockIdx.y * 8 * NT, nslab = (p.N + 15) / 16;
+    const uint32_t s_lo = (uint32_t)((uint64_t)nslab * blockIdx.x / gridDim.x), s_hi = (uint32_t)((uint64_t)nslab * (blockIdx.x + 1) / gridDim.x);
+    const uint32_t total = (s_hi - s_lo) * p.nblk;
+    const uint8_t* wend = p.w + (size_t)p.N * p.row_bytes;
+    grid_dep_launch();
+
+    uint32_t fx = warp, fslot = 0;  // next item to fetch, its ring slot
+    auto fetch = [&]() {
+        if (fx < total) {
+            const uint32_t slab = s_lo + fx / p.nblk, b = fx % p.nblk, n0 = slab * 16;
+            const uint8_t* blk = p.w + (size_t)n0 * p.row_bytes + (size_t)b * BB;
+            uint32_t dst = ring + fslot * SLOT;
+#pragma unroll
+            for (uint32_t q = 0; q < 16; ++q) {
+                copy_block_word<FMT>(dst, blk, wend, lane, n0 + q < p.N, p.w);
+                blk += p.row_bytes;
+                dst += PITCH * 4;
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        fx += KS_WARPS;
+        if (++fslot == DEPTH) fslot = 0;
+    };
+#pragma unroll 1
+    for (uint32_t k = 0; k + 1 < DEPTH; ++k) fetch();
+    if (threadIdx.x < 128 * NT) run[threadIdx.x] = 0.f;
+    grid_dep_wait();
+
+    uint4 bf[NT][4];       // the activation codes of the lane's elements: bit pair g of the code bytes
+    uint32_t bm[NT][2];
+    float d8[NT][2];
+    uint32_t have = 0xFFFFFFFFu, slot = 0;
+    for (uint32_t x0 = 0, rd = 0; x0 < total; x0 += R, ++rd) {
+        float* tab = table + (rd & 1) * R * ITEM;
+#pragma unroll 1
+        for (uint32_t x = x0 + warp; x < min(x0 + R, total); x += KS_WARPS) {
+            fetch();
+            const uint32_t b = x % p.nblk, n0 = (s_lo + x / p.nblk) * 16;
+            if (b != have) {  // stays the same where 16 is a multiple of nblk or nblk is 16
+                have = b;
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) {
+                    const uint32_t m = m_base + 8 * nt + g;
+                    const bool in = m < p.M;
+                    const uint4* src = reinterpret_cast<const uint4*>(p.codes + ((size_t)(in ? m : 0) * p.nblk + b) * 256 + 128 * (t >> 1) + 16 * (t & 1));
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) bf[nt][k] = in ? __ldg(src + 2 * k) : make_uint4(0, 0, 0, 0);
+                    if constexpr (MIN) {
+                        const uint32_t* ms = reinterpret_cast<const uint32_t*>(p.mins + ((size_t)(in ? m : 0) * p.nblk + b) * 32);
+                        bm[nt][0] = in ? __ldg(ms + t) : 0u;
+                        bm[nt][1] = in ? __ldg(ms + 4 + t) : 0u;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const uint32_t mc = m_base + 8 * nt + 2 * t + j;
+                        d8[nt][j] = mc < p.M ? __ldg(p.d8 + (size_t)b * p.M + mc) : 0.f;
+                    }
+                }
+            }
+            asm volatile("cp.async.wait_group %0;" ::"n"(DEPTH - 1) : "memory");
+            __syncwarp();
+            const uint32_t* ra = reinterpret_cast<const uint32_t*>(smem + (warp * DEPTH + slot) * SLOT) + g * PITCH;
+            const uint32_t* rb = ra + 8 * PITCH;
+            uint32_t va[4][4], vb[4][4], dma, dmb;
+            if constexpr (MIN) {
+                q2k_row(ra, t, va);
+                q2k_row(rb, t, vb);
+                dma = ra[20];
+                dmb = rb[20];
+            } else {
+                const uint32_t sha = 8 * (((n0 + g) * p.row_bytes + b * BB) & 2u), shb = 8 * (((n0 + 8 + g) * p.row_bytes + b * BB) & 2u);
+                q3k_row(ra, sha, t, va);
+                q3k_row(rb, shb, t, vb);
+                dma = (ra[27] >> sha) & 0xFFFFu;
+                dmb = (rb[27] >> shb) & 0xFFFFu;
+            }
+            const float da = f16bits_to_f32(dma & 0xFFFF), db = f16bits_to_f32(dmb & 0xFFFF);
+            float* to = tab + (x - x0) * ITEM;
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                int acc[4] = {0, 0, 0, 0};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    mma_s8s8_k32(acc, va[k][0], vb[k][0], va[k][1], vb[k][1], bf[nt][k].x, bf[nt][k].y, acc);
+                    mma_s8s8_k32(acc, va[k][2], vb[k][2], va[k][3], vb[k][3], bf[nt][k].z, bf[nt][k].w, acc);
+                }
+                float tm[4];
+                if constexpr (MIN) {
+                    const uint32_t ma = (ra[t] >> 4) & 0x0F0F0F0Fu, mb = (rb[t] >> 4) & 0x0F0F0F0Fu;
+                    int ms[4] = {0, 0, 0, 0};
+                    mma_u8s8_k32(ms, ma, mb, ma << 4, mb << 4, bm[nt][0], bm[nt][1], ms);
+                    const float na = f16bits_to_f32(dma >> 16), nb = f16bits_to_f32(dmb >> 16);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float d = j < 2 ? da : db, dn = j < 2 ? na : nb, s = d8[nt][j & 1];
+                        tm[j] = __fsub_rn(__fmul_rn(__fmul_rn(d, s), (float)acc[j]), __fmul_rn(__fmul_rn(dn, s), (float)ms[j]));
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) tm[j] = __fmul_rn(__fmul_rn(j < 2 ? -da : -db, d8[nt][j & 1]), (float)acc[j]);
+                }
+                float* tn = to + (8 * nt + 2 * t) * KS_COL + g;
+                tn[0] = tm[0];
+                tn[KS_COL] = tm[1];
+                tn[8] = tm[2];
+                tn[KS_COL + 8] = tm[3];
+            }
+            __syncwarp();  // the slot is refilled by the next fetch
+            if (++slot == DEPTH) slot = 0;
+        }
+        __syncthreads();  // the table of this round is complete; the other one is free again
+        // 128 NT sums (activation row, weight row) by 4 NT warps, another group each round
+        const uint32_t pos = (threadIdx.x + KS_WARPS * 32 - (rd * 128 * NT) % (KS_WARPS * 32)) % (KS_WARPS * 32);
+        if (pos < 128 * NT) {
+            const uint32_t m = m_base + (pos >> 4), row = pos & 15, cnt = min(R, total - x0);
+            const float* tp = tab + (pos >> 4) * KS_COL + row;
+            float s = run[pos];
+            uint32_t b = x0 % p.nblk, n = (s_lo + x0 / p.nblk) * 16 + row;
+#pragma unroll 8
+            for (uint32_t x = 0; x < cnt; ++x) {
+                s = __fadd_rn(s, tp[x * ITEM]);
+                if (++b == p.nblk) {
+                    if (m < p.M && n < p.N) store_as(p.out, p.out_dtype, (size_t)m * p.N + n, s);
+                    s = 0.f;
+                    b = 0;
+                    n += 16;
+                }
+            }
+            run[pos] = s;
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+struct KqScratch {
+    uint8_t *codes, *mins;
+    float* d8;
+};
+KqScratch kq_scratch(void* ws, size_t M, size_t K) {
+    uint8_t* b = static_cast<uint8_t*>(ws);
+    return {b, b + M * K, reinterpret_cast<float*>(b + M * K + M * (K / 256) * 32)};
+}
+
+// Time model of the two kernels, in units of SM cycles per block of K.
+struct KqPlan {
+    uint32_t mt = 0;  // activation rows of a tensor-core tile; 0: the kernel for few activation rows
+    size_t cost = 0;
+};
+KqPlan kq_tc_plan(int fmt, size_t M, size_t N, int sm_count) {
+    KqPlan best;
+    const size_t rt = (N + 127) / 128, fixed = 450, per_row = fmt == FMT_Q2_K ? 7 : 5;
+    for (uint32_t mt = 16; mt <= 128; mt += 16) {
+        const size_t units = rt * ((M + mt - 1) / mt), cost = (units + sm_count - 1) / sm_count * (fixed + per_row * mt);
+        if (!best.mt || cost < best.cost) best = {mt, cost};
+        if (mt >= M) break;
+    }
+    return best;
+}
+KqPlan kq_plan(int fmt, size_t M, size_t K, size_t N, int sm_count) {
+    const KqPlan tc = kq_tc_plan(fmt, M, N, sm_count);
+    const size_t slabs = (N + 15) / 16, nt = M <= 8 ? 1 : M <= 16 ? 2 : 4, groups = (M + 8 * nt - 1) / (8 * nt);
+    const size_t small = (slabs + sm_count - 1) / sm_count * groups * (fmt == FMT_Q2_K ? 90 + 20 * nt : 130 + 20 * nt);
+    const size_t units = (N + 127) / 128 * ((M + 15) / 16);
+    if (M <= 8 || small <= tc.cost || units > (1u << 30) / (K / 256) || !tma_available()) return {0, small};
+    return tc;
+}
+
+template <int FMT>
+cudaError_t launch_tc(const KqTcParams& p, const CUtensorMap& amap, const CUtensorMap& mmap, int sm_count, cudaStream_t st) {
+    static PerDeviceOnce attrs;
+    cudaError_t e = attrs.run([] { return cudaFuncSetAttribute(kq_tc_kernel<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kt_smem(FMT)); });
+    if (e != cudaSuccess) return e;
+    return launch_pdl(kq_tc_kernel<FMT>, dim3(p.nunits < (uint32_t)sm_count ? p.nunits : (uint32_t)sm_count), dim3(KT_THREADS), kt_smem(FMT), st, amap, mmap, p);
+}
+template <int FMT, int NT>
+cudaError_t launch_small(const KqSmallParams& p, int sm_count, cudaStream_t st) {
+    static PerDeviceOnce attrs;
+    cudaError_t e = attrs.run([] { return cudaFuncSetAttribute(kq_small_kernel<FMT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ks_smem(FMT, NT)); });
+    if (e != cudaSuccess) return e;
+    const uint32_t slabs = (p.N + 15) / 16, groups = (p.M + 8 * NT - 1) / (8 * NT);
+    // at most 65535 groups of activation rows in a grid: the rest in further launches
+    for (uint32_t g0 = 0; g0 < groups && e == cudaSuccess; g0 += 65535) {
+        KqSmallParams q = p;
+        q.m_first = g0 * 8 * NT;
+        const uint32_t n = groups - g0 < 65535 ? groups - g0 : 65535;
+        e = launch_pdl(kq_small_kernel<FMT, NT>, dim3(slabs < (uint32_t)sm_count ? slabs : (uint32_t)sm_count, n), dim3(KS_WARPS * 32), ks_smem(FMT, NT), st, q);
+    }
+    return e;
+}
+
+bool encode(CUtensorMap* map, void* base, size_t inner, size_t rows, uint32_t box_inner, uint32_t box_rows, CUtensorMapSwizzle sw) {
+    const cuuint32_t estr[2] = {1, 1}, box[2] = {box_inner, box_rows};
+    const cuuint64_t gdim[2] = {inner, rows}, gstride[1] = {inner};
+    return encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, base, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+}  // namespace
+
+bool kq_lowbit_supported(int fmt, size_t M, size_t K, size_t N) { return (fmt == FMT_Q2_K || fmt == FMT_Q3_K) && M >= 1 && N >= 1 && K % 256 == 0; }
+
+size_t kq_lowbit_workspace_bytes(size_t M, size_t K) { return (M * (K / 256) * RUN_BYTES + 255) & ~(size_t)255; }
+
+// acts_prepared: a previous call with the same activations and scratch left the image there (both formats read the same).
+cudaError_t launch_kq_lowbit(int fmt, const void* act, int act_dtype, const void* w, void* out, int out_dtype, size_t M, size_t K, size_t N, void* ws,
+                             size_t ws_bytes, int sm_count, cudaStream_t st, unsigned int* status, bool* ws_too_small, char* err, size_t err_len,
+                             bool acts_prepared) {
+    *ws_too_small = false;
+    const size_t need = kq_lowbit_workspace_bytes(M, K);
+    if (!ws || ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 15)) {
+        *ws_too_small = true;
+        return cudaSuccess;
+    }
+    if (fmt != FMT_Q2_K && fmt != FMT_Q3_K) return cudaErrorInvalidValue;
+    const KqScratch s = kq_scratch(ws, M, K);
+    const uint32_t nblk = (uint32_t)(K / 256);
+    cudaError_t e;
+    if (!acts_prepared) {
+        size_t grid = (M * nblk + 7) / 8;
+        if (grid > (size_t)sm_count * 8) grid = (size_t)sm_count * 8;
+        e = act_dtype == DT_F32 ? launch_pdl(kq_act_prep_kernel<float>, dim3((unsigned)grid), dim3(256), 0, st, static_cast<const float*>(act), s.codes, s.mins, s.d8, M, nblk)
+                                : launch_pdl(kq_act_prep_kernel<__nv_bfloat16>, dim3((unsigned)grid), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(act), s.codes,
+                                             s.mins, s.d8, M, nblk);
+        note_launch();
+        if (e != cudaSuccess) return e;
+    }
+    const KqPlan plan = kq_plan(fmt, M, K, N, sm_count);
+    if (plan.mt) {
+        KqTcParams p{};
+        p.w = static_cast<const uint8_t*>(w);
+        p.out = out;
+        p.d8 = s.d8;
+        p.M = (uint32_t)M; p.N = (uint32_t)N; p.nblk = nblk;
+        p.mt = plan.mt;
+        p.nct = (uint32_t)((M + plan.mt - 1) / plan.mt);
+        p.nunits = (uint32_t)((N + 127) / 128) * p.nct;
+        p.row_bytes = nblk * (uint32_t)fmt_block_bytes(fmt);
+        p.idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((p.mt >> 3) << 17) | ((128u >> 4) << 24);  // int32 <- s8 x s8, K-major, N = mt, M = 128
+        p.out_dtype = out_dtype;
+        p.neg_zero = 0x8000000080000000ull;
+        p.status = status;
+        CUtensorMap amap, mmap;
+        if (!encode(&amap, s.codes, K, M, 128, plan.mt, CU_TENSOR_MAP_SWIZZLE_128B) ||
+            !encode(&mmap, s.mins, (size_t)nblk * 32, M, 32, plan.mt, CU_TENSOR_MAP_SWIZZLE_32B)) {
+            snprintf(err, err_len, "cuTensorMapEncodeTiled failed (activation image %p, K=%zu, M=%zu)", (void*)s.codes, K, M);
+            return cudaErrorInvalidValue;
+        }
+        e = fmt == FMT_Q2_K ? launch_tc<FMT_Q2_K>(p, amap, mmap, sm_count, st) : launch_tc<FMT_Q3_K>(p, amap, mmap, sm_count, st);
+    } else {
+        KqSmallParams p{};
+        p.w = static_cast<const uint8_t*>(w);
+        p.codes = s.codes; p.mins = s.mins; p.d8 = s.d8;
+        p.out = out;
+        p.M = (uint32_t)M; p.N = (uint32_t)N; p.nblk = nblk;
+        p.row_bytes = nblk * (uint32_t)fmt_block_bytes(fmt);
+        p.out_dtype = out_dtype;
+        const int nt = M <= 8 ? 1 : M <= 16 ? 2 : 4;
+        if (fmt == FMT_Q2_K)
+            e = nt == 1 ? launch_small<FMT_Q2_K, 1>(p, sm_count, st) : nt == 2 ? launch_small<FMT_Q2_K, 2>(p, sm_count, st) : launch_small<FMT_Q2_K, 4>(p, sm_count, st);
+        else
+            e = nt == 1 ? launch_small<FMT_Q3_K, 1>(p, sm_count, st) : nt == 2 ? launch_small<FMT_Q3_K, 2>(p, sm_count, st) : launch_small<FMT_Q3_K, 4>(p, sm_count, st);
+    }
+    note_launch();
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+}  // namespace b200q

@@ -32,6 +32,7 @@
 #include <cstdio>
 
 #include "common.cuh"
+#include "tcgen05_i8.cuh"
 #include "tmap.cuh"
 
 namespace b200q {
@@ -74,81 +75,6 @@ constexpr int OFF_FULL = 0, OFF_EMPTY = 64, OFF_RAW_FULL = 128, OFF_RAW_EMPTY = 
               OFF_SC_FULL = 320, OFF_TMEM = 448, OFF_DEAD = 452, OFF_RED = 456, OFF_LAST = 464, OFF_NSLOT = 472, OFF_XFER = 480, OFF_SLOTS = 512,
               OFF_SC = 1024;  // OFF_SLOTS: two lists of 64 slots
 
-__device__ __noinline__ bool i8_wait_slow(uint32_t bar, uint32_t parity, volatile uint32_t* dead) {
-#pragma unroll 1
-    for (int i = 0; i < 64; ++i)
-        if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t t0 = global_timer_ns();
-#pragma unroll 1
-    for (;;) {
-#pragma unroll 1
-        for (int i = 0; i < 8; ++i)
-            if (mbar_try_wait(bar, parity)) return true;
-        if (*dead || global_timer_ns() - t0 > 2000000000ull) return false;
-        __nanosleep(40);
-    }
-}
-__device__ __forceinline__ bool i8_wait(uint32_t bar, uint32_t parity, volatile uint32_t* dead) {
-    if (mbar_try_wait(bar, parity)) return true;
-    return i8_wait_slow(bar, parity, dead);
-}
-__device__ __noinline__ void i8_fail(volatile uint32_t* dead, unsigned int* status, unsigned int code) {
-    if (!*dead) atomicOr(status, code);
-    *dead = 1;
-}
-__device__ __forceinline__ void tma2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-                 "l"(map), "r"(x), "r"(y), "r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ bool elect_one_lane() {
-    uint32_t pred;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "elect.sync _|p, 0xFFFFFFFF;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(pred));
-    return pred != 0;
-}
-__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit_to(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-// D[128 x N] (int32, tensor memory) = A[128 x 32] (int8, shared) x B[N x 32]^T (int8, shared); never accumulates:
-// every sub-block has its own columns
-__device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, 0, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc)
-        : "memory");
-}
-// K-major operand tile with 128-byte swizzle (rows of 128 bytes, 8-row groups 1024 bytes apart), from the low word
-// ((addr >> 4) | 1 << 16; 32 bytes further along K adds 2)
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t lo) {
-    uint64_t d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"((1024u >> 4) | (1u << 14) | (2u << 29)));
-    return d;
-}
-__device__ __forceinline__ uint32_t desc_lo(uint32_t addr) { return ((addr >> 4) & 0x3FFFu) | (1u << 16); }
-// 16 consecutive 32-bit columns of this thread's lane; the caller waits (tmem_ld_wait) before using them
-__device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld8_async(uint32_t taddr, uint32_t (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
 // One piece of work of a CTA: blocks [b0, b0 + nb) of tile `tile`; slot < 0: the whole tile, written to the output.
 struct I8Unit {
     uint32_t tile, b0, nb;
@@ -173,9 +99,6 @@ __device__ __forceinline__ bool i8_unit(const I8Params& p, uint32_t it, I8Unit& 
     u.slot = u.nb == p.nblk ? -1 : (int)(2 * blockIdx.x + (it == 0 ? 0u : 1u));
     return true;
 }
-
-template <int I>
-__device__ __forceinline__ int ubyte(uint32_t x) { return (int)__byte_perm(x, 0u, 0x4440 | I); }
 
 template <int MP>
 __global__ void __launch_bounds__(I8_THREADS, 1) smallm_i8_q4k_kernel(const __grid_constant__ CUtensorMap tmap_act,
