@@ -29,10 +29,12 @@ namespace {
 
 constexpr uint32_t RUN_BYTES = 292;  // of scratch per (activation row, 256-block): 256 codes, 32 bytes of sums, f32 d8
 
-// Words of a packed block in shared memory.  Blocks are only 4-byte (Q2_K) or 2-byte (Q3_K) aligned in a row: a copy takes
-// the NW words from the 4-byte boundary at or below the block; PITCH is odd, so one word of 32 rows lies in 32 banks.
-__host__ __device__ constexpr uint32_t kq_nw(int fmt) { return fmt == FMT_Q2_K ? 21 : 28; }
-__host__ __device__ constexpr uint32_t kq_pitch(int fmt) { return fmt == FMT_Q2_K ? 21 : 29; }
+// Packed blocks start 4-byte (Q2_K) or 2-byte (Q3_K) aligned in a row and are brought as the 16-byte chunks that hold them:
+// CHUNKS at most, PITCH bytes from row to row in shared memory.  (Copies of 4 bytes - cp.async - ran at about one lane per
+// cycle and took 2-4 us per 128 rows, more than everything else.)  Any such pitch puts one word of 32 rows into eight banks:
+// 112 and 144 use all of these.
+__host__ __device__ constexpr uint32_t kq_chunks(int fmt) { return fmt == FMT_Q2_K ? 6 : 8; }
+__host__ __device__ constexpr uint32_t kq_pitch(int fmt) { return fmt == FMT_Q2_K ? 112 : 144; }
 
 // One warp per (activation row, 256-block): Q8_K codes (d = amax / 127, id = 127 / amax, round half to even), the sums of
 // 16 codes as lo + 16 hi with lo in [-8, 7] (a sum is at most 2048 in size, so hi fits a signed byte), the scale.
@@ -106,53 +108,39 @@ __device__ __forceinline__ uint32_t q3k_scaled(uint32_t w, uint32_t hw, uint32_t
 }
 __device__ __forceinline__ uint32_t byte_of(uint32_t x, uint32_t i) { return __byte_perm(x, 0u, 0x4440u | i); }
 
-// ---------------------------------------------------------------------------------------------------- f32x2 arithmetic
-__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
-    return r;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-// A product that is added to something next.  The assembler fuses a packed multiply (and an FMA with a constant zero) with
-// the packed add behind it, one rounding where the CPU makes two; an FMA with a -0 that it cannot see (a kernel parameter)
-// gives the same value as the product and stays apart.
-__device__ __forceinline__ uint64_t mul2_apart(uint64_t a, uint64_t b, uint64_t neg_zero) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(neg_zero));
-    return r;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t splat2(float x) { return pack2(__float_as_uint(x), __float_as_uint(x)); }
-// Integers below 2^22 in size to f32, exactly: added to the bit pattern of 1.5 * 2^23 they sit in its mantissa.  The sums
-// here are at most 128 * 128 * 256 = 2^22, which this still takes exactly.
-__device__ __forceinline__ uint64_t int2_to_f32(uint32_t a, uint32_t b) {
-    return add2(pack2(a + 0x4B400000u, b + 0x4B400000u), splat2(-12582912.0f));
-}
-
 __device__ __forceinline__ void store_as(void* out, int dt, size_t idx, float v) {
     if (dt == DT_F32) static_cast<float*>(out)[idx] = v;
     else if (dt == DT_BF16) static_cast<__nv_bfloat16*>(out)[idx] = __float2bfloat16_rn(v);
     else static_cast<__half*>(out)[idx] = __float2half_rn(v);
 }
 
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, uint32_t nbytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(nbytes) : "memory");
-}
-// Word `lane` of the block at `blk` (row in range) to dst + 4 lane; the last word is clipped at the tensor's end.
-template <int FMT>
-__device__ __forceinline__ void copy_block_word(uint32_t dst, const uint8_t* blk, const uint8_t* wend, uint32_t lane, bool in, const uint8_t* any) {
-    if (lane >= kq_nw(FMT)) return;
-    const uint8_t* src = blk - (FMT == FMT_Q3_K ? (reinterpret_cast<uintptr_t>(blk) & 2) : 0) + 4 * lane;
-    const uint32_t n = !in ? 0u : (FMT == FMT_Q2_K || src + 4 <= wend) ? 4u : src + 2 <= wend ? 2u : 0u;
-    cp_async4(dst + 4 * lane, in && n ? src : any, n);
+// Eight lanes a row copy the 16-byte chunks of the blocks at blk, blk + row_bytes, ... (ROWS of them, `in` of which exist) to
+// dst, one PITCH apart; each lands at byte (its address & 15) of its slot.  Rows that do not exist are left as they are:
+// their sums are never stored.  `inner`: all exist and none is the tensor's last row, whose last chunk may reach past the
+// end and is clipped there.
+template <int FMT, uint32_t ROWS>
+__device__ __forceinline__ void copy_rows(uint32_t dst, const uint8_t* blk, uint32_t row_bytes, uint32_t lane, bool inner, uint32_t in, const uint8_t* wend) {
+    const uint32_t c = lane & 7, r0 = lane >> 3;
+    if (c >= kq_chunks(FMT)) return;
+    const uint8_t* src = blk + (size_t)r0 * row_bytes;
+    dst += r0 * kq_pitch(FMT) + 16 * c;
+    auto chunk = [&](const uint8_t* q) { return reinterpret_cast<const uint8_t*>((reinterpret_cast<uintptr_t>(q) & ~(uintptr_t)15) + 16 * c); };
+    if (inner) {
+#pragma unroll
+        for (uint32_t q = 0; q < ROWS; q += 4) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + q * kq_pitch(FMT)), "l"(chunk(src)) : "memory");
+            src += 4 * (size_t)row_bytes;
+        }
+        return;
+    }
+#pragma unroll 1
+    for (uint32_t q = r0; q < ROWS && q < in; q += 4) {
+        const uint8_t* s = chunk(src);
+        if (s < wend)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(s), "r"(min(16u, (uint32_t)(wend - s))) : "memory");
+        src += 4 * (size_t)row_bytes;
+        dst += 4 * kq_pitch(FMT);
+    }
 }
 
 // =================================================================================================== tensor-core kernel
@@ -171,9 +159,9 @@ struct KqTcParams {
     uint32_t mt;              // activation rows of a tile: a multiple of 16, at most 128
     uint32_t nct, nunits;     // column tiles; row tiles x column tiles
     uint32_t row_bytes;
+    bool raw_tma;             // rows start 16-byte aligned: packed blocks come by TMA
     uint32_t idesc;
     int out_dtype;
-    uint64_t neg_zero;        // two f32 -0 (mul2_apart)
     unsigned int* status;
 };
 
@@ -188,12 +176,17 @@ constexpr uint32_t KT_REC = 512 + 512;  // the rows' d | dmin, the activation ro
 constexpr int KO_FULL = 0, KO_EMPTY = 16, KO_RAW_FULL = 32, KO_RAW_EMPTY = 64, KO_ACC_FULL = 96, KO_ACC_EMPTY = 112, KO_REC_FULL = 128,
               KO_REC_EMPTY = 160, KO_TMEM = 192, KO_DEAD = 196, KO_RECS = 1024, KO_STAGES = KO_RECS + KT_NQ * KT_REC;
 // a stage: two operand tiles of scaled codes | tile of mins (Q2_K) | two tiles of activation codes | sums of 16 (Q2_K)
-__host__ __device__ constexpr uint32_t kt_stage(int fmt) { return 4 * KT_ATOM + (fmt == FMT_Q2_K ? KT_ATOM + 128 * 32 : 0); }
-__host__ __device__ constexpr uint32_t kt_raw(int fmt) { return 128 * 4 * kq_pitch(fmt); }
+__host__ __device__ constexpr uint32_t kt_stage(int fmt) { return 4 * KT_ATOM + (fmt == FMT_Q2_K ? 128 * 64 + 128 * 32 : 0); }
+__host__ __device__ constexpr uint32_t kt_raw(int fmt) { return 128 * kq_pitch(fmt); }
 __host__ __device__ constexpr size_t kt_smem(int fmt) { return 1024 + KO_STAGES + KT_NS * kt_stage(fmt) + KT_NR * kt_raw(fmt); }
 static_assert(KO_STAGES % 1024 == 0 && kt_stage(FMT_Q2_K) % 1024 == 0 && kt_smem(FMT_Q2_K) <= 232448 && kt_smem(FMT_Q3_K) <= 232448, "shared memory");
 
-// rows of 32 bytes with 32-byte swizzle (8-row groups 256 bytes apart)
+// rows of 64 bytes with 64-byte swizzle (8-row groups 512 bytes apart) and of 32 bytes with 32-byte swizzle
+__device__ __forceinline__ uint64_t desc_sw64(uint32_t lo) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"((512u >> 4) | (1u << 14) | (4u << 29)));
+    return d;
+}
 __device__ __forceinline__ uint64_t desc_sw32(uint32_t lo) {
     uint64_t d;
     asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"((256u >> 4) | (1u << 14) | (6u << 29)));
@@ -202,10 +195,10 @@ __device__ __forceinline__ uint64_t desc_sw32(uint32_t lo) {
 
 template <int FMT>
 __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant__ CUtensorMap tmap_min,
-                                                              const KqTcParams p) {
+                                                              const __grid_constant__ CUtensorMap tmap_w, const KqTcParams p) {
     constexpr bool MIN = FMT == FMT_Q2_K;
     constexpr uint32_t BB = fmt_block_bytes(FMT), PITCH = kq_pitch(FMT), RAW = kt_raw(FMT), STAGE = kt_stage(FMT);
-    constexpr uint32_t OFF_AM = 2 * KT_ATOM, OFF_B = OFF_AM + (MIN ? KT_ATOM : 0), OFF_BM = OFF_B + 2 * KT_ATOM;
+    constexpr uint32_t OFF_AM = 2 * KT_ATOM, OFF_B = OFF_AM + (MIN ? 128 * 64 : 0), OFF_BM = OFF_B + 2 * KT_ATOM;
     constexpr uint32_t ACC_COLS = MIN ? 256 : 128, TMEM_COLS = 2 * ACC_COLS;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);  // the launch reserves 1 KB of slack
@@ -219,7 +212,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
             mbar_init(sbase + KO_EMPTY + 8 * s, 1);  // the commit behind the block's MMAs
         }
         for (uint32_t s = 0; s < KT_NR; ++s) {
-            mbar_init(sbase + KO_RAW_FULL + 8 * s, KT_COPY * 32);  // every copying thread, once its copies have landed
+            mbar_init(sbase + KO_RAW_FULL + 8 * s, p.raw_tma ? 1 : KT_COPY * 32);  // the TMA copy, or every copying thread
             mbar_init(sbase + KO_RAW_EMPTY + 8 * s, 4);
         }
         for (uint32_t s = 0; s < 2; ++s) {
@@ -255,29 +248,34 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
         // ------------------------------------------------------------ packed blocks (do not depend on the previous kernel)
         const uint32_t r0 = (uint32_t)(warp - KT_W_COPY) * (128 / KT_COPY);
         const uint8_t* wend = p.w + (size_t)p.N * p.row_bytes;
-        uint32_t unit = blockIdx.x, b = 0;
+        uint32_t unit = blockIdx.x, b = 0, n0 = unit / p.nct * 128 + r0;
         for (uint32_t i = 0; i < total; ++i) {
             const uint32_t rs = i % KT_NR;
             if (!wait(KO_RAW_EMPTY + 8 * rs, ((i / KT_NR) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) break;
-            const uint32_t n0 = unit / p.nct * 128 + r0;
-            const uint8_t* blk = p.w + (size_t)n0 * p.row_bytes + (size_t)b * BB;
-            uint32_t dst = sbase + OFF_RAW + rs * RAW + r0 * PITCH * 4;
-#pragma unroll 8
-            for (uint32_t q = 0; q < 128 / KT_COPY; ++q) {  // rows past N are zero-filled
-                copy_block_word<FMT>(dst, blk, wend, lane, n0 + q < p.N, p.w);
-                blk += p.row_bytes;
-                dst += PITCH * 4;
+            if (p.raw_tma) {  // one copy a block: rows past N and bytes past the row's end are zero-filled
+                if (warp == KT_W_COPY && lane == 0) {
+                    mbar_expect_tx(sbase + KO_RAW_FULL + 8 * rs, RAW);
+                    tma2d(sbase + OFF_RAW + rs * RAW, &tmap_w, (int)((b * BB & ~15u) / 2), (int)n0, sbase + KO_RAW_FULL + 8 * rs);
+                }
+            } else {
+                copy_rows<FMT, 128 / KT_COPY>(sbase + OFF_RAW + rs * RAW + r0 * PITCH, p.w + (size_t)n0 * p.row_bytes + (size_t)b * BB, p.row_bytes, lane,
+                                              n0 + 128 / KT_COPY < p.N, n0 < p.N ? p.N - n0 : 0u, wend);
             }
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(sbase + KO_RAW_FULL + 8 * rs) : "memory");
-            if (++b == p.nblk) { b = 0; unit += gridDim.x; }
+            if (!p.raw_tma)  // arrives once this thread's copies have landed
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(sbase + KO_RAW_FULL + 8 * rs) : "memory");
+            if (++b == p.nblk) {
+                b = 0;
+                unit += gridDim.x;
+                n0 = unit / p.nct * 128 + r0;
+            }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (warp == KT_W_ACT) {
         // ------------------------------------------------------------ activation codes, sums and scales (previous kernel's output)
         grid_dep_wait();
-        uint32_t unit = blockIdx.x, b = 0;
+        uint32_t unit = blockIdx.x, b = 0, m0 = unit % p.nct * p.mt;
         for (uint32_t i = 0; i < total; ++i) {
-            const uint32_t s = i % KT_NS, q = i % KT_NQ, m0 = unit % p.nct * p.mt;
+            const uint32_t s = i % KT_NS, q = i % KT_NQ;
             if (!wait(KO_EMPTY + 8 * s, ((i / KT_NS) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) break;
             if (lane == 0) {
                 const uint32_t st = st_base + s * STAGE, bar = sbase + KO_FULL + 8 * s;
@@ -290,9 +288,14 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
             if (!wait(KO_REC_EMPTY + 8 * q, ((i / KT_NQ) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) break;
             const uint32_t dst = sbase + KO_RECS + q * KT_REC + 512;
             const float* src = p.d8 + (size_t)b * p.M + m0;
-            for (uint32_t m = lane; m < p.mt; m += 32) cp_async4(dst + 4 * m, m0 + m < p.M ? src + m : p.d8, m0 + m < p.M ? 4u : 0u);
+            for (uint32_t m = lane; m < p.mt; m += 32)  // rows past M are zero-filled
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 4 * m), "l"(m0 + m < p.M ? src + m : p.d8), "r"(m0 + m < p.M ? 4u : 0u) : "memory");
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(sbase + KO_REC_FULL + 8 * q) : "memory");
-            if (++b == p.nblk) { b = 0; unit += gridDim.x; }
+            if (++b == p.nblk) {
+                b = 0;
+                unit += gridDim.x;
+                m0 = unit % p.nct * p.mt;
+            }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
         if (*dead) {  // TMA copies in flight land within microseconds: the CTA's shared memory stays until then
@@ -314,8 +317,8 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
                               k > 0);
                 if constexpr (MIN) {  // sum of 16 = lo + 16 hi: [m | 8 m] . [lo | hi] + [0 | 8 m] . [lo | hi]
                     const uint32_t am = desc_lo(st + OFF_AM), bm = desc_lo(st + OFF_BM);
-                    tc_mma_i8(d + 128, desc_sw128(am), desc_sw32(bm), p.idesc, false);
-                    tc_mma_i8(d + 128, desc_sw128(am + 2), desc_sw32(bm), p.idesc, true);
+                    tc_mma_i8(d + 128, desc_sw64(am), desc_sw32(bm), p.idesc, false);
+                    tc_mma_i8(d + 128, desc_sw64(am + 2), desc_sw32(bm), p.idesc, true);
                 }
                 tc_commit_to(sbase + KO_EMPTY + 8 * s);       // the stage may be overwritten once these MMAs have read it
                 tc_commit_to(sbase + KO_ACC_FULL + 8 * buf);  // and the sums are complete
@@ -325,10 +328,12 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
     } else if (warp < KT_DEC) {
         // ------------------------------------------------------------ decode: one thread per weight row
         const uint32_t r = threadIdx.x & 127, set = threadIdx.x >> 7, x7 = r & 7;
-        for (uint32_t i = set; i < total; i += 2) {
+        uint32_t b = set % p.nblk;  // block of K
+        for (uint32_t i = set; i < total; i += 2, b += 2, b -= b >= p.nblk ? p.nblk : 0, b -= b >= p.nblk ? p.nblk : 0) {
             const uint32_t rs = i % KT_NR, s = i % KT_NS, q = i % KT_NQ;
             if (!wait(KO_RAW_FULL + 8 * rs, (i / KT_NR) & 1, STATUS_TIMEOUT_FULL)) break;
-            const uint32_t* raw = reinterpret_cast<const uint32_t*>(smem + OFF_RAW + rs * RAW) + r * PITCH;
+            const uint32_t at = (r * p.row_bytes + b * BB) & 15u;  // where the row's block sits in its slot (128 rows are a multiple of 16 bytes)
+            const uint32_t* raw = reinterpret_cast<const uint32_t*>(smem + OFF_RAW + rs * RAW + r * PITCH + (at & 12u));
             uint32_t* rec = reinterpret_cast<uint32_t*>(smem + KO_RECS + q * KT_REC) + r;
             uint8_t* a0 = smem + KO_STAGES + s * STAGE + (r >> 3) * 1024 + x7 * 128;
             auto put = [&](uint32_t tile, uint32_t c, uint4 v) { *reinterpret_cast<uint4*>(a0 + tile * KT_ATOM + ((c ^ x7) << 4)) = v; };
@@ -342,10 +347,12 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
                 dm = raw[20];
                 uint4 mn = make_uint4((scw[0] >> 4) & 0x0F0F0F0Fu, (scw[1] >> 4) & 0x0F0F0F0Fu, (scw[2] >> 4) & 0x0F0F0F0Fu, (scw[3] >> 4) & 0x0F0F0F0Fu);
                 const uint4 mn8 = make_uint4(mn.x << 3, mn.y << 3, mn.z << 3, mn.w << 3);
-                put(2, 0, mn);
-                put(2, 1, mn8);
-                put(2, 2, make_uint4(0, 0, 0, 0));
-                put(2, 3, mn8);
+                uint4* am = reinterpret_cast<uint4*>(smem + KO_STAGES + s * STAGE + OFF_AM + r * 64);
+                const uint32_t x3 = (r >> 1) & 3;
+                am[0 ^ x3] = mn;
+                am[1 ^ x3] = mn8;
+                am[2 ^ x3] = make_uint4(0, 0, 0, 0);
+                am[3 ^ x3] = mn8;
 #pragma unroll
                 for (int k = 0; k < 4; ++k) scw[k] &= 0x0F0F0F0Fu;
 #pragma unroll
@@ -363,9 +370,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
                     one(std::integral_constant<int, 3>{});
                 }
             } else {
-                // the row's block sits 0 or 2 bytes into its slot: the low bits of its global address
-                const uint32_t b = i % p.nblk, n0 = (blockIdx.x + i / p.nblk * gridDim.x) / p.nct * 128;
-                const uint32_t sh = 8 * (((n0 + r) * p.row_bytes + b * BB) & 2u);
+                const uint32_t sh = 8 * (at & 2u);
                 auto word = [&](int k) { return __funnelshift_r(raw[k], raw[k + 1], sh); };
                 dm = (raw[27] >> sh) & 0xFFFFu;
                 const uint32_t l0 = word(24), l1 = word(25), hh = word(26);
@@ -409,8 +414,8 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
         // ------------------------------------------------------------ drain: integer sums -> scaled f32 terms, in K order
         const uint32_t quarter = warp & 3, cg = (uint32_t)(warp - KT_DEC) >> 2, r = quarter * 32 + lane;
         const uint32_t t_base = tmem + ((quarter * 32) << 16);
-        uint64_t sum[4][4];  // activation rows 8 (cg + 4 c) + 2 j, + 1
-        grid_dep_wait();     // the output may still be in use by the previous kernel
+        float sum[4][8];  // activation rows 8 (cg + 4 c) + j
+        grid_dep_wait();  // the output may still be in use by the previous kernel
         uint32_t unit = blockIdx.x, b = 0;
         for (uint32_t i = 0; i < total; ++i) {
             const uint32_t q = i % KT_NQ, buf = i & 1;
@@ -418,12 +423,12 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
             const uint8_t* rec = smem + KO_RECS + q * KT_REC;
             const uint32_t dm = reinterpret_cast<const uint32_t*>(rec)[r];
             const float df = f16bits_to_f32(dm & 0xFFFF);
-            const uint64_t d = splat2(MIN ? df : -df), nm = MIN ? splat2(-f16bits_to_f32(dm >> 16)) : 0;
+            const float d = MIN ? df : -df, dmin = MIN ? f16bits_to_f32(dm >> 16) : 0.f;
             if (b == 0)
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) sum[c][j] = 0;
+                    for (int j = 0; j < 8; ++j) sum[c][j] = 0.f;
             if (!wait(KO_ACC_FULL + 8 * buf, (i >> 1) & 1, STATUS_TIMEOUT_MMA)) break;
             tc_after();
 #pragma unroll
@@ -433,15 +438,15 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
                     uint32_t v[8], u[8];
                     tmem_ld8_async(t_base + buf * ACC_COLS + col, v);
                     if constexpr (MIN) tmem_ld8_async(t_base + buf * ACC_COLS + 128 + col, u);
-                    const ulonglong2* d8 = reinterpret_cast<const ulonglong2*>(rec + 512 + 4 * col);
-                    const ulonglong2 d80 = d8[0], d81 = d8[1];
-                    const uint64_t dd[4] = {d80.x, d80.y, d81.x, d81.y};
+                    const float4* d8 = reinterpret_cast<const float4*>(rec + 512 + 4 * col);
+                    const float4 e0 = d8[0], e1 = d8[1];
+                    const float e[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
                     tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        uint64_t t = mul2_apart(mul2(d, dd[j]), int2_to_f32(v[2 * j], v[2 * j + 1]), p.neg_zero);
-                        if constexpr (MIN) t = add2(t, mul2_apart(mul2(nm, dd[j]), int2_to_f32(u[2 * j], u[2 * j + 1]), p.neg_zero));
-                        sum[c][j] = add2(sum[c][j], t);
+                    for (int j = 0; j < 8; ++j) {
+                        float t = __fmul_rn(__fmul_rn(d, e[j]), (float)(int)v[j]);
+                        if constexpr (MIN) t = __fsub_rn(t, __fmul_rn(__fmul_rn(dmin, e[j]), (float)(int)u[j]));
+                        sum[c][j] = __fadd_rn(sum[c][j], t);
                     }
                 }
             }
@@ -462,7 +467,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
                     for (int j = 0; j < 8; ++j) {
                         const uint32_t m = 8 * (cg + 4 * c) + j;
                         if (m < p.mt && m0 + m < p.M)
-                            store_as(p.out, p.out_dtype, (size_t)(m0 + m) * p.N + n, __uint_as_float((uint32_t)(sum[c][j >> 1] >> (32 * (j & 1)))));
+                            store_as(p.out, p.out_dtype, (size_t)(m0 + m) * p.N + n, sum[c][j]);
                     }
         }
     }
@@ -491,12 +496,12 @@ struct KqSmallParams {
     int out_dtype;
 };
 constexpr int KS_WARPS = 16;
-__host__ __device__ constexpr uint32_t ks_depth(int fmt) { return fmt == FMT_Q2_K ? 6 : 4; }      // items in flight per warp
-__host__ __device__ constexpr uint32_t ks_slot(int fmt) { return 16 * 4 * kq_pitch(fmt); }        // bytes of an item
-__host__ __device__ constexpr uint32_t ks_round(int nt) { return 64 / nt; }                       // items between two meetings
+__host__ __device__ constexpr uint32_t ks_depth(int fmt, int nt) { return fmt == FMT_Q2_K ? (nt == 4 ? 5 : 6) : (nt == 4 ? 3 : 5); }  // ring slots of a warp
+__host__ __device__ constexpr uint32_t ks_slot(int fmt) { return 16 * kq_pitch(fmt); }  // bytes of an item
+__host__ __device__ constexpr uint32_t ks_round(int nt) { return nt == 1 ? 32 : 16; }    // items between two meetings
 constexpr uint32_t KS_COL = 20;  // floats from one activation row's 16 terms to the next: 8 lanes x 4 quads hit 32 banks
 __host__ __device__ constexpr uint32_t ks_table(int nt) { return ks_round(nt) * 8 * nt * KS_COL * 4; }
-__host__ __device__ constexpr size_t ks_smem(int fmt, int nt) { return KS_WARPS * ks_depth(fmt) * ks_slot(fmt) + 2 * ks_table(nt) + 128 * nt * 4; }
+__host__ __device__ constexpr size_t ks_smem(int fmt, int nt) { return KS_WARPS * ks_depth(fmt, nt) * ks_slot(fmt) + 2 * ks_table(nt) + 128 * nt * 4; }
 static_assert(ks_smem(FMT_Q2_K, 1) <= 232448 && ks_smem(FMT_Q3_K, 4) <= 232448 && ks_smem(FMT_Q2_K, 4) <= 232448, "shared memory");
 
 // The operand words of one row of an item: v[g][k] = scaled codes of bit pair g, word k of the lane's 16 code bytes.
@@ -538,7 +543,7 @@ __device__ __forceinline__ void q3k_row(const uint32_t* raw, uint32_t sh, uint32
 template <int FMT, int NT>
 __global__ void __launch_bounds__(KS_WARPS * 32, 1) kq_small_kernel(const KqSmallParams p) {
     constexpr bool MIN = FMT == FMT_Q2_K;
-    constexpr uint32_t BB = fmt_block_bytes(FMT), PITCH = kq_pitch(FMT), DEPTH = ks_depth(FMT), SLOT = ks_slot(FMT), R = ks_round(NT);
+    constexpr uint32_t BB = fmt_block_bytes(FMT), PITCH = kq_pitch(FMT), DEPTH = ks_depth(FMT, NT), SLOT = ks_slot(FMT), R = ks_round(NT);
     constexpr uint32_t ITEM = 8 * NT * KS_COL;  // floats of an item's terms
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -551,21 +556,19 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 1) kq_small_kernel(const KqSmal
     const uint8_t* wend = p.w + (size_t)p.N * p.row_bytes;
     grid_dep_launch();
 
-    uint32_t fx = warp, fslot = 0;  // next item to fetch, its ring slot
+    const uint32_t step_s = KS_WARPS / p.nblk, step_b = KS_WARPS % p.nblk;  // KS_WARPS items further, in slabs and blocks
+    uint32_t fx = warp, fb = warp % p.nblk, fn = (s_lo + warp / p.nblk) * 16, fslot = 0;  // next item to fetch: its block, first row and ring slot
     auto fetch = [&]() {
-        if (fx < total) {
-            const uint32_t slab = s_lo + fx / p.nblk, b = fx % p.nblk, n0 = slab * 16;
-            const uint8_t* blk = p.w + (size_t)n0 * p.row_bytes + (size_t)b * BB;
-            uint32_t dst = ring + fslot * SLOT;
-#pragma unroll
-            for (uint32_t q = 0; q < 16; ++q) {
-                copy_block_word<FMT>(dst, blk, wend, lane, n0 + q < p.N, p.w);
-                blk += p.row_bytes;
-                dst += PITCH * 4;
-            }
-        }
+        if (fx < total)
+            copy_rows<FMT, 16>(ring + fslot * SLOT, p.w + (size_t)fn * p.row_bytes + (size_t)fb * BB, p.row_bytes, lane, fn + 16 < p.N, p.N - fn, wend);
         asm volatile("cp.async.commit_group;" ::: "memory");
         fx += KS_WARPS;
+        fn += 16 * step_s;
+        fb += step_b;
+        if (fb >= p.nblk) {
+            fb -= p.nblk;
+            fn += 16;
+        }
         if (++fslot == DEPTH) fslot = 0;
     };
 #pragma unroll 1
@@ -576,13 +579,15 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 1) kq_small_kernel(const KqSmal
     uint4 bf[NT][4];       // the activation codes of the lane's elements: bit pair g of the code bytes
     uint32_t bm[NT][2];
     float d8[NT][2];
-    uint32_t have = 0xFFFFFFFFu, slot = 0;
+    uint32_t have = 0xFFFFFFFFu, slot = 0, xb = warp % p.nblk;  // xb: block of the warp's next item
     for (uint32_t x0 = 0, rd = 0; x0 < total; x0 += R, ++rd) {
         float* tab = table + (rd & 1) * R * ITEM;
 #pragma unroll 1
         for (uint32_t x = x0 + warp; x < min(x0 + R, total); x += KS_WARPS) {
             fetch();
-            const uint32_t b = x % p.nblk, n0 = (s_lo + x / p.nblk) * 16;
+            const uint32_t b = xb;
+            xb += step_b;
+            if (xb >= p.nblk) xb -= p.nblk;
             if (b != have) {  // stays the same where 16 is a multiple of nblk or nblk is 16
                 have = b;
 #pragma unroll
@@ -606,8 +611,9 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 1) kq_small_kernel(const KqSmal
             }
             asm volatile("cp.async.wait_group %0;" ::"n"(DEPTH - 1) : "memory");
             __syncwarp();
-            const uint32_t* ra = reinterpret_cast<const uint32_t*>(smem + (warp * DEPTH + slot) * SLOT) + g * PITCH;
-            const uint32_t* rb = ra + 8 * PITCH;
+            const uint32_t at = (g * p.row_bytes + b * BB) & 15u;  // where the row's block sits in its slot (eight rows are a multiple of 16 bytes)
+            const uint32_t* ra = reinterpret_cast<const uint32_t*>(smem + (warp * DEPTH + slot) * SLOT + g * PITCH + (at & 12u));
+            const uint32_t* rb = ra + 8 * PITCH / 4;
             uint32_t va[4][4], vb[4][4], dma, dmb;
             if constexpr (MIN) {
                 q2k_row(ra, t, va);
@@ -615,11 +621,11 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 1) kq_small_kernel(const KqSmal
                 dma = ra[20];
                 dmb = rb[20];
             } else {
-                const uint32_t sha = 8 * (((n0 + g) * p.row_bytes + b * BB) & 2u), shb = 8 * (((n0 + 8 + g) * p.row_bytes + b * BB) & 2u);
-                q3k_row(ra, sha, t, va);
-                q3k_row(rb, shb, t, vb);
-                dma = (ra[27] >> sha) & 0xFFFFu;
-                dmb = (rb[27] >> shb) & 0xFFFFu;
+                const uint32_t sh = 8 * (at & 2u);
+                q3k_row(ra, sh, t, va);
+                q3k_row(rb, sh, t, vb);
+                dma = (ra[27] >> sh) & 0xFFFFu;
+                dmb = (rb[27] >> sh) & 0xFFFFu;
             }
             const float da = f16bits_to_f32(dma & 0xFFFF), db = f16bits_to_f32(dmb & 0xFFFF);
             float* to = tab + (x - x0) * ITEM;
@@ -713,11 +719,11 @@ KqPlan kq_plan(int fmt, size_t M, size_t K, size_t N, int sm_count) {
 }
 
 template <int FMT>
-cudaError_t launch_tc(const KqTcParams& p, const CUtensorMap& amap, const CUtensorMap& mmap, int sm_count, cudaStream_t st) {
+cudaError_t launch_tc(const KqTcParams& p, const CUtensorMap& amap, const CUtensorMap& mmap, const CUtensorMap& wmap, int sm_count, cudaStream_t st) {
     static PerDeviceOnce attrs;
     cudaError_t e = attrs.run([] { return cudaFuncSetAttribute(kq_tc_kernel<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kt_smem(FMT)); });
     if (e != cudaSuccess) return e;
-    return launch_pdl(kq_tc_kernel<FMT>, dim3(p.nunits < (uint32_t)sm_count ? p.nunits : (uint32_t)sm_count), dim3(KT_THREADS), kt_smem(FMT), st, amap, mmap, p);
+    return launch_pdl(kq_tc_kernel<FMT>, dim3(p.nunits < (uint32_t)sm_count ? p.nunits : (uint32_t)sm_count), dim3(KT_THREADS), kt_smem(FMT), st, amap, mmap, wmap, p);
 }
 template <int FMT, int NT>
 cudaError_t launch_small(const KqSmallParams& p, int sm_count, cudaStream_t st) {
@@ -735,11 +741,12 @@ cudaError_t launch_small(const KqSmallParams& p, int sm_count, cudaStream_t st) 
     return e;
 }
 
-bool encode(CUtensorMap* map, void* base, size_t inner, size_t rows, uint32_t box_inner, uint32_t box_rows, CUtensorMapSwizzle sw) {
+bool encode(CUtensorMap* map, CUtensorMapDataType type, size_t elem, void* base, size_t inner, size_t rows, uint32_t box_inner, uint32_t box_rows,
+            CUtensorMapSwizzle sw) {
     const cuuint32_t estr[2] = {1, 1}, box[2] = {box_inner, box_rows};
-    const cuuint64_t gdim[2] = {inner, rows}, gstride[1] = {inner};
-    return encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, base, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    const cuuint64_t gdim[2] = {inner, rows}, gstride[1] = {inner * elem};
+    return encode_tiled()(map, type, 2, base, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace
@@ -784,15 +791,17 @@ cudaError_t launch_kq_lowbit(int fmt, const void* act, int act_dtype, const void
         p.row_bytes = nblk * (uint32_t)fmt_block_bytes(fmt);
         p.idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((p.mt >> 3) << 17) | ((128u >> 4) << 24);  // int32 <- s8 x s8, K-major, N = mt, M = 128
         p.out_dtype = out_dtype;
-        p.neg_zero = 0x8000000080000000ull;
         p.status = status;
-        CUtensorMap amap, mmap;
-        if (!encode(&amap, s.codes, K, M, 128, plan.mt, CU_TENSOR_MAP_SWIZZLE_128B) ||
-            !encode(&mmap, s.mins, (size_t)nblk * 32, M, 32, plan.mt, CU_TENSOR_MAP_SWIZZLE_32B)) {
-            snprintf(err, err_len, "cuTensorMapEncodeTiled failed (activation image %p, K=%zu, M=%zu)", (void*)s.codes, K, M);
+        p.raw_tma = p.row_bytes % 16 == 0;
+        CUtensorMap amap, mmap, wmap{};
+        if (!encode(&amap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, s.codes, K, M, 128, plan.mt, CU_TENSOR_MAP_SWIZZLE_128B) ||
+            !encode(&mmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, s.mins, (size_t)nblk * 32, M, 32, plan.mt, CU_TENSOR_MAP_SWIZZLE_32B) ||
+            (p.raw_tma && !encode(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void*>(w), p.row_bytes / 2, N, kq_pitch(fmt) / 2, 128,
+                                  CU_TENSOR_MAP_SWIZZLE_NONE))) {
+            snprintf(err, err_len, "cuTensorMapEncodeTiled failed (activation image %p, weight %p, M=%zu K=%zu N=%zu)", (void*)s.codes, w, M, K, N);
             return cudaErrorInvalidValue;
         }
-        e = fmt == FMT_Q2_K ? launch_tc<FMT_Q2_K>(p, amap, mmap, sm_count, st) : launch_tc<FMT_Q3_K>(p, amap, mmap, sm_count, st);
+        e = fmt == FMT_Q2_K ? launch_tc<FMT_Q2_K>(p, amap, mmap, wmap, sm_count, st) : launch_tc<FMT_Q3_K>(p, amap, mmap, wmap, sm_count, st);
     } else {
         KqSmallParams p{};
         p.w = static_cast<const uint8_t*>(w);
