@@ -44,9 +44,9 @@ size_t prefill_workspace_bytes(int fmt, int act_dtype, size_t M, size_t K, size_
 cudaError_t launch_prefill(int fmt, const void* act, int act_dtype, const void* w, void* out, int out_dtype, size_t M,
                            size_t K, size_t N, void* ws, size_t ws_bytes, int sm_count, cudaStream_t st,
                            unsigned int* status, bool* ws_too_small, char* err, size_t err_len, bool acts_prepared);
-bool kq_lowbit_supported(int fmt, size_t M, size_t K, size_t N);
-size_t kq_lowbit_workspace_bytes(size_t M, size_t K);
-cudaError_t launch_kq_lowbit(int fmt, const void* act, int act_dtype, const void* w, void* out, int out_dtype, size_t M, size_t K,
+bool kq_i8_supported(int fmt, size_t M, size_t K, size_t N, int sm_count);
+size_t kq_i8_workspace_bytes(size_t M, size_t K);
+cudaError_t launch_kq_i8(int fmt, const void* act, int act_dtype, const void* w, void* out, int out_dtype, size_t M, size_t K,
                              size_t N, void* ws, size_t ws_bytes, int sm_count, cudaStream_t st, unsigned int* status,
                              bool* ws_too_small, char* err, size_t err_len, bool acts_prepared);
 cudaError_t launch_swiglu_gate(const float* gate, const float* up, void* out, int out_dtype, size_t n, int sm_count,
@@ -174,8 +174,8 @@ bool i8_in_passes(int format, size_t M, size_t K, size_t N);
 size_t workspace_need(int op, int format, int act_dtype, size_t M, size_t K, size_t N) {
     if (!known_format(format) || M == 0 || K == 0 || N == 0 || K % fmt_block_size(format)) return 0;
     const bool swiglu = op == B200Q_OP_QUANT_SWIGLU;
-    if (kq_lowbit_supported(format, M, K, N))  // Q2_K, Q3_K: the Q8_K image (+ gate and up for SwiGLU)
-        return kq_lowbit_workspace_bytes(M, K) + (swiglu ? 2 * ((M * N * sizeof(float) + 255) & ~(size_t)255) : 0);
+    if (kq_i8_supported(format, M, K, N, sm_count_current()))  // the Q8_K image (+ gate and up for SwiGLU)
+        return kq_i8_workspace_bytes(M, K) + (swiglu ? 2 * ((M * N * sizeof(float) + 255) & ~(size_t)255) : 0);
     if (prefill_supported(format, M, K, N)) {
         size_t a = prefill_workspace_bytes(format, act_dtype, M, K, N, sm_count_current());
         // large-M SwiGLU = two prefill GEMMs into scratch, then the gate
@@ -224,7 +224,7 @@ cudaError_t launch_i8_passes(int format, const void* act, int act_dtype, const v
 // share.  The bf16 tensor-core path prepares one form per class of formats (K-quants: Q8_K round trip; others: bf16);
 // the mma.sync small-M kernel one image per format (Q5_K reads Q4_K's).
 int prepared_class(int format, size_t M, size_t K, size_t N) {
-    if (kq_lowbit_supported(format, M, K, N)) return 102;  // Q2_K and Q3_K read one image
+    if (kq_i8_supported(format, M, K, N, sm_count_current())) return format == FMT_Q2_K || format == FMT_Q3_K ? 102 : -1;
     if (prefill_supported(format, M, K, N)) return (format == FMT_Q4_K || format == FMT_Q5_K || format == FMT_Q6_K) ? 101 : 100;
     if (gemv_m1_supported(format, M, K, N, false) || gemv_m1_f32_supported(format, M, K, N)) return -1;
     if (smallm_i8_preferred(format, M, K, N, sm_count_current()) || i8_in_passes(format, M, K, N)) return -1;
@@ -242,9 +242,9 @@ int quant_matmul_impl(int format, const void* act, int act_dtype, const void* w,
     if (!status) return fail(B200Q_ERR_CUDA, "quant_matmul: cannot resolve the device status word");
     bool small = false;
     cudaError_t e;
-    if (kq_lowbit_supported(format, M, K, N)) {
+    if (kq_i8_supported(format, M, K, N, sm_count_current())) {
         char msg[256] = "";
-        e = launch_kq_lowbit(format, act, act_dtype, w, out, out_dtype, M, K, N, ws, ws_bytes, sm_count_current(), st, status, &small, msg, sizeof(msg),
+        e = launch_kq_i8(format, act, act_dtype, w, out, out_dtype, M, K, N, ws, ws_bytes, sm_count_current(), st, status, &small, msg, sizeof(msg),
                              acts_prepared);
         if (e != cudaSuccess && msg[0]) return fail(B200Q_ERR_CUDA, "quant_matmul: %s", msg);
     } else if (prefill_supported(format, M, K, N)) {
@@ -432,7 +432,7 @@ int b200q_quant_swiglu(int format, const void* act, int act_dtype, const void* w
         return fail(B200Q_ERR_WORKSPACE_TOO_SMALL, "quant_swiglu: workspace of %zu bytes is too small, need %zu", ws_bytes, need);
     bool small = false;
     cudaError_t e;
-    if (kq_lowbit_supported(format, M, K, N)) {
+    if (kq_i8_supported(format, M, K, N, sm_count_current())) {
         // two products into f32 scratch (the second reads the first one's Q8_K image), then the gate
         const size_t mn = (M * N * sizeof(float) + 255) & ~(size_t)255;
         float* g = static_cast<float*>(ws);
@@ -440,10 +440,10 @@ int b200q_quant_swiglu(int format, const void* act, int act_dtype, const void* w
         uint8_t* rest = static_cast<uint8_t*>(ws) + 2 * mn;
         const size_t rest_bytes = ws_bytes - 2 * mn;
         char msg[256] = "";
-        e = launch_kq_lowbit(format, act, act_dtype, w_gate, g, DT_F32, M, K, N, rest, rest_bytes, sm_count_current(), st, status, &small, msg, sizeof(msg),
+        e = launch_kq_i8(format, act, act_dtype, w_gate, g, DT_F32, M, K, N, rest, rest_bytes, sm_count_current(), st, status, &small, msg, sizeof(msg),
                              false);
         if (e == cudaSuccess && !small)
-            e = launch_kq_lowbit(format, act, act_dtype, w_up, u, DT_F32, M, K, N, rest, rest_bytes, sm_count_current(), st, status, &small, msg, sizeof(msg),
+            e = launch_kq_i8(format, act, act_dtype, w_up, u, DT_F32, M, K, N, rest, rest_bytes, sm_count_current(), st, status, &small, msg, sizeof(msg),
                                  true);
         if (e != cudaSuccess && msg[0]) return fail(B200Q_ERR_CUDA, "quant_swiglu: %s", msg);
         if (e == cudaSuccess && !small) e = launch_swiglu_gate(g, u, out, out_dtype, M * N, sm_count_current(), st);

@@ -1,19 +1,20 @@
-// Quantized matmul for Q2_K and Q3_K, every number of activation rows, with the bits of boostr's CPU path
-// (src/quant/cpu/kernels/quant_matmul.rs:107-135): each activation row is quantised to Q8_K
+// Quantized matmul of the K-quant formats with the bits of boostr's CPU path
+// (src/quant/cpu/kernels/quant_matmul.rs:107-135) on the integer tensor cores: Q2_K and Q3_K for every number of activation
+// rows, Q4_K and Q5_K between the kernels for few rows and the bf16 path.  Each activation row is quantised to Q8_K
 // (src/quant/cpu/kernels/simd/quantize_act_q8k.rs:26-98), a 256-block contributes
 // (d * d8) * isum - (dmin * d8) * summs with exact integer sums (src/quant/cpu/kernels/simd/fused_q2k_q8k_dot.rs:152-214,
-// fused_q3k_q8k_dot.rs:33-205 in the form x86-64 runs; Q3_K has no min term) and the blocks are added in K order without
-// FMA contraction.
+// fused_q3k_q8k_dot.rs:33-205, fused_q4k_q8k_dot.rs:111-172, fused_q5k_q8k_dot.rs:27-122 in the form x86-64 runs; Q3_K has
+// no min term) and the blocks are added in K order without FMA contraction.
 //
-// What both kernels build on: the PRODUCT of a code and its 16-wide sub-block's scale fits a signed byte (Q2_K: 0..3 times
-// 0..15; Q3_K: -(-4..3) times -32..31 lies in [-128, 124]; the sign is given back by the f32 factor), so the scales go
-// into the operand, a whole 256-block is one K = 256 integer product and only one sum per (row, activation row, block)
-// has to be scaled.  The min term is a second integer product of the mins with the activation's sums of 16 codes, which
-// travel as two bytes, sum = lo + 16 hi.
+// What both kernels build on: the PRODUCT of a code and its sub-block's scale goes into the operand, so a whole 256-block is
+// one K = 256 integer product and only one sum per (row, activation row, block) has to be scaled.  For Q2_K (0..3 times
+// 0..15) and Q3_K (-(-4..3) times -32..31 lies in [-128, 124]; the sign is given back by the f32 factor) it fits a signed
+// byte; for Q4_K and Q5_K (below 2048) it is lo + 128 hi, two operands.  The min term is another integer product, of the
+// mins with the activation's sums of 16 codes, which travel as two bytes, sum = lo + 16 hi.
 //
 //   * kq_act_prep_kernel: codes [M][K], min operand [M][K / 256][lo 16 | hi 16], scales d8 [K / 256][M]: 292 bytes per run;
-//   * kq_tc_kernel<FMT>: tcgen05.mma.kind::i8, tiles of 128 weight rows x up to 128 activation rows;
-//   * kq_small_kernel<FMT, NT>: mma.sync, slabs of 16 weight rows x 8 NT activation rows, for few activation rows.
+//   * kq_tc_kernel<FMT>: tcgen05.mma.kind::i8, tiles of 128 weight rows x up to 128 (Q4_K, Q5_K: 48) activation rows;
+//   * kq_small_kernel<FMT, NT>: mma.sync, slabs of 16 weight rows x 8 NT activation rows, Q2_K / Q3_K with few rows.
 #include <cuda.h>
 
 #include <cstdio>
@@ -33,8 +34,10 @@ constexpr uint32_t RUN_BYTES = 292;  // of scratch per (activation row, 256-bloc
 // CHUNKS at most, PITCH bytes from row to row in shared memory.  (Copies of 4 bytes - cp.async - ran at about one lane per
 // cycle and took 2-4 us per 128 rows, more than everything else.)  Any such pitch puts one word of 32 rows into eight banks:
 // 112 and 144 use all of these.
+// (Rows of Q4_K and Q5_K are whole chunks and always come by TMA.)
 __host__ __device__ constexpr uint32_t kq_chunks(int fmt) { return fmt == FMT_Q2_K ? 6 : 8; }
-__host__ __device__ constexpr uint32_t kq_pitch(int fmt) { return fmt == FMT_Q2_K ? 112 : 144; }
+__host__ __device__ constexpr uint32_t kq_pitch(int fmt) { return fmt == FMT_Q2_K ? 112 : fmt == FMT_Q5_K ? 176 : 144; }
+__host__ __device__ constexpr bool kq_wide(int fmt) { return fmt == FMT_Q4_K || fmt == FMT_Q5_K; }  // two-byte products
 
 // One warp per (activation row, 256-block): Q8_K codes (d = amax / 127, id = 127 / amax, round half to even), the sums of
 // 16 codes as lo + 16 hi with lo in [-8, 7] (a sum is at most 2048 in size, so hi fits a signed byte), the scale.
@@ -106,6 +109,13 @@ __device__ __forceinline__ uint32_t q3k_scaled(uint32_t w, uint32_t hw, uint32_t
     const uint32_t c = ((w >> (2 * G)) & 0x03030303u) | high;
     return (c * neg_s + u4) ^ 0x80808080u;
 }
+// Q4_K, Q5_K: four codes (below 32) times 2 sc (sc below 64) in 16-bit lanes; the high bytes are the products' hi = p >> 7, the
+// low bytes 2 lo, all even, so that one shift of the word halves them in place.
+__device__ __forceinline__ void wide_scaled(uint32_t c, uint32_t sc2, uint32_t& lo, uint32_t& hi) {
+    const uint32_t pe = (c & 0x00FF00FFu) * sc2, po = __byte_perm(c, 0u, 0x4341) * sc2;
+    hi = __byte_perm(pe, po, 0x7351);
+    lo = __byte_perm(pe, po, 0x6240) >> 1;
+}
 __device__ __forceinline__ uint32_t byte_of(uint32_t x, uint32_t i) { return __byte_perm(x, 0u, 0x4440u | i); }
 
 __device__ __forceinline__ void store_as(void* out, int dt, size_t idx, float v) {
@@ -145,9 +155,10 @@ __device__ __forceinline__ void copy_rows(uint32_t dst, const uint8_t* blk, uint
 
 // =================================================================================================== tensor-core kernel
 // One CTA per SM, persistent over (128 weight rows, mt activation rows) tiles, all of K each (the sums grow in K order, so
-// no tile is cut).  Per 256-block: two copy warps bring the 128 packed blocks (cp.async: any row alignment), one of two sets
-// of four decode warps writes the scaled codes as two 128-byte-swizzled K-major operand tiles, the activation codes come by
-// TMA, one thread issues 8 MMAs (+ 2 for the mins) into one of two accumulators, and sixteen drain warps (thread = weight
+// no tile is cut).  Per 256-block: the 128 packed blocks come by TMA (by cp.async from two warps where rows are not 16-byte aligned),
+// two sets of four decode warps, taking the blocks in turn, write the scaled codes as 128-byte-swizzled K-major operand tiles,
+// the activation codes come by TMA, one thread issues 8 MMAs
+// (16 for two-byte products; + 2 for the mins) into one of two accumulators, and sixteen drain warps (thread = weight
 // row x every fourth group of 8 activation rows) scale the sums in packed f32 and add them to their registers.
 // What bounds it: instruction issue - per (128 rows x 256 K) about 300 instructions a row of decode, and 6 (Q2_K) or 3
 // (Q3_K) a sum of drain - ahead of the tensor pipe.
@@ -168,18 +179,22 @@ struct KqTcParams {
 constexpr int KT_DEC = 8, KT_DRAIN = 16, KT_COPY = 2;
 constexpr int KT_W_COPY = KT_DEC + KT_DRAIN, KT_W_ACT = KT_W_COPY + KT_COPY, KT_W_MMA = KT_W_ACT + 1;
 constexpr int KT_THREADS = (KT_W_MMA + 1) * 32;
-// Every ring has an even depth: the decode sets take the blocks in turn, so a slot belongs to one set, which sees every
-// phase of the slot's barriers (a parity wait cannot tell phase k from k - 2).
-constexpr uint32_t KT_NS = 2, KT_NR = 4, KT_NQ = 4;
+constexpr uint32_t KT_NS = 2, KT_NQ = 4;
+__host__ __device__ constexpr uint32_t kt_nr(int fmt) { return kq_wide(fmt) ? 2 : 4; }
 constexpr uint32_t KT_ATOM = 128 * 128;
 constexpr uint32_t KT_REC = 512 + 512;  // the rows' d | dmin, the activation rows' d8
-constexpr int KO_FULL = 0, KO_EMPTY = 16, KO_RAW_FULL = 32, KO_RAW_EMPTY = 64, KO_ACC_FULL = 96, KO_ACC_EMPTY = 112, KO_REC_FULL = 128,
-              KO_REC_EMPTY = 160, KO_TMEM = 192, KO_DEAD = 196, KO_RECS = 1024, KO_STAGES = KO_RECS + KT_NQ * KT_REC;
-// a stage: two operand tiles of scaled codes | tile of mins (Q2_K) | two tiles of activation codes | sums of 16 (Q2_K)
-__host__ __device__ constexpr uint32_t kt_stage(int fmt) { return 4 * KT_ATOM + (fmt == FMT_Q2_K ? 128 * 64 + 128 * 32 : 0); }
+// Every ring has an even depth: the decode sets take the blocks in turn, so a slot belongs to one set, which sees every
+// phase of the slot's barriers (a parity wait cannot tell phase k from k - 2).
+constexpr int KO_FULL = 0, KO_EMPTY = 32, KO_RAW_FULL = 64, KO_RAW_EMPTY = 96, KO_ACC_FULL = 128, KO_ACC_EMPTY = 144, KO_REC_FULL = 160,
+              KO_REC_EMPTY = 192, KO_TMEM = 224, KO_DEAD = 228, KO_RECS = 1024, KO_STAGES = KO_RECS + KT_NQ * KT_REC;
+// a stage: two operand tiles of scaled codes (four of two-byte products) | tile of mins | two tiles of activation codes | sums of 16
+__host__ __device__ constexpr uint32_t kt_mt_max(int fmt) { return kq_wide(fmt) ? 48 : 128; }
+__host__ __device__ constexpr uint32_t kt_stage(int fmt) {
+    return ((kq_wide(fmt) ? 4 : 2) * KT_ATOM + (fmt == FMT_Q3_K ? 0 : 128 * 64) + kt_mt_max(fmt) * (256 + (fmt == FMT_Q3_K ? 0 : 32)) + 1023) / 1024 * 1024;
+}
 __host__ __device__ constexpr uint32_t kt_raw(int fmt) { return 128 * kq_pitch(fmt); }
-__host__ __device__ constexpr size_t kt_smem(int fmt) { return 1024 + KO_STAGES + KT_NS * kt_stage(fmt) + KT_NR * kt_raw(fmt); }
-static_assert(KO_STAGES % 1024 == 0 && kt_stage(FMT_Q2_K) % 1024 == 0 && kt_smem(FMT_Q2_K) <= 232448 && kt_smem(FMT_Q3_K) <= 232448, "shared memory");
+__host__ __device__ constexpr size_t kt_smem(int fmt) { return 1024 + KO_STAGES + KT_NS * kt_stage(fmt) + kt_nr(fmt) * kt_raw(fmt); }
+static_assert(KO_STAGES % 1024 == 0 && kt_smem(FMT_Q2_K) <= 232448 && kt_smem(FMT_Q3_K) <= 232448 && kt_smem(FMT_Q5_K) <= 232448, "shared memory");
 
 // rows of 64 bytes with 64-byte swizzle (8-row groups 512 bytes apart) and of 32 bytes with 32-byte swizzle
 __device__ __forceinline__ uint64_t desc_sw64(uint32_t lo) {
@@ -196,10 +211,12 @@ __device__ __forceinline__ uint64_t desc_sw32(uint32_t lo) {
 template <int FMT>
 __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant__ CUtensorMap tmap_min,
                                                               const __grid_constant__ CUtensorMap tmap_w, const KqTcParams p) {
-    constexpr bool MIN = FMT == FMT_Q2_K;
-    constexpr uint32_t BB = fmt_block_bytes(FMT), PITCH = kq_pitch(FMT), RAW = kt_raw(FMT), STAGE = kt_stage(FMT);
-    constexpr uint32_t OFF_AM = 2 * KT_ATOM, OFF_B = OFF_AM + (MIN ? 128 * 64 : 0), OFF_BM = OFF_B + 2 * KT_ATOM;
-    constexpr uint32_t ACC_COLS = MIN ? 256 : 128, TMEM_COLS = 2 * ACC_COLS;
+    constexpr bool MIN = FMT != FMT_Q3_K, WIDE = kq_wide(FMT);
+    constexpr uint32_t BB = fmt_block_bytes(FMT), PITCH = kq_pitch(FMT), RAW = kt_raw(FMT), STAGE = kt_stage(FMT), NR = kt_nr(FMT);
+    constexpr uint32_t MT_MAX = kt_mt_max(FMT), B_TILE = MT_MAX * 128, CHUNKS = (MT_MAX / 8 + 3) / 4;  // groups of 8 activation rows of a drain warp
+    constexpr uint32_t OFF_AM = (WIDE ? 4 : 2) * KT_ATOM, OFF_B = OFF_AM + (MIN ? 128 * 64 : 0), OFF_BM = OFF_B + 2 * B_TILE;
+    // an accumulator: sums | mins (Q2_K); lo | hi | mins . lo | mins . hi (two-byte products)
+    constexpr uint32_t COL = WIDE ? 64 : 128, ACC_COLS = WIDE ? 256 : MIN ? 256 : 128, TMEM_COLS = 2 * ACC_COLS;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);  // the launch reserves 1 KB of slack
     const uint32_t sbase = smem_u32(smem), st_base = sbase + KO_STAGES;
@@ -211,7 +228,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
             mbar_init(sbase + KO_FULL + 8 * s, 5);   // four decode warps + the activation copies (with their byte count)
             mbar_init(sbase + KO_EMPTY + 8 * s, 1);  // the commit behind the block's MMAs
         }
-        for (uint32_t s = 0; s < KT_NR; ++s) {
+        for (uint32_t s = 0; s < NR; ++s) {
             mbar_init(sbase + KO_RAW_FULL + 8 * s, p.raw_tma ? 1 : KT_COPY * 32);  // the TMA copy, or every copying thread
             mbar_init(sbase + KO_RAW_EMPTY + 8 * s, 4);
         }
@@ -250,14 +267,22 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
         const uint8_t* wend = p.w + (size_t)p.N * p.row_bytes;
         uint32_t unit = blockIdx.x, b = 0, n0 = unit / p.nct * 128 + r0;
         for (uint32_t i = 0; i < total; ++i) {
-            const uint32_t rs = i % KT_NR;
-            if (!wait(KO_RAW_EMPTY + 8 * rs, ((i / KT_NR) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) break;
+            const uint32_t rs = i % NR;
+            if (!wait(KO_RAW_EMPTY + 8 * rs, ((i / NR) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) break;
             if (p.raw_tma) {  // one copy a block: rows past N and bytes past the row's end are zero-filled
-                if (warp == KT_W_COPY && lane == 0) {
+                if (warp == KT_W_COPY + 1) {
+                    // the other copy warp pulls the blocks to come into L2: what is in flight into shared memory does not
+                    // cover the latency of DRAM
+                    if (lane == 0 && i + NR < total) {
+                        const uint32_t ab = b + NR, at_b = ab < p.nblk ? ab : ab % p.nblk, at_n = ab < p.nblk ? n0 - r0 : (unit + ab / p.nblk * gridDim.x) / p.nct * 128;
+                        asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(&tmap_w), "r"((int)((at_b * BB & ~15u) / 2)), "r"((int)at_n)
+                                     : "memory");
+                    }
+                } else if (lane == 0) {
                     mbar_expect_tx(sbase + KO_RAW_FULL + 8 * rs, RAW);
                     tma2d(sbase + OFF_RAW + rs * RAW, &tmap_w, (int)((b * BB & ~15u) / 2), (int)n0, sbase + KO_RAW_FULL + 8 * rs);
                 }
-            } else {
+            } else if constexpr (!WIDE) {
                 copy_rows<FMT, 128 / KT_COPY>(sbase + OFF_RAW + rs * RAW + r0 * PITCH, p.w + (size_t)n0 * p.row_bytes + (size_t)b * BB, p.row_bytes, lane,
                                               n0 + 128 / KT_COPY < p.N, n0 < p.N ? p.N - n0 : 0u, wend);
             }
@@ -276,12 +301,13 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
         uint32_t unit = blockIdx.x, b = 0, m0 = unit % p.nct * p.mt;
         for (uint32_t i = 0; i < total; ++i) {
             const uint32_t s = i % KT_NS, q = i % KT_NQ;
+            const uint32_t st = st_base + s * STAGE;
             if (!wait(KO_EMPTY + 8 * s, ((i / KT_NS) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) break;
             if (lane == 0) {
-                const uint32_t st = st_base + s * STAGE, bar = sbase + KO_FULL + 8 * s;
+                const uint32_t bar = sbase + KO_FULL + 8 * s;
                 mbar_expect_tx(bar, 256 * p.mt + (MIN ? 32 * p.mt : 0));
                 tma2d(st + OFF_B, &tmap_act, (int)(b * 256), (int)m0, bar);
-                tma2d(st + OFF_B + KT_ATOM, &tmap_act, (int)(b * 256 + 128), (int)m0, bar);
+                tma2d(st + OFF_B + B_TILE, &tmap_act, (int)(b * 256 + 128), (int)m0, bar);
                 if constexpr (MIN) tma2d(st + OFF_BM, &tmap_min, (int)(b * 32), (int)m0, bar);
             }
             __syncwarp();
@@ -306,19 +332,23 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
         // ------------------------------------------------------------ MMA issue
         for (uint32_t i = 0; i < total; ++i) {
             const uint32_t s = i % KT_NS, buf = i & 1;
-            if (!wait(KO_FULL + 8 * s, (i / KT_NS) & 1, STATUS_TIMEOUT_FULL)) break;
+            const uint32_t st = st_base + s * STAGE, a_lo = desc_lo(st), b_lo = desc_lo(st + OFF_B), d = tmem + buf * ACC_COLS;
             if (!wait(KO_ACC_EMPTY + 8 * buf, ((i >> 1) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) break;
+            if (!wait(KO_FULL + 8 * s, (i / KT_NS) & 1, STATUS_TIMEOUT_FULL)) break;
             tc_after();
             if (elect_one_lane()) {
-                const uint32_t st = st_base + s * STAGE, a_lo = desc_lo(st), b_lo = desc_lo(st + OFF_B), d = tmem + buf * ACC_COLS;
 #pragma unroll
-                for (uint32_t k = 0; k < 8; ++k)
-                    tc_mma_i8(d, desc_sw128(a_lo + (k >> 2) * (KT_ATOM >> 4) + 2 * (k & 3)), desc_sw128(b_lo + (k >> 2) * (KT_ATOM >> 4) + 2 * (k & 3)), p.idesc,
-                              k > 0);
-                if constexpr (MIN) {  // sum of 16 = lo + 16 hi: [m | 8 m] . [lo | hi] + [0 | 8 m] . [lo | hi]
+                for (uint32_t t = 0; t < (WIDE ? 2 : 1); ++t)
+#pragma unroll
+                    for (uint32_t k = 0; k < 8; ++k)
+                        tc_mma_i8(d + t * COL, desc_sw128(a_lo + (2 * t + (k >> 2)) * (KT_ATOM >> 4) + 2 * (k & 3)),
+                                  desc_sw128(b_lo + (k >> 2) * (B_TILE >> 4) + 2 * (k & 3)), p.idesc, k > 0);
+                if constexpr (MIN) {
+                    // Q2_K: sum of 16 = lo + 16 hi in one accumulator, [m | 8 m] . [lo | hi] + [0 | 8 m] . [lo | hi];
+                    // two-byte products: [m | 0] . [lo | hi] and [0 | m] . [lo | hi] apart
                     const uint32_t am = desc_lo(st + OFF_AM), bm = desc_lo(st + OFF_BM);
-                    tc_mma_i8(d + 128, desc_sw64(am), desc_sw32(bm), p.idesc, false);
-                    tc_mma_i8(d + 128, desc_sw64(am + 2), desc_sw32(bm), p.idesc, true);
+                    tc_mma_i8(d + (WIDE ? 2 * COL : COL), desc_sw64(am), desc_sw32(bm), p.idesc, false);
+                    tc_mma_i8(d + (WIDE ? 3 * COL : COL), desc_sw64(am + 2), desc_sw32(bm), p.idesc, !WIDE);
                 }
                 tc_commit_to(sbase + KO_EMPTY + 8 * s);       // the stage may be overwritten once these MMAs have read it
                 tc_commit_to(sbase + KO_ACC_FULL + 8 * buf);  // and the sums are complete
@@ -326,85 +356,142 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
             __syncwarp();
         }
     } else if (warp < KT_DEC) {
-        // ------------------------------------------------------------ decode: one thread per weight row
-        const uint32_t r = threadIdx.x & 127, set = threadIdx.x >> 7, x7 = r & 7;
+        // ------------------------------------------------------------ decode: one thread per weight row, the sets take blocks in turn
+        const uint32_t r = threadIdx.x & 127, set = (uint32_t)warp >> 2, x7 = r & 7;
         uint32_t b = set % p.nblk;  // block of K
         for (uint32_t i = set; i < total; i += 2, b += 2, b -= b >= p.nblk ? p.nblk : 0, b -= b >= p.nblk ? p.nblk : 0) {
-            const uint32_t rs = i % KT_NR, s = i % KT_NS, q = i % KT_NQ;
-            if (!wait(KO_RAW_FULL + 8 * rs, (i / KT_NR) & 1, STATUS_TIMEOUT_FULL)) break;
+            const uint32_t rs = i % NR, s = i % KT_NS, q = i % KT_NQ;
+            if (!wait(KO_RAW_FULL + 8 * rs, (i / NR) & 1, STATUS_TIMEOUT_FULL)) break;
             const uint32_t at = (r * p.row_bytes + b * BB) & 15u;  // where the row's block sits in its slot (128 rows are a multiple of 16 bytes)
             const uint32_t* raw = reinterpret_cast<const uint32_t*>(smem + OFF_RAW + rs * RAW + r * PITCH + (at & 12u));
             uint32_t* rec = reinterpret_cast<uint32_t*>(smem + KO_RECS + q * KT_REC) + r;
             uint8_t* a0 = smem + KO_STAGES + s * STAGE + (r >> 3) * 1024 + x7 * 128;
-            auto put = [&](uint32_t tile, uint32_t c, uint4 v) { *reinterpret_cast<uint4*>(a0 + tile * KT_ATOM + ((c ^ x7) << 4)) = v; };
-            if (!wait(KO_EMPTY + 8 * s, ((i / KT_NS) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) break;
-            uint32_t dm;
-            // sub-block 8 n + 2 g + h = 16-byte chunk 2 g + h of operand tile n
-            if constexpr (FMT == FMT_Q2_K) {
-                uint32_t scw[4];
+            auto put = [&](uint32_t plane, uint32_t c, uint4 v) { *reinterpret_cast<uint4*>(a0 + plane * KT_ATOM + ((c ^ x7) << 4)) = v; };
+            uint32_t dm = 0;
+            bool lost = false;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) scw[k] = raw[k];
+            for (uint32_t n = 0; n < 2; ++n) {  // the halves of the block: operand tiles n (and 2 + n)
+            // All words of the half leave shared memory before the first store into the operand: nothing waits on a load in the
+            // middle of the arithmetic.
+            uint32_t cw[FMT == FMT_Q4_K || FMT == FMT_Q5_K ? 16 : 8], hw[8], sw[4];  // d (| dmin); codes; high bits; scales
+            if constexpr (FMT == FMT_Q2_K) {
                 dm = raw[20];
-                uint4 mn = make_uint4((scw[0] >> 4) & 0x0F0F0F0Fu, (scw[1] >> 4) & 0x0F0F0F0Fu, (scw[2] >> 4) & 0x0F0F0F0Fu, (scw[3] >> 4) & 0x0F0F0F0Fu);
-                const uint4 mn8 = make_uint4(mn.x << 3, mn.y << 3, mn.z << 3, mn.w << 3);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) sw[k] = raw[k];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) cw[k] = raw[4 + 8 * n + k];
+            } else if constexpr (WIDE) {
+                const uint4* src = reinterpret_cast<const uint4*>(raw);
+                const uint4 h = src[0];
+                dm = h.x;
+                sw[0] = h.y; sw[1] = h.z; sw[2] = h.w;
+                if constexpr (FMT == FMT_Q5_K) {
+                    const uint4 v = src[1 + n];
+                    hw[0] = v.x; hw[1] = v.y; hw[2] = v.z; hw[3] = v.w;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint4 v = src[(FMT == FMT_Q5_K ? 3 : 1) + 4 * n + k];
+                    cw[4 * k] = v.x; cw[4 * k + 1] = v.y; cw[4 * k + 2] = v.z; cw[4 * k + 3] = v.w;
+                }
+            } else {
+                const uint32_t sh = 8 * (at & 2u);
+                uint32_t u[9], v[9], x[4];
+#pragma unroll
+                for (int k = 0; k < 9; ++k) {
+                    u[k] = raw[k];
+                    v[k] = raw[8 + 8 * n + k];
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) x[k] = raw[24 + k];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    hw[k] = __funnelshift_r(u[k], u[k + 1], sh) >> (4 * n);
+                    cw[k] = __funnelshift_r(v[k], v[k + 1], sh);
+                }
+#pragma unroll
+                for (int k = 0; k < 3; ++k) sw[k] = __funnelshift_r(x[k], x[k + 1], sh);
+                dm = (x[3] >> sh) & 0xFFFFu;
+            }
+            if (n == 1) {
+                __syncwarp();
+                if (lane == 0) mbar_arrive(sbase + KO_RAW_EMPTY + 8 * rs);
+            } else if (!wait(KO_EMPTY + 8 * s, ((i / KT_NS) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) {
+                lost = true;
+                break;
+            }
+            if (MIN && n == 0) {  // the tile of mins, 64 bytes a row
+                uint4 mn, m1, m2;
+                if constexpr (FMT == FMT_Q2_K) {
+                    mn = make_uint4((sw[0] >> 4) & 0x0F0F0F0Fu, (sw[1] >> 4) & 0x0F0F0F0Fu, (sw[2] >> 4) & 0x0F0F0F0Fu, (sw[3] >> 4) & 0x0F0F0F0Fu);
+                    m1 = make_uint4(mn.x << 3, mn.y << 3, mn.z << 3, mn.w << 3);
+                    m2 = m1;
+                } else {  // unpack_q4k_q5k_scales, src/quant/cpu/kernels/dequant_k_quants/q4k_q5k.rs:108-122; a min covers two sums of 16
+                    const uint32_t a = sw[1] & 0x3F3F3F3Fu, c = ((sw[2] >> 4) & 0x0F0F0F0Fu) | ((sw[1] >> 2) & 0x30303030u);
+                    mn = make_uint4(__byte_perm(a, 0u, 0x1100), __byte_perm(a, 0u, 0x3322), __byte_perm(c, 0u, 0x1100), __byte_perm(c, 0u, 0x3322));
+                    m1 = make_uint4(0, 0, 0, 0);
+                    m2 = mn;
+                }
                 uint4* am = reinterpret_cast<uint4*>(smem + KO_STAGES + s * STAGE + OFF_AM + r * 64);
                 const uint32_t x3 = (r >> 1) & 3;
                 am[0 ^ x3] = mn;
-                am[1 ^ x3] = mn8;
+                am[1 ^ x3] = m1;
                 am[2 ^ x3] = make_uint4(0, 0, 0, 0);
-                am[3 ^ x3] = mn8;
+                am[3 ^ x3] = m2;
+            }
+            if constexpr (WIDE) {
+                // bytes 32 j .. of low nibbles are sub-block 2 j, of high nibbles sub-block 2 j + 1; Q5_K: bit e of word j of the
+                // fifth bits belongs to element e of sub-block j
+                const uint32_t scw = n ? (sw[2] & 0x0F0F0F0Fu) | ((sw[0] >> 2) & 0x30303030u) : sw[0] & 0x3F3F3F3Fu;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) scw[k] &= 0x0F0F0F0Fu;
+                for (int j = 0; j < 4; ++j) {  // sub-block 4 n + j = 16-byte chunks 2 j, 2 j + 1 of the tile
+                    const uint32_t sc2 = 2 * byte_of(scw, j);
 #pragma unroll
-                for (int nh = 0; nh < 4; ++nh) {
-                    const int n = nh >> 1, h = nh & 1;
-                    const uint32_t w0 = raw[4 + 4 * nh], w1 = raw[5 + 4 * nh], w2 = raw[6 + 4 * nh], w3 = raw[7 + 4 * nh];
-                    auto one = [&](auto gc) {
+                    for (int k = 0; k < 2; ++k) {
+                        uint32_t lo[4], hi[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            uint32_t c = (cw[8 * (j >> 1) + 4 * k + e] >> (4 * (j & 1))) & 0x0F0F0F0Fu;
+                            if constexpr (FMT == FMT_Q5_K) c |= (((hw[j] >> (4 * (4 * k + e))) & 15u) * 0x02040810u) & 0x10101010u;
+                            wide_scaled(c, sc2, lo[e], hi[e]);
+                        }
+                        put(n, 2 * j + k, make_uint4(lo[0], lo[1], lo[2], lo[3]));
+                        put(2 + n, 2 * j + k, make_uint4(hi[0], hi[1], hi[2], hi[3]));
+                    }
+                }
+            } else {
+                uint32_t scw[2];  // the half's eight scales
+                if constexpr (FMT == FMT_Q2_K) {
+                    scw[0] = (n ? sw[2] : sw[0]) & 0x0F0F0F0Fu;
+                    scw[1] = (n ? sw[3] : sw[1]) & 0x0F0F0F0Fu;
+                } else {
+                    scw[0] = ((sw[0] >> (4 * n)) & 0x0F0F0F0Fu) | ((n ? sw[2] : sw[2] << 4) & 0x30303030u);
+                    scw[1] = ((sw[1] >> (4 * n)) & 0x0F0F0F0Fu) | ((n ? sw[2] >> 2 : sw[2] << 2) & 0x30303030u);
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    auto one = [&](auto gc) {  // sub-block 8 n + 2 g + h = 16-byte chunk 2 g + h of the tile
                         constexpr int G = decltype(gc)::value;
-                        const uint32_t sc = byte_of(scw[2 * n + (G >> 1)], 2 * (G & 1) + h);
-                        put(n, 2 * G + h, make_uint4(q2k_scaled<G>(w0, sc), q2k_scaled<G>(w1, sc), q2k_scaled<G>(w2, sc), q2k_scaled<G>(w3, sc)));
+                        const uint32_t sc = byte_of(scw[G >> 1], 2 * (G & 1) + h);
+                        uint32_t v[4];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            if constexpr (FMT == FMT_Q2_K) v[k] = q2k_scaled<G>(cw[4 * h + k], sc);
+                            else v[k] = q3k_scaled<G>(cw[4 * h + k], hw[4 * h + k], 32u - sc, sc * 0x04040404u);
+                        }
+                        put(n, 2 * G + h, make_uint4(v[0], v[1], v[2], v[3]));
                     };
                     one(std::integral_constant<int, 0>{});
                     one(std::integral_constant<int, 1>{});
                     one(std::integral_constant<int, 2>{});
                     one(std::integral_constant<int, 3>{});
                 }
-            } else {
-                const uint32_t sh = 8 * (at & 2u);
-                auto word = [&](int k) { return __funnelshift_r(raw[k], raw[k + 1], sh); };
-                dm = (raw[27] >> sh) & 0xFFFFu;
-                const uint32_t l0 = word(24), l1 = word(25), hh = word(26);
-                const uint32_t scw[4] = {(l0 & 0x0F0F0F0Fu) | ((hh << 4) & 0x30303030u), (l1 & 0x0F0F0F0Fu) | ((hh << 2) & 0x30303030u),
-                                         ((l0 >> 4) & 0x0F0F0F0Fu) | (hh & 0x30303030u), ((l1 >> 4) & 0x0F0F0F0Fu) | ((hh >> 2) & 0x30303030u)};
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    uint32_t hw[4];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) hw[k] = word(4 * h + k);
-#pragma unroll
-                    for (int n = 0; n < 2; ++n) {
-                        uint32_t w[4];
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) w[k] = word(8 + 8 * n + 4 * h + k);
-                        auto one = [&](auto gc) {
-                            constexpr int G = decltype(gc)::value;
-                            const uint32_t u = byte_of(scw[2 * n + (G >> 1)], 2 * (G & 1) + h), ns = 32u - u, u4 = u * 0x04040404u;
-                            put(n, 2 * G + h, make_uint4(q3k_scaled<G>(w[0], hw[0] >> (4 * n), ns, u4), q3k_scaled<G>(w[1], hw[1] >> (4 * n), ns, u4),
-                                                         q3k_scaled<G>(w[2], hw[2] >> (4 * n), ns, u4), q3k_scaled<G>(w[3], hw[3] >> (4 * n), ns, u4)));
-                        };
-                        one(std::integral_constant<int, 0>{});
-                        one(std::integral_constant<int, 1>{});
-                        one(std::integral_constant<int, 2>{});
-                        one(std::integral_constant<int, 3>{});
-                    }
-                }
             }
+            }
+            if (lost) break;
             proxy_fence();  // the operand bytes are read by the tensor core (async proxy)
             __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(sbase + KO_FULL + 8 * s);
-                mbar_arrive(sbase + KO_RAW_EMPTY + 8 * rs);
-            }
+            if (lane == 0) mbar_arrive(sbase + KO_FULL + 8 * s);
             if (!wait(KO_REC_EMPTY + 8 * q, ((i / KT_NQ) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) break;
             *rec = dm;
             __syncwarp();
@@ -414,7 +501,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
         // ------------------------------------------------------------ drain: integer sums -> scaled f32 terms, in K order
         const uint32_t quarter = warp & 3, cg = (uint32_t)(warp - KT_DEC) >> 2, r = quarter * 32 + lane;
         const uint32_t t_base = tmem + ((quarter * 32) << 16);
-        float sum[4][8];  // activation rows 8 (cg + 4 c) + j
+        float sum[CHUNKS][8];  // activation rows 8 (cg + 4 c) + j
         grid_dep_wait();  // the output may still be in use by the previous kernel
         uint32_t unit = blockIdx.x, b = 0;
         for (uint32_t i = 0; i < total; ++i) {
@@ -426,24 +513,31 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
             const float d = MIN ? df : -df, dmin = MIN ? f16bits_to_f32(dm >> 16) : 0.f;
             if (b == 0)
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
+                for (int c = 0; c < (int)CHUNKS; ++c)
 #pragma unroll
                     for (int j = 0; j < 8; ++j) sum[c][j] = 0.f;
             if (!wait(KO_ACC_FULL + 8 * buf, (i >> 1) & 1, STATUS_TIMEOUT_MMA)) break;
             tc_after();
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < (int)CHUNKS; ++c) {
                 const uint32_t col = 8 * (cg + 4 * c);
                 if (col < p.mt) {  // warp-uniform
-                    uint32_t v[8], u[8];
-                    tmem_ld8_async(t_base + buf * ACC_COLS + col, v);
-                    if constexpr (MIN) tmem_ld8_async(t_base + buf * ACC_COLS + 128 + col, u);
+                    uint32_t v[8], u[8], vh[8], uh[8];
+                    const uint32_t tc = t_base + buf * ACC_COLS + col;
+                    tmem_ld8_async(tc, v);
+                    if constexpr (WIDE) tmem_ld8_async(tc + COL, vh);
+                    if constexpr (MIN) tmem_ld8_async(tc + (WIDE ? 2 * COL : COL), u);
+                    if constexpr (WIDE) tmem_ld8_async(tc + 3 * COL, uh);
                     const float4* d8 = reinterpret_cast<const float4*>(rec + 512 + 4 * col);
                     const float4 e0 = d8[0], e1 = d8[1];
                     const float e[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
                     tmem_ld_wait();
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
+                        if constexpr (WIDE) {
+                            v[j] += 128 * vh[j];
+                            u[j] += 16 * uh[j];
+                        }
                         float t = __fmul_rn(__fmul_rn(d, e[j]), (float)(int)v[j]);
                         if constexpr (MIN) t = __fsub_rn(t, __fmul_rn(__fmul_rn(dmin, e[j]), (float)(int)u[j]));
                         sum[c][j] = __fadd_rn(sum[c][j], t);
@@ -462,7 +556,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
             unit += gridDim.x;
             if (n < p.N)
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
+                for (int c = 0; c < (int)CHUNKS; ++c)
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
                         const uint32_t m = 8 * (cg + 4 * c) + j;
@@ -701,16 +795,17 @@ struct KqPlan {
 };
 KqPlan kq_tc_plan(int fmt, size_t M, size_t N, int sm_count) {
     KqPlan best;
-    const size_t rt = (N + 127) / 128, fixed = 450, per_row = fmt == FMT_Q2_K ? 7 : 5;
-    for (uint32_t mt = 16; mt <= 128; mt += 16) {
+    const size_t rt = (N + 127) / 128, fixed = kq_wide(fmt) ? 2200 : 1300, per_row = 7;
+    for (uint32_t mt = 16; mt <= kt_mt_max(fmt); mt += 16) {
         const size_t units = rt * ((M + mt - 1) / mt), cost = (units + sm_count - 1) / sm_count * (fixed + per_row * mt);
-        if (!best.mt || cost < best.cost) best = {mt, cost};
+        if (!best.mt || cost <= best.cost) best = {mt, cost};
         if (mt >= M) break;
     }
     return best;
 }
 KqPlan kq_plan(int fmt, size_t M, size_t K, size_t N, int sm_count) {
     const KqPlan tc = kq_tc_plan(fmt, M, N, sm_count);
+    if (kq_wide(fmt)) return tc;
     const size_t slabs = (N + 15) / 16, nt = M <= 8 ? 1 : M <= 16 ? 2 : 4, groups = (M + 8 * nt - 1) / (8 * nt);
     const size_t small = (slabs + sm_count - 1) / sm_count * groups * (fmt == FMT_Q2_K ? 90 + 20 * nt : 130 + 20 * nt);
     const size_t units = (N + 127) / 128 * ((M + 15) / 16);
@@ -751,21 +846,38 @@ bool encode(CUtensorMap* map, CUtensorMapDataType type, size_t elem, void* base,
 
 }  // namespace
 
-bool kq_lowbit_supported(int fmt, size_t M, size_t K, size_t N) { return (fmt == FMT_Q2_K || fmt == FMT_Q3_K) && M >= 1 && N >= 1 && K % 256 == 0; }
+// Q2_K and Q3_K: every shape.  Q4_K and Q5_K below 64 rows: where one pass here takes less than several passes over the
+// weights by the kernels for few rows (of 16 rows for Q5_K: gemv.cu; of 32 for Q4_K: smallm_i8.cu, which at 17 ... 32 rows
+// is the faster one).  Both sides as fitted to graph replays, in us: here 5 us and 1.15 us + 4 ns a row of the tile per block
+// of K, for every round of tiles; there 4 us and the packed bytes at 2.7 TB/s per pass of 16 rows, and for the passes of 32
+// the larger of 28 + (M - 33) / 5 + 0.35 per block of K and 6 us + 2.4 TB/s per pass.  Measured (here / there): Q5_K 14336 x 4096 at 20 / 37 / 63
+// rows 26 / 37, 28 / 57, 50 / 77; 4096 x 4096 at 37 rows 23 / 26; 4096 x 14336 (32 tiles on 148 SMs) at 37 rows 75 / 56;
+// Q4_K 14336 x 4096 at 37 / 63 rows 25 / 34, 45 / 40; 4096 x 4096 at 37 rows 22 / 33; at 20 rows 24 / 20.
+// K up to 65536 keeps the scratch below 5 MB.
+bool kq_i8_supported(int fmt, size_t M, size_t K, size_t N, int sm_count) {
+    if (M < 1 || N < 1 || K < 256 || K % 256 != 0) return false;
+    if (fmt == FMT_Q2_K || fmt == FMT_Q3_K) return true;
+    if (!kq_wide(fmt) || M < (fmt == FMT_Q5_K ? 17 : 33) || M >= 64 || K > 65536 || N > (1u << 22) || !tma_available()) return false;
+    const size_t mt = kq_tc_plan(fmt, M, N, sm_count).mt, units = (N + 127) / 128 * ((M + mt - 1) / mt), nblk = K / 256;
+    const double here = 5.0 + (double)((units + sm_count - 1) / sm_count * nblk) * (1.15 + 0.004 * mt), mb = (double)(N * nblk * fmt_block_bytes(fmt)) * 1e-6;
+    const double two = 2.0 * (6.0 + mb / 2.4), few = 28.0 + 0.2 * (double)(M - 33) + 0.35 * (double)nblk;
+    const double there = fmt == FMT_Q5_K ? (double)((M + 15) / 16) * (4.0 + mb / 2.7) : two > few ? two : few;
+    return here < 0.95 * there;
+}
 
-size_t kq_lowbit_workspace_bytes(size_t M, size_t K) { return (M * (K / 256) * RUN_BYTES + 255) & ~(size_t)255; }
+size_t kq_i8_workspace_bytes(size_t M, size_t K) { return (M * (K / 256) * RUN_BYTES + 255) & ~(size_t)255; }
 
 // acts_prepared: a previous call with the same activations and scratch left the image there (both formats read the same).
-cudaError_t launch_kq_lowbit(int fmt, const void* act, int act_dtype, const void* w, void* out, int out_dtype, size_t M, size_t K, size_t N, void* ws,
+cudaError_t launch_kq_i8(int fmt, const void* act, int act_dtype, const void* w, void* out, int out_dtype, size_t M, size_t K, size_t N, void* ws,
                              size_t ws_bytes, int sm_count, cudaStream_t st, unsigned int* status, bool* ws_too_small, char* err, size_t err_len,
                              bool acts_prepared) {
     *ws_too_small = false;
-    const size_t need = kq_lowbit_workspace_bytes(M, K);
+    const size_t need = kq_i8_workspace_bytes(M, K);
     if (!ws || ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 15)) {
         *ws_too_small = true;
         return cudaSuccess;
     }
-    if (fmt != FMT_Q2_K && fmt != FMT_Q3_K) return cudaErrorInvalidValue;
+    if (fmt != FMT_Q2_K && fmt != FMT_Q3_K && !kq_wide(fmt)) return cudaErrorInvalidValue;
     const KqScratch s = kq_scratch(ws, M, K);
     const uint32_t nblk = (uint32_t)(K / 256);
     cudaError_t e;
@@ -801,7 +913,10 @@ cudaError_t launch_kq_lowbit(int fmt, const void* act, int act_dtype, const void
             snprintf(err, err_len, "cuTensorMapEncodeTiled failed (activation image %p, weight %p, M=%zu K=%zu N=%zu)", (void*)s.codes, w, M, K, N);
             return cudaErrorInvalidValue;
         }
-        e = fmt == FMT_Q2_K ? launch_tc<FMT_Q2_K>(p, amap, mmap, wmap, sm_count, st) : launch_tc<FMT_Q3_K>(p, amap, mmap, wmap, sm_count, st);
+        e = fmt == FMT_Q2_K   ? launch_tc<FMT_Q2_K>(p, amap, mmap, wmap, sm_count, st)
+            : fmt == FMT_Q3_K ? launch_tc<FMT_Q3_K>(p, amap, mmap, wmap, sm_count, st)
+            : fmt == FMT_Q4_K ? launch_tc<FMT_Q4_K>(p, amap, mmap, wmap, sm_count, st)
+                              : launch_tc<FMT_Q5_K>(p, amap, mmap, wmap, sm_count, st);
     } else {
         KqSmallParams p{};
         p.w = static_cast<const uint8_t*>(w);

@@ -45,6 +45,27 @@ def test_bit_identical(oracle, fmt, m, n, k):
         assert torch.equal(y, out.to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("fmt", ["Q4_K", "Q5_K"])
+@pytest.mark.parametrize("m,n,k", [(17, 9000, 1280), (33, 2050, 512), (37, 4097, 1280), (48, 2100, 768), (49, 20000, 256), (63, 30000, 512)])
+def test_two_byte_products_bit_identical(oracle, fmt, m, n, k):
+    from boostr_b200 import ops
+
+    rng = synth.rng_for(94, seed_of(fmt, m, n, k))
+    act = synth.activations(rng, m, k)
+    act[m // 2] *= 1e-3
+    act[0, :256] = 0.0
+    w = synth.weight_bytes(fmt, rng, n, k)
+    guard = 4096
+    flat = torch.full((2 * guard + m * n,), 4242.0, device="cuda")
+    out = flat[guard:guard + m * n].view(m, n)
+    ops.quant_matmul(torch.from_numpy(act).cuda(), QuantTensor.from_bytes(w, F[fmt], (n, k), device="cuda"), out=out)
+    ops.check_device_status()
+    got = out.cpu().numpy()
+    assert (flat[:guard] == 4242.0).all() and (flat[guard + m * n:] == 4242.0).all(), "guard regions were written"
+    want = oracle.quant_matmul(fmt, act, w, n, threads=os.cpu_count() or 8)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), describe_mismatch(got, want)
+
+
 def test_extreme_codes(oracle):
     """Every scale, code and activation at its largest: the integer sums reach their bounds."""
     from boostr_b200 import ops
