@@ -1006,19 +1006,34 @@ __global__ void __launch_bounds__(512) rmsnorm_kernel(const void* __restrict__ a
     const size_t row = blockIdx.x;
     grid_dep_launch();
     grid_dep_wait();
+    // The first 4096 values stay in registers between the two passes (longer rows are read again) and everything moves in
+    // 16-byte accesses: with one scalar store per value, 32 bytes from lane to lane, 1999 x 4096 took 39 us.
+    float v0[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    const uint32_t k1 = threadIdx.x * 8;
+    if (k1 < K) load_act8(act, act_dtype, row * K + k1, v0);
     float sq = 0.f;
-    for (uint32_t k0 = threadIdx.x * 8; k0 < K; k0 += 512 * 8) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sq = fmaf(v0[i], v0[i], sq);
+    for (uint32_t k0 = k1 + 512 * 8; k0 < K; k0 += 512 * 8) {
         float v[8];
         load_act8(act, act_dtype, row * K + k0, v);
 #pragma unroll
         for (int i = 0; i < 8; ++i) sq = fmaf(v[i], v[i], sq);
     }
+    auto put = [&](uint32_t k0, const float (&v)[8], float rs) {
+        const float4 *w = reinterpret_cast<const float4*>(norm_w + k0), a = __ldg(w), b = __ldg(w + 1);
+        float4* o = reinterpret_cast<float4*>(out + row * K + k0);
+        o[0] = make_float4(__fmul_rn(__fmul_rn(v[0], rs), a.x), __fmul_rn(__fmul_rn(v[1], rs), a.y), __fmul_rn(__fmul_rn(v[2], rs), a.z),
+                           __fmul_rn(__fmul_rn(v[3], rs), a.w));
+        o[1] = make_float4(__fmul_rn(__fmul_rn(v[4], rs), b.x), __fmul_rn(__fmul_rn(v[5], rs), b.y), __fmul_rn(__fmul_rn(v[6], rs), b.z),
+                           __fmul_rn(__fmul_rn(v[7], rs), b.w));
+    };
     const float rs = rms_factor(sq, red, warp, lane, K, eps);
-    for (uint32_t k0 = threadIdx.x * 8; k0 < K; k0 += 512 * 8) {
+    if (k1 < K) put(k1, v0, rs);
+    for (uint32_t k0 = k1 + 512 * 8; k0 < K; k0 += 512 * 8) {
         float v[8];
         load_act8(act, act_dtype, row * K + k0, v);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) out[row * K + k0 + i] = __fmul_rn(__fmul_rn(v[i], rs), __ldg(norm_w + k0 + i));
+        put(k0, v, rs);
     }
 }
 
