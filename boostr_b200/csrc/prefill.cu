@@ -482,6 +482,9 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_acc = *tmem_holder;
+    // Launched while the previous kernel drains (usually the one that prepares the activations): packed weights are fetched
+    // and decoded at once, the activation loads and the epilogue wait for it.
+    grid_dep_launch();
 
     if (warp == 18) {
         // ------------------------------------------------------------ packed weight tiles by TMA
@@ -508,6 +511,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const __grid_con
     } else if (warp == 16) {
         // ------------------------------------------------------------ activation tiles by TMA
         if (lane == 0) {
+            grid_dep_wait();
             uint32_t s = 0, par = 0;
             PfUnit u;
             for (uint32_t it = 0; pf_unit(p, it, u); ++it) {
@@ -576,6 +580,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const __grid_con
         // lane r of the accumulator = weight row n0 + r, column c = activation row m0 + c; a warp reaches the
         // 32 lanes of its quarter (warp & 3)
         const uint32_t quarter = (uint32_t)warp & 3, r = quarter * 32 + lane;
+        grid_dep_wait();  // the output and the scratch may still be in use by the previous kernel
         bool ok = true;
         PfUnit un;
         for (uint32_t it = 0; ok && pf_unit(p, it, un); ++it) {
@@ -755,6 +760,8 @@ constexpr uint32_t PF_RED_ROWS = 8;
 __global__ void __launch_bounds__(128) prefill_reduce_kernel(const PrefillParams p, uint32_t G) {
     __shared__ uint32_t slots[192];
     __shared__ uint32_t nslots;
+    grid_dep_launch();
+    grid_dep_wait();
     const uint32_t t = blockIdx.y, ml0 = blockIdx.x * PF_RED_ROWS, r = threadIdx.x;
     const uint32_t tile = p.nfull + t, n0 = (tile % p.ntn) * 128, m0 = (tile / p.ntn) * p.mt + ml0;
     if (m0 >= p.M) return;  // block-uniform
@@ -808,6 +815,8 @@ __global__ void __launch_bounds__(128) prefill_reduce_kernel(const PrefillParams
 }
 
 __global__ void __launch_bounds__(256) f32_to_bf16_kernel(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, size_t n) {
+    grid_dep_launch();
+    grid_dep_wait();
     const size_t n4 = n / 4;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
         const float4 v = __ldg(reinterpret_cast<const float4*>(in) + i);
@@ -826,6 +835,8 @@ __global__ void __launch_bounds__(256) f32_to_bf16_kernel(const float* __restric
 template <typename InT>
 __global__ void __launch_bounds__(256) act_q8k_to_bf16_kernel(const InT* __restrict__ in, __nv_bfloat16* __restrict__ out, size_t nruns) {
     const int lane = threadIdx.x & 31;
+    grid_dep_launch();
+    grid_dep_wait();
     for (size_t run = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); run < nruns; run += (size_t)gridDim.x * 8) {
         float v[8];
         const size_t base = run * 256 + 8 * lane;
@@ -907,9 +918,9 @@ cudaError_t launch_fmt(const CUtensorMap& map, const CUtensorMap& wmap, const Pr
     static PerDeviceOnce attrs;
     cudaError_t ae = attrs.run([] { return cudaFuncSetAttribute(prefill_kernel<FMT, RAW, Q6BOX>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448 - 1024); });
     if (ae != cudaSuccess) return ae;
-    prefill_kernel<FMT, RAW, Q6BOX><<<grid, PF_THREADS, smem, st>>>(map, wmap, p);
+    const cudaError_t e = launch_pdl(prefill_kernel<FMT, RAW, Q6BOX>, grid, dim3(PF_THREADS), smem, st, map, wmap, p);
     note_launch();
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace
@@ -970,22 +981,23 @@ cudaError_t launch_prefill(int fmt, const void* act, int act_dtype, const void* 
         act_bf16 = ws;  // a previous call with the same activations and scratch left them there (gate, then up)
     } else if (act_dtype != DT_BF16 || kq) {
         const size_t n = M * K;
+        cudaError_t e;
         __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(ws);
         if (kq) {
             const size_t nruns = n / 256;
             int grid = (int)((nruns + 7) / 8);
             if (grid > sm_count * 16) grid = sm_count * 16;
             if (grid < 1) grid = 1;
-            if (act_dtype == DT_F32) act_q8k_to_bf16_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(act), dst, nruns);
-            else act_q8k_to_bf16_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(act), dst, nruns);
+            e = act_dtype == DT_F32 ? launch_pdl(act_q8k_to_bf16_kernel<float>, dim3(grid), dim3(256), 0, st, static_cast<const float*>(act), dst, nruns)
+                                    : launch_pdl(act_q8k_to_bf16_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(act), dst, nruns);
         } else {
             int grid = (int)((n / 4 + 255) / 256);
             if (grid > sm_count * 16) grid = sm_count * 16;
             if (grid < 1) grid = 1;
-            f32_to_bf16_kernel<<<grid, 256, 0, st>>>(static_cast<const float*>(act), dst, n);
+            e = launch_pdl(f32_to_bf16_kernel, dim3(grid), dim3(256), 0, st, static_cast<const float*>(act), dst, n);
         }
         note_launch();
-        cudaError_t e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         act_bf16 = ws;
     }
@@ -1074,9 +1086,9 @@ cudaError_t launch_prefill(int fmt, const void* act, int act_dtype, const void* 
     if (le != cudaSuccess || !pl.split) return le;
     // the K-split tail tiles: add their pieces in K order
     const uint32_t rows = (uint32_t)(M < p.mt ? M : p.mt);
-    prefill_reduce_kernel<<<dim3((rows + PF_RED_ROWS - 1) / PF_RED_ROWS, pl.ntail, 1), 128, 0, st>>>(p, pl.grid);
+    le = launch_pdl(prefill_reduce_kernel, dim3((rows + PF_RED_ROWS - 1) / PF_RED_ROWS, pl.ntail, 1), dim3(128), 0, st, p, pl.grid);
     note_launch();
-    return cudaGetLastError();
+    return le != cudaSuccess ? le : cudaGetLastError();
 }
 
 cudaError_t launch_swiglu_gate(const float* gate, const float* up, void* out, int out_dtype, size_t n, int sm_count,
