@@ -160,8 +160,12 @@ __device__ __forceinline__ void copy_rows(uint32_t dst, const uint8_t* blk, uint
 // the activation codes come by TMA, one thread issues 8 MMAs
 // (16 for two-byte products; + 2 for the mins) into one of two accumulators, and sixteen drain warps (thread = weight
 // row x every fourth group of 8 activation rows) scale the sums in packed f32 and add them to their registers.
-// What bounds it: instruction issue - per (128 rows x 256 K) about 300 instructions a row of decode, and 6 (Q2_K) or 3
-// (Q3_K) a sum of drain - ahead of the tensor pipe.
+// What bounds it: with 128 activation rows a tile the issue slots (63 ... 68 % busy, tensor pipe 19 %, captured with the packed drain below): decode, and 8 (Q2_K) or
+// 5 (Q3_K) instructions a sum of drain; with few the latency of a block's chain through the barriers, the proxy fence and
+// two decode sets, 0.8 us (Q2_K, Q3_K) to 1.2 us (two-byte products) a block.  Measured: 512 rows x 14336 x 4096 Q2_K
+// 99 us, Q3_K 93 us (a layer of such products 0.42 ms; 69 ms with a kernel that took eight rows at a time); Q5_K 37 rows 28 us.  Tried and not kept:
+// packed f32x2 arithmetic in the drain (Q2_K 107 us, Q3_K 87 us; the assembler fuses mul.rn.f32x2 and add.rn.f32x2 into one
+// rounding unless an operand is hidden from it), and halves of a block as stages (4096 x 14336 at 64 rows 49 -> 58 us).
 struct KqTcParams {
     const uint8_t* w;
     void* out;
@@ -371,122 +375,122 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
             bool lost = false;
 #pragma unroll
             for (uint32_t n = 0; n < 2; ++n) {  // the halves of the block: operand tiles n (and 2 + n)
-            // All words of the half leave shared memory before the first store into the operand: nothing waits on a load in the
-            // middle of the arithmetic.
-            uint32_t cw[FMT == FMT_Q4_K || FMT == FMT_Q5_K ? 16 : 8], hw[8], sw[4];  // d (| dmin); codes; high bits; scales
-            if constexpr (FMT == FMT_Q2_K) {
-                dm = raw[20];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) sw[k] = raw[k];
-#pragma unroll
-                for (int k = 0; k < 8; ++k) cw[k] = raw[4 + 8 * n + k];
-            } else if constexpr (WIDE) {
-                const uint4* src = reinterpret_cast<const uint4*>(raw);
-                const uint4 h = src[0];
-                dm = h.x;
-                sw[0] = h.y; sw[1] = h.z; sw[2] = h.w;
-                if constexpr (FMT == FMT_Q5_K) {
-                    const uint4 v = src[1 + n];
-                    hw[0] = v.x; hw[1] = v.y; hw[2] = v.z; hw[3] = v.w;
-                }
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const uint4 v = src[(FMT == FMT_Q5_K ? 3 : 1) + 4 * n + k];
-                    cw[4 * k] = v.x; cw[4 * k + 1] = v.y; cw[4 * k + 2] = v.z; cw[4 * k + 3] = v.w;
-                }
-            } else {
-                const uint32_t sh = 8 * (at & 2u);
-                uint32_t u[9], v[9], x[4];
-#pragma unroll
-                for (int k = 0; k < 9; ++k) {
-                    u[k] = raw[k];
-                    v[k] = raw[8 + 8 * n + k];
-                }
-#pragma unroll
-                for (int k = 0; k < 4; ++k) x[k] = raw[24 + k];
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    hw[k] = __funnelshift_r(u[k], u[k + 1], sh) >> (4 * n);
-                    cw[k] = __funnelshift_r(v[k], v[k + 1], sh);
-                }
-#pragma unroll
-                for (int k = 0; k < 3; ++k) sw[k] = __funnelshift_r(x[k], x[k + 1], sh);
-                dm = (x[3] >> sh) & 0xFFFFu;
-            }
-            if (n == 1) {
-                __syncwarp();
-                if (lane == 0) mbar_arrive(sbase + KO_RAW_EMPTY + 8 * rs);
-            } else if (!wait(KO_EMPTY + 8 * s, ((i / KT_NS) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) {
-                lost = true;
-                break;
-            }
-            if (MIN && n == 0) {  // the tile of mins, 64 bytes a row
-                uint4 mn, m1, m2;
+                // All words of the half leave shared memory before the first store into the operand: nothing waits on a load in the
+                // middle of the arithmetic.
+                uint32_t cw[FMT == FMT_Q4_K || FMT == FMT_Q5_K ? 16 : 8], hw[8], sw[4];  // d (| dmin); codes; high bits; scales
                 if constexpr (FMT == FMT_Q2_K) {
-                    mn = make_uint4((sw[0] >> 4) & 0x0F0F0F0Fu, (sw[1] >> 4) & 0x0F0F0F0Fu, (sw[2] >> 4) & 0x0F0F0F0Fu, (sw[3] >> 4) & 0x0F0F0F0Fu);
-                    m1 = make_uint4(mn.x << 3, mn.y << 3, mn.z << 3, mn.w << 3);
-                    m2 = m1;
-                } else {  // unpack_q4k_q5k_scales, src/quant/cpu/kernels/dequant_k_quants/q4k_q5k.rs:108-122; a min covers two sums of 16
-                    const uint32_t a = sw[1] & 0x3F3F3F3Fu, c = ((sw[2] >> 4) & 0x0F0F0F0Fu) | ((sw[1] >> 2) & 0x30303030u);
-                    mn = make_uint4(__byte_perm(a, 0u, 0x1100), __byte_perm(a, 0u, 0x3322), __byte_perm(c, 0u, 0x1100), __byte_perm(c, 0u, 0x3322));
-                    m1 = make_uint4(0, 0, 0, 0);
-                    m2 = mn;
+                    dm = raw[20];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) sw[k] = raw[k];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) cw[k] = raw[4 + 8 * n + k];
+                } else if constexpr (WIDE) {
+                    const uint4* src = reinterpret_cast<const uint4*>(raw);
+                    const uint4 h = src[0];
+                    dm = h.x;
+                    sw[0] = h.y; sw[1] = h.z; sw[2] = h.w;
+                    if constexpr (FMT == FMT_Q5_K) {
+                        const uint4 v = src[1 + n];
+                        hw[0] = v.x; hw[1] = v.y; hw[2] = v.z; hw[3] = v.w;
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const uint4 v = src[(FMT == FMT_Q5_K ? 3 : 1) + 4 * n + k];
+                        cw[4 * k] = v.x; cw[4 * k + 1] = v.y; cw[4 * k + 2] = v.z; cw[4 * k + 3] = v.w;
+                    }
+                } else {
+                    const uint32_t sh = 8 * (at & 2u);
+                    uint32_t u[9], v[9], x[4];
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) {
+                        u[k] = raw[k];
+                        v[k] = raw[8 + 8 * n + k];
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) x[k] = raw[24 + k];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        hw[k] = __funnelshift_r(u[k], u[k + 1], sh) >> (4 * n);
+                        cw[k] = __funnelshift_r(v[k], v[k + 1], sh);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) sw[k] = __funnelshift_r(x[k], x[k + 1], sh);
+                    dm = (x[3] >> sh) & 0xFFFFu;
                 }
-                uint4* am = reinterpret_cast<uint4*>(smem + KO_STAGES + s * STAGE + OFF_AM + r * 64);
-                const uint32_t x3 = (r >> 1) & 3;
-                am[0 ^ x3] = mn;
-                am[1 ^ x3] = m1;
-                am[2 ^ x3] = make_uint4(0, 0, 0, 0);
-                am[3 ^ x3] = m2;
-            }
-            if constexpr (WIDE) {
-                // bytes 32 j .. of low nibbles are sub-block 2 j, of high nibbles sub-block 2 j + 1; Q5_K: bit e of word j of the
-                // fifth bits belongs to element e of sub-block j
-                const uint32_t scw = n ? (sw[2] & 0x0F0F0F0Fu) | ((sw[0] >> 2) & 0x30303030u) : sw[0] & 0x3F3F3F3Fu;
+                if (n == 1) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(sbase + KO_RAW_EMPTY + 8 * rs);
+                } else if (!wait(KO_EMPTY + 8 * s, ((i / KT_NS) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) {
+                    lost = true;
+                    break;
+                }
+                if (MIN && n == 0) {  // the tile of mins, 64 bytes a row
+                    uint4 mn, m1, m2;
+                    if constexpr (FMT == FMT_Q2_K) {
+                        mn = make_uint4((sw[0] >> 4) & 0x0F0F0F0Fu, (sw[1] >> 4) & 0x0F0F0F0Fu, (sw[2] >> 4) & 0x0F0F0F0Fu, (sw[3] >> 4) & 0x0F0F0F0Fu);
+                        m1 = make_uint4(mn.x << 3, mn.y << 3, mn.z << 3, mn.w << 3);
+                        m2 = m1;
+                    } else {  // unpack_q4k_q5k_scales, src/quant/cpu/kernels/dequant_k_quants/q4k_q5k.rs:108-122; a min covers two sums of 16
+                        const uint32_t a = sw[1] & 0x3F3F3F3Fu, c = ((sw[2] >> 4) & 0x0F0F0F0Fu) | ((sw[1] >> 2) & 0x30303030u);
+                        mn = make_uint4(__byte_perm(a, 0u, 0x1100), __byte_perm(a, 0u, 0x3322), __byte_perm(c, 0u, 0x1100), __byte_perm(c, 0u, 0x3322));
+                        m1 = make_uint4(0, 0, 0, 0);
+                        m2 = mn;
+                    }
+                    uint4* am = reinterpret_cast<uint4*>(smem + KO_STAGES + s * STAGE + OFF_AM + r * 64);
+                    const uint32_t x3 = (r >> 1) & 3;
+                    am[0 ^ x3] = mn;
+                    am[1 ^ x3] = m1;
+                    am[2 ^ x3] = make_uint4(0, 0, 0, 0);
+                    am[3 ^ x3] = m2;
+                }
+                if constexpr (WIDE) {
+                    // bytes 32 j .. of low nibbles are sub-block 2 j, of high nibbles sub-block 2 j + 1; Q5_K: bit e of word j of the
+                    // fifth bits belongs to element e of sub-block j
+                    const uint32_t scw = n ? (sw[2] & 0x0F0F0F0Fu) | ((sw[0] >> 2) & 0x30303030u) : sw[0] & 0x3F3F3F3Fu;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {  // sub-block 4 n + j = 16-byte chunks 2 j, 2 j + 1 of the tile
-                    const uint32_t sc2 = 2 * byte_of(scw, j);
+                    for (int j = 0; j < 4; ++j) {  // sub-block 4 n + j = 16-byte chunks 2 j, 2 j + 1 of the tile
+                        const uint32_t sc2 = 2 * byte_of(scw, j);
 #pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        uint32_t lo[4], hi[4];
+                        for (int k = 0; k < 2; ++k) {
+                            uint32_t lo[4], hi[4];
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            uint32_t c = (cw[8 * (j >> 1) + 4 * k + e] >> (4 * (j & 1))) & 0x0F0F0F0Fu;
-                            if constexpr (FMT == FMT_Q5_K) c |= (((hw[j] >> (4 * (4 * k + e))) & 15u) * 0x02040810u) & 0x10101010u;
-                            wide_scaled(c, sc2, lo[e], hi[e]);
+                            for (int e = 0; e < 4; ++e) {
+                                uint32_t c = (cw[8 * (j >> 1) + 4 * k + e] >> (4 * (j & 1))) & 0x0F0F0F0Fu;
+                                if constexpr (FMT == FMT_Q5_K) c |= (((hw[j] >> (4 * (4 * k + e))) & 15u) * 0x02040810u) & 0x10101010u;
+                                wide_scaled(c, sc2, lo[e], hi[e]);
+                            }
+                            put(n, 2 * j + k, make_uint4(lo[0], lo[1], lo[2], lo[3]));
+                            put(2 + n, 2 * j + k, make_uint4(hi[0], hi[1], hi[2], hi[3]));
                         }
-                        put(n, 2 * j + k, make_uint4(lo[0], lo[1], lo[2], lo[3]));
-                        put(2 + n, 2 * j + k, make_uint4(hi[0], hi[1], hi[2], hi[3]));
+                    }
+                } else {
+                    uint32_t scw[2];  // the half's eight scales
+                    if constexpr (FMT == FMT_Q2_K) {
+                        scw[0] = (n ? sw[2] : sw[0]) & 0x0F0F0F0Fu;
+                        scw[1] = (n ? sw[3] : sw[1]) & 0x0F0F0F0Fu;
+                    } else {
+                        scw[0] = ((sw[0] >> (4 * n)) & 0x0F0F0F0Fu) | ((n ? sw[2] : sw[2] << 4) & 0x30303030u);
+                        scw[1] = ((sw[1] >> (4 * n)) & 0x0F0F0F0Fu) | ((n ? sw[2] >> 2 : sw[2] << 2) & 0x30303030u);
+                    }
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        auto one = [&](auto gc) {  // sub-block 8 n + 2 g + h = 16-byte chunk 2 g + h of the tile
+                            constexpr int G = decltype(gc)::value;
+                            const uint32_t sc = byte_of(scw[G >> 1], 2 * (G & 1) + h);
+                            uint32_t v[4];
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                if constexpr (FMT == FMT_Q2_K) v[k] = q2k_scaled<G>(cw[4 * h + k], sc);
+                                else v[k] = q3k_scaled<G>(cw[4 * h + k], hw[4 * h + k], 32u - sc, sc * 0x04040404u);
+                            }
+                            put(n, 2 * G + h, make_uint4(v[0], v[1], v[2], v[3]));
+                        };
+                        one(std::integral_constant<int, 0>{});
+                        one(std::integral_constant<int, 1>{});
+                        one(std::integral_constant<int, 2>{});
+                        one(std::integral_constant<int, 3>{});
                     }
                 }
-            } else {
-                uint32_t scw[2];  // the half's eight scales
-                if constexpr (FMT == FMT_Q2_K) {
-                    scw[0] = (n ? sw[2] : sw[0]) & 0x0F0F0F0Fu;
-                    scw[1] = (n ? sw[3] : sw[1]) & 0x0F0F0F0Fu;
-                } else {
-                    scw[0] = ((sw[0] >> (4 * n)) & 0x0F0F0F0Fu) | ((n ? sw[2] : sw[2] << 4) & 0x30303030u);
-                    scw[1] = ((sw[1] >> (4 * n)) & 0x0F0F0F0Fu) | ((n ? sw[2] >> 2 : sw[2] << 2) & 0x30303030u);
-                }
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    auto one = [&](auto gc) {  // sub-block 8 n + 2 g + h = 16-byte chunk 2 g + h of the tile
-                        constexpr int G = decltype(gc)::value;
-                        const uint32_t sc = byte_of(scw[G >> 1], 2 * (G & 1) + h);
-                        uint32_t v[4];
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            if constexpr (FMT == FMT_Q2_K) v[k] = q2k_scaled<G>(cw[4 * h + k], sc);
-                            else v[k] = q3k_scaled<G>(cw[4 * h + k], hw[4 * h + k], 32u - sc, sc * 0x04040404u);
-                        }
-                        put(n, 2 * G + h, make_uint4(v[0], v[1], v[2], v[3]));
-                    };
-                    one(std::integral_constant<int, 0>{});
-                    one(std::integral_constant<int, 1>{});
-                    one(std::integral_constant<int, 2>{});
-                    one(std::integral_constant<int, 3>{});
-                }
-            }
             }
             if (lost) break;
             proxy_fence();  // the operand bytes are read by the tensor core (async proxy)
@@ -580,7 +584,9 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
 // 16 x 8 NT terms in a table.  Once per R items the CTA meets and a few warps (in turn) add the terms of every slab in K
 // order.  Inside a block the operand's K order is free: lane t of a quad takes the 16 code bytes 16 t .. of its row, whose
 // four bit pairs belong to four sub-blocks, and the same elements of the activation row (16-byte loads of the code image).
-// What bounds it: instruction issue (about 250 (Q2_K) or 400 (Q3_K) instructions an item of 1.3 or 1.8 KB).
+// What bounds it: shared-memory and integer instructions (issue slots 41 ... 44 % busy, ALU pipe 32 ... 46 %; a lane's words of a
+// row lie in eight banks, 4 cycles a load).  4 rows x 14336 x 4096: Q2_K 13.1 us (1.47 TB/s), Q3_K 16.2 us (1.56 TB/s); with
+// copies of 4 bytes Q3_K 24.8 us.
 struct KqSmallParams {
     const uint8_t *w, *codes, *mins;
     const float* d8;
@@ -788,7 +794,10 @@ KqScratch kq_scratch(void* ws, size_t M, size_t K) {
     return {b, b + M * K, reinterpret_cast<float*>(b + M * K + M * (K / 256) * 32)};
 }
 
-// Time model of the two kernels, in units of SM cycles per block of K.
+// Time of the two kernels per block of K in SM cycles, fitted to graph replays (Q2_K / Q3_K, 1024 ... 14336 weight rows): a round of
+// tensor-core tiles takes 1300 (two-byte products 2200) and 7 a row of the tile; a 16-row slab of the other kernel 90 (Q2_K) or
+// 130 (Q3_K) and 20 per 8 activation rows.  Up to 8 rows the latter always wins (Q3_K 4096 x 4096 at 4 rows 7 us; one round
+// of tiles is 17 us).
 struct KqPlan {
     uint32_t mt = 0;  // activation rows of a tensor-core tile; 0: the kernel for few activation rows
     size_t cost = 0;

@@ -911,7 +911,17 @@ __global__ void __launch_bounds__(256) swiglu_gate_kernel(const float* __restric
     for (size_t i = done + first; i < n; i += step) store_gate(out, out_dtype, i, gate_value(g[i], u[i]));
 }
 
-uint32_t pick_mt(size_t M) { return M >= 256 ? 256u : M > 64 ? 128u : 64u; }
+// Activation rows of a tile.  From 256 rows on 256 (every weight tile is decoded once per column tile), but
+//   * below 1024 rows 128 where the matrix has so few tiles that even these fill less than half of the SMs: the K-split
+//     shares get shorter.  Tile 256 / 128: Q4_K 1024 x 4096 at 256, 512, 900 rows 20.0 / 17.3, 21.4 / 18.0, 24.8 / 22.2 us, 4096 x 4096
+//     at 256 rows 23.7 / 20.8; Q6_K and Q8_0 gain 0 ... 3 us; past that line 128 loses (Q6_K 4096 x 4096 at 300 rows 29 / 31);
+//   * 192 for 257 ... 384 rows, two column tiles either way and a quarter less padding: Q4_K at 300 rows 4096 x 4096 26.8 / 24.7,
+//     4096 x 14336 55.3 / 52.5, 14336 x 4096 51.7 / 50.4; Q6_K 4096 x 14336 at 384 rows 66.4 / 63.4.
+uint32_t pick_mt(size_t M, size_t N, int sm_count) {
+    if (M < 256) return M > 64 ? 128u : 64u;
+    if (M < 1024 && (N + 127) / 128 * ((M + 127) / 128) * 20 <= (size_t)sm_count * 9) return 128u;
+    return M > 256 && M <= 384 ? 192u : 256u;
+}
 
 template <int FMT, bool RAW, bool Q6BOX = false>
 cudaError_t launch_fmt(const CUtensorMap& map, const CUtensorMap& wmap, const PrefillParams& p, dim3 grid, size_t smem, cudaStream_t st) {
@@ -943,7 +953,7 @@ struct PfPlan {
 };
 PfPlan pf_plan(size_t M, size_t K, size_t N, int sm_count) {
     PfPlan pl{};
-    pl.mt = pick_mt(M);
+    pl.mt = pick_mt(M, N, sm_count);
     pl.ntn = (uint32_t)((N + 127) / 128);
     pl.ntiles = pl.ntn * (uint32_t)((M + pl.mt - 1) / pl.mt);
     const uint32_t G = (uint32_t)sm_count, nkt = (uint32_t)(K / BK);
