@@ -270,21 +270,23 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
         const uint32_t r0 = (uint32_t)(warp - KT_W_COPY) * (128 / KT_COPY);
         const uint8_t* wend = p.w + (size_t)p.N * p.row_bytes;
         uint32_t unit = blockIdx.x, b = 0, n0 = unit / p.nct * 128 + r0;
-        for (uint32_t i = 0; i < total; ++i) {
+        // By TMA one warp brings the packed blocks and the other has no part in the ring: a warp that waited on RAW_EMPTY without
+        // being counted in RAW_FULL could miss a phase, and at the end of the work would wait for one that never comes.
+        const uint32_t mine = p.raw_tma && warp != KT_W_COPY ? 0 : total;
+        for (uint32_t i = 0; i < mine; ++i) {
             const uint32_t rs = i % NR;
             if (!wait(KO_RAW_EMPTY + 8 * rs, ((i / NR) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) break;
             if (p.raw_tma) {  // one copy a block: rows past N and bytes past the row's end are zero-filled
-                if (warp == KT_W_COPY + 1) {
-                    // the other copy warp pulls the blocks to come into L2: what is in flight into shared memory does not
-                    // cover the latency of DRAM
-                    if (lane == 0 && i + NR < total) {
-                        const uint32_t ab = b + NR, at_b = ab < p.nblk ? ab : ab % p.nblk, at_n = ab < p.nblk ? n0 - r0 : (unit + ab / p.nblk * gridDim.x) / p.nct * 128;
+                if (lane == 0) {
+                    mbar_expect_tx(sbase + KO_RAW_FULL + 8 * rs, RAW);
+                    tma2d(sbase + OFF_RAW + rs * RAW, &tmap_w, (int)((b * BB & ~15u) / 2), (int)n0, sbase + KO_RAW_FULL + 8 * rs);
+                    // The block that this slot takes next goes to L2: what is in flight into shared memory does not cover the
+                    // latency of DRAM.
+                    if (i + NR < total) {
+                        const uint32_t ab = b + NR, at_b = ab < p.nblk ? ab : ab % p.nblk, at_n = ab < p.nblk ? n0 : (unit + ab / p.nblk * gridDim.x) / p.nct * 128;
                         asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(&tmap_w), "r"((int)((at_b * BB & ~15u) / 2)), "r"((int)at_n)
                                      : "memory");
                     }
-                } else if (lane == 0) {
-                    mbar_expect_tx(sbase + KO_RAW_FULL + 8 * rs, RAW);
-                    tma2d(sbase + OFF_RAW + rs * RAW, &tmap_w, (int)((b * BB & ~15u) / 2), (int)n0, sbase + KO_RAW_FULL + 8 * rs);
                 }
             } else if constexpr (!WIDE) {
                 copy_rows<FMT, 128 / KT_COPY>(sbase + OFF_RAW + rs * RAW + r0 * PITCH, p.w + (size_t)n0 * p.row_bytes + (size_t)b * BB, p.row_bytes, lane,
@@ -945,3 +947,10 @@ cudaError_t launch_kq_i8(int fmt, const void* act, int act_dtype, const void* w,
 }
 
 }  // namespace b200q
+
+// Activation rows of the tensor-core tile that a product takes (0: the kernel for few rows, -1: another path).  Not part of
+// the C ABI: the tests hold their shapes to the tiles that they are meant for.
+extern "C" __attribute__((visibility("default"))) int b200q_kq_tile_rows(int fmt, size_t M, size_t K, size_t N, int sm_count) {
+    if (!b200q::kq_i8_supported(fmt, M, K, N, sm_count)) return -1;
+    return (int)b200q::kq_plan(fmt, M, K, N, sm_count).mt;
+}

@@ -6,7 +6,7 @@ import os
 import numpy as np
 import pytest
 
-from boostr_b200 import synth
+from boostr_b200 import _cabi, synth
 from boostr_b200.format import QuantFormat as F
 from boostr_b200.tensor import QuantTensor
 from util import describe_mismatch, seed_of
@@ -43,6 +43,43 @@ def test_bit_identical(oracle, fmt, m, n, k):
     pair = ops.quant_matmul_batch(x, [qt, qt], out_dtype=torch.bfloat16)
     for y in pair:
         assert torch.equal(y, out.to(torch.bfloat16))
+
+
+def _tile_rows(fmt, m, n, k):
+    """The tile that the library's own rule picks (0: kernel for few rows, -1: another path)."""
+    import ctypes
+
+    f = _cabi.lib().b200q_kq_tile_rows
+    f.restype, f.argtypes = ctypes.c_int, [ctypes.c_int, ctypes.c_size_t, ctypes.c_size_t, ctypes.c_size_t, ctypes.c_int]
+    return f(F[fmt].format_id, m, k, n, torch.cuda.get_device_properties(0).multi_processor_count)
+
+
+@pytest.mark.parametrize("fmt,m,n,k,tile", [
+    ("Q2_K", 48, 18900, 1024, 48), ("Q2_K", 112, 18900, 1024, 112), ("Q2_K", 128, 18900, 2048, 128), ("Q2_K", 129, 18900, 1024, 80),
+    ("Q2_K", 300, 5001, 4096, 112), ("Q2_K", 512, 4096, 2048, 128),
+    ("Q3_K", 24, 18900, 2048, 32), ("Q3_K", 112, 18900, 2048, 112), ("Q3_K", 128, 18900, 2048, 128), ("Q3_K", 300, 4001, 2048, 80),
+    ("Q3_K", 512, 4096, 4096, 128), ("Q4_K", 33, 18900, 2048, 48), ("Q4_K", 48, 14336, 2048, 48), ("Q4_K", 63, 20000, 1024, 32),
+    ("Q4_K", 40, 18900, 256, 48), ("Q5_K", 17, 2050, 256, 16), ("Q5_K", 20, 18900, 2048, 32), ("Q5_K", 37, 13825, 5120, 48), ("Q5_K", 48, 18900, 256, 48)])
+def test_weight_tiles_by_tma(oracle, fmt, m, n, k, tile):
+    """Rows that are a multiple of 16 bytes, as in every real matrix: the packed blocks come by TMA.  Whole and partial tiles,
+    every CTA with one unit or several, one block of K up to twenty; the ring of packed blocks must end with the work (a
+    bounded wait that ran out would show in the status word), also over many launches of the shortest work."""
+    from boostr_b200 import ops
+
+    assert _tile_rows(fmt, m, n, k) == tile and k // 256 * F[fmt].block_bytes % 16 == 0
+    rng = synth.rng_for(96, seed_of(fmt, m, n, k))
+    act = synth.activations(rng, m, k)
+    w = synth.weight_bytes(fmt, rng, n, k)
+    x, qt = torch.from_numpy(act).cuda(), QuantTensor.from_bytes(w, F[fmt], (n, k), device="cuda")
+    out = ops.quant_matmul(x, qt)
+    again = torch.empty_like(out)
+    for _ in range(200 if k == 256 else 3):
+        ops.quant_matmul(x, qt, out=again)
+    ops.check_device_status()
+    assert torch.equal(out.view(torch.int32), again.view(torch.int32))
+    got = out.cpu().numpy()
+    want = oracle.quant_matmul(fmt, act, w, n, threads=os.cpu_count() or 8)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), describe_mismatch(got, want)
 
 
 @pytest.mark.parametrize("fmt", ["Q4_K", "Q5_K"])
