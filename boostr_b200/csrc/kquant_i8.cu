@@ -45,8 +45,10 @@ template <typename InT>
 __global__ void __launch_bounds__(256) kq_act_prep_kernel(const InT* __restrict__ act, uint8_t* __restrict__ codes, uint8_t* __restrict__ mins,
                                                           float* __restrict__ d8, size_t M, uint32_t nblk) {
     const int lane = threadIdx.x & 31;
-    grid_dep_launch();
     grid_dep_wait();  // the activations may be the previous kernel's output; the image may still be read by it
+    // In this order: the products read their packed weights as soon as they are started, and these may have been written
+    // by whatever ran before this kernel.
+    grid_dep_launch();
     const size_t nruns = M * nblk;
     for (size_t run = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); run < nruns; run += (size_t)gridDim.x * 8) {
         float v[8];
@@ -266,7 +268,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
     const uint32_t units = (p.nunits - blockIdx.x + gridDim.x - 1) / gridDim.x, total = units * p.nblk;
 
     if (warp >= KT_W_COPY && warp < KT_W_ACT) {
-        // ------------------------------------------------------------ packed blocks (do not depend on the previous kernel)
+        // ------------------------------------------------------------ packed blocks (do not depend on the kernel that is still running)
         const uint32_t r0 = (uint32_t)(warp - KT_W_COPY) * (128 / KT_COPY);
         const uint8_t* wend = p.w + (size_t)p.N * p.row_bytes;
         uint32_t unit = blockIdx.x, b = 0, n0 = unit / p.nct * 128 + r0;

@@ -482,8 +482,9 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_acc = *tmem_holder;
-    // Launched while the previous kernel drains (usually the one that prepares the activations): packed weights are fetched
-    // and decoded at once, the activation loads and the epilogue wait for it.
+    // Launched while the previous kernel of the same call drains: packed weights are fetched and decoded at once, the activation
+    // loads and the epilogue wait for it.  The weights may have been written by whatever ran before the call, so that has
+    // to be over by now: the kernel that prepares the activations lets this one start only after its own wait.
     grid_dep_launch();
 
     if (warp == 18) {
@@ -815,8 +816,8 @@ __global__ void __launch_bounds__(128) prefill_reduce_kernel(const PrefillParams
 }
 
 __global__ void __launch_bounds__(256) f32_to_bf16_kernel(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, size_t n) {
-    grid_dep_launch();
     grid_dep_wait();
+    grid_dep_launch();  // in this order: see prefill_kernel
     const size_t n4 = n / 4;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
         const float4 v = __ldg(reinterpret_cast<const float4*>(in) + i);
@@ -835,8 +836,8 @@ __global__ void __launch_bounds__(256) f32_to_bf16_kernel(const float* __restric
 template <typename InT>
 __global__ void __launch_bounds__(256) act_q8k_to_bf16_kernel(const InT* __restrict__ in, __nv_bfloat16* __restrict__ out, size_t nruns) {
     const int lane = threadIdx.x & 31;
-    grid_dep_launch();
     grid_dep_wait();
+    grid_dep_launch();  // in this order: see prefill_kernel
     for (size_t run = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); run < nruns; run += (size_t)gridDim.x * 8) {
         float v[8];
         const size_t base = run * 256 + 8 * lane;
@@ -924,11 +925,13 @@ uint32_t pick_mt(size_t M, size_t N, int sm_count) {
 }
 
 template <int FMT, bool RAW, bool Q6BOX = false>
-cudaError_t launch_fmt(const CUtensorMap& map, const CUtensorMap& wmap, const PrefillParams& p, dim3 grid, size_t smem, cudaStream_t st) {
+cudaError_t launch_fmt(const CUtensorMap& map, const CUtensorMap& wmap, const PrefillParams& p, dim3 grid, size_t smem, cudaStream_t st, bool early) {
     static PerDeviceOnce attrs;
     cudaError_t ae = attrs.run([] { return cudaFuncSetAttribute(prefill_kernel<FMT, RAW, Q6BOX>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448 - 1024); });
     if (ae != cudaSuccess) return ae;
-    const cudaError_t e = launch_pdl(prefill_kernel<FMT, RAW, Q6BOX>, grid, dim3(PF_THREADS), smem, st, map, wmap, p);
+    cudaError_t e = cudaSuccess;
+    if (early) e = launch_pdl(prefill_kernel<FMT, RAW, Q6BOX>, grid, dim3(PF_THREADS), smem, st, map, wmap, p);
+    else prefill_kernel<FMT, RAW, Q6BOX><<<grid, PF_THREADS, smem, st>>>(map, wmap, p);
     note_launch();
     return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -1083,14 +1086,16 @@ cudaError_t launch_prefill(int fmt, const void* act, int act_dtype, const void* 
         }
     }
     dim3 grid(pl.grid, 1, 1);
+    // only behind a kernel of this call (its own preparation, or the product that shares the prepared activations)
+    const bool early = acts_prepared || act_bf16 != act;
     cudaError_t le;
     switch (fmt) {
-    case FMT_Q4_0: le = raw ? launch_fmt<FMT_Q4_0, true>(map, wmap, p, grid, smem, st) : launch_fmt<FMT_Q4_0, false>(map, wmap, p, grid, smem, st); break;
-    case FMT_Q5_0: le = raw ? launch_fmt<FMT_Q5_0, true>(map, wmap, p, grid, smem, st) : launch_fmt<FMT_Q5_0, false>(map, wmap, p, grid, smem, st); break;
-    case FMT_Q8_0: le = raw ? launch_fmt<FMT_Q8_0, true>(map, wmap, p, grid, smem, st) : launch_fmt<FMT_Q8_0, false>(map, wmap, p, grid, smem, st); break;
-    case FMT_Q4_K: le = launch_fmt<FMT_Q4_K, true>(map, wmap, p, grid, smem, st); break;
-    case FMT_Q5_K: le = launch_fmt<FMT_Q5_K, true>(map, wmap, p, grid, smem, st); break;
-    case FMT_Q6_K: le = q6box ? launch_fmt<FMT_Q6_K, true, true>(map, wmap, p, grid, smem, st) : launch_fmt<FMT_Q6_K, true>(map, wmap, p, grid, smem, st); break;
+    case FMT_Q4_0: le = raw ? launch_fmt<FMT_Q4_0, true>(map, wmap, p, grid, smem, st, early) : launch_fmt<FMT_Q4_0, false>(map, wmap, p, grid, smem, st, early); break;
+    case FMT_Q5_0: le = raw ? launch_fmt<FMT_Q5_0, true>(map, wmap, p, grid, smem, st, early) : launch_fmt<FMT_Q5_0, false>(map, wmap, p, grid, smem, st, early); break;
+    case FMT_Q8_0: le = raw ? launch_fmt<FMT_Q8_0, true>(map, wmap, p, grid, smem, st, early) : launch_fmt<FMT_Q8_0, false>(map, wmap, p, grid, smem, st, early); break;
+    case FMT_Q4_K: le = launch_fmt<FMT_Q4_K, true>(map, wmap, p, grid, smem, st, early); break;
+    case FMT_Q5_K: le = launch_fmt<FMT_Q5_K, true>(map, wmap, p, grid, smem, st, early); break;
+    case FMT_Q6_K: le = q6box ? launch_fmt<FMT_Q6_K, true, true>(map, wmap, p, grid, smem, st, early) : launch_fmt<FMT_Q6_K, true>(map, wmap, p, grid, smem, st, early); break;
     default: return cudaErrorInvalidValue;
     }
     if (le != cudaSuccess || !pl.split) return le;
