@@ -762,7 +762,6 @@ __global__ void __launch_bounds__(128) prefill_reduce_kernel(const PrefillParams
     __shared__ uint32_t slots[192];
     __shared__ uint32_t nslots;
     grid_dep_launch();
-    grid_dep_wait();
     const uint32_t t = blockIdx.y, ml0 = blockIdx.x * PF_RED_ROWS, r = threadIdx.x;
     const uint32_t tile = p.nfull + t, n0 = (tile % p.ntn) * 128, m0 = (tile / p.ntn) * p.mt + ml0;
     if (m0 >= p.M) return;  // block-uniform
@@ -1101,9 +1100,12 @@ cudaError_t launch_prefill(int fmt, const void* act, int act_dtype, const void* 
     if (le != cudaSuccess || !pl.split) return le;
     // the K-split tail tiles: add their pieces in K order
     const uint32_t rows = (uint32_t)(M < p.mt ? M : p.mt);
-    le = launch_pdl(prefill_reduce_kernel, dim3((rows + PF_RED_ROWS - 1) / PF_RED_ROWS, pl.ntail, 1), dim3(128), 0, st, p, pl.grid);
+    // In plain order: launched early, its blocks took room and slots beside the product that they wait for.  1024 x 4096, early /
+    // plain: Q4_K 64, 128, 200 rows 14.1 / 13.0, 17.3 / 13.9, 16.8 / 15.4 us, Q8_0 128 rows 18.3 / 15.6; 240 prompt products in
+    // the mean 0.925 / 0.913 of the time without any early launch.
+    prefill_reduce_kernel<<<dim3((rows + PF_RED_ROWS - 1) / PF_RED_ROWS, pl.ntail, 1), 128, 0, st>>>(p, pl.grid);
     note_launch();
-    return le != cudaSuccess ? le : cudaGetLastError();
+    return cudaGetLastError();
 }
 
 cudaError_t launch_swiglu_gate(const float* gate, const float* up, void* out, int out_dtype, size_t n, int sm_count,
