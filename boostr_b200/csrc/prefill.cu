@@ -59,6 +59,7 @@ struct PrefillParams {
     uint32_t nfull, ntail, split, gran, gpt;
     float* part;
     int out_dtype;
+    bool first;  // of the kernels of its call
     unsigned int* status;
 };
 
@@ -482,9 +483,11 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_acc = *tmem_holder;
-    // Launched while the previous kernel of the same call drains: packed weights are fetched and decoded at once, the activation
-    // loads and the epilogue wait for it.  The weights may have been written by whatever ran before the call, so that has
-    // to be over by now: the kernel that prepares the activations lets this one start only after its own wait.
+    // Launched while the kernel before it drains.  Behind a kernel of the same call the packed weights are fetched and decoded at
+    // once; the activation loads and the epilogue wait for it.  The weights may have been written by whatever ran before the
+    // call, so that has to be over by now: the kernel that prepares the activations lets this one start only after
+    // its own wait, and a product that comes first in its call waits here, before it lets the next kernel start.
+    if (p.first) grid_dep_wait();
     grid_dep_launch();
 
     if (warp == 18) {
@@ -924,13 +927,11 @@ uint32_t pick_mt(size_t M, size_t N, int sm_count) {
 }
 
 template <int FMT, bool RAW, bool Q6BOX = false>
-cudaError_t launch_fmt(const CUtensorMap& map, const CUtensorMap& wmap, const PrefillParams& p, dim3 grid, size_t smem, cudaStream_t st, bool early) {
+cudaError_t launch_fmt(const CUtensorMap& map, const CUtensorMap& wmap, const PrefillParams& p, dim3 grid, size_t smem, cudaStream_t st) {
     static PerDeviceOnce attrs;
     cudaError_t ae = attrs.run([] { return cudaFuncSetAttribute(prefill_kernel<FMT, RAW, Q6BOX>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448 - 1024); });
     if (ae != cudaSuccess) return ae;
-    cudaError_t e = cudaSuccess;
-    if (early) e = launch_pdl(prefill_kernel<FMT, RAW, Q6BOX>, grid, dim3(PF_THREADS), smem, st, map, wmap, p);
-    else prefill_kernel<FMT, RAW, Q6BOX><<<grid, PF_THREADS, smem, st>>>(map, wmap, p);
+    const cudaError_t e = launch_pdl(prefill_kernel<FMT, RAW, Q6BOX>, grid, dim3(PF_THREADS), smem, st, map, wmap, p);
     note_launch();
     return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -1053,6 +1054,7 @@ cudaError_t launch_prefill(int fmt, const void* act, int act_dtype, const void* 
     p.nfull = pl.nfull; p.ntail = pl.ntail; p.split = pl.split; p.gran = pl.gran; p.gpt = pl.gpt;
     p.part = pl.split ? reinterpret_cast<float*>(static_cast<uint8_t*>(ws) + act_bytes) : nullptr;
     p.out_dtype = out_dtype;
+    p.first = !acts_prepared && act_bf16 == act;  // neither its own preparation nor the product that shares the activations ran before
     p.status = status;
     const size_t smem = 2048 + raw_bytes + (size_t)nsb * b_tile;
 
@@ -1085,16 +1087,14 @@ cudaError_t launch_prefill(int fmt, const void* act, int act_dtype, const void* 
         }
     }
     dim3 grid(pl.grid, 1, 1);
-    // only behind a kernel of this call (its own preparation, or the product that shares the prepared activations)
-    const bool early = acts_prepared || act_bf16 != act;
     cudaError_t le;
     switch (fmt) {
-    case FMT_Q4_0: le = raw ? launch_fmt<FMT_Q4_0, true>(map, wmap, p, grid, smem, st, early) : launch_fmt<FMT_Q4_0, false>(map, wmap, p, grid, smem, st, early); break;
-    case FMT_Q5_0: le = raw ? launch_fmt<FMT_Q5_0, true>(map, wmap, p, grid, smem, st, early) : launch_fmt<FMT_Q5_0, false>(map, wmap, p, grid, smem, st, early); break;
-    case FMT_Q8_0: le = raw ? launch_fmt<FMT_Q8_0, true>(map, wmap, p, grid, smem, st, early) : launch_fmt<FMT_Q8_0, false>(map, wmap, p, grid, smem, st, early); break;
-    case FMT_Q4_K: le = launch_fmt<FMT_Q4_K, true>(map, wmap, p, grid, smem, st, early); break;
-    case FMT_Q5_K: le = launch_fmt<FMT_Q5_K, true>(map, wmap, p, grid, smem, st, early); break;
-    case FMT_Q6_K: le = q6box ? launch_fmt<FMT_Q6_K, true, true>(map, wmap, p, grid, smem, st, early) : launch_fmt<FMT_Q6_K, true>(map, wmap, p, grid, smem, st, early); break;
+    case FMT_Q4_0: le = raw ? launch_fmt<FMT_Q4_0, true>(map, wmap, p, grid, smem, st) : launch_fmt<FMT_Q4_0, false>(map, wmap, p, grid, smem, st); break;
+    case FMT_Q5_0: le = raw ? launch_fmt<FMT_Q5_0, true>(map, wmap, p, grid, smem, st) : launch_fmt<FMT_Q5_0, false>(map, wmap, p, grid, smem, st); break;
+    case FMT_Q8_0: le = raw ? launch_fmt<FMT_Q8_0, true>(map, wmap, p, grid, smem, st) : launch_fmt<FMT_Q8_0, false>(map, wmap, p, grid, smem, st); break;
+    case FMT_Q4_K: le = launch_fmt<FMT_Q4_K, true>(map, wmap, p, grid, smem, st); break;
+    case FMT_Q5_K: le = launch_fmt<FMT_Q5_K, true>(map, wmap, p, grid, smem, st); break;
+    case FMT_Q6_K: le = q6box ? launch_fmt<FMT_Q6_K, true, true>(map, wmap, p, grid, smem, st) : launch_fmt<FMT_Q6_K, true>(map, wmap, p, grid, smem, st); break;
     default: return cudaErrorInvalidValue;
     }
     if (le != cudaSuccess || !pl.split) return le;
