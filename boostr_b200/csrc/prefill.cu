@@ -4,7 +4,7 @@
 // scalar decode + FFMA, no tensor cores).  Here the contraction runs on tcgen05.mma with the accumulator
 // in tensor memory:
 //   * orientation: the WEIGHT tile is the MMA's A operand (128 weight rows = the 128 TMEM lanes), the
-//     ACTIVATION tile is the B operand (MT = 64/128/256 activation rows = TMEM columns).  The packed
+//     ACTIVATION tile is the B operand (MT = 64/128/192/256 activation rows = TMEM columns).  The packed
 //     weights are decoded once per (128 x MT) output tile, so a larger MT amortises the decode.
 //   * persistent: one CTA per SM walks the output tiles; tensor memory holds TWO accumulators, so four
 //     epilogue warps drain tile i (tcgen05.ld: lane = weight row, columns = activation rows; out[m, n]
@@ -914,16 +914,28 @@ __global__ void __launch_bounds__(256) swiglu_gate_kernel(const float* __restric
     for (size_t i = done + first; i < n; i += step) store_gate(out, out_dtype, i, gate_value(g[i], u[i]));
 }
 
-// Activation rows of a tile.  From 256 rows on 256 (every weight tile is decoded once per column tile), but
-//   * below 1024 rows 128 where the matrix has so few tiles that even these fill less than half of the SMs: the K-split
-//     shares get shorter.  Tile 256 / 128: Q4_K 1024 x 4096 at 256, 512, 900 rows 20.0 / 17.3, 21.4 / 18.0, 24.8 / 22.2 us, 4096 x 4096
-//     at 256 rows 23.7 / 20.8; Q6_K and Q8_0 gain 0 ... 3 us; past that line 128 loses (Q6_K 4096 x 4096 at 300 rows 29 / 31);
+// Activation rows of a tile.  From 256 rows on 256 (every weight tile is decoded once per column tile), but below 1024 rows
+//   * 128 where there are so few tiles that the shorter shares of the K split and half the partial sums outweigh the second
+//     decoding.  The line is a share of the SMs that falls with K and lies lower where the decoding costs more (Q8_0, Q6_K, most
+//     of all Q6_K rows that are copied 4 bytes at a time) and where the other choice is the tile of 192.  Tile 256 / 128 at
+//     256 rows, us: 1024 x 4096 Q4_K 16.7 / 15.6, Q8_0 18.6 / 17.3; 4096 x 4096 23.8 / 21.0, 25.4 / 24.8; 2048 x 8192
+//     22.2 / 21.7, 25.1 / 26.4; 4096 x 14336 38.8 / 43.3, 44.5 / 56.4; Q6_K 3072 x 1024 16.1 / 18.3, 4096 x 11008 51.8 / 76.6.
+//     928 products of 256 ... 900 rows lie 0.2 % in the mean above the better of both, at most 11 %;
 //   * 192 for 257 ... 384 rows, two column tiles either way and a quarter less padding: Q4_K at 300 rows 4096 x 4096 26.8 / 24.7,
 //     4096 x 14336 55.3 / 52.5, 14336 x 4096 51.7 / 50.4; Q6_K 4096 x 14336 at 384 rows 66.4 / 63.4.
-uint32_t pick_mt(size_t M, size_t N, int sm_count) {
+uint32_t pick_mt(int fmt, size_t M, size_t K, size_t N, int sm_count) {
     if (M < 256) return M > 64 ? 128u : 64u;
-    if (M < 1024 && (N + 127) / 128 * ((M + 127) / 128) * 20 <= (size_t)sm_count * 9) return 128u;
-    return M > 256 && M <= 384 ? 192u : 256u;
+    const bool mid = M > 256 && M <= 384, light = fmt != FMT_Q8_0 && fmt != FMT_Q6_K, copied = fmt == FMT_Q6_K && K % 2048 != 0;
+    const bool low = copied || (mid && !light);
+    const uint32_t share = K < 2048    ? 40u  // of 180 SMs
+                           : K <= 4096 ? (low ? 40u : 81u)
+                           : K <= 6144 ? (light ? 60u : 40u)
+                           : K <= 8192 && light ? 40u
+                           : low       ? 15u
+                                       : 30u;
+    const size_t tiles = (N + 127) / 128 * ((M + 127) / 128);
+    if (M < 1024 && tiles * 180 <= (size_t)sm_count * share) return 128u;
+    return mid ? 192u : 256u;
 }
 
 template <int FMT, bool RAW, bool Q6BOX = false>
@@ -954,9 +966,9 @@ struct PfPlan {
     uint32_t mt, ntn, ntiles, grid, nfull, ntail, split, gran, gpt;
     size_t part_bytes;
 };
-PfPlan pf_plan(size_t M, size_t K, size_t N, int sm_count) {
+PfPlan pf_plan(int fmt, size_t M, size_t K, size_t N, int sm_count) {
     PfPlan pl{};
-    pl.mt = pick_mt(M, N, sm_count);
+    pl.mt = pick_mt(fmt, M, K, N, sm_count);
     pl.ntn = (uint32_t)((N + 127) / 128);
     pl.ntiles = pl.ntn * (uint32_t)((M + pl.mt - 1) / pl.mt);
     const uint32_t G = (uint32_t)sm_count, nkt = (uint32_t)(K / BK);
@@ -978,7 +990,7 @@ PfPlan pf_plan(size_t M, size_t K, size_t N, int sm_count) {
 size_t prefill_workspace_bytes(int fmt, int act_dtype, size_t M, size_t K, size_t N, int sm_count) {
     const bool kq = (fmt == FMT_Q4_K || fmt == FMT_Q5_K || fmt == FMT_Q6_K);  // always re-quantised (see act_q8k_to_bf16_kernel)
     const size_t acts = (act_dtype == DT_BF16 && !kq) ? 0 : ((M * K * 2 + 255) & ~(size_t)255);
-    return acts + pf_plan(M, K, N, sm_count).part_bytes;
+    return acts + pf_plan(fmt, M, K, N, sm_count).part_bytes;
 }
 
 cudaError_t launch_prefill(int fmt, const void* act, int act_dtype, const void* w, void* out, int out_dtype, size_t M,
@@ -987,7 +999,7 @@ cudaError_t launch_prefill(int fmt, const void* act, int act_dtype, const void* 
     *ws_too_small = false;
     const void* act_bf16 = act;
     const bool kq = (fmt == FMT_Q4_K || fmt == FMT_Q5_K || fmt == FMT_Q6_K);
-    const PfPlan pl = pf_plan(M, K, N, sm_count);
+    const PfPlan pl = pf_plan(fmt, M, K, N, sm_count);
     const size_t need = prefill_workspace_bytes(fmt, act_dtype, M, K, N, sm_count), act_bytes = need - pl.part_bytes;
     if (need && (!ws || ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 15))) { *ws_too_small = true; return cudaSuccess; }
     if ((act_dtype != DT_BF16 || kq) && acts_prepared) {

@@ -13,7 +13,8 @@ torch = pytest.importorskip("torch")
 
 @pytest.mark.parametrize("fmt", ["Q4_K", "Q6_K", "Q8_0"])
 @pytest.mark.parametrize("m,n,k", [(255, 300, 1024), (256, 300, 2048), (257, 20000, 256), (300, 9000, 1024), (384, 8193, 512), (385, 9000, 512),
-                                   (384, 1024, 2048), (900, 130, 4096), (1023, 1024, 512), (1024, 1024, 512)])
+                                   (384, 1024, 2048), (900, 130, 4096), (1023, 1024, 512), (1024, 1024, 512),
+                                   (256, 4096, 4096), (256, 4000, 4352), (512, 1000, 6144), (300, 700, 6400), (700, 200, 8448)])
 def test_tile_rule(oracle, fmt, m, n, k):
     from boostr_b200 import ops
 
