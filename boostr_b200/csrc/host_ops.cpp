@@ -59,9 +59,12 @@ WeightRef* ref_of(PyObject* qt) {
     return r;
 }
 
-// Scratch buffers: one per (device, stream), grown on demand.  Calls on one stream run in order, so they may share a
-// buffer; the entry's mutex keeps the launches of two threads on one stream from interleaving inside a call, and the
-// call's own reference keeps a buffer that another thread replaces alive until its launches are enqueued.
+// Scratch buffers of eager calls: one per (device, stream), grown on demand.  Calls on one stream run in order, so they may
+// share a buffer; the entry's mutex keeps the launches of two threads on one stream from interleaving inside a call, and
+// the call's own reference keeps a buffer that another thread replaces alive until its launches are enqueued.
+// A call that is being captured into a graph takes none of them: a replay runs whenever and on whichever stream its owner
+// launches it, beside eager calls and other graphs, and its addresses outlive the growth of a shared buffer.  Its
+// scratch is allocated for the call, from the memory pool of the graph, which keeps it.
 struct Scratch {
     std::mutex m;
     at::Tensor buf;
@@ -142,40 +145,46 @@ struct DeviceScope {
     }
 };
 
+bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;
+    cudaGetLastError();  // the legacy stream beside another thread's capture: the launch itself will say so
+    return false;
+}
+
+// Other Python threads run while this lives.
+struct NoGil {
+    PyThreadState* state = PyEval_SaveThread();
+    NoGil() = default;
+    NoGil(const NoGil&) = delete;
+    ~NoGil() { PyEval_RestoreThread(state); }
+};
+
 // Runs call(scratch pointer, scratch bytes, stream) without the GIL, with at least `need` bytes of scratch.
 template <typename F>
 int with_scratch(c10::Device dev, size_t need, F&& call) {
     const cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
     if (!need) {
-        int rc;
-        Py_BEGIN_ALLOW_THREADS
-        rc = call(static_cast<void*>(nullptr), (size_t)0, st);
-        Py_END_ALLOW_THREADS
-        return rc;
+        NoGil nogil;
+        return call(static_cast<void*>(nullptr), (size_t)0, st);
+    }
+    if (capturing(st)) {
+        const at::Tensor buf = empty({(int64_t)need}, at::kByte, dev);
+        NoGil nogil;
+        return call(buf.data_ptr(), need, st);
     }
     Scratch& s = scratch_of(dev.index(), st);
-    int rc = B200Q_OK;
-    bool oom = false;
-    Py_BEGIN_ALLOW_THREADS
-    {
-        std::lock_guard<std::mutex> g(s.m);
-        if (!s.buf.defined() || (size_t)s.buf.numel() < need) {
-            s.buf = at::Tensor();  // back to the allocator first: a grown buffer may reuse its memory
-            try {
-                s.buf = empty({(int64_t)std::max<size_t>(need, (size_t)1 << 20)}, at::kByte, dev);
-            } catch (...) {
-                oom = true;
-            }
-        }
-        if (!oom) rc = call(s.buf.data_ptr(), (size_t)s.buf.numel(), st);
+    NoGil nogil;
+    std::lock_guard<std::mutex> g(s.m);
+    if (!s.buf.defined() || (size_t)s.buf.numel() < need) {
+        s.buf = at::Tensor();  // back to the allocator first: a grown buffer may reuse its memory
+        s.buf = empty({(int64_t)std::max<size_t>(need, (size_t)1 << 20)}, at::kByte, dev);
     }
-    Py_END_ALLOW_THREADS
-    return oom ? -1 : rc;  // -1: no scratch; the Python form retries and raises torch's own error
+    return call(s.buf.data_ptr(), (size_t)s.buf.numel(), st);
 }
 
 PyObject* not_served() { Py_RETURN_NOTIMPLEMENTED; }
 PyObject* result(int rc, const at::Tensor& out) {
-    if (rc == -1) return not_served();
     if (rc != B200Q_OK) return PyLong_FromLong(rc);
     return THPVariable_Wrap(out);
 }
@@ -282,7 +291,6 @@ PyObject* quant_matmul_batch(PyObject*, PyObject* const* args, Py_ssize_t nargs)
                 return b200q_rmsnorm_quant_matmul_batch((int)nw, fmts, wp, ns, op, a.t->data_ptr(), norm, eps, a.dt, (int)odt, a.m, a.k, ws, bytes, st);
             return b200q_quant_matmul_batch((int)nw, fmts, wp, ns, op, a.t->data_ptr(), a.dt, (int)odt, a.m, a.k, ws, bytes, st);
         });
-        if (rc == -1) return not_served();
         if (rc != B200Q_OK) return PyLong_FromLong(rc);
         PyObject* list = PyList_New(nw);
         if (!list) return nullptr;

@@ -3,7 +3,8 @@
 Mirrors the contract of boostr's graph-mode decode (src/inference/decode_graph.rs:1-48,
 src/model/llama/model/forward_graph.rs:22-73): every tensor the host touches between replays is allocated
 BEFORE capture and keeps its address; per-step values reach the kernels through device memory that is
-updated with stream-ordered copies on the compute stream; the captured step allocates nothing.
+updated with stream-ordered copies on the compute stream; the captured step allocates nothing but the scratch of
+its calls, which comes from the graph's own memory pool and lives as long as the graph.
 
 ``DecodeGraph`` owns that discipline for a step function built from this library's operators:
 

@@ -47,7 +47,10 @@ def _require_cuda(t: torch.Tensor, what: str) -> None:
 
 
 def workspace(nbytes: int, device) -> torch.Tensor:
-    """Scratch buffer reused across calls on one device (grown on demand, never shrunk)."""
+    """Scratch buffer reused across eager calls on one device and stream (grown on demand, never shrunk).  A call that is
+    being captured gets one of its own from the graph's memory pool: its replays run beside eager calls and other graphs."""
+    if torch.cuda.is_current_stream_capturing():
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
     key = (torch.device(device).index, torch.cuda.current_stream().cuda_stream)
     buf = _workspaces.get(key)
     if buf is None or buf.numel() < nbytes:
