@@ -46,18 +46,22 @@ WeightRef* ref_of_capsule(PyObject* o) {
     if (!PyCapsule_CheckExact(o)) return nullptr;
     return static_cast<WeightRef*>(PyCapsule_GetPointer(o, CAPSULE));
 }
-// The WeightRef of a QuantTensor; nullptr (no Python error) when the object has none.
-WeightRef* ref_of(PyObject* qt) {
-    PyObject* c = PyObject_GetAttr(qt, s_ref);
-    if (!c) {
-        PyErr_Clear();
-        return nullptr;
+// The WeightRef of a QuantTensor, held with its capsule until the end of the call (the attribute is made by the first call
+// that asks for it, on any thread); none (and no Python error) when the object has none.
+class Ref {
+    PyObject* capsule_;
+    WeightRef* w_ = nullptr;
+
+  public:
+    explicit Ref(PyObject* qt) : capsule_(PyObject_GetAttr(qt, s_ref)) {
+        if (capsule_) w_ = ref_of_capsule(capsule_);
+        if (!w_) PyErr_Clear();
     }
-    WeightRef* r = ref_of_capsule(c);
-    if (!r) PyErr_Clear();
-    Py_DECREF(c);  // the QuantTensor keeps it alive for the duration of the call
-    return r;
-}
+    Ref(const Ref&) = delete;
+    ~Ref() { Py_XDECREF(capsule_); }
+    explicit operator bool() const { return w_ != nullptr; }
+    WeightRef* operator->() const { return w_; }
+};
 
 // Scratch buffers of eager calls: one per (device, stream), grown on demand.  Calls on one stream run in order, so they may
 // share a buffer; the entry's mutex keeps the launches of two threads on one stream from interleaving inside a call, and
@@ -116,7 +120,7 @@ bool act_of(PyObject* o, Act& a) {
     a.dev = t.device();
     return true;
 }
-bool weight_fits(const WeightRef* w, const Act& a) { return w && w->matrix && w->k == a.k && w->storage.device() == a.dev; }
+bool weight_fits(const Ref& w, const Act& a) { return w && w->matrix && w->k == a.k && w->storage.device() == a.dev; }
 
 // The output: `given` (validated) or a new tensor [..., n]; false: `given` does not fit.
 bool out_of(PyObject* given, const Act& a, size_t n, at::ScalarType t, at::Tensor& out) {
@@ -226,7 +230,7 @@ PyObject* quant_matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject* {
         Act a;
         if (nargs != 4 || !act_of(args[0], a)) return not_served();
-        WeightRef* w = ref_of(args[1]);
+        const Ref w(args[1]);
         if (!weight_fits(w, a)) return not_served();
         const long odt = PyLong_AsLong(args[2]);
         DeviceScope dev(a.dev);
@@ -261,7 +265,7 @@ PyObject* quant_matmul_batch(PyObject*, PyObject* const* args, Py_ssize_t nargs)
         at::Tensor outs[16];
         size_t need = 0;
         for (Py_ssize_t i = 0; i < nw; ++i) {
-            WeightRef* w = ref_of(PySequence_Fast_GET_ITEM(seq, i));
+            const Ref w(PySequence_Fast_GET_ITEM(seq, i));
             if (!weight_fits(w, a)) return not_served();
             fmts[i] = w->format;
             wp[i] = w->storage.data_ptr();
@@ -311,7 +315,7 @@ PyObject* quant_swiglu(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject* {
         Act a;
         if (nargs != 5 || !act_of(args[0], a)) return not_served();
-        WeightRef *g = ref_of(args[1]), *u = ref_of(args[2]);
+        const Ref g(args[1]), u(args[2]);
         if (!weight_fits(g, a) || !weight_fits(u, a) || g->format != u->format || g->n != u->n) return not_served();
         const long odt = PyLong_AsLong(args[3]);
         DeviceScope dev(a.dev);
@@ -331,7 +335,7 @@ PyObject* quant_mlp(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject* {
         Act a;
         if (nargs != 6 || !act_of(args[0], a)) return not_served();
-        WeightRef *g = ref_of(args[1]), *u = ref_of(args[2]), *d = ref_of(args[3]);
+        const Ref g(args[1]), u(args[2]), d(args[3]);
         if (!weight_fits(g, a) || !weight_fits(u, a) || g->format != u->format || g->n != u->n || !d || !d->matrix || d->k != g->n ||
             d->storage.device() != a.dev)
             return not_served();
@@ -352,7 +356,7 @@ PyObject* quant_mlp(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 PyObject* dequantize(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject* {
         if (nargs != 2) return not_served();
-        WeightRef* w = ref_of(args[0]);
+        const Ref w(args[0]);
         if (!w || !w->storage.is_cuda()) return not_served();
         const long odt = PyLong_AsLong(args[1]);
         const c10::Device d = w->storage.device();

@@ -5,6 +5,7 @@ buffer, the block format, and the LOGICAL element shape.  Blocks run along the l
 """
 from __future__ import annotations
 
+import warnings
 from typing import Sequence
 
 import numpy as np
@@ -15,6 +16,17 @@ from .format import QuantError, QuantFormat
 _hostops = None
 
 
+class _PythonForms:
+    """Stands in for the compiled entry points where they are not built: every call is declined and takes its Python form,
+    which enters the same kernels with 10 us more host time."""
+
+    @staticmethod
+    def _decline(*args):
+        return NotImplemented
+
+    quant_matmul = quant_matmul_batch = quant_swiglu = quant_mlp = dequantize = _decline
+
+
 def hostops():
     """The compiled Python entry points (``csrc/host_ops.cpp``)."""
     global _hostops
@@ -22,8 +34,9 @@ def hostops():
         try:
             from . import _hostops as mod
         except ImportError as e:
-            raise ImportError("boostr_b200/_hostops.so cannot be loaded: build it with `python -m boostr_b200.build` "
-                              "(needs nvcc and g++; no GPU required)") from e
+            warnings.warn(f"boostr_b200/_hostops.so cannot be loaded ({e}): calls take their slower Python form. "
+                          "Build it with `python -m boostr_b200.build` (needs nvcc and g++; no GPU required)", RuntimeWarning, stacklevel=3)
+            mod = _PythonForms
         _hostops = mod
     return _hostops
 
@@ -33,8 +46,14 @@ class QuantTensor:
         self._storage = storage
         self._format = fmt
         self._shape = tuple(int(x) for x in shape)
-        # what the compiled entry points need of this tensor, read once
-        self._ref = hostops().make_ref(storage, fmt.format_id, self._shape)
+
+    def __getattr__(self, name: str):
+        # ``_ref``: what the compiled entry points need of this tensor, read once by its first call.  A tensor that is only made,
+        # read from a file or sharded on the host never asks for them.
+        if name != "_ref":
+            raise AttributeError(f"{type(self).__name__!r} object has no attribute {name!r}")
+        self._ref = ref = hostops().make_ref(self._storage, self._format.format_id, self._shape)
+        return ref
 
     @classmethod
     def from_bytes(cls, data, fmt, shape: Sequence[int], device="cuda") -> "QuantTensor":
