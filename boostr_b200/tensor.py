@@ -55,6 +55,10 @@ class QuantTensor:
         self._ref = ref = hostops().make_ref(self._storage, self._format.format_id, self._shape)
         return ref
 
+    def __getstate__(self) -> dict:
+        """For copies, pickles and ``torch.save``: ``_ref`` points into this process and to this tensor's storage."""
+        return {k: v for k, v in vars(self).items() if k != "_ref"}
+
     @classmethod
     def from_bytes(cls, data, fmt, shape: Sequence[int], device="cuda") -> "QuantTensor":
         """src/quant/tensor.rs:44-92 — validates the last dimension and the exact byte count."""

@@ -40,3 +40,31 @@ with warnings.catch_warnings(record=True) as seen:
 assert len(seen) == 1 and "slower Python form" in str(seen[0].message)
 """
     subprocess.run([sys.executable, "-c", code], cwd=ROOT, check=True)
+
+
+def _tensor():
+    return QuantTensor.from_bytes(synth.weight_bytes("Q6_K", synth.rng_for(2), 6, 512), "Q6_K", (6, 512), device="cpu")
+
+
+def _same(a, b):
+    return a.format is b.format and a.shape == b.shape and torch.equal(a.storage, b.storage)
+
+
+@pytest.mark.parametrize("used", [False, True])
+def test_copied_and_saved(used):
+    """Also a tensor that a compiled call has used, whose handle of native memory stays behind."""
+    qt = _tensor()
+    if used:
+        qt._ref = lambda: None  # like the real handle, nothing that can be copied or saved
+    lin = QuantLinear(qt, torch.arange(6.0))
+    deep = copy.deepcopy(qt)
+    assert _same(deep, qt) and deep.storage.data_ptr() != qt.storage.data_ptr()
+    flat = copy.copy(qt)
+    assert _same(flat, qt) and flat.storage.data_ptr() == qt.storage.data_ptr()
+    for other in (pickle.loads(pickle.dumps(qt)), pickle.loads(pickle.dumps(lin)).weight, copy.deepcopy(lin).weight):
+        assert _same(other, qt)
+    f = io.BytesIO()
+    torch.save({"w": qt}, f)
+    f.seek(0)
+    assert _same(torch.load(f, weights_only=False)["w"], qt)
+    assert all("_ref" not in vars(x) for x in (deep, flat))
