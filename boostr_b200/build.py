@@ -1,12 +1,13 @@
-"""Compiles the CUDA sources into ``boostr_b200/libb200q.so`` for sm_100a with nvcc.
+"""Compiles the CUDA sources into ``boostr_b200/libb200q.so`` for sm_100a with nvcc, and the Python entry points
+(``host_ops.cpp``) into the extension module ``boostr_b200/_hostops`` against torch's headers.
 
-and the Python entry points (``host_ops.cpp``) into ``boostr_b200/_hostops.so`` against torch's
-headers.  No GPU is needed to build.  ``python -m boostr_b200.build`` (or ``build()``) recompiles
-only the translation units whose sources changed.
+No GPU is needed to build.  ``python -m boostr_b200.build`` (or ``build()``) recompiles only the translation units whose
+sources changed, and the extension also when Python or torch did; ``-f`` recompiles everything.
 """
 from __future__ import annotations
 
 import concurrent.futures
+import importlib.metadata
 import os
 import shutil
 import subprocess
@@ -17,7 +18,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJDIR = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libb200q.so")
-HOST_LIB = os.path.join(HERE, "_hostops.so")
+HOST_LIB = os.path.join(HERE, "_hostops" + sysconfig.get_config_var("EXT_SUFFIX"))  # the name carries Python's ABI
+HOST_STAMP = os.path.join(OBJDIR, "_hostops.stamp")
 HOST_SOURCE = os.path.join(CSRC, "host_ops.cpp")
 SOURCES = ["api.cu", "dequant.cu", "gemv.cu", "gemv_m1.cu", "gemv_m1_f32.cu", "kquant_i8.cu", "prefill.cu", "smallm_i8.cu"]
 NVCC_FLAGS = [
@@ -55,9 +57,21 @@ def _compile(src: str, verbose: bool) -> str:
     return obj
 
 
-def _build_host() -> None:
+def _host_stamp() -> str:
+    """What the extension is compiled against."""
+    return f"{os.path.basename(HOST_LIB)} torch {importlib.metadata.version('torch')}"
+
+
+def _host_current() -> bool:
     header = os.path.join(HERE, "..", "include", "b200q.h")
-    if os.path.exists(HOST_LIB) and os.path.getmtime(HOST_LIB) >= max(os.path.getmtime(HOST_SOURCE), os.path.getmtime(header)):
+    if not (os.path.exists(HOST_LIB) and os.path.exists(HOST_STAMP)):
+        return False
+    with open(HOST_STAMP) as f:
+        return f.read() == _host_stamp() and os.path.getmtime(HOST_LIB) >= max(os.path.getmtime(HOST_SOURCE), os.path.getmtime(header))
+
+
+def _build_host() -> None:
+    if _host_current():
         return
     import torch
     from torch.utils.cpp_extension import include_paths
@@ -72,6 +86,11 @@ def _build_host() -> None:
     if r.returncode:
         sys.stderr.write(r.stdout + r.stderr)
         raise RuntimeError("g++ failed on host_ops.cpp")
+    untagged = os.path.join(HERE, "_hostops.so")
+    if os.path.exists(untagged):  # of a build without Python's ABI in the name
+        os.remove(untagged)
+    with open(HOST_STAMP, "w") as f:
+        f.write(_host_stamp())
 
 
 def build(verbose: bool = False, force: bool = False) -> str:

@@ -17,6 +17,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/version.h>
 
 #include <algorithm>
 #include <map>
@@ -384,5 +385,7 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_hostops", nullptr, -1, methods};
 
 PyMODINIT_FUNC PyInit__hostops(void) {
     s_ref = PyUnicode_InternFromString("_ref");
-    return PyModule_Create(&module);
+    PyObject* m = PyModule_Create(&module);
+    if (m && PyModule_AddStringConstant(m, "torch_version", TORCH_VERSION) != 0) Py_CLEAR(m);
+    return m;
 }

@@ -33,8 +33,11 @@ def hostops():
     if _hostops is None:
         try:
             from . import _hostops as mod
+
+            if not torch.__version__.startswith(mod.torch_version):
+                raise ImportError(f"compiled against torch {mod.torch_version}, running torch {torch.__version__}")
         except ImportError as e:
-            warnings.warn(f"boostr_b200/_hostops.so cannot be loaded ({e}): calls take their slower Python form. "
+            warnings.warn(f"the compiled entry points boostr_b200._hostops cannot be used ({e}): calls take their slower Python form. "
                           "Build it with `python -m boostr_b200.build` (needs nvcc and g++; no GPU required)", RuntimeWarning, stacklevel=3)
             mod = _PythonForms
         _hostops = mod
