@@ -64,6 +64,25 @@ class Ref {
     WeightRef* operator->() const { return w_; }
 };
 
+// The objects of a list or tuple at the time of the call, held until its end: reading an attribute of one of them runs Python,
+// and other threads run during the launches, so the list itself may change meanwhile.
+struct Items {
+    static constexpr Py_ssize_t MAX = 16;
+    PyObject* o[MAX];
+    Py_ssize_t n = 0;
+    Items() = default;
+    Items(const Items&) = delete;
+    ~Items() {
+        for (Py_ssize_t i = 0; i < n; ++i) Py_DECREF(o[i]);
+    }
+    bool take(PyObject* seq) {
+        if (!PyList_CheckExact(seq) && !PyTuple_CheckExact(seq)) return false;
+        if (PySequence_Fast_GET_SIZE(seq) > MAX) return false;
+        for (; n < PySequence_Fast_GET_SIZE(seq); ++n) o[n] = Py_NewRef(PySequence_Fast_GET_ITEM(seq, n));
+        return true;
+    }
+};
+
 // Scratch buffers of eager calls: one per (device, stream), grown on demand.  Calls on one stream run in order, so they may
 // share a buffer; the entry's mutex keeps the launches of two threads on one stream from interleaving inside a call, and
 // the call's own reference keeps a buffer that another thread replaces alive until its launches are enqueued.
@@ -251,22 +270,19 @@ PyObject* quant_matmul_batch(PyObject*, PyObject* const* args, Py_ssize_t nargs)
     return guarded([&]() -> PyObject* {
         Act a;
         if (nargs != 6 || !act_of(args[0], a)) return not_served();
-        PyObject* seq = args[3];
-        if (!PyList_CheckExact(seq) && !PyTuple_CheckExact(seq)) return not_served();
-        const Py_ssize_t nw = PySequence_Fast_GET_SIZE(seq);
-        if (nw < 1 || nw > 16) return not_served();
-        PyObject* given = args[5];
-        if (given != Py_None && ((!PyList_CheckExact(given) && !PyTuple_CheckExact(given)) || PySequence_Fast_GET_SIZE(given) != nw)) return not_served();
+        Items weights, given;
+        if (!weights.take(args[3]) || weights.n < 1 || (args[5] != Py_None && (!given.take(args[5]) || given.n != weights.n))) return not_served();
+        const Py_ssize_t nw = weights.n;
         const long odt = PyLong_AsLong(args[4]);
         DeviceScope dev(a.dev);
-        int fmts[16];
-        const void* wp[16];
-        size_t ns[16];
-        void* op[16];
-        at::Tensor outs[16];
+        int fmts[Items::MAX];
+        const void* wp[Items::MAX];
+        size_t ns[Items::MAX];
+        void* op[Items::MAX];
+        at::Tensor outs[Items::MAX];
         size_t need = 0;
         for (Py_ssize_t i = 0; i < nw; ++i) {
-            const Ref w(PySequence_Fast_GET_ITEM(seq, i));
+            const Ref w(weights.o[i]);
             if (!weight_fits(w, a)) return not_served();
             fmts[i] = w->format;
             wp[i] = w->storage.data_ptr();
@@ -288,7 +304,7 @@ PyObject* quant_matmul_batch(PyObject*, PyObject* const* args, Py_ssize_t nargs)
             return not_served();
         }
         for (Py_ssize_t i = 0; i < nw; ++i) {
-            if (!out_of(given == Py_None ? Py_None : PySequence_Fast_GET_ITEM(given, i), a, ns[i], scalar_type(odt), outs[i])) return not_served();
+            if (!out_of(given.n ? given.o[i] : Py_None, a, ns[i], scalar_type(odt), outs[i])) return not_served();
             op[i] = outs[i].data_ptr();
         }
         const int rc = with_scratch(a.dev, need, [&](void* ws, size_t bytes, cudaStream_t st) {
@@ -300,7 +316,7 @@ PyObject* quant_matmul_batch(PyObject*, PyObject* const* args, Py_ssize_t nargs)
         PyObject* list = PyList_New(nw);
         if (!list) return nullptr;
         for (Py_ssize_t i = 0; i < nw; ++i) {
-            PyObject* o = given == Py_None ? THPVariable_Wrap(outs[i]) : Py_NewRef(PySequence_Fast_GET_ITEM(given, i));
+            PyObject* o = given.n ? Py_NewRef(given.o[i]) : THPVariable_Wrap(outs[i]);
             if (!o) {
                 Py_DECREF(list);
                 return nullptr;

@@ -1,0 +1,46 @@
+"""The compiled Python entry points (``csrc/host_ops.cpp``): what they take, what they leave to the Python form, and the scratch
+that they share between calls."""
+import pytest
+
+from boostr_b200 import synth
+from boostr_b200.format import QuantFormat as F
+from boostr_b200.tensor import QuantTensor, hostops
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from boostr_b200 import ops as o
+
+    assert hostops().__name__ == "boostr_b200._hostops", "the compiled entry points are not built"
+    return o
+
+
+def _gen(seed):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    return g
+
+
+def test_lists_that_change_during_the_call(ops):
+    """The entry points read an attribute of every weight, which may run Python code that shrinks the lists of the call."""
+    gen = _gen(1)
+    outs = []
+
+    class Shrinking(QuantTensor):
+        @property
+        def _ref(self):
+            del outs[1:], weights[1:]
+            return hostops().make_ref(self.storage, self.format.format_id, self.shape)
+
+    base = [synth.device_weight("Q4_K", 64, 256, gen) for _ in range(3)]
+    weights = [Shrinking(w.storage, w.format, w.shape) for w in base]
+    x = torch.randn(2, 256, device="cuda", generator=gen)
+    outs.extend(torch.empty(2, 64, device="cuda") for _ in range(3))
+    kept = list(outs)
+    got = ops.quant_matmul_batch(x, weights, outs=outs)
+    assert len(got) == 3 and all(a is b for a, b in zip(got, kept))
+    for y, w in zip(got, base):
+        assert torch.equal(y, ops.quant_matmul(x, w))
