@@ -374,12 +374,13 @@ PyObject* dequantize(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject* {
         if (nargs != 2) return not_served();
         const Ref w(args[0]);
-        if (!w || !w->storage.is_cuda()) return not_served();
+        const size_t block = w ? b200q_block_size(w->format) : 0;
+        if (!block || !w->storage.is_cuda()) return not_served();  // 0: not a format of this library
         const long odt = PyLong_AsLong(args[1]);
         const c10::Device d = w->storage.device();
         DeviceScope dev(d);
         at::Tensor out = empty(w->shape, scalar_type(odt), d);
-        const size_t nblocks = w->numel / b200q_block_size(w->format);
+        const size_t nblocks = w->numel / block;
         const int rc = with_scratch(d, 0, [&](void*, size_t, cudaStream_t st) {
             return b200q_dequantize(w->format, w->storage.data_ptr(), nblocks, out.data_ptr(), (int)odt, st);
         });

@@ -44,3 +44,14 @@ def test_lists_that_change_during_the_call(ops):
     assert len(got) == 3 and all(a is b for a, b in zip(got, kept))
     for y, w in zip(got, base):
         assert torch.equal(y, ops.quant_matmul(x, w))
+
+
+def test_unknown_format_is_an_error(ops):
+    class Fmt:  # Q4_1, which the library does not read
+        format_id, block_size, block_bytes, name = 1, 32, 20, "Q4_1"
+
+    qt = QuantTensor(torch.zeros(20 * 8, dtype=torch.uint8, device="cuda"), Fmt(), (8, 32))
+    with pytest.raises(RuntimeError, match="unsupported format id 1"):
+        ops.dequantize(qt)
+    with pytest.raises(RuntimeError, match="unsupported format id 1"):
+        ops.quant_matmul(torch.zeros(1, 32, device="cuda"), qt)
