@@ -103,6 +103,24 @@ def test_two_byte_products_bit_identical(oracle, fmt, m, n, k):
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), describe_mismatch(got, want)
 
 
+def test_batch_shares_one_image():
+    """The Q2_K, Q3_K and Q5_K weights of a batch read one image of the activations."""
+    from boostr_b200 import ops
+
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(7)
+    m, k = 37, 1280
+    ws = [synth.device_weight(fmt, n, k, gen) for fmt, n in (("Q5_K", 4097), ("Q3_K", 300), ("Q2_K", 300), ("Q5_K", 4100))]
+    assert all(_tile_rows(w.format.name, m, *w.shape) >= 0 for w in ws)
+    x = torch.randn(m, k, device="cuda", generator=gen)
+    want = [ops.quant_matmul(x, w) for w in ws]
+    before = ops.launch_count()
+    got = ops.quant_matmul_batch(x, ws)
+    assert ops.launch_count() - before == 1 + len(ws)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
 def test_extreme_codes(oracle):
     """Every scale, code and activation at its largest: the integer sums reach their bounds."""
     from boostr_b200 import ops
