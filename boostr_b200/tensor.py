@@ -58,6 +58,11 @@ class QuantTensor:
         self._ref = ref = hostops().make_ref(self._storage, self._format.format_id, self._shape)
         return ref
 
+    def __setattr__(self, name: str, value) -> None:
+        object.__setattr__(self, name, value)
+        if name in ("_storage", "_format", "_shape"):
+            vars(self).pop("_ref", None)
+
     def __getstate__(self) -> dict:
         """For copies, pickles and ``torch.save``: ``_ref`` points into this process and to this tensor's storage."""
         return {k: v for k, v in vars(self).items() if k != "_ref"}

@@ -55,3 +55,14 @@ def test_unknown_format_is_an_error(ops):
         ops.dequantize(qt)
     with pytest.raises(RuntimeError, match="unsupported format id 1"):
         ops.quant_matmul(torch.zeros(1, 32, device="cuda"), qt)
+
+
+def test_replaced_storage_is_read(ops):
+    """A tensor whose storage is exchanged after a call: the next call reads the new one."""
+    gen = _gen(2)
+    a, b = (synth.device_weight("Q4_K", 64, 512, gen) for _ in range(2))
+    x = torch.randn(3, 512, device="cuda", generator=gen)
+    want = ops.quant_matmul(x, b), ops.dequantize(b)
+    ops.quant_matmul(x, a), ops.dequantize(a)
+    a._storage = b.storage.clone()
+    assert torch.equal(ops.quant_matmul(x, a), want[0]) and torch.equal(ops.dequantize(a), want[1])
