@@ -316,7 +316,7 @@ PyObject* quant_matmul_batch(PyObject*, PyObject* const* args, Py_ssize_t nargs)
         PyObject* list = PyList_New(nw);
         if (!list) return nullptr;
         for (Py_ssize_t i = 0; i < nw; ++i) {
-            PyObject* o = given.n ? Py_NewRef(given.o[i]) : THPVariable_Wrap(outs[i]);
+            PyObject* o = THPVariable_Wrap(outs[i]);  // the given tensor itself, or the new one where None was given
             if (!o) {
                 Py_DECREF(list);
                 return nullptr;

@@ -66,3 +66,13 @@ def test_replaced_storage_is_read(ops):
     ops.quant_matmul(x, a), ops.dequantize(a)
     a._storage = b.storage.clone()
     assert torch.equal(ops.quant_matmul(x, a), want[0]) and torch.equal(ops.dequantize(a), want[1])
+
+
+def test_outputs_given_in_part(ops):
+    """None among the outputs of a batch: that one is allocated, and returned."""
+    gen = _gen(5)
+    w = synth.device_weight("Q4_K", 64, 512, gen)
+    x = torch.randn(3, 512, device="cuda", generator=gen)
+    y = torch.empty(3, 64, device="cuda")
+    got = ops.quant_matmul_batch(x, [w, w], outs=[None, y])
+    assert got[1] is y and torch.equal(got[0], y) and torch.equal(y, ops.quant_matmul(x, w))
