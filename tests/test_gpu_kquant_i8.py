@@ -1,6 +1,7 @@
-"""Q2_K / Q3_K products at the edges of their kernels' tiles, bit for bit against the CPU oracle (integer sums, blocks added
-in K order): row counts around the multiples of 8 and 16 of the mma.sync kernel and of 16 ... 128 of the tensor-core
-kernel, partial row tiles, one block and odd block counts (rows of every alignment), more tiles than SMs, long K."""
+"""The integer tensor-core products of the K-quants, bit for bit against the CPU oracle (integer sums, blocks added in K order).
+``test_bit_identical``: Q2_K / Q3_K around the multiples of 8 and 16 rows of the mma.sync kernel (which takes all of its shapes but
+the two of 300 and 512 rows), partial row tiles, one block and odd block counts (rows of every alignment), long K.
+``test_weight_tiles_by_tma``: the tensor-core kernel on tiles of 16 ... 128 rows, held to the rule that picks them."""
 import os
 
 import numpy as np
@@ -139,3 +140,54 @@ def test_extreme_codes(oracle):
             got = ops.quant_matmul(torch.from_numpy(act[:rows]).cuda(), QuantTensor.from_bytes(w, F[fmt], (n, k), device="cuda")).cpu().numpy()
             want = oracle.quant_matmul(fmt, act[:rows], w, n, threads=4)
             assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), describe_mismatch(got, want)
+
+
+@pytest.mark.parametrize("fmt,m,n,k", [("Q2_K", 512, 4096, 1024), ("Q3_K", 512, 4096, 2048), ("Q4_K", 48, 14336, 1024), ("Q5_K", 48, 14336, 1024),
+                                       ("Q5_K", 20, 4100, 512)])
+@pytest.mark.parametrize("fill", [0xFF, 0x00, 0xF0, 0x0F])
+def test_extreme_codes_in_tiles(oracle, fmt, m, n, k, fill):
+    """The same in the tensor-core kernel: every code, scale and min at an end of its range, activations of one sign and of
+    alternating ones, so that the sums of one-byte and of two-byte products reach their bounds."""
+    from boostr_b200 import ops
+
+    assert _tile_rows(fmt, m, n, k) > 0
+    w = np.full((n * k // 256, F[fmt].block_bytes), fill, np.uint8)
+    one = np.frombuffer(np.array([1.0], np.float16).tobytes(), np.uint8)
+    for at in {"Q2_K": (80, 82), "Q3_K": (108,), "Q4_K": (0, 2), "Q5_K": (0, 2)}[fmt]:
+        w[:, at:at + 2] = one
+    act = np.ones((m, k), np.float32)
+    act[1::3] = -1.0
+    act[2::3, ::2] = -1.0
+    got = ops.quant_matmul(torch.from_numpy(act).cuda(), QuantTensor.from_bytes(w.reshape(-1), F[fmt], (n, k), device="cuda")).cpu().numpy()
+    ops.check_device_status()
+    want = oracle.quant_matmul(fmt, act, w.reshape(-1), n, threads=os.cpu_count() or 8)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), describe_mismatch(got, want)
+
+
+@pytest.mark.parametrize("fmt,m,n,k", [("Q2_K", 5, 131, 512), ("Q3_K", 300, 4001, 256), ("Q4_K", 37, 8193, 512), ("Q5_K", 21, 4099, 512), ("Q4_K", 65, 131, 256)])
+def test_swiglu_and_its_output(fmt, m, n, k):
+    """SwiGLU is silu(gate) * up of the two products; the last kernel takes outputs of any 4-byte alignment, an element count
+    that is no multiple of four, and 16-bit results that are one rounding of the f32 ones."""
+    from boostr_b200 import ops
+
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(seed_of(fmt, m, n, k))
+    g, u = synth.device_weight(fmt, n, k, gen), synth.device_weight(fmt, n, k, gen)
+    x = torch.randn(m, k, device="cuda", generator=gen)
+    a, b = ops.quant_matmul(x, g).double(), ops.quant_matmul(x, u).double()
+    want = a / (1 + torch.exp(-a)) * b
+    out = ops.quant_swiglu(x, g, u)
+    # expf is within 2 ulp, the sum, the quotient and the product within half a one each: below 4 * 2^-23; past -88 expf overflows
+    # and the result is 0 in place of less than 1e-36 |b|
+    assert ((out.double() - want).abs() <= 5e-7 * want.abs() + 1e-36 * b.abs()).all()
+    for shift in (1, 2, 3):
+        buf = torch.full((m * n + 8,), 77.0, device="cuda")
+        y = ops.quant_swiglu(x, g, u, out=buf[shift:shift + m * n].view(m, n))
+        assert torch.equal(y, out) and (buf[:shift] == 77.0).all() and (buf[shift + m * n:] == 77.0).all()
+    for dt in (torch.bfloat16, torch.float16):
+        assert torch.equal(ops.quant_swiglu(x, g, u, out_dtype=dt), out.to(dt))
+    d = synth.device_weight("Q6_K", 64, 8192, gen)
+    if n >= 8192:  # the feed-forward block on these kernels: SwiGLU, then the down product
+        g8, u8 = (QuantTensor(t.storage[:F[fmt].storage_bytes(8192 * k)], t.format, (8192, k)) for t in (g, u))
+        assert torch.equal(ops.quant_mlp(x, g8, u8, d), ops.quant_matmul(ops.quant_swiglu(x, g8, u8), d))
+    ops.check_device_status()
