@@ -24,7 +24,7 @@ class _PythonForms:
     def _decline(*args):
         return NotImplemented
 
-    quant_matmul = quant_matmul_batch = quant_swiglu = quant_mlp = dequantize = _decline
+    make_ref = quant_matmul = quant_matmul_batch = quant_swiglu = quant_mlp = dequantize = _decline
 
 
 def hostops():
@@ -46,13 +46,14 @@ def hostops():
 
 class QuantTensor:
     def __init__(self, storage: torch.Tensor, fmt: QuantFormat, shape: Sequence[int]):
-        self._storage = storage
-        self._format = fmt
-        self._shape = tuple(int(x) for x in shape)
+        own = vars(self)
+        own.update(_storage=storage, _format=fmt, _shape=tuple(int(x) for x in shape))
+        if storage.is_cuda:  # with the tensor, not in its first call
+            own["_ref"] = hostops().make_ref(storage, fmt.format_id, own["_shape"])
 
     def __getattr__(self, name: str):
-        # ``_ref``: what the compiled entry points need of this tensor, read once by its first call.  A tensor that is only made,
-        # read from a file or sharded on the host never asks for them.
+        # ``_ref``: what the compiled entry points need of this tensor.  A tensor that is made, read from a file or sharded on the
+        # host never asks for them.
         if name != "_ref":
             raise AttributeError(f"{type(self).__name__!r} object has no attribute {name!r}")
         self._ref = ref = hostops().make_ref(self._storage, self._format.format_id, self._shape)
