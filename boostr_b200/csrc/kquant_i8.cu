@@ -161,13 +161,15 @@ __device__ __forceinline__ void copy_rows(uint32_t dst, const uint8_t* blk, uint
 // two sets of four decode warps, taking the blocks in turn, write the scaled codes as 128-byte-swizzled K-major operand tiles,
 // the activation codes come by TMA, one thread issues 8 MMAs
 // (16 for two-byte products; + 2 for the mins) into one of two accumulators, and sixteen drain warps (thread = weight
-// row x every fourth group of 8 activation rows) scale the sums in packed f32 and add them to their registers.
-// What bounds it: with 128 activation rows a tile the issue slots (63 ... 68 % busy, tensor pipe 19 %, captured with the packed drain below): decode, and 8 (Q2_K) or
-// 5 (Q3_K) instructions a sum of drain; with few the latency of a block's chain through the barriers, the proxy fence and
-// two decode sets, 0.8 us (Q2_K, Q3_K) to 1.2 us (two-byte products) a block.  Measured: 512 rows x 14336 x 4096 Q2_K
-// 99 us, Q3_K 93 us (a layer of such products 0.42 ms; 69 ms with a kernel that took eight rows at a time); Q5_K 37 rows 28 us.  Tried and not kept:
-// packed f32x2 arithmetic in the drain (Q2_K 107 us, Q3_K 87 us; the assembler fuses mul.rn.f32x2 and add.rn.f32x2 into one
-// rounding unless an operand is hidden from it), and halves of a block as stages (4096 x 14336 at 64 rows 49 -> 58 us).
+// row x every fourth group of 8 activation rows) scale the sums and add them to their registers.
+// What bounds it: with 128 activation rows a tile the issue slots (Q2_K 72 %, Q3_K 67 % busy; ALU pipe 41 / 55 %, tensor pipe
+// 20 / 18 %): decode, and 8 (Q2_K) or 5 (Q3_K) instructions a sum of drain; with few the latency of a block's chain through
+// the barriers, the proxy fence and two decode sets (two-byte products: issue slots 60 ... 64 %, ALU pipe 51 ... 54 %), 0.8 us (Q2_K,
+// Q3_K) to 1.2 us (two-byte products) a block.  Measured: 512 rows x 14336 x 4096 Q2_K 99 us, Q3_K 93 us (a layer of such
+// products 0.42 ms; 69 ms with a kernel that took eight rows at a time); Q5_K 37 rows 28 us.  Tried and not kept: packed f32x2
+// arithmetic in the drain, which suits one format and not the other (Q2_K 107, Q3_K 87 us) and needs an operand hidden from
+// the assembler, which else makes one rounding of mul.rn.f32x2 and add.rn.f32x2; and halves of a block as stages
+// (4096 x 14336 at 64 rows 49 -> 58 us).
 struct KqTcParams {
     const uint8_t* w;
     void* out;

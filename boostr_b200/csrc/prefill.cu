@@ -24,9 +24,8 @@
 // Measured (M = 8192, N = 14336, K = 4096): 814 TFLOP/s; with the decode arithmetic and the tile stores
 // switched off the same pipeline reaches 980 TFLOP/s, cuBLAS bf16 on the same shape 1455 TFLOP/s, so
 // the single-CTA (cta_group::1) pipeline itself, not the decode, is the larger part of the gap.
-// Output tiles are dealt round-robin, whole.  Cutting the tiles of the last, incomplete round along K (each SM an equal
-// share of K steps, partial accumulators handed to the neighbouring CTA through global memory) was built and measured:
-// it executed the same number of instructions but ran 5-8 % slower on every shape, so it was taken out again.
+// Output tiles are dealt round-robin; where the last round fills less than two thirds of the SMs its tiles are cut along K, each
+// SM an equal share of K steps, and a small kernel adds the partial accumulators in K order (PrefillParams).
 // Every mbarrier wait is bounded; on a timeout the CTA records a status code, skips the work that
 // depended on the wait and still frees its tensor memory.
 #include <cuda.h>
@@ -44,7 +43,7 @@ struct PrefillParams {
     void* out;
     uint32_t M, N, K;
     uint32_t row_bytes;
-    uint32_t mt;      // activation rows per tile (MMA N): 64, 128 or 256
+    uint32_t mt;      // activation rows per tile (MMA N): 64, 128, 192 or 256
     uint32_t idesc;   // tcgen05 instruction descriptor
     uint32_t nkt;     // K / 64
     uint32_t ns;      // ring depth: stage s = ks decoded weight tiles in tensor memory + ks activation tiles in shared memory
@@ -454,7 +453,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const __grid_con
     const uint32_t raw_bytes = RAW_TMA ? p.nr * RAW_TILE_BYTES : 0;
     const uint32_t raw_tiles = sbase + 1024, b_tiles = raw_tiles + raw_bytes;
     // Tensor memory (all 512 columns): nacc accumulators of mt columns (two while they fit beside the weight stages,
-    // one at mt = 256), then the decoded weight tiles of 32 columns (128 rows x 64 bf16, two per column).
+    // one at mt = 192 and 256), then the decoded weight tiles of 32 columns (128 rows x 64 bf16, two per column).
     const uint32_t tmem_cols = 512, nacc = p.mt <= 128 ? 2u : 1u, a_col0 = nacc * p.mt;
 
     if (threadIdx.x == 0) {

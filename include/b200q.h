@@ -13,6 +13,10 @@
  *     default stream) and the call returns without synchronising;
  *   - weights are packed blocks, row-major [N, K] with blocks along K and no row
  *     padding (src/quant/format.rs:5-20); `w` must be 16-byte aligned;
+ *   - weights are constants: products of up to 63 rows (other than Q2_K and Q3_K) begin to read `w` while the
+ *     kernel before the call is finishing.  A weight that a KERNEL writes must be complete (its stream
+ *     synchronised) before the first such call; products of 64 rows and more, Q2_K and Q3_K products and
+ *     dequantize read it in stream order;
  *   - activations are contiguous row-major [M, K]; outputs are row-major [M, N];
  *   - every function returns a b200q_status; on failure `b200q_last_error()` gives the
  *     reason for the calling thread (the counterpart of Error::QuantError { reason },
