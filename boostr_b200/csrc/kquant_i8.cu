@@ -43,12 +43,14 @@ __host__ __device__ constexpr bool kq_wide(int fmt) { return fmt == FMT_Q4_K || 
 // 16 codes as lo + 16 hi with lo in [-8, 7] (a sum is at most 2048 in size, so hi fits a signed byte), the scale.
 template <typename InT>
 __global__ void __launch_bounds__(256) kq_act_prep_kernel(const InT* __restrict__ act, uint8_t* __restrict__ codes, uint8_t* __restrict__ mins,
-                                                          float* __restrict__ d8, size_t M, uint32_t nblk) {
+                                                          float* __restrict__ d8, size_t M, uint32_t nblk, bool early) {
     const int lane = threadIdx.x & 31;
+    // The product reads its packed weights as soon as it is started.  Q2_K and Q3_K weights may have been written by whatever ran
+    // before this kernel; those of the other formats are complete before a call of so few rows (include/b200q.h), and their
+    // product starts beside that kernel's tail: 2 us of 25 ... 36 a call.
+    if (early) grid_dep_launch();
     grid_dep_wait();  // the activations may be the previous kernel's output; the image may still be read by it
-    // In this order: the products read their packed weights as soon as they are started, and these may have been written
-    // by whatever ran before this kernel.
-    grid_dep_launch();
+    if (!early) grid_dep_launch();
     const size_t nruns = M * nblk;
     for (size_t run = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); run < nruns; run += (size_t)gridDim.x * 8) {
         float v[8];
@@ -259,7 +261,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
     __syncthreads();
     tc_after();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(smem + KO_TMEM);
-    grid_dep_launch();
+    if constexpr (!WIDE) grid_dep_launch();
     // A wait of a whole warp: all lanes leave together; on a timeout the CTA is marked dead and every role ends.
     auto wait = [&](uint32_t off, uint32_t parity, unsigned int code) {
         const bool ok = __all_sync(0xFFFFFFFFu, i8_wait(sbase + off, parity, dead));
@@ -308,6 +310,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
     } else if (warp == KT_W_ACT) {
         // ------------------------------------------------------------ activation codes, sums and scales (previous kernel's output)
         grid_dep_wait();
+        if constexpr (WIDE) grid_dep_launch();  // not before: the next product of a batch may be one that reads its weights in order
         uint32_t unit = blockIdx.x, b = 0, m0 = unit % p.nct * p.mt;
         for (uint32_t i = 0; i < total; ++i) {
             const uint32_t s = i % KT_NS, q = i % KT_NQ;
@@ -899,9 +902,10 @@ cudaError_t launch_kq_i8(int fmt, const void* act, int act_dtype, const void* w,
     if (!acts_prepared) {
         size_t grid = (M * nblk + 7) / 8;
         if (grid > (size_t)sm_count * 8) grid = (size_t)sm_count * 8;
-        e = act_dtype == DT_F32 ? launch_pdl(kq_act_prep_kernel<float>, dim3((unsigned)grid), dim3(256), 0, st, static_cast<const float*>(act), s.codes, s.mins, s.d8, M, nblk)
+        const bool early = kq_wide(fmt);
+        e = act_dtype == DT_F32 ? launch_pdl(kq_act_prep_kernel<float>, dim3((unsigned)grid), dim3(256), 0, st, static_cast<const float*>(act), s.codes, s.mins, s.d8, M, nblk, early)
                                 : launch_pdl(kq_act_prep_kernel<__nv_bfloat16>, dim3((unsigned)grid), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(act), s.codes,
-                                             s.mins, s.d8, M, nblk);
+                                             s.mins, s.d8, M, nblk, early);
         note_launch();
         if (e != cudaSuccess) return e;
     }
