@@ -21,7 +21,7 @@ LIB = os.path.join(HERE, "libb200q.so")
 HOST_LIB = os.path.join(HERE, "_hostops" + sysconfig.get_config_var("EXT_SUFFIX"))  # the name carries Python's ABI
 HOST_STAMP = os.path.join(OBJDIR, "_hostops.stamp")
 HOST_SOURCE = os.path.join(CSRC, "host_ops.cpp")
-SOURCES = ["api.cu", "dequant.cu", "gemv.cu", "gemv_m1.cu", "gemv_m1_f32.cu", "kquant_i8.cu", "prefill.cu", "smallm_i8.cu"]
+SOURCES = ["api.cu", "dequant.cu", "gemv.cu", "gemv_m1.cu", "gemv_m1_f32.cu", "kquant_few.cu", "kquant_i8.cu", "prefill.cu", "smallm_i8.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "--expt-relaxed-constexpr",

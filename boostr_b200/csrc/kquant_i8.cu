@@ -26,6 +26,9 @@
 
 namespace b200q {
 
+bool kq_few_supported(int fmt, size_t M, size_t K, size_t N);
+int kq_few_tile_rows(int fmt, size_t M, size_t K, size_t N, int sm_count);
+
 namespace {
 
 constexpr uint32_t RUN_BYTES = 292;  // of scratch per (activation row, 256-block): 256 codes, 32 bytes of sums, f32 d8
@@ -43,7 +46,7 @@ __host__ __device__ constexpr bool kq_wide(int fmt) { return fmt == FMT_Q4_K || 
 // 16 codes as lo + 16 hi with lo in [-8, 7] (a sum is at most 2048 in size, so hi fits a signed byte), the scale.
 template <typename InT>
 __global__ void __launch_bounds__(256) kq_act_prep_kernel(const InT* __restrict__ act, uint8_t* __restrict__ codes, uint8_t* __restrict__ mins,
-                                                          float* __restrict__ d8, size_t M, uint32_t nblk, bool early) {
+                                                          float* __restrict__ d8, __half* __restrict__ sums, size_t M, uint32_t nblk, bool early) {
     const int lane = threadIdx.x & 31;
     // The product reads its packed weights as soon as it is started.  Q2_K and Q3_K weights may have been written by whatever ran
     // before this kernel; those of the other formats are complete before a call of so few rows (include/b200q.h), and their
@@ -89,6 +92,7 @@ __global__ void __launch_bounds__(256) kq_act_prep_kernel(const InT* __restrict_
             const int hi = (s + 8) >> 4;
             mins[run * 32 + (lane >> 1)] = (uint8_t)(s - 16 * hi);
             mins[run * 32 + 16 + (lane >> 1)] = (uint8_t)hi;
+            if (sums) sums[run * 16 + (lane >> 1)] = __int2half_rn(s);  // at most 2048 in size: exact
         }
         const size_t m = run / nblk, b = run % nblk;
         if (lane == 0) d8[b * M + m] = __fdiv_rn(amax, 127.0f);
@@ -797,10 +801,13 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 1) kq_small_kernel(const KqSmal
 struct KqScratch {
     uint8_t *codes, *mins;
     float* d8;
+    __half* sums;  // the sums of 16 codes as f16, where kquant_few.cu may read the image too
 };
+bool kq_has_sums(size_t M, size_t K) { return M < 64 && K <= 65536; }
+size_t kq_sums_at(size_t M, size_t K) { return (M * (K / 256) * RUN_BYTES + 15) & ~(size_t)15; }
 KqScratch kq_scratch(void* ws, size_t M, size_t K) {
     uint8_t* b = static_cast<uint8_t*>(ws);
-    return {b, b + M * K, reinterpret_cast<float*>(b + M * K + M * (K / 256) * 32)};
+    return {b, b + M * K, reinterpret_cast<float*>(b + M * K + M * (K / 256) * 32), kq_has_sums(M, K) ? reinterpret_cast<__half*>(b + kq_sums_at(M, K)) : nullptr};
 }
 
 // Time of the two kernels per block of K in SM cycles, fitted to graph replays (Q2_K / Q3_K, 1024 ... 14336 weight rows): a round of
@@ -883,7 +890,31 @@ bool kq_i8_supported(int fmt, size_t M, size_t K, size_t N, int sm_count) {
     return here < 0.95 * there;
 }
 
-size_t kq_i8_workspace_bytes(size_t M, size_t K) { return (M * (K / 256) * RUN_BYTES + 255) & ~(size_t)255; }
+size_t kq_i8_workspace_bytes(size_t M, size_t K) {
+    const size_t image = M * (K / 256) * RUN_BYTES;
+    return ((kq_has_sums(M, K) ? kq_sums_at(M, K) + M * (K / 256) * 32 : image) + 255) & ~(size_t)255;
+}
+
+// Writes the image of the activations that all K-quant products of up to 63 rows (and those of Q2_K and Q3_K) read; early: the
+// product may start before this kernel's wait (kq_act_prep_kernel).
+cudaError_t launch_kq_prep(const void* act, int act_dtype, size_t M, size_t K, void* ws, bool early, int sm_count, cudaStream_t st) {
+    const KqScratch s = kq_scratch(ws, M, K);
+    const uint32_t nblk = (uint32_t)(K / 256);
+    size_t grid = (M * nblk + 7) / 8;
+    if (grid > (size_t)sm_count * 8) grid = (size_t)sm_count * 8;
+    const cudaError_t e = act_dtype == DT_F32 ? launch_pdl(kq_act_prep_kernel<float>, dim3((unsigned)grid), dim3(256), 0, st, static_cast<const float*>(act), s.codes,
+                                                           s.mins, s.d8, s.sums, M, nblk, early)
+                                              : launch_pdl(kq_act_prep_kernel<__nv_bfloat16>, dim3((unsigned)grid), dim3(256), 0, st,
+                                                           static_cast<const __nv_bfloat16*>(act), s.codes, s.mins, s.d8, s.sums, M, nblk, early);
+    note_launch();
+    return e;
+}
+void kq_image(void* ws, size_t M, size_t K, uint8_t** codes, __half** sums, float** d8) {
+    const KqScratch s = kq_scratch(ws, M, K);
+    *codes = s.codes;
+    *sums = s.sums;
+    *d8 = s.d8;
+}
 
 // acts_prepared: a previous call with the same activations and scratch left the image there (both formats read the same).
 cudaError_t launch_kq_i8(int fmt, const void* act, int act_dtype, const void* w, void* out, int out_dtype, size_t M, size_t K, size_t N, void* ws,
@@ -900,13 +931,7 @@ cudaError_t launch_kq_i8(int fmt, const void* act, int act_dtype, const void* w,
     const uint32_t nblk = (uint32_t)(K / 256);
     cudaError_t e;
     if (!acts_prepared) {
-        size_t grid = (M * nblk + 7) / 8;
-        if (grid > (size_t)sm_count * 8) grid = (size_t)sm_count * 8;
-        const bool early = kq_wide(fmt);
-        e = act_dtype == DT_F32 ? launch_pdl(kq_act_prep_kernel<float>, dim3((unsigned)grid), dim3(256), 0, st, static_cast<const float*>(act), s.codes, s.mins, s.d8, M, nblk, early)
-                                : launch_pdl(kq_act_prep_kernel<__nv_bfloat16>, dim3((unsigned)grid), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(act), s.codes,
-                                             s.mins, s.d8, M, nblk, early);
-        note_launch();
+        e = launch_kq_prep(act, act_dtype, M, K, ws, kq_wide(fmt), sm_count, st);
         if (e != cudaSuccess) return e;
     }
     const KqPlan plan = kq_plan(fmt, M, K, N, sm_count);
@@ -959,6 +984,7 @@ cudaError_t launch_kq_i8(int fmt, const void* act, int act_dtype, const void* w,
 // Activation rows of the tensor-core tile that a product takes (0: the kernel for few rows, -1: another path).  Not part of
 // the C ABI: the tests hold their shapes to the tiles that they are meant for.
 extern "C" __attribute__((visibility("default"))) int b200q_kq_tile_rows(int fmt, size_t M, size_t K, size_t N, int sm_count) {
+    if (b200q::kq_few_supported(fmt, M, K, N)) return b200q::kq_few_tile_rows(fmt, M, K, N, sm_count);
     if (!b200q::kq_i8_supported(fmt, M, K, N, sm_count)) return -1;
     return (int)b200q::kq_plan(fmt, M, K, N, sm_count).mt;
 }

@@ -1,0 +1,91 @@
+"""The K-quant kernel for 17 ... 63 activation rows (csrc/kquant_few.cu) against the CPU oracle: the CPU's bits up to K = 4096
+(blocks added in K order also where a cluster shares a tile), 2e-6 of the largest result beyond, where the shares of a cluster
+are added as sums (the grouping of at most 64 f32 terms)."""
+import os
+
+import numpy as np
+import pytest
+
+from boostr_b200 import synth
+from boostr_b200.format import QuantFormat as F
+from boostr_b200.tensor import QuantTensor
+from util import describe_mismatch, rel_err, seed_of
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+# tiles of 16, 32, 48 activation rows and two of them, one and several blocks, clusters of 2, 4, 8 and whole tiles, weight rows
+# around multiples of 128, Q6_K rows of every alignment
+SHAPES = [(17, 1, 256), (18, 129, 512), (31, 127, 768), (20, 1000, 4096), (17, 256, 1280), (32, 2500, 2048), (33, 300, 3840), (48, 1300, 4096),
+          (49, 128, 512), (63, 4100, 1024), (19, 20000, 512), (32, 19100, 256), (40, 19000, 1536), (37, 700, 14336), (24, 4096, 4352), (63, 900, 8192)]
+
+
+@pytest.mark.parametrize("fmt", ["Q4_K", "Q5_K", "Q6_K"])
+@pytest.mark.parametrize("m,n,k", SHAPES)
+def test_products(oracle, fmt, m, n, k):
+    from boostr_b200 import ops
+
+    rng = synth.rng_for(101, seed_of(fmt, m, n, k))
+    act = synth.activations(rng, m, k)
+    act[m // 2] *= 1e-3  # rows of different scale
+    act[0, :256] = 0.0   # a block without a maximum
+    w = synth.weight_bytes(fmt, rng, n, k)
+    guard = 4096
+    flat = torch.full((2 * guard + m * n,), 4242.0, device="cuda")
+    out = flat[guard:guard + m * n].view(m, n)
+    x, qt = torch.from_numpy(act).cuda(), QuantTensor.from_bytes(w, F[fmt], (n, k), device="cuda")
+    ops.quant_matmul(x, qt, out=out)
+    ops.check_device_status()
+    got = out.cpu().numpy()
+    assert (flat[:guard] == 4242.0).all() and (flat[guard + m * n:] == 4242.0).all(), "guard regions were written"
+    want = oracle.quant_matmul(fmt, act, w, n, threads=os.cpu_count() or 8)
+    if k <= 4096:
+        assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), describe_mismatch(got, want)
+    else:
+        assert rel_err(got, want)[0] <= 2e-6, describe_mismatch(got, want)
+    for _ in range(20):
+        again = ops.quant_matmul(x, qt)
+    assert torch.equal(again.view(torch.int32), out.view(torch.int32))
+    ops.check_device_status()
+
+
+@pytest.mark.parametrize("fmt", ["Q4_K", "Q5_K", "Q6_K"])
+@pytest.mark.parametrize("fill", [0xFF, 0x00, 0xF0, 0x0F, 0x80, 0x7F])
+def test_largest_sums(oracle, fmt, fill):
+    """Every code, scale and min at an end of its range, activations of one sign and of alternating ones."""
+    from boostr_b200 import ops
+
+    m, n, k = 48, 140, 1024
+    w = np.full((n * k // 256, F[fmt].block_bytes), fill, np.uint8)
+    for at in (208,) if fmt == "Q6_K" else (0, 2):
+        w[:, at:at + 2] = np.frombuffer(np.array([1.0], np.float16).tobytes(), np.uint8)
+    act = np.ones((m, k), np.float32)
+    act[1::3] = -1.0
+    act[2::3, ::2] = -1.0
+    w = w.reshape(-1)
+    for rows in (20, m):
+        got = ops.quant_matmul(torch.from_numpy(act[:rows]).cuda(), QuantTensor.from_bytes(w, F[fmt], (n, k), device="cuda")).cpu().numpy()
+        want = oracle.quant_matmul(fmt, act[:rows], w, n, threads=4)
+        assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), describe_mismatch(got, want)
+    ops.check_device_status()
+
+
+@pytest.mark.parametrize("fmt", ["Q4_K", "Q5_K", "Q6_K"])
+@pytest.mark.parametrize("m,n,k", [(18, 65, 512), (24, 9500, 1280), (33, 500, 4096), (20, 1000, 5120)])
+def test_swiglu(fmt, m, n, k):
+    """silu(gate) * up of the two products, to the rounding of one f32 expression."""
+    from boostr_b200 import ops
+
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(seed_of(fmt, m, n, k))
+    g, u = synth.device_weight(fmt, n, k, gen), synth.device_weight(fmt, n, k, gen)
+    x = torch.randn(m, k, device="cuda", generator=gen)
+    a, b = ops.quant_matmul(x, g).double(), ops.quant_matmul(x, u).double()
+    got = ops.quant_swiglu(x, g, u)
+    ops.check_device_status()
+    want = a / (1 + torch.exp(-a)) * b
+    # K <= 4096: the same products; expf within 2 ulp, three more roundings (4 * 2^-23); beyond, other shares of K (2e-6 of the largest)
+    if k <= 4096:
+        assert ((got.double() - want).abs() <= 5e-7 * want.abs() + 1e-36 * b.abs()).all()
+    else:
+        assert (got.double() - want).abs().max() <= 1e-5 * want.abs().max()
