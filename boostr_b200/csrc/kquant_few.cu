@@ -1,4 +1,4 @@
-// Quantized matmul of the K-quants for 17 ... 63 activation rows with the bits of boostr's CPU path
+// Quantized matmul of the K-quants for 9 ... 63 activation rows with the bits of boostr's CPU path
 // (src/quant/cpu/kernels/quant_matmul.rs:107-135): activations quantised to Q8_K (quantize_act_q8k.rs:26-98), per 256-block
 // (d * d8) * isum - (dmin * d8) * summs with exact integer sums (fused_q4k_q8k_dot.rs:111-172, fused_q5k_q8k_dot.rs:27-122,
 // fused_q6k_q8k_dot.rs:27-154 under src/quant/cpu/kernels/simd; Q6_K has no min term), blocks added in K order.
@@ -37,6 +37,7 @@
 
 namespace b200q {
 
+bool smallm_i8_preferred(int fmt, size_t M, size_t K, size_t N, int sm_count);
 size_t kq_i8_workspace_bytes(size_t M, size_t K);
 cudaError_t launch_kq_prep(const void* act, int act_dtype, size_t M, size_t K, void* ws, bool early, int sm_count, cudaStream_t st);
 void kq_image(void* ws, size_t M, size_t K, uint8_t** codes, __half** sums, float** d8);
@@ -604,6 +605,7 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
 struct KfPlan {
     uint32_t mt = 0, cs = 1;
     bool terms = false;
+    double us = 0;  // expected time behind the first block
 };
 constexpr uint32_t KF_SMEM = 232448;
 uint32_t kf_x_bytes(const KfPlan& pl, uint32_t nblk, bool swiglu) {
@@ -656,13 +658,13 @@ uint32_t kf_clusters(uint32_t cs) {
 }
 
 // Tile and cluster of least time, in us: blocks of K one after the other x the time of one (a line in mt, measured at 14336 x
-// 4096: 16 / 32 / 48 rows Q4_K 0.86 / 0.99 / 1.14, Q5_K 1.02 / 1.18 / 1.32, Q6_K 1.31 / 1.37 / 1.45), and 3.4 for the meeting of a
+// 4096: 16 / 32 / 48 rows Q4_K 0.86 / 0.99 / 1.14, Q5_K 1.02 / 1.18 / 1.32, Q6_K 1.31 / 1.37 / 1.45, or 1.97 where
+// its rows are no multiple of 16 bytes: 13825 x 5120), and 3.4 for the meeting of a
 // cluster (2048 x 2048 and 4096 x 4096 against whole tiles).
-KfPlan kf_plan(int fmt, size_t M, size_t K, size_t row_tiles, bool swiglu, int sm_count) {
+KfPlan kf_plan(int fmt, size_t M, size_t K, size_t row_tiles, bool swiglu, int sm_count, bool estimate = false) {
     KfPlan best;
     const uint32_t nblk = (uint32_t)(K / 256);
-    const double c0 = fmt == FMT_Q4_K ? 0.72 : fmt == FMT_Q5_K ? 0.87 : 1.24, c1 = fmt == FMT_Q4_K ? 0.0088 : fmt == FMT_Q5_K ? 0.0094 : 0.0044;
-    double best_cost = 0;
+    const double c0 = fmt == FMT_Q4_K ? 0.72 : fmt == FMT_Q5_K ? 0.87 : nblk % 8 ? 1.9 : 1.24, c1 = fmt == FMT_Q4_K ? 0.0088 : fmt == FMT_Q5_K ? 0.0094 : 0.0044;
     for (uint32_t mt = 16; mt <= KF_MT_MAX; mt += 16) {
         const size_t units = row_tiles * ((M + mt - 1) / mt);
         for (uint32_t cs = 1; cs <= 8 && cs <= nblk; cs *= 2) {
@@ -670,13 +672,10 @@ KfPlan kf_plan(int fmt, size_t M, size_t K, size_t row_tiles, bool swiglu, int s
             c.mt = mt;
             c.cs = cs;
             c.terms = cs > 1 && nblk <= 16;
-            if (cs > 1 && (units > kf_clusters(cs) || kf_ring(fmt, c, nblk, swiglu) < 2)) continue;
+            if (cs > 1 && (units * cs > (size_t)sm_count || kf_ring(fmt, c, nblk, swiglu) < 2 || (!estimate && units > kf_clusters(cs)))) continue;
             const size_t blocks = cs > 1 ? (nblk + cs - 1) / cs : (units + sm_count - 1) / sm_count * nblk;
-            const double cost = (double)blocks * (c0 + c1 * mt) + (cs > 1 ? 3.4 : 0.0);
-            if (!best.mt || cost < best_cost) {
-                best = c;
-                best_cost = cost;
-            }
+            c.us = (double)blocks * (c0 + c1 * mt) + (cs > 1 ? 3.4 : 0.0);
+            if (!best.mt || c.us < best.us) best = c;
         }
         if (mt >= M) break;
     }
@@ -716,11 +715,21 @@ cudaError_t kf_launch(const CUtensorMap& am, const CUtensorMap& sm, const CUtens
 }  // namespace
 
 // From 17 rows on one pass here beats passes of 16 rows by mma.sync (gemv.cu); of 91 products between 24 and 63 rows two are 1 ... 2 %
-// slower (1024 x 4096 at 24 rows, Q5_K 11.25 -> 11.4 us, Q6_K 11.55 -> 11.8), the mean takes 0.69 of the time.  At 16 rows the two are about
-// even (14336 x 4096: Q4_K 16.3 there, 17.7 here; Q5_K 23.3, 20.4; Q6_K 24.2, 25.0), at 8 rows mma.sync is 1.1 ... 1.9 times as fast.
-bool kq_few_supported(int fmt, size_t M, size_t K, size_t N) {
-    return (fmt == FMT_Q4_K || fmt == FMT_Q5_K || fmt == FMT_Q6_K) && M >= 17 && M < 64 && K >= 256 && K % 256 == 0 && K <= 65536 && N >= 1 &&
-           N <= (1u << 22) && tma_available();
+// slower (1024 x 4096 at 24 rows, Q5_K 11.25 -> 11.4 us, Q6_K 11.55 -> 11.8), the mean takes 0.69 of the time.  At 9 ... 16 rows the two are
+// even on most shapes (14336 x 4096 at 16 rows: Q6_K 24.2 there, 25.0 here) and this kernel wins where the other's fixed shares of K (chunks of 16
+// blocks; 5 + 0.13 ... 0.155 us a tile of 128 rows and chunk) are badly filled: 13825 x 5120 at 13 rows Q4_K 30.6 -> 21.1, Q5_K 34.9 -> 24.4; 14336 x
+// 2048 Q5_K 20.1 -> 12.4, Q6_K 20.1 -> 14.3; SwiGLU 2 x 5632 x 2048 17.8 -> 12.4, 20.7 -> 14.0, 19.5 -> 14.9.  Up to 8 rows mma.sync is 1.1 ... 1.9 times as fast.
+bool kq_few_supported(int fmt, size_t M, size_t K, size_t N, bool swiglu, int sm_count) {
+    if ((fmt != FMT_Q4_K && fmt != FMT_Q5_K && fmt != FMT_Q6_K) || M < 9 || M >= 64 || K < 256 || K % 256 != 0 || K > 65536 || N < 1 || N > (1u << 22) ||
+        !tma_available())
+        return false;
+    if (M >= 17) return true;
+    if (smallm_i8_preferred(fmt, M, K, N, sm_count)) return false;
+    const size_t nblk = K / 256, tiles = (N + 127) / 128 * (swiglu ? 2 : 1);
+    const double there = 5.0 + (double)(tiles * ((nblk + 15) / 16)) * (fmt == FMT_Q4_K ? 0.128 : fmt == FMT_Q5_K ? 0.155 : 0.13);
+    const size_t row_tiles = swiglu ? (N + 63) / 64 : (N + 127) / 128;
+    // (the estimate spares shapes that stay with the other kernel the question how many clusters fit, which loads this one)
+    return 4.0 + kf_plan(fmt, M, K, row_tiles, swiglu, sm_count, true).us < 0.95 * there && 4.0 + kf_plan(fmt, M, K, row_tiles, swiglu, sm_count).us < 0.95 * there;
 }
 int kq_few_tile_rows(int fmt, size_t M, size_t K, size_t N, int sm_count) { return (int)kf_plan(fmt, M, K, (N + 127) / 128, false, sm_count).mt; }
 

@@ -26,7 +26,7 @@
 
 namespace b200q {
 
-bool kq_few_supported(int fmt, size_t M, size_t K, size_t N);
+bool kq_few_supported(int fmt, size_t M, size_t K, size_t N, bool swiglu, int sm_count);
 int kq_few_tile_rows(int fmt, size_t M, size_t K, size_t N, int sm_count);
 
 namespace {
@@ -984,7 +984,7 @@ cudaError_t launch_kq_i8(int fmt, const void* act, int act_dtype, const void* w,
 // Activation rows of the tensor-core tile that a product takes (0: the kernel for few rows, -1: another path).  Not part of
 // the C ABI: the tests hold their shapes to the tiles that they are meant for.
 extern "C" __attribute__((visibility("default"))) int b200q_kq_tile_rows(int fmt, size_t M, size_t K, size_t N, int sm_count) {
-    if (b200q::kq_few_supported(fmt, M, K, N)) return b200q::kq_few_tile_rows(fmt, M, K, N, sm_count);
+    if (b200q::kq_few_supported(fmt, M, K, N, false, sm_count)) return b200q::kq_few_tile_rows(fmt, M, K, N, sm_count);
     if (!b200q::kq_i8_supported(fmt, M, K, N, sm_count)) return -1;
     return (int)b200q::kq_plan(fmt, M, K, N, sm_count).mt;
 }
