@@ -44,7 +44,7 @@ size_t prefill_workspace_bytes(int fmt, int act_dtype, size_t M, size_t K, size_
 cudaError_t launch_prefill(int fmt, const void* act, int act_dtype, const void* w, void* out, int out_dtype, size_t M,
                            size_t K, size_t N, void* ws, size_t ws_bytes, int sm_count, cudaStream_t st,
                            unsigned int* status, bool* ws_too_small, char* err, size_t err_len, bool acts_prepared);
-bool kq_i8_supported(int fmt, size_t M, size_t K, size_t N, int sm_count);
+bool kq_i8_supported(int fmt, size_t M, size_t K, size_t N);
 size_t kq_i8_workspace_bytes(size_t M, size_t K);
 cudaError_t launch_kq_i8(int fmt, const void* act, int act_dtype, const void* w, void* out, int out_dtype, size_t M, size_t K,
                              size_t N, void* ws, size_t ws_bytes, int sm_count, cudaStream_t st, unsigned int* status,
@@ -179,7 +179,7 @@ size_t workspace_need(int op, int format, int act_dtype, size_t M, size_t K, siz
     if (!known_format(format) || M == 0 || K == 0 || N == 0 || K % fmt_block_size(format)) return 0;
     const bool swiglu = op == B200Q_OP_QUANT_SWIGLU;
     if (kq_few_supported(format, M, K, N, swiglu, sm_count_current())) return kq_i8_workspace_bytes(M, K);  // the Q8_K image
-    if (kq_i8_supported(format, M, K, N, sm_count_current()))  // the Q8_K image (+ gate and up for SwiGLU)
+    if (kq_i8_supported(format, M, K, N))  // the Q8_K image (+ gate and up for SwiGLU)
         return kq_i8_workspace_bytes(M, K) + (swiglu ? 2 * ((M * N * sizeof(float) + 255) & ~(size_t)255) : 0);
     if (prefill_supported(format, M, K, N)) {
         size_t a = prefill_workspace_bytes(format, act_dtype, M, K, N, sm_count_current());
@@ -231,7 +231,7 @@ cudaError_t launch_i8_passes(int format, const void* act, int act_dtype, const v
 // (K-quants: Q8_K round trip; others: bf16);
 // the mma.sync small-M kernel one image per format (Q5_K reads Q4_K's).
 int prepared_class(int format, size_t M, size_t K, size_t N) {
-    if (kq_few_supported(format, M, K, N, false, sm_count_current()) || kq_i8_supported(format, M, K, N, sm_count_current()))
+    if (kq_few_supported(format, M, K, N, false, sm_count_current()) || kq_i8_supported(format, M, K, N))
         return M <= 32 || format == FMT_Q2_K || format == FMT_Q3_K || format == FMT_Q5_K ? 102 : -1;
     if (prefill_supported(format, M, K, N)) return (format == FMT_Q4_K || format == FMT_Q5_K || format == FMT_Q6_K) ? 101 : 100;
     if (gemv_m1_supported(format, M, K, N, false) || gemv_m1_f32_supported(format, M, K, N)) return -1;
@@ -255,7 +255,7 @@ int quant_matmul_impl(int format, const void* act, int act_dtype, const void* w,
         e = launch_kq_few(format, act, act_dtype, 1, &w, &out, &N, false, out_dtype, M, K, ws, ws_bytes, sm_count_current(), st, status, &small, msg, sizeof(msg),
                           acts_prepared);
         if (e != cudaSuccess && msg[0]) return fail(B200Q_ERR_CUDA, "quant_matmul: %s", msg);
-    } else if (kq_i8_supported(format, M, K, N, sm_count_current())) {
+    } else if (kq_i8_supported(format, M, K, N)) {
         char msg[256] = "";
         e = launch_kq_i8(format, act, act_dtype, w, out, out_dtype, M, K, N, ws, ws_bytes, sm_count_current(), st, status, &small, msg, sizeof(msg),
                              acts_prepared);
@@ -452,7 +452,7 @@ int b200q_quant_swiglu(int format, const void* act, int act_dtype, const void* w
         const size_t nn[2] = {N, N};
         e = launch_kq_few(format, act, act_dtype, 2, ww, oo, nn, true, out_dtype, M, K, ws, ws_bytes, sm_count_current(), st, status, &small, msg, sizeof(msg), false);
         if (e != cudaSuccess && msg[0]) return fail(B200Q_ERR_CUDA, "quant_swiglu: %s", msg);
-    } else if (kq_i8_supported(format, M, K, N, sm_count_current())) {
+    } else if (kq_i8_supported(format, M, K, N)) {
         // two products into f32 scratch (the second reads the first one's Q8_K image), then the gate
         const size_t mn = (M * N * sizeof(float) + 255) & ~(size_t)255;
         float* g = static_cast<float*>(ws);

@@ -720,7 +720,7 @@ cudaError_t kf_launch(const CUtensorMap& am, const CUtensorMap& sm, const CUtens
 // blocks; 5 + 0.13 ... 0.155 us a tile of 128 rows and chunk) are badly filled: 13825 x 5120 at 13 rows Q4_K 30.6 -> 21.1, Q5_K 34.9 -> 24.4; 14336 x
 // 2048 Q5_K 20.1 -> 12.4, Q6_K 20.1 -> 14.3; SwiGLU 2 x 5632 x 2048 17.8 -> 12.4, 20.7 -> 14.0, 19.5 -> 14.9.  Up to 8 rows mma.sync is 1.1 ... 1.9 times as fast.
 bool kq_few_supported(int fmt, size_t M, size_t K, size_t N, bool swiglu, int sm_count) {
-    if ((fmt != FMT_Q4_K && fmt != FMT_Q5_K && fmt != FMT_Q6_K) || M < 9 || M >= 64 || K < 256 || K % 256 != 0 || K > 65536 || N < 1 || N > (1u << 22) ||
+    if ((fmt != FMT_Q4_K && fmt != FMT_Q5_K && fmt != FMT_Q6_K) || M < 9 || M >= 64 || K < 256 || K % 256 != 0 || K > 65536 || N < 1 ||
         !tma_available())
         return false;
     if (M >= 17) return true;

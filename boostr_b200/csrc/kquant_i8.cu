@@ -1,19 +1,19 @@
 // Quantized matmul of the K-quant formats with the bits of boostr's CPU path
 // (src/quant/cpu/kernels/quant_matmul.rs:107-135) on the integer tensor cores: Q2_K and Q3_K for every number of activation
-// rows, Q4_K and Q5_K between the kernels for few rows and the bf16 path.  Each activation row is quantised to Q8_K
+// rows (Q4_K, Q5_K and Q6_K with few rows: kquant_few.cu, which reads the same image).  Each activation row is quantised to Q8_K
 // (src/quant/cpu/kernels/simd/quantize_act_q8k.rs:26-98), a 256-block contributes
 // (d * d8) * isum - (dmin * d8) * summs with exact integer sums (src/quant/cpu/kernels/simd/fused_q2k_q8k_dot.rs:152-214,
-// fused_q3k_q8k_dot.rs:33-205, fused_q4k_q8k_dot.rs:111-172, fused_q5k_q8k_dot.rs:27-122 in the form x86-64 runs; Q3_K has
-// no min term) and the blocks are added in K order without FMA contraction.
+// fused_q3k_q8k_dot.rs:33-205 in the form x86-64 runs; Q3_K has no min term) and the blocks are added in K order without FMA contraction.
 //
 // What both kernels build on: the PRODUCT of a code and its sub-block's scale goes into the operand, so a whole 256-block is
 // one K = 256 integer product and only one sum per (row, activation row, block) has to be scaled.  For Q2_K (0..3 times
 // 0..15) and Q3_K (-(-4..3) times -32..31 lies in [-128, 124]; the sign is given back by the f32 factor) it fits a signed
-// byte; for Q4_K and Q5_K (below 2048) it is lo + 128 hi, two operands.  The min term is another integer product, of the
-// mins with the activation's sums of 16 codes, which travel as two bytes, sum = lo + 16 hi.
+// byte.  The min term is another integer product, of the mins with the activation's sums of 16 codes, which travel as two
+// bytes, sum = lo + 16 hi.
 //
-//   * kq_act_prep_kernel: codes [M][K], min operand [M][K / 256][lo 16 | hi 16], scales d8 [K / 256][M]: 292 bytes per run;
-//   * kq_tc_kernel<FMT>: tcgen05.mma.kind::i8, tiles of 128 weight rows x up to 128 (Q4_K, Q5_K: 48) activation rows;
+//   * kq_act_prep_kernel: codes [M][K], min operand [M][K / 256][lo 16 | hi 16], scales d8 [K / 256][M]: 292 bytes per run; below
+//     64 rows the sums of 16 also as f16, for kquant_few.cu;
+//   * kq_tc_kernel<FMT>: tcgen05.mma.kind::i8, tiles of 128 weight rows x up to 128 activation rows;
 //   * kq_small_kernel<FMT, NT>: mma.sync, slabs of 16 weight rows x 8 NT activation rows, Q2_K / Q3_K with few rows.
 #include <cuda.h>
 
@@ -37,10 +37,8 @@ constexpr uint32_t RUN_BYTES = 292;  // of scratch per (activation row, 256-bloc
 // CHUNKS at most, PITCH bytes from row to row in shared memory.  (Copies of 4 bytes - cp.async - ran at about one lane per
 // cycle and took 2-4 us per 128 rows, more than everything else.)  Any such pitch puts one word of 32 rows into eight banks:
 // 112 and 144 use all of these.
-// (Rows of Q4_K and Q5_K are whole chunks and always come by TMA.)
 __host__ __device__ constexpr uint32_t kq_chunks(int fmt) { return fmt == FMT_Q2_K ? 6 : 8; }
-__host__ __device__ constexpr uint32_t kq_pitch(int fmt) { return fmt == FMT_Q2_K ? 112 : fmt == FMT_Q5_K ? 176 : 144; }
-__host__ __device__ constexpr bool kq_wide(int fmt) { return fmt == FMT_Q4_K || fmt == FMT_Q5_K; }  // two-byte products
+__host__ __device__ constexpr uint32_t kq_pitch(int fmt) { return fmt == FMT_Q2_K ? 112 : 144; }
 
 // One warp per (activation row, 256-block): Q8_K codes (d = amax / 127, id = 127 / amax, round half to even), the sums of
 // 16 codes as lo + 16 hi with lo in [-8, 7] (a sum is at most 2048 in size, so hi fits a signed byte), the scale.
@@ -117,13 +115,6 @@ __device__ __forceinline__ uint32_t q3k_scaled(uint32_t w, uint32_t hw, uint32_t
     const uint32_t c = ((w >> (2 * G)) & 0x03030303u) | high;
     return (c * neg_s + u4) ^ 0x80808080u;
 }
-// Q4_K, Q5_K: four codes (below 32) times 2 sc (sc below 64) in 16-bit lanes; the high bytes are the products' hi = p >> 7, the
-// low bytes 2 lo, all even, so that one shift of the word halves them in place.
-__device__ __forceinline__ void wide_scaled(uint32_t c, uint32_t sc2, uint32_t& lo, uint32_t& hi) {
-    const uint32_t pe = (c & 0x00FF00FFu) * sc2, po = __byte_perm(c, 0u, 0x4341) * sc2;
-    hi = __byte_perm(pe, po, 0x7351);
-    lo = __byte_perm(pe, po, 0x6240) >> 1;
-}
 __device__ __forceinline__ uint32_t byte_of(uint32_t x, uint32_t i) { return __byte_perm(x, 0u, 0x4440u | i); }
 
 __device__ __forceinline__ void store_as(void* out, int dt, size_t idx, float v) {
@@ -166,13 +157,12 @@ __device__ __forceinline__ void copy_rows(uint32_t dst, const uint8_t* blk, uint
 // no tile is cut).  Per 256-block: the 128 packed blocks come by TMA (by cp.async from two warps where rows are not 16-byte aligned),
 // two sets of four decode warps, taking the blocks in turn, write the scaled codes as 128-byte-swizzled K-major operand tiles,
 // the activation codes come by TMA, one thread issues 8 MMAs
-// (16 for two-byte products; + 2 for the mins) into one of two accumulators, and sixteen drain warps (thread = weight
+// (+ 2 for the mins) into one of two accumulators, and sixteen drain warps (thread = weight
 // row x every fourth group of 8 activation rows) scale the sums and add them to their registers.
 // What bounds it: with 128 activation rows a tile the issue slots (Q2_K 72 %, Q3_K 67 % busy; ALU pipe 41 / 55 %, tensor pipe
 // 20 / 18 %): decode, and 8 (Q2_K) or 5 (Q3_K) instructions a sum of drain; with few the latency of a block's chain through
-// the barriers, the proxy fence and two decode sets (two-byte products: issue slots 60 ... 64 %, ALU pipe 51 ... 54 %), 0.8 us (Q2_K,
-// Q3_K) to 1.2 us (two-byte products) a block.  Measured: 512 rows x 14336 x 4096 Q2_K 99 us, Q3_K 93 us (a layer of such
-// products 0.42 ms; 69 ms with a kernel that took eight rows at a time); Q5_K 37 rows 28 us.  Tried and not kept: packed f32x2
+// the barriers, the proxy fence and two decode sets, 0.8 us a block.  Measured: 512 rows x 14336 x 4096 Q2_K 99 us, Q3_K 93 us (a layer of such
+// products 0.42 ms; 69 ms with a kernel that took eight rows at a time).  Tried and not kept: packed f32x2
 // arithmetic in the drain, which suits one format and not the other (Q2_K 107, Q3_K 87 us) and needs an operand hidden from
 // the assembler, which else makes one rounding of mul.rn.f32x2 and add.rn.f32x2; and halves of a block as stages
 // (4096 x 14336 at 64 rows 49 -> 58 us).
@@ -194,21 +184,21 @@ constexpr int KT_DEC = 8, KT_DRAIN = 16, KT_COPY = 2;
 constexpr int KT_W_COPY = KT_DEC + KT_DRAIN, KT_W_ACT = KT_W_COPY + KT_COPY, KT_W_MMA = KT_W_ACT + 1;
 constexpr int KT_THREADS = (KT_W_MMA + 1) * 32;
 constexpr uint32_t KT_NS = 2, KT_NQ = 4;
-__host__ __device__ constexpr uint32_t kt_nr(int fmt) { return kq_wide(fmt) ? 2 : 4; }
+constexpr uint32_t KT_NR = 4;
 constexpr uint32_t KT_ATOM = 128 * 128;
 constexpr uint32_t KT_REC = 512 + 512;  // the rows' d | dmin, the activation rows' d8
 // Every ring has an even depth: the decode sets take the blocks in turn, so a slot belongs to one set, which sees every
 // phase of the slot's barriers (a parity wait cannot tell phase k from k - 2).
 constexpr int KO_FULL = 0, KO_EMPTY = 32, KO_RAW_FULL = 64, KO_RAW_EMPTY = 96, KO_ACC_FULL = 128, KO_ACC_EMPTY = 144, KO_REC_FULL = 160,
               KO_REC_EMPTY = 192, KO_TMEM = 224, KO_DEAD = 228, KO_RECS = 1024, KO_STAGES = KO_RECS + KT_NQ * KT_REC;
-// a stage: two operand tiles of scaled codes (four of two-byte products) | tile of mins | two tiles of activation codes | sums of 16
-__host__ __device__ constexpr uint32_t kt_mt_max(int fmt) { return kq_wide(fmt) ? 48 : 128; }
+// a stage: two operand tiles of scaled codes | tile of mins | two tiles of activation codes | sums of 16
+constexpr uint32_t KT_MT_MAX = 128;
 __host__ __device__ constexpr uint32_t kt_stage(int fmt) {
-    return ((kq_wide(fmt) ? 4 : 2) * KT_ATOM + (fmt == FMT_Q3_K ? 0 : 128 * 64) + kt_mt_max(fmt) * (256 + (fmt == FMT_Q3_K ? 0 : 32)) + 1023) / 1024 * 1024;
+    return (2 * KT_ATOM + (fmt == FMT_Q3_K ? 0 : 128 * 64) + KT_MT_MAX * (256 + (fmt == FMT_Q3_K ? 0 : 32)) + 1023) / 1024 * 1024;
 }
 __host__ __device__ constexpr uint32_t kt_raw(int fmt) { return 128 * kq_pitch(fmt); }
-__host__ __device__ constexpr size_t kt_smem(int fmt) { return 1024 + KO_STAGES + KT_NS * kt_stage(fmt) + kt_nr(fmt) * kt_raw(fmt); }
-static_assert(KO_STAGES % 1024 == 0 && kt_smem(FMT_Q2_K) <= 232448 && kt_smem(FMT_Q3_K) <= 232448 && kt_smem(FMT_Q5_K) <= 232448, "shared memory");
+__host__ __device__ constexpr size_t kt_smem(int fmt) { return 1024 + KO_STAGES + KT_NS * kt_stage(fmt) + KT_NR * kt_raw(fmt); }
+static_assert(KO_STAGES % 1024 == 0 && kt_smem(FMT_Q2_K) <= 232448 && kt_smem(FMT_Q3_K) <= 232448, "shared memory");
 
 // rows of 64 bytes with 64-byte swizzle (8-row groups 512 bytes apart) and of 32 bytes with 32-byte swizzle
 __device__ __forceinline__ uint64_t desc_sw64(uint32_t lo) {
@@ -225,12 +215,12 @@ __device__ __forceinline__ uint64_t desc_sw32(uint32_t lo) {
 template <int FMT>
 __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant__ CUtensorMap tmap_min,
                                                               const __grid_constant__ CUtensorMap tmap_w, const KqTcParams p) {
-    constexpr bool MIN = FMT != FMT_Q3_K, WIDE = kq_wide(FMT);
-    constexpr uint32_t BB = fmt_block_bytes(FMT), PITCH = kq_pitch(FMT), RAW = kt_raw(FMT), STAGE = kt_stage(FMT), NR = kt_nr(FMT);
-    constexpr uint32_t MT_MAX = kt_mt_max(FMT), B_TILE = MT_MAX * 128, CHUNKS = (MT_MAX / 8 + 3) / 4;  // groups of 8 activation rows of a drain warp
-    constexpr uint32_t OFF_AM = (WIDE ? 4 : 2) * KT_ATOM, OFF_B = OFF_AM + (MIN ? 128 * 64 : 0), OFF_BM = OFF_B + 2 * B_TILE;
-    // an accumulator: sums | mins (Q2_K); lo | hi | mins . lo | mins . hi (two-byte products)
-    constexpr uint32_t COL = WIDE ? 64 : 128, ACC_COLS = WIDE ? 256 : MIN ? 256 : 128, TMEM_COLS = 2 * ACC_COLS;
+    constexpr bool MIN = FMT != FMT_Q3_K;
+    constexpr uint32_t BB = fmt_block_bytes(FMT), PITCH = kq_pitch(FMT), RAW = kt_raw(FMT), STAGE = kt_stage(FMT), NR = KT_NR;
+    constexpr uint32_t MT_MAX = KT_MT_MAX, B_TILE = MT_MAX * 128, CHUNKS = (MT_MAX / 8 + 3) / 4;  // groups of 8 activation rows of a drain warp
+    constexpr uint32_t OFF_AM = 2 * KT_ATOM, OFF_B = OFF_AM + (MIN ? 128 * 64 : 0), OFF_BM = OFF_B + 2 * B_TILE;
+    // an accumulator: sums (| mins)
+    constexpr uint32_t COL = 128, ACC_COLS = MIN ? 256 : 128, TMEM_COLS = 2 * ACC_COLS;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);  // the launch reserves 1 KB of slack
     const uint32_t sbase = smem_u32(smem), st_base = sbase + KO_STAGES;
@@ -265,7 +255,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
     __syncthreads();
     tc_after();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(smem + KO_TMEM);
-    if constexpr (!WIDE) grid_dep_launch();
+    grid_dep_launch();
     // A wait of a whole warp: all lanes leave together; on a timeout the CTA is marked dead and every role ends.
     auto wait = [&](uint32_t off, uint32_t parity, unsigned int code) {
         const bool ok = __all_sync(0xFFFFFFFFu, i8_wait(sbase + off, parity, dead));
@@ -298,7 +288,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
                                      : "memory");
                     }
                 }
-            } else if constexpr (!WIDE) {
+            } else {
                 copy_rows<FMT, 128 / KT_COPY>(sbase + OFF_RAW + rs * RAW + r0 * PITCH, p.w + (size_t)n0 * p.row_bytes + (size_t)b * BB, p.row_bytes, lane,
                                               n0 + 128 / KT_COPY < p.N, n0 < p.N ? p.N - n0 : 0u, wend);
             }
@@ -314,7 +304,6 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
     } else if (warp == KT_W_ACT) {
         // ------------------------------------------------------------ activation codes, sums and scales (previous kernel's output)
         grid_dep_wait();
-        if constexpr (WIDE) grid_dep_launch();  // not before: the next product of a batch may be one that reads its weights in order
         uint32_t unit = blockIdx.x, b = 0, m0 = unit % p.nct * p.mt;
         for (uint32_t i = 0; i < total; ++i) {
             const uint32_t s = i % KT_NS, q = i % KT_NQ;
@@ -355,17 +344,13 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
             tc_after();
             if (elect_one_lane()) {
 #pragma unroll
-                for (uint32_t t = 0; t < (WIDE ? 2 : 1); ++t)
-#pragma unroll
-                    for (uint32_t k = 0; k < 8; ++k)
-                        tc_mma_i8(d + t * COL, desc_sw128(a_lo + (2 * t + (k >> 2)) * (KT_ATOM >> 4) + 2 * (k & 3)),
-                                  desc_sw128(b_lo + (k >> 2) * (B_TILE >> 4) + 2 * (k & 3)), p.idesc, k > 0);
+                for (uint32_t k = 0; k < 8; ++k)
+                    tc_mma_i8(d, desc_sw128(a_lo + (k >> 2) * (KT_ATOM >> 4) + 2 * (k & 3)), desc_sw128(b_lo + (k >> 2) * (B_TILE >> 4) + 2 * (k & 3)), p.idesc, k > 0);
                 if constexpr (MIN) {
-                    // Q2_K: sum of 16 = lo + 16 hi in one accumulator, [m | 8 m] . [lo | hi] + [0 | 8 m] . [lo | hi];
-                    // two-byte products: [m | 0] . [lo | hi] and [0 | m] . [lo | hi] apart
+                    // sum of 16 = lo + 16 hi in one accumulator, [m | 8 m] . [lo | hi] + [0 | 8 m] . [lo | hi]
                     const uint32_t am = desc_lo(st + OFF_AM), bm = desc_lo(st + OFF_BM);
-                    tc_mma_i8(d + (WIDE ? 2 * COL : COL), desc_sw64(am), desc_sw32(bm), p.idesc, false);
-                    tc_mma_i8(d + (WIDE ? 3 * COL : COL), desc_sw64(am + 2), desc_sw32(bm), p.idesc, !WIDE);
+                    tc_mma_i8(d + COL, desc_sw64(am), desc_sw32(bm), p.idesc, false);
+                    tc_mma_i8(d + COL, desc_sw64(am + 2), desc_sw32(bm), p.idesc, true);
                 }
                 tc_commit_to(sbase + KO_EMPTY + 8 * s);       // the stage may be overwritten once these MMAs have read it
                 tc_commit_to(sbase + KO_ACC_FULL + 8 * buf);  // and the sums are complete
@@ -390,27 +375,13 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
             for (uint32_t n = 0; n < 2; ++n) {  // the halves of the block: operand tiles n (and 2 + n)
                 // All words of the half leave shared memory before the first store into the operand: nothing waits on a load in the
                 // middle of the arithmetic.
-                uint32_t cw[FMT == FMT_Q4_K || FMT == FMT_Q5_K ? 16 : 8], hw[8], sw[4];  // d (| dmin); codes; high bits; scales
+                uint32_t cw[8], hw[8], sw[4];  // d (| dmin); codes; high bits; scales
                 if constexpr (FMT == FMT_Q2_K) {
                     dm = raw[20];
 #pragma unroll
                     for (int k = 0; k < 4; ++k) sw[k] = raw[k];
 #pragma unroll
                     for (int k = 0; k < 8; ++k) cw[k] = raw[4 + 8 * n + k];
-                } else if constexpr (WIDE) {
-                    const uint4* src = reinterpret_cast<const uint4*>(raw);
-                    const uint4 h = src[0];
-                    dm = h.x;
-                    sw[0] = h.y; sw[1] = h.z; sw[2] = h.w;
-                    if constexpr (FMT == FMT_Q5_K) {
-                        const uint4 v = src[1 + n];
-                        hw[0] = v.x; hw[1] = v.y; hw[2] = v.z; hw[3] = v.w;
-                    }
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const uint4 v = src[(FMT == FMT_Q5_K ? 3 : 1) + 4 * n + k];
-                        cw[4 * k] = v.x; cw[4 * k + 1] = v.y; cw[4 * k + 2] = v.z; cw[4 * k + 3] = v.w;
-                    }
                 } else {
                     const uint32_t sh = 8 * (at & 2u);
                     uint32_t u[9], v[9], x[4];
@@ -438,45 +409,16 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
                     break;
                 }
                 if (MIN && n == 0) {  // the tile of mins, 64 bytes a row
-                    uint4 mn, m1, m2;
-                    if constexpr (FMT == FMT_Q2_K) {
-                        mn = make_uint4((sw[0] >> 4) & 0x0F0F0F0Fu, (sw[1] >> 4) & 0x0F0F0F0Fu, (sw[2] >> 4) & 0x0F0F0F0Fu, (sw[3] >> 4) & 0x0F0F0F0Fu);
-                        m1 = make_uint4(mn.x << 3, mn.y << 3, mn.z << 3, mn.w << 3);
-                        m2 = m1;
-                    } else {  // unpack_q4k_q5k_scales, src/quant/cpu/kernels/dequant_k_quants/q4k_q5k.rs:108-122; a min covers two sums of 16
-                        const uint32_t a = sw[1] & 0x3F3F3F3Fu, c = ((sw[2] >> 4) & 0x0F0F0F0Fu) | ((sw[1] >> 2) & 0x30303030u);
-                        mn = make_uint4(__byte_perm(a, 0u, 0x1100), __byte_perm(a, 0u, 0x3322), __byte_perm(c, 0u, 0x1100), __byte_perm(c, 0u, 0x3322));
-                        m1 = make_uint4(0, 0, 0, 0);
-                        m2 = mn;
-                    }
+                    const uint4 mn = make_uint4((sw[0] >> 4) & 0x0F0F0F0Fu, (sw[1] >> 4) & 0x0F0F0F0Fu, (sw[2] >> 4) & 0x0F0F0F0Fu, (sw[3] >> 4) & 0x0F0F0F0Fu);
+                    const uint4 m8 = make_uint4(mn.x << 3, mn.y << 3, mn.z << 3, mn.w << 3);
                     uint4* am = reinterpret_cast<uint4*>(smem + KO_STAGES + s * STAGE + OFF_AM + r * 64);
                     const uint32_t x3 = (r >> 1) & 3;
                     am[0 ^ x3] = mn;
-                    am[1 ^ x3] = m1;
+                    am[1 ^ x3] = m8;
                     am[2 ^ x3] = make_uint4(0, 0, 0, 0);
-                    am[3 ^ x3] = m2;
+                    am[3 ^ x3] = m8;
                 }
-                if constexpr (WIDE) {
-                    // bytes 32 j .. of low nibbles are sub-block 2 j, of high nibbles sub-block 2 j + 1; Q5_K: bit e of word j of the
-                    // fifth bits belongs to element e of sub-block j
-                    const uint32_t scw = n ? (sw[2] & 0x0F0F0F0Fu) | ((sw[0] >> 2) & 0x30303030u) : sw[0] & 0x3F3F3F3Fu;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {  // sub-block 4 n + j = 16-byte chunks 2 j, 2 j + 1 of the tile
-                        const uint32_t sc2 = 2 * byte_of(scw, j);
-#pragma unroll
-                        for (int k = 0; k < 2; ++k) {
-                            uint32_t lo[4], hi[4];
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                uint32_t c = (cw[8 * (j >> 1) + 4 * k + e] >> (4 * (j & 1))) & 0x0F0F0F0Fu;
-                                if constexpr (FMT == FMT_Q5_K) c |= (((hw[j] >> (4 * (4 * k + e))) & 15u) * 0x02040810u) & 0x10101010u;
-                                wide_scaled(c, sc2, lo[e], hi[e]);
-                            }
-                            put(n, 2 * j + k, make_uint4(lo[0], lo[1], lo[2], lo[3]));
-                            put(2 + n, 2 * j + k, make_uint4(hi[0], hi[1], hi[2], hi[3]));
-                        }
-                    }
-                } else {
+                {
                     uint32_t scw[2];  // the half's eight scales
                     if constexpr (FMT == FMT_Q2_K) {
                         scw[0] = (n ? sw[2] : sw[0]) & 0x0F0F0F0Fu;
@@ -539,22 +481,16 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_tc_kernel(const __grid_const
             for (int c = 0; c < (int)CHUNKS; ++c) {
                 const uint32_t col = 8 * (cg + 4 * c);
                 if (col < p.mt) {  // warp-uniform
-                    uint32_t v[8], u[8], vh[8], uh[8];
+                    uint32_t v[8], u[8];
                     const uint32_t tc = t_base + buf * ACC_COLS + col;
                     tmem_ld8_async(tc, v);
-                    if constexpr (WIDE) tmem_ld8_async(tc + COL, vh);
-                    if constexpr (MIN) tmem_ld8_async(tc + (WIDE ? 2 * COL : COL), u);
-                    if constexpr (WIDE) tmem_ld8_async(tc + 3 * COL, uh);
+                    if constexpr (MIN) tmem_ld8_async(tc + COL, u);
                     const float4* d8 = reinterpret_cast<const float4*>(rec + 512 + 4 * col);
                     const float4 e0 = d8[0], e1 = d8[1];
                     const float e[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
                     tmem_ld_wait();
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        if constexpr (WIDE) {
-                            v[j] += 128 * vh[j];
-                            u[j] += 16 * uh[j];
-                        }
                         float t = __fmul_rn(__fmul_rn(d, e[j]), (float)(int)v[j]);
                         if constexpr (MIN) t = __fsub_rn(t, __fmul_rn(__fmul_rn(dmin, e[j]), (float)(int)u[j]));
                         sum[c][j] = __fadd_rn(sum[c][j], t);
@@ -811,7 +747,7 @@ KqScratch kq_scratch(void* ws, size_t M, size_t K) {
 }
 
 // Time of the two kernels per block of K in SM cycles, fitted to graph replays (Q2_K / Q3_K, 1024 ... 14336 weight rows): a round of
-// tensor-core tiles takes 1300 (two-byte products 2200) and 7 a row of the tile; a 16-row slab of the other kernel 90 (Q2_K) or
+// tensor-core tiles takes 1300 and 7 a row of the tile; a 16-row slab of the other kernel 90 (Q2_K) or
 // 130 (Q3_K) and 20 per 8 activation rows.  Up to 8 rows the latter always wins (Q3_K 4096 x 4096 at 4 rows 7 us; one round
 // of tiles is 17 us).
 struct KqPlan {
@@ -820,8 +756,8 @@ struct KqPlan {
 };
 KqPlan kq_tc_plan(int fmt, size_t M, size_t N, int sm_count) {
     KqPlan best;
-    const size_t rt = (N + 127) / 128, fixed = kq_wide(fmt) ? 2200 : 1300, per_row = 7;
-    for (uint32_t mt = 16; mt <= kt_mt_max(fmt); mt += 16) {
+    const size_t rt = (N + 127) / 128, fixed = 1300, per_row = 7;
+    for (uint32_t mt = 16; mt <= KT_MT_MAX; mt += 16) {
         const size_t units = rt * ((M + mt - 1) / mt), cost = (units + sm_count - 1) / sm_count * (fixed + per_row * mt);
         if (!best.mt || cost <= best.cost) best = {mt, cost};
         if (mt >= M) break;
@@ -830,7 +766,6 @@ KqPlan kq_tc_plan(int fmt, size_t M, size_t N, int sm_count) {
 }
 KqPlan kq_plan(int fmt, size_t M, size_t K, size_t N, int sm_count) {
     const KqPlan tc = kq_tc_plan(fmt, M, N, sm_count);
-    if (kq_wide(fmt)) return tc;
     const size_t slabs = (N + 15) / 16, nt = M <= 8 ? 1 : M <= 16 ? 2 : 4, groups = (M + 8 * nt - 1) / (8 * nt);
     const size_t small = (slabs + sm_count - 1) / sm_count * groups * (fmt == FMT_Q2_K ? 90 + 20 * nt : 130 + 20 * nt);
     const size_t units = (N + 127) / 128 * ((M + 15) / 16);
@@ -871,23 +806,9 @@ bool encode(CUtensorMap* map, CUtensorMapDataType type, size_t elem, void* base,
 
 }  // namespace
 
-// Q2_K and Q3_K: every shape.  Q4_K and Q5_K below 64 rows: where one pass here takes less than several passes over the
-// weights by the kernels for few rows (of 16 rows for Q5_K: gemv.cu; of 32 for Q4_K: smallm_i8.cu, which at 17 ... 32 rows
-// is the faster one).  Both sides as fitted to graph replays, in us: here 5 us and 1.15 us + 4 ns a row of the tile per block
-// of K, for every round of tiles; there 4 us and the packed bytes at 2.7 TB/s per pass of 16 rows, and for the passes of 32
-// the larger of 28 + (M - 33) / 5 + 0.35 per block of K and 6 us + 2.4 TB/s per pass.  Measured (here / there): Q5_K 14336 x 4096 at 20 / 37 / 63
-// rows 26 / 37, 28 / 57, 50 / 77; 4096 x 4096 at 37 rows 23 / 26; 4096 x 14336 (32 tiles on 148 SMs) at 37 rows 75 / 56;
-// Q4_K 14336 x 4096 at 37 / 63 rows 25 / 34, 45 / 40; 4096 x 4096 at 37 rows 22 / 33; at 20 rows 24 / 20.
-// K up to 65536 keeps the scratch below 5 MB.
-bool kq_i8_supported(int fmt, size_t M, size_t K, size_t N, int sm_count) {
-    if (M < 1 || N < 1 || K < 256 || K % 256 != 0) return false;
-    if (fmt == FMT_Q2_K || fmt == FMT_Q3_K) return true;
-    if (!kq_wide(fmt) || M < (fmt == FMT_Q5_K ? 17 : 33) || M >= 64 || K > 65536 || N > (1u << 22) || !tma_available()) return false;
-    const size_t mt = kq_tc_plan(fmt, M, N, sm_count).mt, units = (N + 127) / 128 * ((M + mt - 1) / mt), nblk = K / 256;
-    const double here = 5.0 + (double)((units + sm_count - 1) / sm_count * nblk) * (1.15 + 0.004 * mt), mb = (double)(N * nblk * fmt_block_bytes(fmt)) * 1e-6;
-    const double two = 2.0 * (6.0 + mb / 2.4), few = 28.0 + 0.2 * (double)(M - 33) + 0.35 * (double)nblk;
-    const double there = fmt == FMT_Q5_K ? (double)((M + 15) / 16) * (4.0 + mb / 2.7) : two > few ? two : few;
-    return here < 0.95 * there;
+// Q2_K and Q3_K: every shape.
+bool kq_i8_supported(int fmt, size_t M, size_t K, size_t N) {
+    return (fmt == FMT_Q2_K || fmt == FMT_Q3_K) && M >= 1 && N >= 1 && K >= 256 && K % 256 == 0;
 }
 
 size_t kq_i8_workspace_bytes(size_t M, size_t K) {
@@ -926,12 +847,12 @@ cudaError_t launch_kq_i8(int fmt, const void* act, int act_dtype, const void* w,
         *ws_too_small = true;
         return cudaSuccess;
     }
-    if (fmt != FMT_Q2_K && fmt != FMT_Q3_K && !kq_wide(fmt)) return cudaErrorInvalidValue;
+    if (fmt != FMT_Q2_K && fmt != FMT_Q3_K) return cudaErrorInvalidValue;
     const KqScratch s = kq_scratch(ws, M, K);
     const uint32_t nblk = (uint32_t)(K / 256);
     cudaError_t e;
     if (!acts_prepared) {
-        e = launch_kq_prep(act, act_dtype, M, K, ws, kq_wide(fmt), sm_count, st);
+        e = launch_kq_prep(act, act_dtype, M, K, ws, false, sm_count, st);
         if (e != cudaSuccess) return e;
     }
     const KqPlan plan = kq_plan(fmt, M, K, N, sm_count);
@@ -958,9 +879,7 @@ cudaError_t launch_kq_i8(int fmt, const void* act, int act_dtype, const void* w,
             return cudaErrorInvalidValue;
         }
         e = fmt == FMT_Q2_K   ? launch_tc<FMT_Q2_K>(p, amap, mmap, wmap, sm_count, st)
-            : fmt == FMT_Q3_K ? launch_tc<FMT_Q3_K>(p, amap, mmap, wmap, sm_count, st)
-            : fmt == FMT_Q4_K ? launch_tc<FMT_Q4_K>(p, amap, mmap, wmap, sm_count, st)
-                              : launch_tc<FMT_Q5_K>(p, amap, mmap, wmap, sm_count, st);
+                              : launch_tc<FMT_Q3_K>(p, amap, mmap, wmap, sm_count, st);
     } else {
         KqSmallParams p{};
         p.w = static_cast<const uint8_t*>(w);
@@ -985,6 +904,6 @@ cudaError_t launch_kq_i8(int fmt, const void* act, int act_dtype, const void* w,
 // the C ABI: the tests hold their shapes to the tiles that they are meant for.
 extern "C" __attribute__((visibility("default"))) int b200q_kq_tile_rows(int fmt, size_t M, size_t K, size_t N, int sm_count) {
     if (b200q::kq_few_supported(fmt, M, K, N, false, sm_count)) return b200q::kq_few_tile_rows(fmt, M, K, N, sm_count);
-    if (!b200q::kq_i8_supported(fmt, M, K, N, sm_count)) return -1;
+    if (!b200q::kq_i8_supported(fmt, M, K, N)) return -1;
     return (int)b200q::kq_plan(fmt, M, K, N, sm_count).mt;
 }

@@ -1,4 +1,4 @@
-// Small-M quantized matmul (2 <= M <= 32) for Q4_K on the 5th-generation tensor cores' INTEGER path:
+// Small-M quantized matmul (2 <= M <= 16) for Q4_K on the 5th-generation tensor cores' INTEGER path:
 //   out[M,N] = act[M,K] x W[N,K]^T  with boostr's CPU arithmetic (activations quantised to Q8_K,
 //   src/quant/cpu/kernels/simd/quantize_act_q8k.rs:26-98; per 256-block (d*d8)*sumi - (dmin*d8)*sumi_mins with exact
 //   integer sums, src/quant/cpu/kernels/simd/fused_q4k_q8k_dot.rs:111-172).
@@ -8,7 +8,7 @@
 // tcgen05.mma.kind::i8 (128 weight rows x MP activation rows x 32 K) computes the integer dot products of a whole
 // 32-wide sub-block for 128 rows, and the per-sub-block scales are applied by the warps that drain the accumulator:
 //   * tile = 128 weight rows (the MMA's M = the 128 lanes of tensor memory); the activations are the B operand,
-//     MP = 16 or 32 rows (MMA N); every 32-wide sub-block j of a 256-block gets its OWN accumulator columns
+//     MP = 16 rows (MMA N); every 32-wide sub-block j of a 256-block gets its OWN accumulator columns
 //     [MP j, MP j + MP), so no scale has to enter the tensor core; tensor memory holds two such accumulators;
 //   * packed weight blocks arrive by TMA as tiles of 128 rows x 144 bytes (conflict-free 16-byte reads, one thread
 //     per row); two sets of four decode warps, taking the blocks in turn, split the nibbles into bytes and write them
@@ -843,7 +843,7 @@ struct I8Layout {
 };
 I8Layout i8_layout(size_t M, size_t K, size_t N, int sm_count) {
     I8Layout l{};
-    l.MP = M <= 16 ? 16u : 32u;
+    l.MP = 16u;
     l.nblk = (uint32_t)(K / 256);
     l.ntiles = (uint32_t)((N + 127) / 128);
     l.Q = l.ntiles * l.nblk;
@@ -962,24 +962,22 @@ cudaError_t launch_smallm_q8_0(const void* act, int act_dtype, const void* w, vo
 
 }  // namespace
 
-// Shapes the integer tensor-core kernels take.  Q4_K: 2 <= M <= 32, whole 256-blocks (rows are multiples of 16 bytes:
+// Shapes the integer tensor-core kernels take.  Q4_K: 2 <= M <= 16, whole 256-blocks (rows are multiples of 16 bytes:
 // 144-byte blocks), pair counts within 32 bits.  Q8_0: 17 <= M <= 32 (up to 16 rows the mma.sync kernel is as fast), K a multiple
 // of 256 (rows of whole 272-byte runs), whole tiles only.
 bool smallm_i8_supported(int fmt, size_t M, size_t K, size_t N) {
     if (M < 2 || M > 32 || K % 256 != 0 || K < 256 || N < 1 || (N + 127) / 128 * (K / 256) >= (1u << 30)) return false;
-    return (fmt == FMT_Q8_0 && M > 16) || (fmt == FMT_Q4_K && K / 256 <= 64);
+    return (fmt == FMT_Q8_0 && M > 16) || (fmt == FMT_Q4_K && M <= 16 && K / 256 <= 64);
 }
 size_t smallm_i8_workspace_bytes(int fmt, size_t M, size_t K, size_t N, int sm_count) {
     return fmt == FMT_Q8_0 ? q8_layout(M, K, N, sm_count).total : i8_layout(M, K, N, sm_count).total;
 }
 // Where they beat the mma.sync kernel (measured).  Q4_K: matrices with enough 128-row tiles to give every SM whole tiles
-// (nothing to hand over), from 8 activation rows on; and every shape above 16 rows, which the mma.sync kernel takes in
-// two passes over the weights.  Q8_0: above 16 rows (one pass over the weights instead of two), matrices with enough
+// (nothing to hand over), from 8 activation rows on.  Q8_0: above 16 rows (one pass over the weights instead of two), matrices with enough
 // tiles to occupy half of the SMs (only whole tiles are dealt).
 bool smallm_i8_preferred(int fmt, size_t M, size_t K, size_t N, int sm_count) {
     if (!smallm_i8_supported(fmt, M, K, N)) return false;
     if (fmt == FMT_Q8_0) return M > 16 && (N + 127) / 128 >= (size_t)sm_count / 2;
-    if (M > 16) return true;
     const I8Layout l = i8_layout(M, K, N, sm_count);
     return M >= 8 && l.unit == l.nblk && l.ntiles >= (uint32_t)sm_count * 3 / 4;
 }
@@ -1064,14 +1062,9 @@ cudaError_t launch_smallm_i8(int fmt, const void* act, int act_dtype, const void
         }
     }
     static PerDeviceOnce attrs;
-    cudaError_t e = attrs.run([] {
-        cudaError_t a = cudaFuncSetAttribute(smallm_i8_q4k_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
-        if (a == cudaSuccess) a = cudaFuncSetAttribute(smallm_i8_q4k_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
-        return a;
-    });
+    cudaError_t e = attrs.run([] { return cudaFuncSetAttribute(smallm_i8_q4k_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448); });
     if (e != cudaSuccess) return e;
-    e = p.MP == 16 ? launch_pdl(smallm_i8_q4k_kernel<16>, dim3(l.grid), dim3(I8_THREADS), smem, st, amap, wmap, p)
-                   : launch_pdl(smallm_i8_q4k_kernel<32>, dim3(l.grid), dim3(I8_THREADS), smem, st, amap, wmap, p);
+    e = launch_pdl(smallm_i8_q4k_kernel<16>, dim3(l.grid), dim3(I8_THREADS), smem, st, amap, wmap, p);
     note_launch();
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
