@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
             if (!wait(KF_RAW_FULL + 8 * rs, rpar, STATUS_TIMEOUT_FULL)) break;
             const uint32_t col = a_col0 + HALF * st;
             uint32_t dm = 0;
-            // all columns of this half may be overwritten
+            // all columns of this half may be overwritten: the MMAs that read them have completed, and the stores stay behind that
             auto take = [&]() { return x < p.ns || wait(KF_SET_EMPTY + 8 * set, ((x - p.ns) >> 2) & 1, STATUS_TIMEOUT_EMPTY); };
             auto release = [&]() {
                 __syncwarp();
@@ -372,6 +372,7 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
 #pragma unroll
                 for (int k = 0; k < 2; ++k) sw[k] = __funnelshift_r(sw[k], sw[k + 1], sh);
                 if (!take()) break;
+                tc_after();
 #pragma unroll
                 for (int part = 0; part < 2; ++part) {
                     uint32_t lw[9];
@@ -409,6 +410,7 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
                 const uint32_t scw = h ? (hd.w & 0x0F0F0F0Fu) | ((hd.y >> 2) & 0x30303030u) : hd.y & 0x3F3F3F3Fu;
                 const uint32_t slw = scw & 0x07070707u, shw = (scw >> 3) & 0x07070707u;
                 if (!take()) break;
+                tc_after();
 #pragma unroll
                 for (int part = 0; part < 2; ++part) {  // 32 bytes of nibbles: sub-blocks 4 h + 2 part and the next
                     uint32_t cw[8];
