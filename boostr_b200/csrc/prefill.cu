@@ -735,6 +735,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const __grid_con
                     pf_fail(dead_flag, p.status, STATUS_TIMEOUT_EMPTY);
                     ok = false;
                 }
+                tc_fence_after();  // the store stays behind the MMAs that read the stage
                 // the thread's 64 bf16 go to its own lane (= weight row) of the stage's tensor-memory tile, 32 columns.
                 // Executed by the whole warp (dead warps store what they hold: nobody reads it).
                 tmem_st32(tmem_acc + ((((uint32_t)warp & 3u) * 32u) << 16) + a_col0 + 32 * (p.ks * s + sub), o);

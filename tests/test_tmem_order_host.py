@@ -1,6 +1,7 @@
 """Tensor memory is read and written by the tensor core out of the threads' order: an access behind a barrier on which its
 MMAs (or another warp's accesses) were waited for needs ``tcgen05.fence::after_thread_sync`` between the two, stores that
 overwrite an operand as well as loads and MMAs.  No run can show a missing fence for sure; the text of the kernels can."""
+import glob
 import os
 import re
 
@@ -28,7 +29,7 @@ def _unfenced(text):
     return bad
 
 
-@pytest.mark.parametrize("name", ["kquant_few.cu", "kquant_i8.cu", "smallm_i8.cu"])
+@pytest.mark.parametrize("name", sorted(os.path.basename(f) for f in glob.glob(os.path.join(CSRC, "*.cu"))))
 def test_accesses_are_fenced_behind_waits(name):
     with open(os.path.join(CSRC, name)) as f:
         text = re.sub(r"//[^\n]*", "", f.read())
