@@ -50,9 +50,9 @@ cudaError_t launch_kq_i8(int fmt, const void* act, int act_dtype, const void* w,
                              size_t N, void* ws, size_t ws_bytes, int sm_count, cudaStream_t st, unsigned int* status,
                              bool* ws_too_small, char* err, size_t err_len, bool acts_prepared);
 bool kq_few_supported(int fmt, size_t M, size_t K, size_t N, bool swiglu, int sm_count);
-cudaError_t launch_kq_few(int fmt, const void* act, int act_dtype, int nseg, const void* const* w, void* const* out, const size_t* N, bool swiglu,
-                          int out_dtype, size_t M, size_t K, void* ws, size_t ws_bytes, int sm_count, cudaStream_t st, unsigned int* status,
-                          bool* ws_too_small, char* err, size_t err_len, bool acts_prepared);
+cudaError_t launch_kq_few(int fmt, const void* act, int act_dtype, const void* w, const void* w_up, void* out, int out_dtype, size_t M, size_t K,
+                          size_t N, void* ws, size_t ws_bytes, int sm_count, cudaStream_t st, unsigned int* status, bool* ws_too_small, char* err,
+                          size_t err_len, bool acts_prepared);
 cudaError_t launch_swiglu_gate(const float* gate, const float* up, void* out, int out_dtype, size_t n, int sm_count,
                                cudaStream_t st);
 bool smallm_i8_supported(int fmt, size_t M, size_t K, size_t N);
@@ -252,7 +252,7 @@ int quant_matmul_impl(int format, const void* act, int act_dtype, const void* w,
     cudaError_t e;
     if (kq_few_supported(format, M, K, N, false, sm_count_current())) {
         char msg[256] = "";
-        e = launch_kq_few(format, act, act_dtype, 1, &w, &out, &N, false, out_dtype, M, K, ws, ws_bytes, sm_count_current(), st, status, &small, msg, sizeof(msg),
+        e = launch_kq_few(format, act, act_dtype, w, nullptr, out, out_dtype, M, K, N, ws, ws_bytes, sm_count_current(), st, status, &small, msg, sizeof(msg),
                           acts_prepared);
         if (e != cudaSuccess && msg[0]) return fail(B200Q_ERR_CUDA, "quant_matmul: %s", msg);
     } else if (kq_i8_supported(format, M, K, N)) {
@@ -447,10 +447,8 @@ int b200q_quant_swiglu(int format, const void* act, int act_dtype, const void* w
     cudaError_t e;
     if (kq_few_supported(format, M, K, N, true, sm_count_current())) {
         char msg[256] = "";
-        const void* ww[2] = {w_gate, w_up};
-        void* oo[2] = {out, out};
-        const size_t nn[2] = {N, N};
-        e = launch_kq_few(format, act, act_dtype, 2, ww, oo, nn, true, out_dtype, M, K, ws, ws_bytes, sm_count_current(), st, status, &small, msg, sizeof(msg), false);
+        e = launch_kq_few(format, act, act_dtype, w_gate, w_up, out, out_dtype, M, K, N, ws, ws_bytes, sm_count_current(), st, status, &small, msg, sizeof(msg),
+                          false);
         if (e != cudaSuccess && msg[0]) return fail(B200Q_ERR_CUDA, "quant_swiglu: %s", msg);
     } else if (kq_i8_supported(format, M, K, N)) {
         // two products into f32 scratch (the second reads the first one's Q8_K image), then the gate

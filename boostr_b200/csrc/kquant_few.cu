@@ -49,17 +49,11 @@ __host__ __device__ constexpr uint32_t kf_half_cols(int fmt) { return fmt == FMT
 __host__ __device__ constexpr bool kf_min(int fmt) { return fmt != FMT_Q6_K; }
 __host__ __device__ constexpr uint32_t kf_raw(int fmt) { return 128 * kf_pitch(fmt); }
 
-struct KfSeg {
-    const uint8_t* w;
-    void* out;
-    uint32_t N;
-    uint32_t rt0;  // its first row tile among those of all segments
-};
 struct KfParams {
-    KfSeg seg[3];
-    uint32_t nseg;
+    const uint8_t *w, *w_up;  // w_up: SwiGLU (w is gate)
+    void* out;
     const float* d8;  // [nblk][M]
-    uint32_t M, nblk, row_bytes;
+    uint32_t M, N, nblk, row_bytes;
     uint32_t mt, nct, nunits;  // activation rows of a tile; column tiles; row tiles x column tiles
     uint32_t cs;               // CTAs per tile (a cluster), each with a share of K
     uint32_t ns, nr, nb;       // ring depths: operand halves in tensor memory, packed blocks (even), activation blocks
@@ -162,7 +156,7 @@ __device__ __forceinline__ void kf_copy_q6(uint32_t dst, const uint8_t* blk, uin
 template <int FMT>
 __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant__ CUtensorMap tmap_sum,
                                                                const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
-                                                               const __grid_constant__ CUtensorMap tmap_w2, const KfParams p) {
+                                                               const KfParams p) {
     constexpr bool MIN = kf_min(FMT), Q6 = FMT == FMT_Q6_K;
     constexpr uint32_t BB = fmt_block_bytes(FMT), PITCH = kf_pitch(FMT), RAW = kf_raw(FMT), HI_SHIFT = Q6 ? 8 : 3, HALF = kf_half_cols(FMT);
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -215,7 +209,6 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
     const uint32_t k0 = rank * p.nblk / p.cs, nb = (rank + 1) * p.nblk / p.cs - k0;
     const uint32_t units = (p.nunits - unit0 + stride - 1) / stride, total = units * nb;
     const uint32_t rows = p.swiglu ? 64 : 128;  // weight rows of a row tile (SwiGLU: as many of gate and of up)
-    auto seg_of = [&](uint32_t rt) { return (p.nseg > 1 && rt >= p.seg[1].rt0 ? 1u : 0u) + (p.nseg > 2 && rt >= p.seg[2].rt0 ? 1u : 0u); };
 
     // Two warps issue the MMAs, one for the even and one for the odd blocks, where the second copying warp has nothing to copy and
     // every operand half has a slot of its own (a slot then belongs to one of them).
@@ -229,20 +222,20 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
         uint32_t unit = unit0, b = k0, rs = 0, par = 1;
         for (uint32_t i = 0; i < mine; ++i) {
             if (!wait(KF_RAW_EMPTY + 8 * rs, par, STATUS_TIMEOUT_EMPTY)) break;
-            const uint32_t rt = unit / p.nct, sg = p.swiglu ? 0 : seg_of(rt), n0 = (rt - p.seg[sg].rt0) * rows;
+            const uint32_t n0 = unit / p.nct * rows;
             const uint32_t dst = sbase + p.off_raw + rs * RAW, bar = sbase + KF_RAW_FULL + 8 * rs;
             if (p.raw_tma) {
                 if (lane == 0) {
                     mbar_expect_tx(bar, RAW);
                     const int x = (int)((b * BB & ~15u) / 2);
-                    tma2d(dst, sg == 0 ? &tmap_w0 : sg == 1 ? &tmap_w1 : &tmap_w2, x, (int)n0, bar);
+                    tma2d(dst, &tmap_w0, x, (int)n0, bar);
                     if (p.swiglu) tma2d(dst + RAW / 2, &tmap_w1, x, (int)n0, bar);  // boxes of 64 rows
                 }
             } else if constexpr (Q6) {
-                const KfSeg& s = p.seg[p.swiglu ? half : sg];
+                const uint8_t* w = p.swiglu && half ? p.w_up : p.w;
                 const uint32_t r0 = p.swiglu ? n0 : n0 + 64 * half;
-                kf_copy_q6(dst + half * (RAW / 2), s.w + (size_t)r0 * p.row_bytes + (size_t)b * BB, p.row_bytes, lane, r0 < s.N ? s.N - r0 : 0,
-                           s.w + (size_t)s.N * p.row_bytes);
+                kf_copy_q6(dst + half * (RAW / 2), w + (size_t)r0 * p.row_bytes + (size_t)b * BB, p.row_bytes, lane, r0 < p.N ? p.N - r0 : 0,
+                           w + (size_t)p.N * p.row_bytes);
                 asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
             }
             if (++b == k0 + nb) {
@@ -533,7 +526,7 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
             }
             if (++b < nb) continue;
             b = 0;
-            const uint32_t rt = unit / p.nct, sg = p.swiglu ? 0 : seg_of(rt), n = (rt - p.seg[sg].rt0) * rows + r, N = p.seg[sg].N;
+            const uint32_t n = unit / p.nct * rows + r;
             unit += stride;
             if (p.cs > 1) {
                 if (!p.terms)
@@ -563,13 +556,13 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
                         for (int j = 0; j < 8; ++j)
                             if (8 * (cg + 2 * c) < p.mt) sum[c][j] = kf_gate(sum[c][j], to[(8 * (cg + 2 * c) + j) * 64]);
             }
-            if (n < N && (!p.swiglu || r < 64))
+            if (n < p.N && (!p.swiglu || r < 64))
 #pragma unroll
                 for (int c = 0; c < CHUNKS; ++c)
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
                         const uint32_t m = 8 * (cg + 2 * c) + j;
-                        if (m < p.mt && m0 + m < p.M) kf_store(p.seg[sg].out, p.out_dtype, (size_t)(m0 + m) * N + n, sum[c][j]);
+                        if (m < p.mt && m0 + m < p.M) kf_store(p.out, p.out_dtype, (size_t)(m0 + m) * p.N + n, sum[c][j]);
                     }
         }
     }
@@ -578,8 +571,7 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
         // The shares of K meet: CTA `rank` adds them for every cs-th activation row of the tile and writes the results.
         cluster_sync_all();
         if (!*dead) {
-            const uint32_t m0 = unit0 % p.nct * p.mt, in = min(p.mt, p.M - m0), rt = unit0 / p.nct, sg = p.swiglu ? 0 : seg_of(rt);
-            const uint32_t n0 = (rt - p.seg[sg].rt0) * rows, N = p.seg[sg].N, x0 = sbase + p.off_x;
+            const uint32_t m0 = unit0 % p.nct * p.mt, in = min(p.mt, p.M - m0), n0 = unit0 / p.nct * rows, x0 = sbase + p.off_x;
             for (uint32_t t = threadIdx.x; t < (in > rank ? (in - rank + p.cs - 1) / p.cs : 0) * rows; t += KF_THREADS) {
                 const uint32_t m = rank + t / rows * p.cs, r = t % rows;
                 float s[2] = {0.f, 0.f};
@@ -591,7 +583,7 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
                         if (p.swiglu) s[1] = __fadd_rn(s[1], ld_cluster(from + j * p.mt * 512 + 256));
                     }
                 }
-                if (n0 + r < N) kf_store(p.seg[sg].out, p.out_dtype, (size_t)(m0 + m) * N + n0 + r, p.swiglu ? kf_gate(s[0], s[1]) : s[0]);
+                if (n0 + r < p.N) kf_store(p.out, p.out_dtype, (size_t)(m0 + m) * p.N + n0 + r, p.swiglu ? kf_gate(s[0], s[1]) : s[0]);
             }
         }
         cluster_sync_all();  // nobody's shared memory goes before all have read it
@@ -709,7 +701,7 @@ cudaError_t kf_launch(const CUtensorMap& am, const CUtensorMap& sm, const CUtens
     at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = p.cs > 1 ? 2 : 1;
-    e = cudaLaunchKernelEx(&cfg, kq_few_kernel<FMT>, am, sm, wm[0], wm[1], wm[2], p);
+    e = cudaLaunchKernelEx(&cfg, kq_few_kernel<FMT>, am, sm, wm[0], wm[1], p);
     note_launch();
     return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -735,10 +727,10 @@ bool kq_few_supported(int fmt, size_t M, size_t K, size_t N, bool swiglu, int sm
 }
 int kq_few_tile_rows(int fmt, size_t M, size_t K, size_t N, int sm_count) { return (int)kf_plan(fmt, M, K, (N + 127) / 128, false, sm_count).mt; }
 
-// nseg products of one format with the same activations (swiglu: nseg = 2, gate and up, one output).
-cudaError_t launch_kq_few(int fmt, const void* act, int act_dtype, int nseg, const void* const* w, void* const* out, const size_t* N, bool swiglu,
-                          int out_dtype, size_t M, size_t K, void* ws, size_t ws_bytes, int sm_count, cudaStream_t st, unsigned int* status,
-                          bool* ws_too_small, char* err, size_t err_len, bool acts_prepared) {
+// w_up: SwiGLU of the products with w (gate) and w_up; else null.
+cudaError_t launch_kq_few(int fmt, const void* act, int act_dtype, const void* w, const void* w_up, void* out, int out_dtype, size_t M, size_t K,
+                          size_t N, void* ws, size_t ws_bytes, int sm_count, cudaStream_t st, unsigned int* status, bool* ws_too_small, char* err,
+                          size_t err_len, bool acts_prepared) {
     *ws_too_small = false;
     if (!ws || ws_bytes < kq_i8_workspace_bytes(M, K) || (reinterpret_cast<uintptr_t>(ws) & 15)) {
         *ws_too_small = true;
@@ -754,14 +746,13 @@ cudaError_t launch_kq_few(int fmt, const void* act, int act_dtype, int nseg, con
         if (e != cudaSuccess) return e;
     }
     KfParams p{};
-    const uint32_t rows = swiglu ? 64 : 128;
-    uint32_t rt = 0;
-    for (int i = 0; i < nseg; ++i) {
-        p.seg[i] = {static_cast<const uint8_t*>(w[i]), out[i], (uint32_t)N[i], swiglu ? 0 : rt};
-        if (i == 0 || !swiglu) rt += (uint32_t)((N[i] + rows - 1) / rows);
-    }
+    const bool swiglu = w_up != nullptr;
+    const uint32_t rows = swiglu ? 64 : 128, rt = (uint32_t)((N + rows - 1) / rows);
     const KfPlan pl = kf_plan(fmt, M, K, rt, swiglu, sm_count);
-    p.nseg = (uint32_t)nseg;
+    p.w = static_cast<const uint8_t*>(w);
+    p.w_up = static_cast<const uint8_t*>(w_up);
+    p.out = out;
+    p.N = (uint32_t)N;
     p.d8 = d8;
     p.M = (uint32_t)M;
     p.nblk = nblk;
@@ -784,12 +775,12 @@ cudaError_t launch_kq_few(int fmt, const void* act, int act_dtype, int nseg, con
     p.raw_tma = p.row_bytes % 16 == 0;
     p.swiglu = swiglu;
     p.status = status;
-    CUtensorMap am, sm, wm[3];
+    CUtensorMap am, sm, wm[2];
     bool ok = kf_encode(&am, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, codes, K, M, 128, p.mt, CU_TENSOR_MAP_SWIZZLE_128B) &&
               kf_encode(&sm, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, sums, (size_t)nblk * 16, M, 16, p.mt, CU_TENSOR_MAP_SWIZZLE_32B);
-    for (int i = 0; i < 3 && ok; ++i) {
-        if (p.raw_tma && i < nseg)
-            ok = kf_encode(&wm[i], CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, w[i], p.row_bytes / 2, N[i], kf_pitch(fmt) / 2, rows, CU_TENSOR_MAP_SWIZZLE_NONE);
+    for (int i = 0; i < 2 && ok; ++i) {
+        if (p.raw_tma && (i == 0 || swiglu))
+            ok = kf_encode(&wm[i], CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, i ? w_up : w, p.row_bytes / 2, N, kf_pitch(fmt) / 2, rows, CU_TENSOR_MAP_SWIZZLE_NONE);
         else
             wm[i] = am;
     }
