@@ -17,9 +17,11 @@
 // into TENSOR MEMORY (tcgen05.st; the MMA takes its A operand from there): no swizzled shared-memory stores, no proxy fence,
 // and shared memory is left to the packed blocks in flight.  A stage is HALF a block (128 codes); four sets of four decode
 // warps take the halves in turn.
-// Work: whole tiles dealt round-robin, or, where a matrix has few tiles, a thread-block cluster of 2, 4 or 8 CTAs per tile, each
-// with a share of K.  The shares meet in distributed shared memory: up to 16 blocks as the blocks' terms, added in K order
-// (the CPU's bits), beyond as one sum per share.
+// Work: whole tiles dealt round-robin, or, where a matrix has few tiles, a thread-block cluster of 2, 4 or 8 CTAs per tile, which
+// takes that many blocks of K at a time, one per CTA.  Each CTA adds up some of the tile's weight rows: the terms of a round come
+// to it from all CTAs by st.async into shared memory and are added in K order while the next round is drained, so the results
+// have the CPU's bits at every K.  (Shares of K added as sums, which have other bits, are up to 15 % faster at K = 14336: 4096 x 14336 at 37
+// rows Q4_K 25.7 against 27.1 us.  Up to K = 4096 the exchange by rounds is the faster one too: 4096 x 4096 at 37 rows Q4_K 14.8 -> 11.1 us.)
 // What bounds it: instructions.  A block costs some 4600 (Q4_K) or 6800 (Q6_K) warp instructions, issue slots 58 % busy, the ALU
 // pipe 38 / 61 %; the MMAs themselves take 10 ... 20 cycles each with the A operand in tensor memory (34 ... 38 from shared memory).  One
 // MMA-issuing warp spent 90 cycles on each and set the pace (2.0 us a Q4_K block instead of 0.9 at 16 rows), hence two.
@@ -55,12 +57,12 @@ struct KfParams {
     const float* d8;  // [nblk][M]
     uint32_t M, N, nblk, row_bytes;
     uint32_t mt, nct, nunits;  // activation rows of a tile; column tiles; row tiles x column tiles
-    uint32_t cs;               // CTAs per tile (a cluster), each with a share of K
+    uint32_t cs, cs_log;       // CTAs per tile: a cluster of 2^cs_log, each of which takes every cs-th block of K
     uint32_t ns, nr, nb;       // ring depths: operand halves in tensor memory, packed blocks (even), activation blocks
     uint32_t off_rec, off_raw, off_x;  // of shared memory
     uint32_t idesc_i, idesc_h;
     int out_dtype;
-    bool raw_tma, swiglu, terms;
+    bool raw_tma, swiglu;
     unsigned int* status;
 };
 
@@ -70,7 +72,7 @@ constexpr int KF_THREADS = (KF_W_MMA + 1) * 32;
 constexpr uint32_t KF_NQ = 4, KF_REC = 1024;  // 128 x (d | dmin), then the activation rows' d8
 constexpr uint32_t KF_MT_MAX = 48;
 constexpr int KF_FULL = 0, KF_SET_EMPTY = 32, KF_RAW_FULL = 64, KF_RAW_EMPTY = 160, KF_B_FULL = 256, KF_B_EMPTY = 288, KF_ACC_FULL = 320,
-              KF_ACC_EMPTY = 336, KF_REC_FULL = 352, KF_REC_EMPTY = 384, KF_MEET = 416, KF_TMEM = 424, KF_DEAD = 428, KF_STAGES = 1024;
+              KF_ACC_EMPTY = 336, KF_REC_FULL = 352, KF_REC_EMPTY = 384, KF_MEET = 416, KF_TMEM = 424, KF_DEAD = 428, KF_READY = 432, KF_FREE = 448, KF_STAGES = 1024;
 constexpr uint32_t KF_NR_MAX = 12;
 __host__ __device__ constexpr uint32_t kf_btile(uint32_t mt) { return (mt * 288 + 1023) / 1024 * 1024; }
 
@@ -119,19 +121,22 @@ __device__ __forceinline__ uint32_t cluster_rank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
-__device__ __forceinline__ float ld_cluster(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-    return v;
+// A store to a CTA of the cluster that counts its bytes at a barrier there: nothing waits for it on this side, while stores
+// released by an arrival (st.shared::cluster, mbarrier.arrive.release.cluster) cost 2 us a round.
+__device__ __forceinline__ void st_async4(uint32_t addr, float a, float b, float c, float d, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "f"(a), "f"(b), "f"(c),
+                 "f"(d), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
 }
 // silu(g) u as in swiglu_gate_kernel
 __device__ __forceinline__ float kf_gate(float g, float u) { return g / (1.0f + expf(-g)) * u; }
@@ -153,7 +158,7 @@ __device__ __forceinline__ void kf_copy_q6(uint32_t dst, const uint8_t* blk, uin
     }
 }
 
-template <int FMT>
+template <int FMT, bool CLUSTER>
 __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_constant__ CUtensorMap tmap_act, const __grid_constant__ CUtensorMap tmap_sum,
                                                                const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
                                                                const KfParams p) {
@@ -166,6 +171,15 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
     volatile uint32_t* dead = reinterpret_cast<volatile uint32_t*>(smem + KF_DEAD);
     // tensor memory: two accumulators (lo | hi (| mins), mt columns each), ns operand halves (lo 32 | hi 32 (| fifth bits 32)), two tiles of mins
     const uint32_t acc_cols = (MIN ? 3 : 2) * p.mt, a_col0 = 2 * acc_cols, m_col0 = a_col0 + HALF * p.ns;
+    // Blocks of this CTA: all of the units blockIdx.x, + gridDim.x, ..., or of one unit the blocks rank, + cs, ...
+    const uint32_t cs = CLUSTER ? p.cs : 1, cs_log = CLUSTER ? p.cs_log : 0, rank = CLUSTER ? cluster_rank() : 0;
+    const uint32_t stride = gridDim.x >> cs_log, unit0 = blockIdx.x >> cs_log, nb = (p.nblk - rank + cs - 1) >> cs_log;
+    const uint32_t units = (p.nunits - unit0 + stride - 1) / stride, total = units * nb;
+    const uint32_t rows = p.swiglu ? 64 : 128;  // weight rows of a row tile (SwiGLU: as many of gate and of up)
+    const uint32_t in = min(p.mt, p.M - unit0 % p.nct * p.mt);  // activation rows of a cluster's tile
+    // round i of a cluster is one block per CTA: how many there are, and the bytes of their terms that one CTA gets
+    auto round_blocks = [&](uint32_t i) { return i << cs_log < p.nblk ? min(cs, p.nblk - (i << cs_log)) : 0u; };
+    auto round_bytes = [&](uint32_t i) { return round_blocks(i) * (((in + 7) & ~7u) >> cs_log) * 512; };
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < 4; ++s) {
             mbar_init(sbase + KF_FULL + 8 * s, 4);       // the four warps of the set that wrote the half
@@ -186,8 +200,16 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
             mbar_init(sbase + KF_REC_EMPTY + 8 * s, KF_DRAIN);
         }
         mbar_init(sbase + KF_MEET, KF_DRAIN);
+        if constexpr (CLUSTER)
+            for (uint32_t s = 0; s < 2; ++s) {
+                mbar_init(sbase + KF_READY + 8 * s, 1);              // the bytes of a round's terms
+                mbar_init(sbase + KF_FREE + 8 * s, KF_DRAIN << p.cs_log);  // the drain warps of the whole cluster
+            }
         *dead = 0;
         mbar_fence_init();
+        if constexpr (CLUSTER)
+            for (uint32_t s = 0; s < 2; ++s)
+                if (round_bytes(s)) mbar_expect_tx(sbase + KF_READY + 8 * s, round_bytes(s));
     }
     if (warp == KF_W_MMA) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + KF_TMEM), "r"(512u) : "memory");
@@ -204,11 +226,7 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
         if (!ok && lane == 0) i8_fail(dead, p.status, code);
         return ok;
     };
-    // Blocks of this CTA: all of K of the units blockIdx.x, + gridDim.x, ..., or a share [k0, k0 + nb) of one unit's.
-    const uint32_t rank = p.cs > 1 ? cluster_rank() : 0, stride = gridDim.x / p.cs, unit0 = blockIdx.x / p.cs;
-    const uint32_t k0 = rank * p.nblk / p.cs, nb = (rank + 1) * p.nblk / p.cs - k0;
-    const uint32_t units = (p.nunits - unit0 + stride - 1) / stride, total = units * nb;
-    const uint32_t rows = p.swiglu ? 64 : 128;  // weight rows of a row tile (SwiGLU: as many of gate and of up)
+    if constexpr (CLUSTER) cluster_arrive();  // this CTA's barriers exist
 
     // Two warps issue the MMAs, one for the even and one for the odd blocks, where the second copying warp has nothing to copy and
     // every operand half has a slot of its own (a slot then belongs to one of them).
@@ -219,7 +237,7 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
         // ------------------------------------------------------------ packed blocks (do not depend on the kernel that is still running)
         const uint32_t half = (uint32_t)(warp - KF_W_COPY);
         const uint32_t mine = p.raw_tma && half ? 0 : total;  // by TMA one warp brings all
-        uint32_t unit = unit0, b = k0, rs = 0, par = 1;
+        uint32_t unit = unit0, b = rank, rs = 0, par = 1;
         for (uint32_t i = 0; i < mine; ++i) {
             if (!wait(KF_RAW_EMPTY + 8 * rs, par, STATUS_TIMEOUT_EMPTY)) break;
             const uint32_t n0 = unit / p.nct * rows;
@@ -238,8 +256,9 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
                            w + (size_t)p.N * p.row_bytes);
                 asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
             }
-            if (++b == k0 + nb) {
-                b = k0;
+            b += cs;
+            if (b >= p.nblk) {
+                b = rank;
                 unit += stride;
             }
             if (++rs == p.nr) {
@@ -252,7 +271,7 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
         // ------------------------------------------------------------ activation codes, sums and scales (previous kernel's output)
         grid_dep_wait();
         grid_dep_launch();  // not before: the next product of a batch may be one that reads its weights in order
-        uint32_t unit = unit0, b = k0, bs = 0, par = 1;
+        uint32_t unit = unit0, b = rank, bs = 0, par = 1;
         const uint32_t btile = kf_btile(p.mt);
         for (uint32_t i = 0; i < total; ++i) {
             const uint32_t q = i % KF_NQ, m0 = unit % p.nct * p.mt, dst = sbase + KF_STAGES + bs * btile, bar = sbase + KF_B_FULL + 8 * bs;
@@ -270,8 +289,9 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
             for (uint32_t m = lane; m < p.mt; m += 32)  // rows past M are zero-filled
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(rec + 4 * m), "l"(m0 + m < p.M ? src + m : p.d8), "r"(m0 + m < p.M ? 4u : 0u) : "memory");
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(sbase + KF_REC_FULL + 8 * q) : "memory");
-            if (++b == k0 + nb) {
-                b = k0;
+            b += cs;
+            if (b >= p.nblk) {
+                b = rank;
                 unit += stride;
             }
             if (++bs == p.nb) {
@@ -336,8 +356,8 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
         // ------------------------------------------------------------ decode: one thread per weight row, the sets take the half blocks in turn
         const uint32_t r = threadIdx.x & 127, set = (uint32_t)warp >> 2, h = set & 1;
         const uint32_t lanes = tmem + (((uint32_t)warp & 3) << 21);
-        uint32_t b = k0 + (set >> 1) % nb, st = set % p.ns, rs = set >> 1, rpar = 0;
-        const uint32_t b_step = 2 % nb, st_step = 4 % p.ns;
+        uint32_t b = rank + cs * ((set >> 1) % nb), st = set % p.ns, rs = set >> 1, rpar = 0;
+        const uint32_t b_step = cs * (2 % nb), b_end = rank + cs * nb, st_step = 4 % p.ns;
         for (uint32_t i = set >> 1; i < total; i += 2) {
             const uint32_t q = i % KF_NQ, x = 2 * i + h;
             if (!wait(KF_RAW_FULL + 8 * rs, rpar, STATUS_TIMEOUT_FULL)) break;
@@ -459,7 +479,7 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
                 if (lane == 0) mbar_arrive(sbase + KF_REC_FULL + 8 * q);
             }
             b += b_step;
-            if (b >= k0 + nb) b -= nb;
+            if (b >= b_end) b -= cs * nb;
             st += st_step;
             if (st >= p.ns) st -= p.ns;
             rs += 2;
@@ -473,22 +493,82 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
         const uint32_t quarter = warp & 3, cg = (uint32_t)(warp - KF_W_DRAIN) >> 2, r = quarter * 32 + lane;
         const uint32_t t_base = tmem + ((quarter * 32) << 16);
         constexpr int CHUNKS = KF_MT_MAX / 16;
-        float sum[CHUNKS][8];  // activation rows 8 (cg + 2 c) + j
+        float sum[CHUNKS][8];  // activation rows 8 (cg + 2 c) + j; in a cluster the units of `from`
         float* xch = reinterpret_cast<float*>(smem + p.off_x);
         grid_dep_wait();  // the output may still be in use by the previous kernel
+        // Cluster: in a round every CTA drains one block.  The weight rows of the tile are shared out; their CTA gets the round's terms from
+        // all, [buffer][CTA][activation rows / 4][weight row][4], and adds them in the CTAs' order, which is K order, while the next round
+        // is drained.  A buffer is written again once all CTAs have added what was in theirs.
+        const uint32_t dt = threadIdx.x - KF_W_DRAIN * 32, rounds = CLUSTER ? (p.nblk + cs - 1) >> cs_log : total;
+        const uint32_t own = rows >> cs_log, own_log = (p.swiglu ? 6 : 7) - cs_log, lines = 128 >> cs_log;  // its weight rows; with those of up
+        const uint32_t line = (r & (own - 1)) + (r >= rows ? own : 0), owner = CLUSTER ? (r & (rows - 1)) >> own_log : 0;
+        const uint32_t to = CLUSTER ? mapa(sbase + p.off_x + (rank * (p.mt / 4) * lines + line) * 16, owner) : 0;
+        const uint32_t to_bar = CLUSTER ? mapa(sbase + KF_READY, owner) : 0;
+        // what this thread adds: units (4 activation rows of a weight row) dt, dt + 256, dt + 512; SwiGLU: dt, dt + 256 of gate (0, 1) and of up (2, 3)
+        auto unit_of = [&](int q) { return dt + 256 * (p.swiglu ? q & 1 : q); };
+        uint32_t from[4] = {};  // addresses of the units (0: none) in the first buffer
+        if constexpr (CLUSTER)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if ((unit_of(q) >> own_log) * 4 < in && (q < 3 || p.swiglu))
+                    from[q] = sbase + p.off_x + ((unit_of(q) >> own_log) * lines + (unit_of(q) & (own - 1)) + (p.swiglu && q >= 2 ? own : 0)) * 16;
+        constexpr uint32_t ZERO = 0x80000000u;  // -0.0: x + -0.0 is x
+        auto collect = [&](uint32_t i) {
+            if (!wait(KF_READY + 8 * (i & 1), (i >> 1) & 1, STATUS_TIMEOUT_FULL)) return false;
+            if (dt == 0 && round_bytes(i + 2)) mbar_expect_tx(sbase + KF_READY + 8 * (i & 1), round_bytes(i + 2));
+            const uint32_t cnt = round_blocks(i), step = p.mt * lines * 4;
+#pragma unroll
+            for (int q = 0; q < 4; q += 2) {
+                if (!from[q]) continue;
+                uint32_t a = (i & 1) * p.mt * 512;
+#pragma unroll 1
+                for (uint32_t c = 0; c < cnt; c += 2, a += 2 * step) {  // two units of two blocks are on their way together
+                    uint4 v[2][2];
+#pragma unroll
+                    for (int k = 0; k < 2; ++k)
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) v[k][u] = from[q + u] && c + k < cnt ? sld128(from[q + u] + a + k * step) : make_uint4(ZERO, ZERO, ZERO, ZERO);
+#pragma unroll
+                    for (int k = 0; k < 2; ++k)
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            float* s = &sum[q >> 1][u * 4];
+                            s[0] = __fadd_rn(s[0], __uint_as_float(v[k][u].x));
+                            s[1] = __fadd_rn(s[1], __uint_as_float(v[k][u].y));
+                            s[2] = __fadd_rn(s[2], __uint_as_float(v[k][u].z));
+                            s[3] = __fadd_rn(s[3], __uint_as_float(v[k][u].w));
+                        }
+                }
+            }
+            __syncwarp();
+            if ((uint32_t)lane < cs) mbar_arrive_remote(mapa(sbase + KF_FREE + 8 * (i & 1), lane));
+            return true;
+        };
+        if constexpr (CLUSTER) cluster_wait();  // the barriers of all CTAs exist
         uint32_t unit = unit0, b = 0, tiles = 0;
+        bool ok = true;
         for (uint32_t i = 0; i < total; ++i) {
             const uint32_t q = i % KF_NQ, buf = i & 1, m0 = unit % p.nct * p.mt;
-            if (!wait(KF_REC_FULL + 8 * q, (i / KF_NQ) & 1, STATUS_TIMEOUT_FULL)) break;
+            if (!wait(KF_REC_FULL + 8 * q, (i / KF_NQ) & 1, STATUS_TIMEOUT_FULL)) {
+                ok = false;
+                break;
+            }
             const uint8_t* rec = smem + p.off_rec + q * KF_REC;
             const uint32_t dm = reinterpret_cast<const uint32_t*>(rec)[r];
             const float d = f16bits_to_f32(dm & 0xFFFF), dmin = f16bits_to_f32(dm >> 16);
-            if (b == 0)
+            if (CLUSTER ? i == 0 : b == 0)
 #pragma unroll
                 for (int c = 0; c < CHUNKS; ++c)
 #pragma unroll
                     for (int j = 0; j < 8; ++j) sum[c][j] = 0.f;
-            if (!wait(KF_ACC_FULL + 8 * buf, (i >> 1) & 1, STATUS_TIMEOUT_MMA)) break;
+            if (CLUSTER && i >= 2 && !wait(KF_FREE + 8 * buf, ((i >> 1) & 1) ^ 1, STATUS_TIMEOUT_EMPTY)) {
+                ok = false;
+                break;
+            }
+            if (!wait(KF_ACC_FULL + 8 * buf, (i >> 1) & 1, STATUS_TIMEOUT_MMA)) {
+                ok = false;
+                break;
+            }
             tc_after();
 #pragma unroll
             for (int c = 0; c < CHUNKS; ++c) {
@@ -509,9 +589,10 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
                         t[j] = __fmul_rn(__fmul_rn(d, e[j]), (float)(int)(v[j] + (vh[j] << HI_SHIFT)));
                         if constexpr (MIN) t[j] = __fsub_rn(t[j], __fmul_rn(__fmul_rn(dmin, e[j]), __uint_as_float(u[j])));
                     }
-                    if (p.terms) {
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) xch[(b * p.mt + col + j) * 128 + r] = t[j];
+                    if constexpr (CLUSTER) {
+                        const uint32_t dst = to + (buf * p.mt * 128 + col * lines) * 4, bar = to_bar + 8 * buf;
+                        st_async4(dst, t[0], t[1], t[2], t[3], bar);
+                        st_async4(dst + lines * 16, t[4], t[5], t[6], t[7], bar);
                     } else {
 #pragma unroll
                         for (int j = 0; j < 8; ++j) sum[c][j] = __fadd_rn(sum[c][j], t[j]);
@@ -524,19 +605,17 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
                 mbar_arrive(sbase + KF_ACC_EMPTY + 8 * buf);
                 mbar_arrive(sbase + KF_REC_EMPTY + 8 * q);
             }
+            if constexpr (CLUSTER) {
+                if (i > 0 && !collect(i - 1)) {
+                    ok = false;
+                    break;
+                }
+                continue;
+            }
             if (++b < nb) continue;
             b = 0;
             const uint32_t n = unit / p.nct * rows + r;
             unit += stride;
-            if (p.cs > 1) {
-                if (!p.terms)
-#pragma unroll
-                    for (int c = 0; c < CHUNKS; ++c)
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            if (8 * (cg + 2 * c) < p.mt) xch[(8 * (cg + 2 * c) + j) * 128 + r] = sum[c][j];
-                continue;
-            }
             if (p.swiglu) {  // the lanes of up hand their sums to those of gate; two buffers, so one meeting a tile is enough
                 float* to = xch + (tiles & 1) * p.mt * 64 + (r & 63);
                 if (r >= 64)
@@ -565,28 +644,29 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
                         if (m < p.mt && m0 + m < p.M) kf_store(p.out, p.out_dtype, (size_t)(m0 + m) * p.N + n, sum[c][j]);
                     }
         }
-    }
-    __syncwarp();
-    if (p.cs > 1) {
-        // The shares of K meet: CTA `rank` adds them for every cs-th activation row of the tile and writes the results.
-        cluster_sync_all();
-        if (!*dead) {
-            const uint32_t m0 = unit0 % p.nct * p.mt, in = min(p.mt, p.M - m0), n0 = unit0 / p.nct * rows, x0 = sbase + p.off_x;
-            for (uint32_t t = threadIdx.x; t < (in > rank ? (in - rank + p.cs - 1) / p.cs : 0) * rows; t += KF_THREADS) {
-                const uint32_t m = rank + t / rows * p.cs, r = t % rows;
-                float s[2] = {0.f, 0.f};
-                for (uint32_t c = 0; c < p.cs; ++c) {
-                    const uint32_t cnt = p.terms ? (c + 1) * p.nblk / p.cs - c * p.nblk / p.cs : 1, from = mapa(x0, c) + (m * 128 + r) * 4;
-#pragma unroll 4
-                    for (uint32_t j = 0; j < cnt; ++j) {
-                        s[0] = __fadd_rn(s[0], ld_cluster(from + j * p.mt * 512));
-                        if (p.swiglu) s[1] = __fadd_rn(s[1], ld_cluster(from + j * p.mt * 512 + 256));
+        // the rounds that are left: the last one, and the one before where this CTA had no block in the last
+        if (CLUSTER)
+            for (uint32_t i = total - 1; ok && i < rounds; ++i) ok = collect(i);
+        if (CLUSTER && ok) {
+            const uint32_t n0 = unit0 / p.nct * rows + (rank << own_log), m0 = unit0 % p.nct * p.mt;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const uint32_t n = n0 + (unit_of(q) & (own - 1)), m = (unit_of(q) >> own_log) * 4;
+                if (n < p.N && from[q] && (q < 2 || !p.swiglu))
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        float v = sum[q >> 1][(q & 1) * 4 + j];
+                        if (q < 2 && p.swiglu) v = kf_gate(v, sum[1][(q & 1) * 4 + j]);
+                        if (m + j < in) kf_store(p.out, p.out_dtype, (size_t)(m0 + m + j) * p.N + n, v);
                     }
-                }
-                if (n0 + r < p.N) kf_store(p.out, p.out_dtype, (size_t)(m0 + m) * p.N + n0 + r, p.swiglu ? kf_gate(s[0], s[1]) : s[0]);
             }
         }
-        cluster_sync_all();  // nobody's shared memory goes before all have read it
+    }
+    __syncwarp();
+    if constexpr (CLUSTER) {  // nobody's shared memory goes before all have done with it
+        if (warp < KF_W_DRAIN || warp >= KF_W_COPY) cluster_wait();  // (the drain warps have waited for the barriers to exist)
+        cluster_arrive();
+        cluster_wait();
     }
     tc_before();
     __syncthreads();
@@ -598,13 +678,10 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
 
 struct KfPlan {
     uint32_t mt = 0, cs = 1;
-    bool terms = false;
     double us = 0;  // expected time behind the first block
 };
 constexpr uint32_t KF_SMEM = 232448;
-uint32_t kf_x_bytes(const KfPlan& pl, uint32_t nblk, bool swiglu) {
-    return pl.cs > 1 ? (pl.terms ? (nblk + pl.cs - 1) / pl.cs : 1u) * pl.mt * 512 : swiglu ? pl.mt * 512 : 0u;
-}
+uint32_t kf_x_bytes(const KfPlan& pl, bool swiglu) { return pl.cs > 1 ? 2 * pl.mt * 512 : swiglu ? pl.mt * 512 : 0u; }
 // Operand halves in tensor memory: at most one ahead of every set (KF_SET_EMPTY); activation blocks in shared memory.
 uint32_t kf_stages(int fmt, uint32_t mt) {
     const uint32_t n = (512 - 2 * (kf_min(fmt) ? 3 : 2) * mt - 16) / kf_half_cols(fmt);
@@ -612,17 +689,16 @@ uint32_t kf_stages(int fmt, uint32_t mt) {
 }
 uint32_t kf_acts(int fmt, uint32_t mt) { return kf_stages(fmt, mt) == 4 || mt <= 32 ? 4 : 3; }
 // packed blocks that fit beside the rest (even: a slot belongs to the sets of one block parity)
-uint32_t kf_ring(int fmt, const KfPlan& pl, uint32_t nblk, bool swiglu) {
-    const uint32_t fixed = 2048 + kf_acts(fmt, pl.mt) * kf_btile(pl.mt) + KF_NQ * KF_REC + kf_x_bytes(pl, nblk, swiglu);
-    if (fixed >= KF_SMEM) return 0;
+uint32_t kf_ring(int fmt, const KfPlan& pl, bool swiglu) {
+    const uint32_t fixed = 2048 + kf_acts(fmt, pl.mt) * kf_btile(pl.mt) + KF_NQ * KF_REC + kf_x_bytes(pl, swiglu);
     const uint32_t nr = (KF_SMEM - fixed) / kf_raw(fmt) & ~1u;
     return nr > KF_NR_MAX ? KF_NR_MAX : nr;
 }
 
-template <int FMT>
+template <int FMT, bool CLUSTER>
 cudaError_t kf_attr() {
     static PerDeviceOnce attrs;
-    return attrs.run([] { return cudaFuncSetAttribute(kq_few_kernel<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KF_SMEM); });
+    return attrs.run([] { return cudaFuncSetAttribute(kq_few_kernel<FMT, CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KF_SMEM); });
 }
 // Tiles of `cs` CTAs that can run at the same time.
 uint32_t kf_clusters(uint32_t cs) {
@@ -643,7 +719,7 @@ uint32_t kf_clusters(uint32_t cs) {
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (kf_attr<FMT_Q4_K>() != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kq_few_kernel<FMT_Q4_K>, &cfg) != cudaSuccess) {
+    if (kf_attr<FMT_Q4_K, true>() != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kq_few_kernel<FMT_Q4_K, true>, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -653,8 +729,8 @@ uint32_t kf_clusters(uint32_t cs) {
 
 // Tile and cluster of least time, in us: blocks of K one after the other x the time of one (a line in mt, measured at 14336 x
 // 4096: 16 / 32 / 48 rows Q4_K 0.86 / 0.99 / 1.14, Q5_K 1.02 / 1.18 / 1.32, Q6_K 1.31 / 1.37 / 1.45, or 1.97 where
-// its rows are no multiple of 16 bytes: 13825 x 5120), and 3.4 for the meeting of a
-// cluster (2048 x 2048 and 4096 x 4096 against whole tiles).
+// its rows are no multiple of 16 bytes: 13825 x 5120).  In a cluster the exchange of a block's terms takes 0.15 + 0.0075 a row more, and 0.7 once
+// (fitted to 512 ... 9216 weight rows, K = 1024 ... 14336).
 KfPlan kf_plan(int fmt, size_t M, size_t K, size_t row_tiles, bool swiglu, int sm_count, bool estimate = false) {
     KfPlan best;
     const uint32_t nblk = (uint32_t)(K / 256);
@@ -665,10 +741,9 @@ KfPlan kf_plan(int fmt, size_t M, size_t K, size_t row_tiles, bool swiglu, int s
             KfPlan c;
             c.mt = mt;
             c.cs = cs;
-            c.terms = cs > 1 && nblk <= 16;
-            if (cs > 1 && (units * cs > (size_t)sm_count || kf_ring(fmt, c, nblk, swiglu) < 2 || (!estimate && units > kf_clusters(cs)))) continue;
+            if (cs > 1 && (units * cs > (size_t)sm_count || (!estimate && units > kf_clusters(cs)))) continue;
             const size_t blocks = cs > 1 ? (nblk + cs - 1) / cs : (units + sm_count - 1) / sm_count * nblk;
-            c.us = (double)blocks * (c0 + c1 * mt) + (cs > 1 ? 3.4 : 0.0);
+            c.us = (double)blocks * (c0 + c1 * mt + (cs > 1 ? 0.15 + 0.0075 * mt : 0.0)) + (cs > 1 ? 0.7 : 0.0);
             if (!best.mt || c.us < best.us) best = c;
         }
         if (mt >= M) break;
@@ -684,9 +759,9 @@ bool kf_encode(CUtensorMap* map, CUtensorMapDataType type, size_t elem, const vo
                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int FMT>
+template <int FMT, bool CLUSTER>
 cudaError_t kf_launch(const CUtensorMap& am, const CUtensorMap& sm, const CUtensorMap* wm, const KfParams& p, uint32_t grid, size_t smem, cudaStream_t st) {
-    cudaError_t e = kf_attr<FMT>();
+    cudaError_t e = kf_attr<FMT, CLUSTER>();
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
@@ -700,8 +775,8 @@ cudaError_t kf_launch(const CUtensorMap& am, const CUtensorMap& sm, const CUtens
     at[1].val.clusterDim.x = p.cs;
     at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = p.cs > 1 ? 2 : 1;
-    e = cudaLaunchKernelEx(&cfg, kq_few_kernel<FMT>, am, sm, wm[0], wm[1], p);
+    cfg.numAttrs = CLUSTER ? 2 : 1;
+    e = cudaLaunchKernelEx(&cfg, kq_few_kernel<FMT, CLUSTER>, am, sm, wm[0], wm[1], p);
     note_launch();
     return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -761,10 +836,10 @@ cudaError_t launch_kq_few(int fmt, const void* act, int act_dtype, const void* w
     p.nct = (uint32_t)((M + pl.mt - 1) / pl.mt);
     p.nunits = rt * p.nct;
     p.cs = pl.cs;
-    p.terms = pl.cs > 1 && pl.terms;
+    p.cs_log = pl.cs == 8 ? 3 : pl.cs == 4 ? 2 : pl.cs == 2 ? 1 : 0;
     p.ns = kf_stages(fmt, pl.mt);
     p.nb = kf_acts(fmt, pl.mt);
-    p.nr = kf_ring(fmt, pl, nblk, swiglu);
+    p.nr = kf_ring(fmt, pl, swiglu);
     p.off_rec = KF_STAGES + p.nb * kf_btile(pl.mt);
     p.off_raw = p.off_rec + KF_NQ * KF_REC;
     p.off_x = p.off_raw + p.nr * kf_raw(fmt);
@@ -789,10 +864,14 @@ cudaError_t launch_kq_few(int fmt, const void* act, int act_dtype, const void* w
         return cudaErrorInvalidValue;
     }
     const uint32_t grid = pl.cs > 1 ? p.nunits * pl.cs : p.nunits < (uint32_t)sm_count ? p.nunits : (uint32_t)sm_count;
-    const size_t smem = 1024 + p.off_x + kf_x_bytes(pl, nblk, swiglu);
-    return fmt == FMT_Q4_K   ? kf_launch<FMT_Q4_K>(am, sm, wm, p, grid, smem, st)
-           : fmt == FMT_Q5_K ? kf_launch<FMT_Q5_K>(am, sm, wm, p, grid, smem, st)
-                             : kf_launch<FMT_Q6_K>(am, sm, wm, p, grid, smem, st);
+    const size_t smem = 1024 + p.off_x + kf_x_bytes(pl, swiglu);
+    if (pl.cs > 1)
+        return fmt == FMT_Q4_K   ? kf_launch<FMT_Q4_K, true>(am, sm, wm, p, grid, smem, st)
+               : fmt == FMT_Q5_K ? kf_launch<FMT_Q5_K, true>(am, sm, wm, p, grid, smem, st)
+                                 : kf_launch<FMT_Q6_K, true>(am, sm, wm, p, grid, smem, st);
+    return fmt == FMT_Q4_K   ? kf_launch<FMT_Q4_K, false>(am, sm, wm, p, grid, smem, st)
+           : fmt == FMT_Q5_K ? kf_launch<FMT_Q5_K, false>(am, sm, wm, p, grid, smem, st)
+                             : kf_launch<FMT_Q6_K, false>(am, sm, wm, p, grid, smem, st);
 }
 
 }  // namespace b200q

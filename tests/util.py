@@ -30,3 +30,18 @@ def seed_of(*parts) -> int:
     import zlib
 
     return zlib.crc32(repr(parts).encode()) % 1000
+
+
+def kq_tile_rows(fmt, m, n, k):
+    """Activation rows of the tensor-core tile that the library's own rule gives a K-quant product (0: kernel for few rows, -1: another
+    path)."""
+    import ctypes
+
+    import torch
+
+    from boostr_b200 import _cabi
+    from boostr_b200.format import QuantFormat
+
+    f = _cabi.lib().b200q_kq_tile_rows
+    f.restype, f.argtypes = ctypes.c_int, [ctypes.c_int, ctypes.c_size_t, ctypes.c_size_t, ctypes.c_size_t, ctypes.c_int]
+    return f(QuantFormat[fmt].format_id, m, k, n, torch.cuda.get_device_properties(0).multi_processor_count)
