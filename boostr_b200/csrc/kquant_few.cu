@@ -616,26 +616,31 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
             b = 0;
             const uint32_t n = unit / p.nct * rows + r;
             unit += stride;
-            if (p.swiglu) {  // the lanes of up hand their sums to those of gate; two buffers, so one meeting a tile is enough
-                float* to = xch + (tiles & 1) * p.mt * 64 + (r & 63);
-                if (r >= 64)
+            if (p.swiglu) {
+                // A lane of gate and its lane of up swap half of their sums, so that both gate and store half of the row's results; two
+                // buffers, so one meeting a tile is enough.
+                const bool up = r >= 64;  // warp-uniform
+                float* swap = xch + (tiles & 1) * p.mt * 64 + (r & 63);
 #pragma unroll
-                    for (int c = 0; c < CHUNKS; ++c)
+                for (int c = 0; c < CHUNKS; ++c)
 #pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            if (8 * (cg + 2 * c) < p.mt) to[(8 * (cg + 2 * c) + j) * 64] = sum[c][j];
+                    for (int j = 0; j < 4; ++j)
+                        if (8 * (cg + 2 * c) < p.mt) swap[(8 * (cg + 2 * c) + j + (up ? 0 : 4)) * 64] = up ? sum[c][j] : sum[c][j + 4];
                 __syncwarp();
                 if (lane == 0) mbar_arrive(sbase + KF_MEET);
                 if (!wait(KF_MEET, tiles & 1, STATUS_TIMEOUT_EMPTY)) break;
                 ++tiles;
-                if (r < 64)
 #pragma unroll
-                    for (int c = 0; c < CHUNKS; ++c)
+                for (int c = 0; c < CHUNKS; ++c)
 #pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            if (8 * (cg + 2 * c) < p.mt) sum[c][j] = kf_gate(sum[c][j], to[(8 * (cg + 2 * c) + j) * 64]);
-            }
-            if (n < p.N && (!p.swiglu || r < 64))
+                    for (int j = 0; j < 4; ++j) {
+                        const uint32_t mr = 8 * (cg + 2 * c) + j + (up ? 4 : 0);
+                        if (mr < p.mt && m0 + mr < p.M && n - (up ? 64 : 0) < p.N) {
+                            const float other = swap[mr * 64], own_sum = up ? sum[c][j + 4] : sum[c][j];
+                            kf_store(p.out, p.out_dtype, (size_t)(m0 + mr) * p.N + n - (up ? 64 : 0), up ? kf_gate(other, own_sum) : kf_gate(own_sum, other));
+                        }
+                    }
+            } else if (n < p.N) {
 #pragma unroll
                 for (int c = 0; c < CHUNKS; ++c)
 #pragma unroll
@@ -643,6 +648,7 @@ __global__ void __launch_bounds__(KF_THREADS, 1) kq_few_kernel(const __grid_cons
                         const uint32_t m = 8 * (cg + 2 * c) + j;
                         if (m < p.mt && m0 + m < p.M) kf_store(p.out, p.out_dtype, (size_t)(m0 + m) * p.N + n, sum[c][j]);
                     }
+            }
         }
         // the rounds that are left: the last one, and the one before where this CTA had no block in the last
         if (CLUSTER)
