@@ -33,6 +33,7 @@
 
 #include <cstdio>
 
+#include "../../include/b200q.h"
 #include "common.cuh"
 #include "tcgen05_i8.cuh"
 #include "tmap.cuh"
@@ -41,6 +42,7 @@ namespace b200q {
 
 bool smallm_i8_preferred(int fmt, size_t M, size_t K, size_t N, int sm_count);
 size_t kq_i8_workspace_bytes(size_t M, size_t K);
+size_t gemv_workspace_bytes(int fmt, size_t M, size_t K, size_t N, bool swiglu, int sm_count);
 cudaError_t launch_kq_prep(const void* act, int act_dtype, size_t M, size_t K, void* ws, bool early, int sm_count, cudaStream_t st);
 void kq_image(void* ws, size_t M, size_t K, uint8_t** codes, __half** sums, float** d8);
 
@@ -789,8 +791,10 @@ cudaError_t kf_launch(const CUtensorMap& am, const CUtensorMap& sm, const CUtens
 
 }  // namespace
 
-// From 17 rows on one pass here beats passes of 16 rows by mma.sync (gemv.cu); of 91 products between 24 and 63 rows two are 1 ... 2 %
-// slower (1024 x 4096 at 24 rows, Q5_K 11.25 -> 11.4 us, Q6_K 11.55 -> 11.8), the mean takes 0.69 of the time.  At 9 ... 16 rows the two are
+// From 17 rows on one pass here beats passes of 16 rows by mma.sync (gemv.cu), except where K is long and the matrix has so few tiles that
+// clusters of 8 leave SMs idle, which the other kernel's chunks of K occupy (5 us a pass, and 0.12 ... 0.15 more for every tile of 128 rows
+// and chunk past the tenth): Q6_K at 17 rows 64 x 28672 13.4 us there, 24.3 here, 512 x 14336 13.9 and 15.2, 1024 x 14336 18.8 and 16.3; at 48 rows 512 x 14336
+// 20.4 and 15.4.  At 9 ... 16 rows the two are
 // even on most shapes (14336 x 4096 at 16 rows: Q6_K 24.2 there, 25.0 here) and this kernel wins where the other's fixed shares of K (chunks of 16
 // blocks; 5 + 0.13 ... 0.155 us a tile of 128 rows and chunk) are badly filled: 13825 x 5120 at 13 rows Q4_K 30.6 -> 21.1, Q5_K 34.9 -> 24.4; 14336 x
 // 2048 Q5_K 20.1 -> 12.4, Q6_K 20.1 -> 14.3; SwiGLU 2 x 5632 x 2048 17.8 -> 12.4, 20.7 -> 14.0, 19.5 -> 14.9.  Up to 8 rows mma.sync is 1.1 ... 1.9 times as fast.
@@ -798,11 +802,17 @@ bool kq_few_supported(int fmt, size_t M, size_t K, size_t N, bool swiglu, int sm
     if ((fmt != FMT_Q4_K && fmt != FMT_Q5_K && fmt != FMT_Q6_K) || M < 9 || M >= 64 || K < 256 || K % 256 != 0 || K > 65536 || N < 1 ||
         !tma_available())
         return false;
-    if (M >= 17) return true;
+    const size_t nblk = K / 256, row_tiles = swiglu ? (N + 63) / 64 : (N + 127) / 128, tiles = (N + 127) / 128 * (swiglu ? 2 : 1), chunks = tiles * ((nblk + 15) / 16);
+    if (M >= 17) {
+        if (swiglu || 8 * tiles > (size_t)sm_count) return true;
+        const double pass = fmt == FMT_Q4_K ? 4.6 : fmt == FMT_Q5_K ? 5.0 : 5.2, more = fmt == FMT_Q4_K ? 0.12 : fmt == FMT_Q5_K ? 0.14 : 0.15;
+        const double there = 2.5 + (double)((M + 15) / 16) * (pass + (chunks > 10 ? more * (double)(chunks - 10) : 0.0));
+        // (a call without scratch of its own must not come to need more than there is: its partial sums grow with K, M and N)
+        return 4.2 + kf_plan(fmt, M, K, row_tiles, false, sm_count, true).us < 1.05 * there ||
+               gemv_workspace_bytes(fmt, M, K, N, false, sm_count) > B200Q_STATIC_SCRATCH_BYTES;
+    }
     if (smallm_i8_preferred(fmt, M, K, N, sm_count)) return false;
-    const size_t nblk = K / 256, tiles = (N + 127) / 128 * (swiglu ? 2 : 1);
-    const double there = 5.0 + (double)(tiles * ((nblk + 15) / 16)) * (fmt == FMT_Q4_K ? 0.128 : fmt == FMT_Q5_K ? 0.155 : 0.13);
-    const size_t row_tiles = swiglu ? (N + 63) / 64 : (N + 127) / 128;
+    const double there = 5.0 + (double)chunks * (fmt == FMT_Q4_K ? 0.128 : fmt == FMT_Q5_K ? 0.155 : 0.13);
     // (the estimate spares shapes that stay with the other kernel the question how many clusters fit, which loads this one)
     return 4.0 + kf_plan(fmt, M, K, row_tiles, swiglu, sm_count, true).us < 0.95 * there && 4.0 + kf_plan(fmt, M, K, row_tiles, swiglu, sm_count).us < 0.95 * there;
 }

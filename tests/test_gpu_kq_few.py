@@ -39,14 +39,30 @@ def test_products(oracle, fmt, m, n, k):
     got = out.cpu().numpy()
     assert (flat[:guard] == 4242.0).all() and (flat[guard + m * n:] == 4242.0).all(), "guard regions were written"
     want = oracle.quant_matmul(fmt, act, w, n, threads=os.cpu_count() or 8)
-    if kq_tile_rows(fmt, m, n, k) > 0:
+    if m > 16 or kq_tile_rows(fmt, m, n, k) > 0:
         assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), describe_mismatch(got, want)
     else:  # mma.sync is expected to be faster: its chunks of K are added as sums
-        assert m <= 16 and rel_err(got, want)[0] <= 2e-6, describe_mismatch(got, want)
+        assert rel_err(got, want)[0] <= 2e-6, describe_mismatch(got, want)
     for _ in range(20):
         again = ops.quant_matmul(x, qt)
     assert torch.equal(again.view(torch.int32), out.view(torch.int32))
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("fmt", ["Q4_K", "Q5_K", "Q6_K"])
+@pytest.mark.parametrize("m,n,k", [(17, 64, 28672), (20, 130, 28672), (32, 256, 28672), (33, 100, 28672), (63, 1, 65536), (17, 400, 65536)])
+def test_few_weight_rows_of_long_k(oracle, fmt, m, n, k):
+    """Too few tiles for the chip: mma.sync shares K out over all of it, and its chunks of K are added as sums."""
+    from boostr_b200 import ops
+
+    assert kq_tile_rows(fmt, m, n, k) == -1
+    rng = synth.rng_for(103, seed_of(fmt, m, n, k))
+    act = synth.activations(rng, m, k)
+    w = synth.weight_bytes(fmt, rng, n, k)
+    got = ops.quant_matmul(torch.from_numpy(act).cuda(), QuantTensor.from_bytes(w, F[fmt], (n, k), device="cuda")).cpu().numpy()
+    ops.check_device_status()
+    want = oracle.quant_matmul(fmt, act, w, n, threads=os.cpu_count() or 8)
+    assert rel_err(got, want)[0] <= 2e-6, describe_mismatch(got, want)
 
 
 @pytest.mark.parametrize("fmt", ["Q4_K", "Q5_K", "Q6_K"])
