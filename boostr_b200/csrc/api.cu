@@ -226,13 +226,11 @@ cudaError_t launch_i8_passes(int format, const void* act, int act_dtype, const v
 }
 
 // Which prepared form of the activations (in scratch) a product reads; -1: none that another weight of a batch could
-// share.  The integer tensor-core K-quant paths have one image, which depends on M and K only (above 32 rows the launches of a
-// batch are what they were before Q4_K and Q6_K read it: those prepare their own); the bf16 tensor-core path prepares one form per class of formats
-// (K-quants: Q8_K round trip; others: bf16);
+// share.  The integer tensor-core K-quant paths have one image, which depends on M and K only; the bf16 tensor-core path prepares
+// one form per class of formats (K-quants: Q8_K round trip; others: bf16);
 // the mma.sync small-M kernel one image per format (Q5_K reads Q4_K's).
 int prepared_class(int format, size_t M, size_t K, size_t N) {
-    if (kq_few_supported(format, M, K, N, false, sm_count_current()) || kq_i8_supported(format, M, K, N))
-        return M <= 32 || format == FMT_Q2_K || format == FMT_Q3_K || format == FMT_Q5_K ? 102 : -1;
+    if (kq_few_supported(format, M, K, N, false, sm_count_current()) || kq_i8_supported(format, M, K, N)) return 102;
     if (prefill_supported(format, M, K, N)) return (format == FMT_Q4_K || format == FMT_Q5_K || format == FMT_Q6_K) ? 101 : 100;
     if (gemv_m1_supported(format, M, K, N, false) || gemv_m1_f32_supported(format, M, K, N)) return -1;
     if (smallm_i8_preferred(format, M, K, N, sm_count_current()) || i8_in_passes(format, M, K, N)) return -1;

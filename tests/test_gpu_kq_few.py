@@ -102,3 +102,45 @@ def test_swiglu(fmt, m, n, k):
     want = a / (1 + torch.exp(-a)) * b
     # the same products; expf within 2 ulp, three more roundings (4 * 2^-23)
     assert ((got.double() - want).abs() <= 5e-7 * want.abs() + 1e-36 * b.abs()).all()
+
+
+@pytest.mark.parametrize("reverse", [False, True])
+@pytest.mark.parametrize("m", [17, 24, 32, 33, 48, 63])
+def test_batch_shares_one_image(m, reverse):
+    """All K-quant weights of a batch of 17 ... 63 rows read one image of the activations, whatever their order, and give the bits of
+    separate calls."""
+    from boostr_b200 import ops
+
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(m)
+    k = 1536
+    specs = [("Q4_K", 1500), ("Q6_K", 300), ("Q2_K", 300), ("Q5_K", 2100), ("Q3_K", 200), ("Q4_K", 129), ("Q6_K", 2049)]
+    ws = [synth.device_weight(fmt, n, k, gen) for fmt, n in (reversed(specs) if reverse else specs)]
+    x = torch.randn(m, k, device="cuda", generator=gen)
+    want = [ops.quant_matmul(x, w) for w in ws]
+    before = ops.launch_count()
+    got = ops.quant_matmul_batch(x, ws)
+    assert ops.launch_count() - before == 1 + len(ws)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    ops.check_device_status()
+
+
+@pytest.mark.parametrize("reverse", [False, True])
+@pytest.mark.parametrize("m", [9, 13, 16])
+def test_batch_that_changes_the_kernel(m, reverse):
+    """At 9 ... 16 rows the weights of a batch go to this kernel and to mma.sync in turn: each finds its own image in the scratch."""
+    from boostr_b200 import ops
+
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(m)
+    k = 2048
+    specs = [("Q5_K", 14336), ("Q5_K", 1024), ("Q6_K", 14336), ("Q4_K", 1024), ("Q2_K", 300), ("Q5_K", 14336), ("Q6_K", 512), ("Q4_K", 200)]
+    ws = [synth.device_weight(fmt, n, k, gen) for fmt, n in (reversed(specs) if reverse else specs)]
+    tiles = [kq_tile_rows(w.format.name, m, *w.shape) for w in ws if w.format is not F.Q2_K]
+    assert max(tiles) > 0 and min(tiles) < 0
+    x = torch.randn(m, k, device="cuda", generator=gen)
+    want = [ops.quant_matmul(x, w) for w in ws]
+    for a, b in zip(ops.quant_matmul_batch(x, ws), want):
+        assert torch.equal(a, b)
+    ops.check_device_status()
