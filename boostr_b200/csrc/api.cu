@@ -193,8 +193,9 @@ size_t workspace_need(int op, int format, int act_dtype, size_t M, size_t K, siz
     // small-M kernel: the activation image, plus split-K partial sums when K is long
     if (smallm_i8_preferred(format, M, K, N, sm_count_current()))  // integer tensor-core kernel (+ gate and up for SwiGLU)
         return smallm_i8_workspace_bytes(format, M, K, N, sm_count_current()) + (swiglu ? 2 * ((M * N * sizeof(float) + 255) & ~(size_t)255) : 0);
-    if (!swiglu && i8_in_passes(format, M, K, N)) {  // passes of 32 rows; a last pass of one row uses the mma.sync kernel's scratch
-        const size_t a = smallm_i8_workspace_bytes(format, 32, K, N, sm_count_current()), b = gemv_workspace_bytes(format, 1, K, N, false, sm_count_current());
+    if (!swiglu && i8_in_passes(format, M, K, N)) {  // 32 rows, then the rest: up to 16 rows of it by the mma.sync kernel
+        const size_t a = smallm_i8_workspace_bytes(format, 32, K, N, sm_count_current());
+        const size_t b = M - 32 <= 16 ? gemv_workspace_bytes(format, M - 32, K, N, false, sm_count_current()) : 0;
         return a > b ? a : b;
     }
     return gemv_workspace_bytes(format, M, K, N, swiglu, sm_count_current());
@@ -216,10 +217,10 @@ cudaError_t launch_i8_passes(int format, const void* act, int act_dtype, const v
         const size_t rows = M - m0 < 32 ? M - m0 : 32;
         const void* a = static_cast<const uint8_t*>(act) + m0 * K * dtype_bytes(act_dtype);
         void* o = static_cast<uint8_t*>(out) + m0 * N * dtype_bytes(out_dtype);
-        if (rows >= 2 && smallm_i8_supported(format, rows, K, N))
+        if (smallm_i8_supported(format, rows, K, N))
             e = launch_smallm_i8(format, a, act_dtype, w, o, out_dtype, rows, K, N, ws, ws_bytes, sm_count_current(), st, status, small, msg, msg_len,
                                  false);
-        else  // a last pass of one row (or of a row count the kernels do not take): the mma.sync kernel
+        else  // a last pass of up to 16 rows: the mma.sync kernel
             e = launch_gemv(format, a, act_dtype, w, nullptr, o, out_dtype, rows, K, N, ws, ws_bytes, false, sm_count_current(), st, status, small);
     }
     return e;

@@ -241,3 +241,24 @@ def test_33_to_63_rows_in_passes_of_32(ops, oracle, fmt, m, n, k, tol):
         assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), describe_mismatch(got, want)
     else:
         assert rel_err(got, want)[0] <= tol, describe_mismatch(got, want)
+
+
+@pytest.mark.parametrize("m", [33, 40, 48, 49, 63])
+def test_passes_fit_the_scratch_they_ask_for(ops, oracle, m):
+    # the last pass may be one of the mma.sync kernel, whose partial sums of a long K need more than the images of 32 rows
+    from boostr_b200 import _cabi
+    from boostr_b200.tensor import QuantTensor
+
+    n, k, fid = 9600, 8192, F.Q8_0.format_id
+    rng = synth.rng_for(99, m)
+    act, w = synth.activations(rng, m, k), synth.weight_bytes("Q8_0", rng, n, k)
+    qt, x, out = QuantTensor.from_bytes(w, F.Q8_0, (n, k), device="cuda"), torch.from_numpy(act).cuda(), torch.empty(m, n, device="cuda")
+    lib = _cabi.lib()
+    need = lib.b200q_workspace_bytes(_cabi.OP_QUANT_MATMUL, fid, m, k, n)
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+    rc = lib.b200q_quant_matmul(fid, x.data_ptr(), _cabi.DT_F32, qt.storage.data_ptr(), out.data_ptr(), _cabi.DT_F32, m, k, n, ws.data_ptr(), need,
+                                torch.cuda.current_stream().cuda_stream)
+    assert rc == 0, lib.b200q_last_error()
+    ops.check_device_status()
+    want = oracle.quant_matmul("Q8_0", act, w, n, threads=_threads())
+    assert rel_err(out.cpu().numpy(), want)[0] <= 1e-4
