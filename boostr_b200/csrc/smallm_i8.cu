@@ -1,12 +1,11 @@
-// Small-M quantized matmul (2 <= M <= 16) for Q4_K on the 5th-generation tensor cores' INTEGER path:
+// Small-M quantized matmul (8 <= M <= 16) for Q4_K on the 5th-generation tensor cores' INTEGER path:
 //   out[M,N] = act[M,K] x W[N,K]^T  with boostr's CPU arithmetic (activations quantised to Q8_K,
 //   src/quant/cpu/kernels/simd/quantize_act_q8k.rs:26-98; per 256-block (d*d8)*sumi - (dmin*d8)*sumi_mins with exact
 //   integer sums, src/quant/cpu/kernels/simd/fused_q4k_q8k_dot.rs:111-172).
 //
 // The mma.sync kernel (gemv.cu) spends ~540 warp instructions per (16 weight rows x 256 K x 16 activation rows), is bound
-// by instruction issue, and takes more than 16 activation rows in several passes over the weights.  Here ONE
-// tcgen05.mma.kind::i8 (128 weight rows x MP activation rows x 32 K) computes the integer dot products of a whole
-// 32-wide sub-block for 128 rows, and the per-sub-block scales are applied by the warps that drain the accumulator:
+// by instruction issue.  Here ONE tcgen05.mma.kind::i8 (128 weight rows x 16 activation rows x 32 K) computes the integer dot
+// products of a whole 32-wide sub-block for 128 rows, and the per-sub-block scales are applied by the warps that drain the accumulator:
 //   * tile = 128 weight rows (the MMA's M = the 128 lanes of tensor memory); the activations are the B operand,
 //     MP = 16 rows (MMA N); every 32-wide sub-block j of a 256-block gets its OWN accumulator columns
 //     [MP j, MP j + MP), so no scale has to enter the tensor core; tensor memory holds two such accumulators;
@@ -20,10 +19,7 @@
 //     weight row and half of the activation rows), read the 8 x MP integer sums from tensor memory, form
 //     sumi = sum_j sc_j dot_j and sumi_mins = sum_j m_j bsum_j in integers and the block's f32 term; the running f32
 //     sums pass from team to team through shared memory, so the blocks are still added in K order;
-//   * work = (tile, block) pairs dealt to the CTAs as equal contiguous ranges.  Where the matrix has enough tiles the
-//     ranges are whole tiles and the result has the CPU's bits.  Otherwise a range may cut a tile along K: such pieces
-//     go to scratch as f32 partial tiles and the CTA that writes a tile's last piece (a counter per tile) adds them in
-//     K order; a cut tile differs from the CPU's bits by f32 rounding only (the grouping of the sum).
+//   * work = whole tiles, dealt to the CTAs as equal contiguous ranges: the result has the CPU's bits.
 // What bounds it: the drain is ~200 instructions per (weight row, 8 activation rows, block), about 2600 warp
 // instructions per (128 rows x 256 K x 16 activation rows) for the whole CTA against ~4300 in the mma.sync kernel.
 // Every mbarrier wait is bounded; on a timeout the CTA records a status code and still frees its tensor memory.
@@ -38,18 +34,11 @@
 namespace b200q {
 
 struct I8Params {
-    const uint8_t* w;
     void* out;
-    float* part;          // [slot][MP][128] f32 pieces of cut tiles
-    unsigned int* cnt;    // [ntiles] pieces of a cut tile that have been written; 0 between calls
-    const uint8_t* aux;   // [nblk][aux_bytes(MP)]: per block the eight int16 sums of 32 codes of every activation row, then the rows' Q8_K scales
-    uint32_t M, N, K;
-    uint32_t MP;          // activation rows of the MMA (16 or 32)
-    uint32_t nblk;        // K / 256
-    uint32_t ntiles;      // ceil(N / 128)
-    uint32_t Q;           // ntiles * nblk (tile, block) pairs
-    uint32_t unit;        // pairs are dealt in items of `unit` pairs: 1, or nblk (whole tiles: nothing is cut)
-    uint32_t qbase, qrem; // items / grid and items % grid: CTA c takes items [c qbase + min(c, qrem), ...)
+    const uint8_t* aux;     // [nblk][AUX_BYTES]: per block the eight int16 sums of 32 codes of every activation row, then the rows' Q8_K scales
+    uint32_t M, N;
+    uint32_t nblk;          // K / 256
+    uint32_t tbase, trem;   // tiles / grid and tiles % grid: CTA c takes tiles [c tbase + min(c, trem), ...)
     uint32_t ns;          // ring depth of operand stages (one 256-block each)
     uint32_t nr;          // ring depth of packed-weight tiles
     uint32_t nsc;         // ring depth of the scale records
@@ -68,39 +57,16 @@ constexpr uint32_t RAW_PITCH = 144, RAW_TILE = 128 * RAW_PITCH;  // 18432 = 18 x
 constexpr uint32_t A_ATOM = 128 * 128;                            // 128 rows x 128 codes
 constexpr uint32_t SC_WORDS = 5;                                  // d|dmin, 8 scales, 8 mins
 constexpr uint32_t SC_REC = 128 * SC_WORDS * 4;                  // the 128 row records of a block
-constexpr uint32_t SC_SLOT = SC_REC + 32 * 20;                    // + the activation side of the block (aux_bytes(32))
-__host__ __device__ constexpr uint32_t aux_bytes(uint32_t MP) { return MP * 20; }  // per block: MP x 8 int16 block sums | MP x f32 d8
+constexpr uint32_t I8_MP = 16;                                    // activation rows of the MMA
+constexpr uint32_t AUX_BYTES = I8_MP * 20;                        // per block: MP x 8 int16 block sums | MP x f32 d8
+constexpr uint32_t SC_SLOT = SC_REC + AUX_BYTES;
 // barriers (8 bytes each) at the start of dynamic shared memory
 constexpr int OFF_FULL = 0, OFF_EMPTY = 64, OFF_RAW_FULL = 128, OFF_RAW_EMPTY = 192, OFF_ACC_FULL = 256, OFF_ACC_EMPTY = 272,
-              OFF_SC_FULL = 320, OFF_TMEM = 448, OFF_DEAD = 452, OFF_RED = 456, OFF_LAST = 464, OFF_NSLOT = 472, OFF_XFER = 480, OFF_SLOTS = 512,
-              OFF_SC = 1024;  // OFF_SLOTS: two lists of 64 slots
+              OFF_SC_FULL = 320, OFF_TMEM = 448, OFF_DEAD = 452, OFF_XFER = 480, OFF_SC = 1024;
 
-// One piece of work of a CTA: blocks [b0, b0 + nb) of tile `tile`; slot < 0: the whole tile, written to the output.
-struct I8Unit {
-    uint32_t tile, b0, nb;
-    int slot;
-};
-// First (tile, block) pair of CTA c: the first qrem CTAs take one item more than the others
-__device__ __forceinline__ uint32_t i8_range_begin(const I8Params& p, uint32_t c) { return (c * p.qbase + min(c, p.qrem)) * p.unit; }
-// The CTA whose range holds pair x
-__device__ __forceinline__ uint32_t i8_cta_of(const I8Params& p, uint32_t x) {
-    const uint32_t y = x / p.unit, big = p.qrem * (p.qbase + 1);
-    return y < big ? y / (p.qbase + 1) : p.qrem + (y - big) / p.qbase;
-}
-// The it-th unit of this CTA (every role walks the same list): the CTA's range cut at the tile boundaries
-__device__ __forceinline__ bool i8_unit(const I8Params& p, uint32_t it, I8Unit& u) {
-    const uint32_t a = i8_range_begin(p, blockIdx.x), b = i8_range_begin(p, blockIdx.x + 1);
-    const uint32_t t = a / p.nblk + it;
-    const uint32_t lo = max(a, t * p.nblk), hi = min(b, (t + 1) * p.nblk);
-    if (t >= p.ntiles || lo >= hi) return false;
-    u.tile = t;
-    u.b0 = lo - t * p.nblk;
-    u.nb = hi - lo;
-    u.slot = u.nb == p.nblk ? -1 : (int)(2 * blockIdx.x + (it == 0 ? 0u : 1u));
-    return true;
-}
+// First tile of CTA c: the first trem CTAs take one more than the others
+__device__ __forceinline__ uint32_t i8_tile_begin(const I8Params& p, uint32_t c) { return c * p.tbase + min(c, p.trem); }
 
-template <int MP>
 __global__ void __launch_bounds__(I8_THREADS, 1) smallm_i8_q4k_kernel(const __grid_constant__ CUtensorMap tmap_act,
                                                                       const __grid_constant__ CUtensorMap tmap_w, const I8Params p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -112,7 +78,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) smallm_i8_q4k_kernel(const __gr
                    bar_sc_full = sbase + OFF_SC_FULL;
     volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(smem + OFF_TMEM);
     volatile uint32_t* dead = reinterpret_cast<volatile uint32_t*>(smem + OFF_DEAD);
-    constexpr uint32_t NACC = 2, ACC_COLS = 8 * MP, TMEM_COLS = NACC * ACC_COLS < 32 ? 32 : NACC * ACC_COLS;  // 256 or 512
+    constexpr uint32_t MP = I8_MP, NACC = 2, ACC_COLS = 8 * MP, TMEM_COLS = NACC * ACC_COLS;  // 256
     constexpr uint32_t B_ATOM = MP * 128, STAGE = 2 * A_ATOM + 2 * B_ATOM;
     // shared memory: barriers | scale records | exchange buffer of the drain teams | packed tiles | operand stages (A atom
     // 0, A atom 1, B atom 0, B atom 1)
@@ -136,7 +102,6 @@ __global__ void __launch_bounds__(I8_THREADS, 1) smallm_i8_q4k_kernel(const __gr
             mbar_init(sbase + OFF_XFER + 8 * s, team_warps);  // the team's running sums are in the exchange buffer
         }
         for (uint32_t s = 0; s < p.nsc; ++s) mbar_init(bar_sc_full + 8 * s, 5);  // four decode warps write the records, one copy brings the activation side
-        mbar_init(sbase + OFF_RED, 2 * team_warps);  // both teams meet here around the hand-over of a cut tile
         *dead = 0;
         mbar_fence_init();
     }
@@ -149,20 +114,20 @@ __global__ void __launch_bounds__(I8_THREADS, 1) smallm_i8_q4k_kernel(const __gr
     tc_after();
     const uint32_t tmem = *tmem_holder;
     grid_dep_launch();
+    const uint32_t t_begin = i8_tile_begin(p, blockIdx.x), t_end = i8_tile_begin(p, blockIdx.x + 1);
 
     if (warp == W_RAW) {
         // ------------------------------------------------------------ packed weight tiles (do not depend on the previous kernel)
         if (lane == 0) {
             uint32_t s = 0, par = 0;
-            I8Unit u;
-            for (uint32_t it = 0; i8_unit(p, it, u) && !*dead; ++it) {
-                for (uint32_t j = 0; j < u.nb; ++j) {
+            for (uint32_t tile = t_begin; tile < t_end && !*dead; ++tile) {
+                for (uint32_t j = 0; j < p.nblk; ++j) {
                     if (!i8_wait(bar_raw_empty + 8 * s, par ^ 1, dead)) {
                         i8_fail(dead, p.status, STATUS_TIMEOUT_EMPTY);
                         break;
                     }
                     mbar_expect_tx(bar_raw_full + 8 * s, RAW_TILE);
-                    tma2d(sbase + raw_off + s * RAW_TILE, &tmap_w, (int)((u.b0 + j) * RAW_PITCH), (int)(u.tile * 128), bar_raw_full + 8 * s);
+                    tma2d(sbase + raw_off + s * RAW_TILE, &tmap_w, (int)(j * RAW_PITCH), (int)(tile * 128), bar_raw_full + 8 * s);
                     if (++s == p.nr) { s = 0; par ^= 1; }
                 }
             }
@@ -172,21 +137,20 @@ __global__ void __launch_bounds__(I8_THREADS, 1) smallm_i8_q4k_kernel(const __gr
         if (lane == 0) {
             grid_dep_wait();
             uint32_t s = 0, par = 0, i = 0;
-            I8Unit u;
-            for (uint32_t it = 0; i8_unit(p, it, u) && !*dead; ++it) {
-                for (uint32_t j = 0; j < u.nb; ++j, ++i) {
+            for (uint32_t tile = t_begin; tile < t_end && !*dead; ++tile) {
+                for (uint32_t j = 0; j < p.nblk; ++j, ++i) {
                     if (!i8_wait(bar_empty + 8 * s, par ^ 1, dead)) {
                         i8_fail(dead, p.status, STATUS_TIMEOUT_EMPTY);
                         break;
                     }
                     const uint32_t b0 = sbase + st_off + s * STAGE + 2 * A_ATOM;
                     mbar_expect_tx(bar_full + 8 * s, 2 * B_ATOM);
-                    tma2d(b0, &tmap_act, (int)((u.b0 + j) * 256), 0, bar_full + 8 * s);
-                    tma2d(b0 + B_ATOM, &tmap_act, (int)((u.b0 + j) * 256 + 128), 0, bar_full + 8 * s);
+                    tma2d(b0, &tmap_act, (int)(j * 256), 0, bar_full + 8 * s);
+                    tma2d(b0 + B_ATOM, &tmap_act, (int)(j * 256 + 128), 0, bar_full + 8 * s);
                     // block sums and scales of the activation rows, next to the row records (same life time)
                     const uint32_t q = i % p.nsc;
-                    mbar_expect_tx(bar_sc_full + 8 * q, aux_bytes(MP));
-                    bulk_g2s(sbase + sc_off + q * SC_SLOT + SC_REC, p.aux + (size_t)(u.b0 + j) * aux_bytes(MP), aux_bytes(MP), bar_sc_full + 8 * q);
+                    mbar_expect_tx(bar_sc_full + 8 * q, AUX_BYTES);
+                    bulk_g2s(sbase + sc_off + q * SC_SLOT + SC_REC, p.aux + (size_t)j * AUX_BYTES, AUX_BYTES, bar_sc_full + 8 * q);
                     if (++s == p.ns) { s = 0; par ^= 1; }
                 }
             }
@@ -195,9 +159,8 @@ __global__ void __launch_bounds__(I8_THREADS, 1) smallm_i8_q4k_kernel(const __gr
         // ------------------------------------------------------------ MMA issue: 8 sub-blocks, 8 column groups
         uint32_t s = 0, par = 0, i = 0;
         bool ok = true;
-        I8Unit u;
-        for (uint32_t it = 0; ok && i8_unit(p, it, u); ++it) {
-            for (uint32_t j = 0; j < u.nb; ++j, ++i) {
+        for (uint32_t tile = t_begin; ok && tile < t_end; ++tile) {
+            for (uint32_t j = 0; j < p.nblk; ++j, ++i) {
                 const uint32_t buf = i % NACC, use = i / NACC;
                 if (!i8_wait(bar_full + 8 * s, par, dead)) {
                     if (lane == 0) i8_fail(dead, p.status, STATUS_TIMEOUT_FULL);
@@ -230,11 +193,10 @@ __global__ void __launch_bounds__(I8_THREADS, 1) smallm_i8_q4k_kernel(const __gr
         const uint32_t r = threadIdx.x & 127, set = threadIdx.x >> 7;
         const uint32_t row_sw = (r >> 3) * 1024 + (r & 7) * 128, x7 = r & 7;
         bool ok = true;
-        I8Unit u;
         uint32_t i = 0;
-        for (uint32_t it = 0; i8_unit(p, it, u); ++it) {
-            const bool row_ok = u.tile * 128 + r < p.N;
-            for (uint32_t j = 0; j < u.nb; ++j, ++i) {
+        for (uint32_t tile = t_begin; tile < t_end; ++tile) {
+            const bool row_ok = tile * 128 + r < p.N;
+            for (uint32_t j = 0; j < p.nblk; ++j, ++i) {
                 if (i % (DEC_WARPS / 4) != set) continue;
                 const uint32_t rs = i % p.nr, rpar = (i / p.nr) & 1, s = i % p.ns, par = (i / p.ns) & 1;
                 if (ok && !i8_wait(bar_raw_full + 8 * rs, rpar, dead)) {
@@ -291,18 +253,12 @@ __global__ void __launch_bounds__(I8_THREADS, 1) smallm_i8_q4k_kernel(const __gr
         // of two blocks overlap.  In a team, a thread owns one weight row (two warps per quarter of the rows) and MH of
         // the activation rows; warps whose rows do not exist have nothing to do.  The f32 sums still grow block by block,
         // in K order: the running sums of a tile pass from team to team through a buffer in shared memory.
-        // The CTA's pairs are the contiguous range [xa, xb): pair x = block x % nblk of tile x / nblk.
         const uint32_t dw = (uint32_t)warp - DEC_WARPS, team = dw >> 3, quarter = dw & 3, r = quarter * 32 + lane, m_lo = ((dw >> 2) & 1) * MH;
         const bool rows_exist = m_lo < p.M;
         const uint32_t lane_addr = (quarter * 32) << 16;
-        const uint32_t xa = i8_range_begin(p, blockIdx.x), xb = i8_range_begin(p, blockIdx.x + 1);
-        const uint32_t bar_red = sbase + OFF_RED, bar_x = sbase + OFF_XFER;
-        volatile uint32_t* last_flag = reinterpret_cast<volatile uint32_t*>(smem + OFF_LAST);   // [2]
-        volatile uint32_t* nslot = reinterpret_cast<volatile uint32_t*>(smem + OFF_NSLOT);      // [2]
-        volatile uint32_t* slot_list = reinterpret_cast<volatile uint32_t*>(smem + OFF_SLOTS);  // [2][64]
+        const uint32_t nblocks = (t_end - t_begin) * p.nblk, bar_x = sbase + OFF_XFER;
         float* xch = reinterpret_cast<float*>(smem + x_off) + m_lo * 128 + r;                   // [activation row][weight row]
-        grid_dep_wait();  // the output and the scratch may still be in use by the previous kernel
-        uint32_t red_phase = 0;
+        grid_dep_wait();  // the output may still be in use by the previous kernel
         bool ok = true;
         auto store_out = [&](uint32_t n, uint32_t m, float v) {
             const size_t idx = (size_t)m * p.N + n;
@@ -310,23 +266,8 @@ __global__ void __launch_bounds__(I8_THREADS, 1) smallm_i8_q4k_kernel(const __gr
             else if (p.out_dtype == DT_BF16) static_cast<__nv_bfloat16*>(p.out)[idx] = __float2bfloat16_rn(v);
             else static_cast<__half*>(p.out)[idx] = __float2half_rn(v);
         };
-        // the drain warps meet (bounded: a warp that gave up marks the CTA dead and the others leave too)
-        auto meet = [&]() {
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_red);
-            if (!i8_wait(bar_red, red_phase & 1, dead)) {
-                i8_fail(dead, p.status, STATUS_TIMEOUT_EMPTY);
-                ok = false;
-            }
-            ++red_phase;
-        };
-        // pieces of cut tiles this CTA writes: of its first tile (0) and / or of its last one (1)
-        const uint32_t t_first = xa / p.nblk, t_last = xb > xa ? (xb - 1) / p.nblk : t_first;
-        const bool have[2] = {xb > xa && (xa != t_first * p.nblk || xb < (t_first + 1) * p.nblk), t_last != t_first && xb != (t_last + 1) * p.nblk};
-        const uint32_t cut_tile[2] = {t_first, t_last};
-        for (uint32_t x = xa + team; x < xb && ok && rows_exist; x += 2) {
-            const uint32_t i = x - xa, buf = team, use = i >> 1, q = i % p.nsc;
-            const uint32_t tile = x / p.nblk, blk = x - tile * p.nblk;
+        for (uint32_t i = team; i < nblocks && ok && rows_exist; i += 2) {
+            const uint32_t buf = team, use = i >> 1, q = i % p.nsc, tile = t_begin + i / p.nblk, blk = i % p.nblk;
             if (!i8_wait(bar_sc_full + 8 * q, (i / p.nsc) & 1, dead)) {
                 i8_fail(dead, p.status, STATUS_TIMEOUT_FULL);
                 ok = false;
@@ -353,10 +294,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) smallm_i8_q4k_kernel(const __gr
             for (int g = 0; g < 8 / GB; ++g) {
                 uint32_t v[GB][MH];
 #pragma unroll
-                for (int k = 0; k < GB; ++k) {
-                    if constexpr (MH == 16) tmem_ld16_async(t0 + MP * (GB * g + k), v[k]);
-                    else tmem_ld8_async(t0 + MP * (GB * g + k), v[k]);
-                }
+                for (int k = 0; k < GB; ++k) tmem_ld8_async(t0 + MP * (GB * g + k), v[k]);
                 tmem_ld_wait();
 #pragma unroll
                 for (int k = 0; k < GB; ++k)
@@ -378,85 +316,26 @@ __global__ void __launch_bounds__(I8_THREADS, 1) smallm_i8_q4k_kernel(const __gr
             }
             // the running sums after the previous block (the other team's); every block waits for its predecessor, so the
             // teams never drift apart by more than one block
-            const bool first_of_tile = blk == 0 || x == xa;
             if (i > 0 && !i8_wait(bar_x + 8 * (team ^ 1), ((i - 1) >> 1) & 1, dead)) {
                 i8_fail(dead, p.status, STATUS_TIMEOUT_EMPTY);
                 ok = false;
                 break;
             }
-            if (!first_of_tile)
+            if (blk > 0)
 #pragma unroll
                 for (int m = 0; m < MH; ++m) term[m] = __fadd_rn(xch[m * 128], term[m]);
-            const bool last_of_tile = blk + 1 == p.nblk || x + 1 == xb;
+            const bool last_of_tile = blk + 1 == p.nblk;
             if (!last_of_tile)
 #pragma unroll
                 for (int m = 0; m < MH; ++m) xch[m * 128] = term[m];
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_x + 8 * team);
             if (!last_of_tile) continue;
-            // ---- the CTA's last block of this tile
             const uint32_t n = tile * 128 + r;
-            const bool whole = (tile * p.nblk >= xa) && ((tile + 1) * p.nblk <= xb);
-            if (whole) {
-                if (n < p.N)
+            if (n < p.N)
 #pragma unroll
-                    for (int m = 0; m < MH; ++m)
-                        if (m_lo + m < p.M) store_out(n, m_lo + m, term[m]);
-            } else {
-                // a piece of a cut tile goes to scratch; the hand-over follows when all blocks are done
-                const uint32_t which = tile == t_first ? 0u : 1u;
-                float* part = p.part + ((size_t)(2 * blockIdx.x + which) * MP + m_lo) * 128;
-#pragma unroll
-                for (int m = 0; m < MH; ++m) part[m * 128 + r] = term[m];
-            }
-        }
-        // ---- cut tiles: whoever writes a tile's last piece adds all of them, in K order, and stores the rows
-        if (ok && rows_exist && (have[0] || have[1])) {
-            meet();  // every drain thread's pieces are written
-            if (ok && warp == DEC_WARPS && lane == 0) {
-                uint32_t old[2] = {0, 0}, np[2] = {0, 0};
-#pragma unroll
-                for (uint32_t which = 0; which < 2; ++which) {
-                    if (!have[which]) continue;
-                    // the CTAs whose ranges meet the tile's pairs [x0, x1), in order
-                    const uint32_t tile = cut_tile[which], x0 = tile * p.nblk, x1 = x0 + p.nblk, G = gridDim.x;
-                    uint32_t k = 0;
-                    for (uint32_t cc = i8_cta_of(p, x0); cc < G && k < 64; ++cc) {
-                        const uint32_t a = i8_range_begin(p, cc);
-                        if (a >= x1) break;
-                        slot_list[64 * which + k++] = 2 * cc + (tile == a / p.nblk ? 0u : 1u);
-                    }
-                    nslot[which] = np[which] = k;
-                    // release: the pieces (seen through the meeting) are visible to whoever reads the count; acquire: the
-                    // pieces counted before are visible here.  The two counts are on their way together.
-                    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old[which]) : "l"(p.cnt + tile) : "memory");
-                }
-#pragma unroll
-                for (uint32_t which = 0; which < 2; ++which) {
-                    const bool last = have[which] && old[which] + 1 == np[which];
-                    if (last) p.cnt[cut_tile[which]] = 0;  // ready for the next call
-                    last_flag[which] = last ? 1u : 0u;
-                }
-            }
-            meet();
-            // the rows of a tile are shared out over both teams: team t adds the activation rows of its parity
-            for (uint32_t which = 0; ok && which < 2; ++which) {
-                if (!have[which] || !last_flag[which]) continue;
-                const uint32_t ns = nslot[which], n = cut_tile[which] * 128 + r;
-                for (uint32_t m = m_lo + team; m < m_lo + MH && m < p.M; m += 2) {
-                    float tot = 0.f;
-                    for (uint32_t k0 = 0; k0 < ns; k0 += 8) {
-                        float v[8];
-#pragma unroll
-                        for (uint32_t k = 0; k < 8; ++k)
-                            if (k0 + k < ns) v[k] = __ldcg(p.part + ((size_t)slot_list[64 * which + k0 + k] * MP + m) * 128 + r);
-#pragma unroll
-                        for (uint32_t k = 0; k < 8; ++k)
-                            if (k0 + k < ns) tot = k0 + k == 0 ? v[k] : __fadd_rn(tot, v[k]);
-                    }
-                    if (n < p.N) store_out(n, m, tot);
-                }
-            }
+                for (int m = 0; m < MH; ++m)
+                    if (m_lo + m < p.M) store_out(n, m_lo + m, term[m]);
         }
     }
     tc_before();
@@ -469,15 +348,13 @@ __global__ void __launch_bounds__(I8_THREADS, 1) smallm_i8_q4k_kernel(const __gr
 
 // One warp per (activation row, 256-block): Q8_K codes (quantize_act_q8k.rs:26-98: d = amax / 127, id = 127 / amax,
 // round half to even) into the int8 image [M][K]; the eight sums of 32 codes and the scale go to the block's record in
-// `aux` (aux_bytes).  Also clears the piece counters of the main kernel.
+// `aux` (AUX_BYTES).
 template <typename InT>
 __global__ void __launch_bounds__(256) i8_act_prep_kernel(const InT* __restrict__ act, uint8_t* __restrict__ codes, uint8_t* __restrict__ aux,
-                                                          unsigned int* __restrict__ cnt, uint32_t ntiles, uint32_t M, uint32_t nblk,
-                                                          uint32_t MP) {
+                                                          uint32_t M, uint32_t nblk) {
     const int lane = threadIdx.x & 31;
     grid_dep_launch();
     grid_dep_wait();  // the activations may be the previous kernel's output; the image may still be read by it
-    for (uint32_t t = blockIdx.x * 256 + threadIdx.x; t < ntiles; t += gridDim.x * 256) cnt[t] = 0;  // piece counters of the cut tiles
     const uint32_t run = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (run >= M * nblk) return;
     const uint32_t m = run / nblk, b = run % nblk;
@@ -514,9 +391,9 @@ __global__ void __launch_bounds__(256) i8_act_prep_kernel(const InT* __restrict_
     *reinterpret_cast<uint2*>(codes + base) = make_uint2(w0, w1);
     s += __shfl_xor_sync(0xFFFFFFFFu, s, 1);  // 32 codes = four lanes
     s += __shfl_xor_sync(0xFFFFFFFFu, s, 2);
-    uint8_t* ab = aux + (size_t)b * aux_bytes(MP);
+    uint8_t* ab = aux + (size_t)b * AUX_BYTES;
     if ((lane & 3) == 0) reinterpret_cast<short*>(ab)[m * 8 + (lane >> 2)] = (short)s;
-    if (lane == 0) reinterpret_cast<float*>(ab + MP * 16)[m] = __fdiv_rn(amax, 127.0f);
+    if (lane == 0) reinterpret_cast<float*>(ab + I8_MP * 16)[m] = __fdiv_rn(amax, 127.0f);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -528,7 +405,7 @@ __global__ void __launch_bounds__(256) i8_act_prep_kernel(const InT* __restrict_
 // above with these differences: an accumulator holds the four blocks of half a 256-run (one 128-byte operand tile, 256
 // columns), so a stage feeds both accumulators and each is reused every block; all sixteen drain warps work on every
 // accumulator (four groups of four warps, 8 activation rows each) and keep their sums in registers for the whole tile;
-// only whole tiles are dealt (no hand-over).
+// whole tiles are dealt round-robin.
 struct Q8Params {
     const uint8_t* w;
     void* out;
@@ -838,27 +715,16 @@ __global__ void __launch_bounds__(256) q8_act_prep_kernel(const InT* __restrict_
 }
 
 struct I8Layout {
-    uint32_t MP, nblk, ntiles, Q, grid, unit;
-    size_t codes_bytes, aux_off, part_off, cnt_off, total;
+    uint32_t nblk, ntiles, grid;
+    size_t aux_off, total;
 };
 I8Layout i8_layout(size_t M, size_t K, size_t N, int sm_count) {
     I8Layout l{};
-    l.MP = 16u;
     l.nblk = (uint32_t)(K / 256);
     l.ntiles = (uint32_t)((N + 127) / 128);
-    l.Q = l.ntiles * l.nblk;
-    // Whole tiles per CTA (nothing to hand over) unless cutting the tiles along K shortens the longest CTA by more than
-    // the hand-over costs (about eight blocks' worth of time).
-    const uint32_t G = (uint32_t)sm_count;
-    const uint32_t whole_cost = (l.ntiles + G - 1) / G * l.nblk, cut_cost = (l.Q + G - 1) / G + 8;
-    l.unit = whole_cost <= cut_cost ? l.nblk : 1u;
-    const uint32_t items = l.Q / l.unit;
-    l.grid = items < G ? items : G;
-    l.codes_bytes = (M * K + 255) & ~(size_t)255;
-    l.aux_off = l.codes_bytes;
-    l.part_off = l.aux_off + (((size_t)l.nblk * aux_bytes(l.MP) + 255) & ~(size_t)255);
-    l.cnt_off = l.part_off + (size_t)2 * l.grid * l.MP * 128 * 4;
-    l.total = l.cnt_off + (((size_t)l.ntiles * 4 + 255) & ~(size_t)255);
+    l.grid = l.ntiles < (uint32_t)sm_count ? l.ntiles : (uint32_t)sm_count;
+    l.aux_off = (M * K + 255) & ~(size_t)255;
+    l.total = l.aux_off + (((size_t)l.nblk * AUX_BYTES + 255) & ~(size_t)255);
     return l;
 }
 
@@ -962,24 +828,24 @@ cudaError_t launch_smallm_q8_0(const void* act, int act_dtype, const void* w, vo
 
 }  // namespace
 
-// Shapes the integer tensor-core kernels take.  Q4_K: 2 <= M <= 16, whole 256-blocks (rows are multiples of 16 bytes:
-// 144-byte blocks), pair counts within 32 bits.  Q8_0: 17 <= M <= 32 (up to 16 rows the mma.sync kernel is as fast), K a multiple
-// of 256 (rows of whole 272-byte runs), whole tiles only.
+// Shapes the integer tensor-core kernels take.  Q4_K: 8 <= M <= 16, whole 256-blocks (rows are multiples of 16 bytes:
+// 144-byte blocks), (tile, block) pairs within 32 bits.  Q8_0: 17 <= M <= 32 (up to 16 rows the mma.sync kernel is as fast), K a multiple
+// of 256 (rows of whole 272-byte runs).  Both deal whole tiles only.
 bool smallm_i8_supported(int fmt, size_t M, size_t K, size_t N) {
-    if (M < 2 || M > 32 || K % 256 != 0 || K < 256 || N < 1 || (N + 127) / 128 * (K / 256) >= (1u << 30)) return false;
-    return (fmt == FMT_Q8_0 && M > 16) || (fmt == FMT_Q4_K && M <= 16 && K / 256 <= 64);
+    if (K % 256 != 0 || K < 256 || N < 1 || (N + 127) / 128 * (K / 256) >= (1u << 30)) return false;
+    return (fmt == FMT_Q8_0 && M > 16 && M <= 32) || (fmt == FMT_Q4_K && M >= 8 && M <= 16 && K / 256 <= 64);
 }
 size_t smallm_i8_workspace_bytes(int fmt, size_t M, size_t K, size_t N, int sm_count) {
     return fmt == FMT_Q8_0 ? q8_layout(M, K, N, sm_count).total : i8_layout(M, K, N, sm_count).total;
 }
-// Where they beat the mma.sync kernel (measured).  Q4_K: matrices with enough 128-row tiles to give every SM whole tiles
-// (nothing to hand over), from 8 activation rows on.  Q8_0: above 16 rows (one pass over the weights instead of two), matrices with enough
-// tiles to occupy half of the SMs (only whole tiles are dealt).
+// Where they beat the mma.sync kernel (measured).  Q4_K: matrices with enough 128-row tiles for whole tiles on every SM: the longest CTA
+// has at most eight blocks more than an even share would give it.  Q8_0: one pass over the weights instead of two,
+// matrices with enough tiles to occupy half of the SMs.
 bool smallm_i8_preferred(int fmt, size_t M, size_t K, size_t N, int sm_count) {
     if (!smallm_i8_supported(fmt, M, K, N)) return false;
-    if (fmt == FMT_Q8_0) return M > 16 && (N + 127) / 128 >= (size_t)sm_count / 2;
-    const I8Layout l = i8_layout(M, K, N, sm_count);
-    return M >= 8 && l.unit == l.nblk && l.ntiles >= (uint32_t)sm_count * 3 / 4;
+    const size_t tiles = (N + 127) / 128, sms = (size_t)sm_count, nblk = K / 256;
+    if (fmt == FMT_Q8_0) return tiles >= sms / 2;
+    return (tiles + sms - 1) / sms * nblk <= (tiles * nblk + sms - 1) / sms + 8 && tiles >= sms * 3 / 4;
 }
 
 // acts_prepared: a previous call with the same activations and scratch left the image there (gate, then up).
@@ -994,14 +860,13 @@ cudaError_t launch_smallm_i8(int fmt, const void* act, int act_dtype, const void
     uint8_t* base = static_cast<uint8_t*>(ws);
     uint8_t* codes = base;
     uint8_t* aux = base + l.aux_off;
-    unsigned int* cnt = reinterpret_cast<unsigned int*>(base + l.cnt_off);
     if (!acts_prepared) {
         const uint32_t runs = (uint32_t)M * l.nblk;
         const dim3 pg((runs + 7) / 8);
         cudaError_t e = act_dtype == DT_F32
-                            ? launch_pdl(i8_act_prep_kernel<float>, pg, dim3(256), 0, st, static_cast<const float*>(act), codes, aux, cnt, l.ntiles, (uint32_t)M, l.nblk, l.MP)
-                            : launch_pdl(i8_act_prep_kernel<__nv_bfloat16>, pg, dim3(256), 0, st, static_cast<const __nv_bfloat16*>(act), codes, aux, cnt,
-                                         l.ntiles, (uint32_t)M, l.nblk, l.MP);
+                            ? launch_pdl(i8_act_prep_kernel<float>, pg, dim3(256), 0, st, static_cast<const float*>(act), codes, aux, (uint32_t)M, l.nblk)
+                            : launch_pdl(i8_act_prep_kernel<__nv_bfloat16>, pg, dim3(256), 0, st, static_cast<const __nv_bfloat16*>(act), codes, aux,
+                                         (uint32_t)M, l.nblk);
         note_launch();
         if (e != cudaSuccess) return e;
     }
@@ -1011,23 +876,19 @@ cudaError_t launch_smallm_i8(int fmt, const void* act, int act_dtype, const void
         return cudaErrorNotSupported;
     }
     I8Params p{};
-    p.w = static_cast<const uint8_t*>(w);
     p.out = out;
-    p.part = reinterpret_cast<float*>(base + l.part_off);
-    p.cnt = cnt;
     p.aux = aux;
-    p.M = (uint32_t)M; p.N = (uint32_t)N; p.K = (uint32_t)K;
-    p.MP = l.MP; p.nblk = l.nblk; p.ntiles = l.ntiles; p.Q = l.Q;
-    p.unit = l.unit;
-    p.qbase = (l.Q / l.unit) / l.grid; p.qrem = (l.Q / l.unit) % l.grid;
+    p.M = (uint32_t)M; p.N = (uint32_t)N;
+    p.nblk = l.nblk;
+    p.tbase = l.ntiles / l.grid; p.trem = l.ntiles % l.grid;
     // int32 accumulator, signed 8-bit x signed 8-bit, both K-major, N = MP, M = 128
-    p.idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((p.MP >> 3) << 17) | ((128u >> 4) << 24);
+    p.idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((I8_MP >> 3) << 17) | ((128u >> 4) << 24);
     p.out_dtype = out_dtype;
     p.status = status;
-    const uint32_t stage = 2 * A_ATOM + 2 * p.MP * 128;
+    const uint32_t stage = 2 * A_ATOM + 2 * I8_MP * 128;
     p.ns = 3;
     p.nsc = p.ns + 2 + 2;
-    const uint32_t fixed = 1024 + ((p.nsc * SC_SLOT + 128 * p.MP * 4 + 1023u) & ~1023u) + p.ns * stage;
+    const uint32_t fixed = 1024 + ((p.nsc * SC_SLOT + 128 * I8_MP * 4 + 1023u) & ~1023u) + p.ns * stage;
     // The ring of packed tiles must have an EVEN depth: block i lives in slot i % nr and is read by decode set i & 1, so with
     // an even depth a slot always belongs to one set and that set sees every phase of the slot's barrier.  With an odd depth
     // the sets would alternate on a slot, a set would wait for phase k having last seen phase k - 2, and a parity wait cannot
@@ -1041,7 +902,7 @@ cudaError_t launch_smallm_i8(int fmt, const void* act, int act_dtype, const void
     {
         const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)M};
         const cuuint64_t gstride[1] = {(cuuint64_t)K};
-        const cuuint32_t box[2] = {128u, p.MP};
+        const cuuint32_t box[2] = {128u, I8_MP};
         CUresult cr = enc(&amap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, codes, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (cr != CUDA_SUCCESS) {
@@ -1062,9 +923,9 @@ cudaError_t launch_smallm_i8(int fmt, const void* act, int act_dtype, const void
         }
     }
     static PerDeviceOnce attrs;
-    cudaError_t e = attrs.run([] { return cudaFuncSetAttribute(smallm_i8_q4k_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448); });
+    cudaError_t e = attrs.run([] { return cudaFuncSetAttribute(smallm_i8_q4k_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448); });
     if (e != cudaSuccess) return e;
-    e = launch_pdl(smallm_i8_q4k_kernel<16>, dim3(l.grid), dim3(I8_THREADS), smem, st, amap, wmap, p);
+    e = launch_pdl(smallm_i8_q4k_kernel, dim3(l.grid), dim3(I8_THREADS), smem, st, amap, wmap, p);
     note_launch();
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
