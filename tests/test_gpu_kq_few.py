@@ -144,3 +144,36 @@ def test_batch_that_changes_the_kernel(m, reverse):
     for a, b in zip(ops.quant_matmul_batch(x, ws), want):
         assert torch.equal(a, b)
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("fmt", ["Q4_K", "Q5_K", "Q6_K"])
+@pytest.mark.parametrize("m,n,k", [(24, 700, 2048), (37, 1300, 5120), (63, 19000, 256), (17, 1000, 768)])
+def test_16_bit_activations_and_results(oracle, fmt, m, n, k):
+    from boostr_b200 import ops
+
+    assert kq_tile_rows(fmt, m, n, k) > 0
+    rng = synth.rng_for(102, seed_of(fmt, m, n, k))
+    x = torch.from_numpy(synth.activations(rng, m, k)).cuda().to(torch.bfloat16)
+    w = synth.weight_bytes(fmt, rng, n, k)
+    qt = QuantTensor.from_bytes(w, F[fmt], (n, k), device="cuda")
+    got = ops.quant_matmul(x, qt, out_dtype=torch.float32)
+    want = oracle.quant_matmul(fmt, x.float().cpu().numpy(), w, n, threads=os.cpu_count() or 8)
+    assert np.array_equal(got.cpu().numpy().view(np.uint32), want.view(np.uint32)), describe_mismatch(got.cpu().numpy(), want)
+    for dt in (torch.bfloat16, torch.float16):  # one rounding of the f32 results
+        assert torch.equal(ops.quant_matmul(x, qt, out_dtype=dt), got.to(dt))
+    ops.check_device_status()
+
+
+def test_more_weight_rows_than_2_to_the_22():
+    """The last rows of a weight of more than 2^22 rows have the bits that they have in a weight of their own."""
+    from boostr_b200 import ops
+
+    m, n, k, tail = 17, (1 << 22) + 200, 256, 300
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(22)
+    w = synth.device_weight("Q4_K", n, k, gen)
+    x = torch.randn(m, k, device="cuda", generator=gen)
+    block = F.Q4_K.block_bytes
+    part = QuantTensor(w.storage[(n - tail) * block:n * block].clone(), w.format, (tail, k))
+    assert torch.equal(ops.quant_matmul(x, w)[:, n - tail:], ops.quant_matmul(x, part))
+    ops.check_device_status()

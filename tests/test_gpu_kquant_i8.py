@@ -1,4 +1,5 @@
-"""The integer tensor-core products of the K-quants, bit for bit against the CPU oracle (integer sums, blocks added in K order).
+"""The integer tensor-core products of the K-quants, bit for bit against the CPU oracle (integer sums, blocks added in K order): Q2_K and
+Q3_K (csrc/kquant_i8.cu), Q4_K and Q5_K with 17 ... 63 rows (csrc/kquant_few.cu).
 ``test_bit_identical``: Q2_K / Q3_K around the multiples of 8 and 16 rows of the mma.sync kernel (which takes all of its shapes but
 the two of 300 and 512 rows), partial row tiles, one block and odd block counts (rows of every alignment), long K.
 ``test_weight_tiles_by_tma``: the tensor-core kernel on tiles of 16 ... 128 rows, held to the rule that picks them."""
@@ -7,10 +8,10 @@ import os
 import numpy as np
 import pytest
 
-from boostr_b200 import _cabi, synth
+from boostr_b200 import synth
 from boostr_b200.format import QuantFormat as F
 from boostr_b200.tensor import QuantTensor
-from util import describe_mismatch, seed_of
+from util import describe_mismatch, kq_tile_rows, seed_of
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -46,15 +47,6 @@ def test_bit_identical(oracle, fmt, m, n, k):
         assert torch.equal(y, out.to(torch.bfloat16))
 
 
-def _tile_rows(fmt, m, n, k):
-    """The tile that the library's own rule picks (0: kernel for few rows, -1: another path)."""
-    import ctypes
-
-    f = _cabi.lib().b200q_kq_tile_rows
-    f.restype, f.argtypes = ctypes.c_int, [ctypes.c_int, ctypes.c_size_t, ctypes.c_size_t, ctypes.c_size_t, ctypes.c_int]
-    return f(F[fmt].format_id, m, k, n, torch.cuda.get_device_properties(0).multi_processor_count)
-
-
 @pytest.mark.parametrize("fmt,m,n,k,tile", [
     ("Q2_K", 48, 18900, 1024, 48), ("Q2_K", 112, 18900, 1024, 112), ("Q2_K", 128, 18900, 2048, 128), ("Q2_K", 129, 18900, 1024, 80),
     ("Q2_K", 300, 5001, 4096, 112), ("Q2_K", 512, 4096, 2048, 128),
@@ -67,7 +59,7 @@ def test_weight_tiles_by_tma(oracle, fmt, m, n, k, tile):
     bounded wait that ran out would show in the status word), also over many launches of the shortest work."""
     from boostr_b200 import ops
 
-    assert _tile_rows(fmt, m, n, k) == tile and k // 256 * F[fmt].block_bytes % 16 == 0
+    assert kq_tile_rows(fmt, m, n, k) == tile and k // 256 * F[fmt].block_bytes % 16 == 0
     rng = synth.rng_for(96, seed_of(fmt, m, n, k))
     act = synth.activations(rng, m, k)
     w = synth.weight_bytes(fmt, rng, n, k)
@@ -85,7 +77,7 @@ def test_weight_tiles_by_tma(oracle, fmt, m, n, k, tile):
 
 @pytest.mark.parametrize("fmt", ["Q4_K", "Q5_K"])
 @pytest.mark.parametrize("m,n,k", [(17, 9000, 1280), (33, 2050, 512), (37, 4097, 1280), (48, 2100, 768), (49, 20000, 256), (63, 30000, 512)])
-def test_two_byte_products_bit_identical(oracle, fmt, m, n, k):
+def test_q4_k_and_q5_k_bit_identical(oracle, fmt, m, n, k):
     from boostr_b200 import ops
 
     rng = synth.rng_for(94, seed_of(fmt, m, n, k))
@@ -112,7 +104,7 @@ def test_batch_shares_one_image():
     gen.manual_seed(7)
     m, k = 37, 1280
     ws = [synth.device_weight(fmt, n, k, gen) for fmt, n in (("Q5_K", 4097), ("Q3_K", 300), ("Q2_K", 300), ("Q5_K", 4100))]
-    assert all(_tile_rows(w.format.name, m, *w.shape) >= 0 for w in ws)
+    assert all(kq_tile_rows(w.format.name, m, *w.shape) >= 0 for w in ws)
     x = torch.randn(m, k, device="cuda", generator=gen)
     want = [ops.quant_matmul(x, w) for w in ws]
     before = ops.launch_count()
@@ -147,10 +139,10 @@ def test_extreme_codes(oracle):
 @pytest.mark.parametrize("fill", [0xFF, 0x00, 0xF0, 0x0F])
 def test_extreme_codes_in_tiles(oracle, fmt, m, n, k, fill):
     """The same in the tensor-core kernel: every code, scale and min at an end of its range, activations of one sign and of
-    alternating ones, so that the sums of one-byte and of two-byte products reach their bounds."""
+    alternating ones, so that the sums reach their bounds."""
     from boostr_b200 import ops
 
-    assert _tile_rows(fmt, m, n, k) > 0
+    assert kq_tile_rows(fmt, m, n, k) > 0
     w = np.full((n * k // 256, F[fmt].block_bytes), fill, np.uint8)
     one = np.frombuffer(np.array([1.0], np.float16).tobytes(), np.uint8)
     for at in {"Q2_K": (80, 82), "Q3_K": (108,), "Q4_K": (0, 2), "Q5_K": (0, 2)}[fmt]:
