@@ -8,7 +8,7 @@ import re
 import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "boostr_b200", "csrc")
-EVENT = re.compile(r"(?<!\w)(?P<wait>(?:i8_wait|pf_wait|mbar_wait|wait|take)\()|(?P<fence>tc_(?:fence_)?after\(\)|tcgen05\.fence::after_thread_sync)"
+EVENT = re.compile(r"(?<!\w)(?P<wait>(?:i8_wait|pf_wait|mbar_wait|wait|wait_cluster|take)\()|(?P<fence>tc_(?:fence_)?after\(\)|tcgen05\.fence::after_thread_sync)"
                    r"|(?P<access>tmem_st\d+\(|tmem_ld\d+(?:_async)?\(|tc_mma_\w+\(|mma_\w+_ts\()")
 
 
