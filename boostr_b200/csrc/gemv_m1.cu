@@ -29,6 +29,8 @@
 
 namespace b200q {
 
+bool gemv_m1_f32_supported(int fmt, size_t M, size_t K, size_t N);
+int gemv_m1_f32_ring_depth(int fmt, size_t K);
 
 // Where the launch AFTER this one starts to read, so that this launch can pull those bytes into L2 while its
 // own ring drains.  A space is the virtual row range of up to three weights (or gate + up) that the next
@@ -700,6 +702,10 @@ bool gemv_m1_supported(int fmt, size_t M, size_t K, size_t N, bool swiglu) {
 }
 
 constexpr size_t M1_SMEM_MAX = 232448 - 1024;
+// RING_GROUPS: the rings of the one-row kernels are a multiple of the four warp groups deep, so that a slot belongs to ONE group, which
+// sees every phase of its barriers.  In a ring of 13 (K = 3840) the groups took turns at a slot; a group some five fills ahead of another
+// could wait for phase k while the slot was still in phase k - 1, which a wait by parity takes for done, and read, release and refill a
+// slot that others had yet to fill: copies could still be on their way when their CTA left.
 
 // Fills in the Q6_K parameters for a launch on at most `max_grid` CTAs; returns the grid, 0 if none.
 static size_t setup_q6k(GemvM1Q6Params& p, uint32_t& nchunk, size_t& smem, const void* act, int act_dtype, const void* w, void* out,
@@ -721,6 +727,7 @@ static size_t setup_q6k(GemvM1Q6Params& p, uint32_t& nchunk, size_t& smem, const
     p.stage_off = (p.act_off + p.nblk * ACT6_STRIDE + 127) & ~127u;
     p.nstages = (uint32_t)((M1_SMEM_MAX - p.stage_off - 64) / p.stage_bytes);
     if (p.nstages > 16) p.nstages = 16;
+    p.nstages &= ~3u;  // see RING_GROUPS
     // never fewer than ~16 rows per CTA
     size_t grid = (N + 15) / 16;
     if (grid > max_grid) grid = max_grid;
@@ -760,6 +767,7 @@ static size_t setup_q4k(GemvM1Params& p, size_t& smem, const void* act, int act_
     p.stage_off = (p.act_off + 16 * ACT_STRIDE + 127) & ~127u;
     p.nstages = (uint32_t)((M1_SMEM_MAX - p.stage_off) / p.stage_bytes);
     if (p.nstages > 16) p.nstages = 16;
+    p.nstages &= ~3u;  // see RING_GROUPS
     size_t grid = (N + 15) / 16;
     if (grid > max_grid) grid = max_grid;
     p.rows_per_cta = (uint32_t)((N + grid - 1) / grid);
@@ -1069,3 +1077,22 @@ cudaError_t launch_tp_all_reduce(float* data, size_t count, const PeerComm& comm
 }
 
 }  // namespace b200q
+
+// Ring depth of the one-row kernels (0: another path).  Not part of the C ABI: a test holds it to a multiple of the warp groups.
+extern "C" __attribute__((visibility("default"))) int b200q_m1_ring_depth(int fmt, size_t K, int swiglu) {
+    using namespace b200q;
+    if (gemv_m1_f32_supported(fmt, 1, K, 1)) return swiglu ? 0 : gemv_m1_f32_ring_depth(fmt, K);
+    if (!gemv_m1_supported(fmt, 1, K, 1, swiglu != 0)) return 0;
+    size_t smem, n = 4096;
+    void* out = nullptr;
+    const void* w = nullptr;
+    uint32_t nchunk;
+    if (fmt == FMT_Q6_K) {
+        GemvM1Q6Params p;
+        setup_q6k(p, nchunk, smem, nullptr, DT_F32, w, nullptr, DT_F32, K, n, 148, nullptr);
+        return (int)p.nstages;
+    }
+    GemvM1Params p;
+    setup_q4k(p, smem, nullptr, DT_F32, 1, &w, &n, &out, swiglu ? &n : nullptr, DT_F32, K, 148, nullptr);
+    return (int)p.nstages;
+}

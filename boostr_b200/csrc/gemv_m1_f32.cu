@@ -447,15 +447,11 @@ bool gemv_m1_f32_supported(int fmt, size_t M, size_t K, size_t N) {
     return M == 1 && N >= 1 && (fmt == FMT_Q8_0 || fmt == FMT_Q4_0) && K % 32 == 0 && K >= 32 && K <= 8192;
 }
 
-cudaError_t launch_gemv_m1_f32(int fmt, const void* act, int act_dtype, const void* w, void* out, int out_dtype, size_t K,
-                               size_t N, int sm_count, cudaStream_t st, unsigned int* status) {
-    constexpr size_t SMEM_MAX = 232448 - 1024;
-    GemvM1F32Params p{};
-    p.w = static_cast<const uint8_t*>(w);
-    p.act = act;
-    p.out = out;
+namespace {
+constexpr size_t SMEM_MAX = 232448 - 1024;
+// Geometry of the ring.  Its depth is a multiple of the four warp groups, so that a slot belongs to one of them (gemv_m1.cu, RING_GROUPS).
+void setup_f32(GemvM1F32Params& p, int fmt, size_t K) {
     p.K = (uint32_t)K;
-    p.N = (uint32_t)N;
     p.nblk = (uint32_t)(K / 32);
     p.row_bytes = p.nblk * (fmt == FMT_Q8_0 ? 34u : 18u);
     p.rpw = 18432 / (4 * p.row_bytes);  // fills of about 18 KB
@@ -468,6 +464,24 @@ cudaError_t launch_gemv_m1_f32(int fmt, const void* act, int act_dtype, const vo
     p.stage_off = pieces ? (p.part_off + 16 * 4 * p.rpw * 16 + 127) & ~127u : (p.x_off + p.nblk * 36 * 4 + 127) & ~127u;
     p.nstages = (uint32_t)((SMEM_MAX - p.stage_off - 64) / p.stage_bytes);
     if (p.nstages > 16) p.nstages = 16;
+    p.nstages &= ~3u;
+}
+}  // namespace
+int gemv_m1_f32_ring_depth(int fmt, size_t K) {
+    GemvM1F32Params p{};
+    setup_f32(p, fmt, K);
+    return (int)p.nstages;
+}
+
+cudaError_t launch_gemv_m1_f32(int fmt, const void* act, int act_dtype, const void* w, void* out, int out_dtype, size_t K,
+                               size_t N, int sm_count, cudaStream_t st, unsigned int* status) {
+    GemvM1F32Params p{};
+    p.w = static_cast<const uint8_t*>(w);
+    p.act = act;
+    p.out = out;
+    p.N = (uint32_t)N;
+    setup_f32(p, fmt, K);
+    const bool pieces = K % 256 == 0;
     size_t grid = (N + 15) / 16;
     if (grid > (size_t)sm_count) grid = sm_count;
     p.rows_per_cta = (uint32_t)((N + grid - 1) / grid);
