@@ -142,7 +142,7 @@ __device__ __forceinline__ void fill_contiguous(uint32_t dst_s, uint8_t* dst_g, 
 // stream is still draining (launch_pdl below).  grid_dep_launch() lets the NEXT grid start early;
 // grid_dep_wait() blocks until the PREVIOUS grid has completed and its writes are visible — it
 // must precede the first read of activations and the first write of any output or scratch.
-// Packed weights: the kernels for few rows (gemv*.cu, smallm_i8.cu, Q4_K and Q5_K in kquant_i8.cu) fetch them before the wait,
+// Packed weights: the kernels for few rows (gemv*.cu, smallm_i8.cu, kquant_few.cu) fetch them before the wait,
 // so a weight that the kernel before the call is still writing must be ordered by the caller (include/b200q.h).  Prompt
 // products and Q2_K / Q3_K products fetch theirs early only behind a kernel of the same call, which has itself waited for what
 // came before.

@@ -22,12 +22,13 @@
 // to it from all CTAs by st.async into shared memory and are added in K order while the next round is drained, so the results
 // have the CPU's bits at every K.  (Shares of K added as sums, which have other bits, are up to 15 % faster at K = 14336: 4096 x 14336 at 37
 // rows Q4_K 25.7 against 27.1 us.  Up to K = 4096 the exchange by rounds is the faster one too: 4096 x 4096 at 37 rows Q4_K 14.8 -> 11.1 us.)
-// What bounds it: instructions.  A block costs some 4600 (Q4_K) or 6800 (Q6_K) warp instructions, issue slots 58 % busy, the ALU
-// pipe 38 / 61 %; the MMAs themselves take 10 ... 20 cycles each with the A operand in tensor memory (34 ... 38 from shared memory).  One
-// MMA-issuing warp spent 90 cycles on each and set the pace (2.0 us a Q4_K block instead of 0.9 at 16 rows), hence two.
-// Measured, us (graph replays, before -> now): 14336 x 4096 at 24 / 37 / 63 rows Q4_K 20.5 / 25.2 / 40.3 -> 19.8 / 22.3 / 36.8, Q5_K 26.2 / 28.3 /
-// 49.5 -> 23.0 / 25.4 / 42.6, Q6_K 41.9 / 60.3 / 81.0 -> 26.0 / 27.4 / 47.0; 4096 x 14336 at 37 rows 47.9, 56.3, 60.0 -> 25.2, 27.6, 30.4; SwiGLU
-// 2 x 14336 x 4096 at 37 rows 52.9, 59.2, 118 -> 48.9, 56.8, 53.1; Q6_K 128256 x 4096 at 37 rows 378 -> 158.
+// What bounds it: instructions.  At 37 rows a block costs some 5500 (Q4_K), 6700 (Q5_K) or 7200 (Q6_K) warp instructions, in a cluster 1600 more; issue
+// slots 59 ... 63 % busy, the ALU pipe 36 / 44 / 59 %; the MMAs themselves take 10 ... 20 cycles each with the A operand in tensor memory (34 ... 38 from
+// shared memory).  One MMA-issuing warp spent 90 cycles on each and set the pace (2.0 us a Q4_K block instead of 0.9 at 16 rows), hence two.
+// Measured, us (graph replays; the kernels that took these rows before -> here): 14336 x 4096 at 24 / 40 / 63 rows Q4_K 21.2 / 25.5 / 41.2 -> 18.7 / 21.2 / 34.5,
+// Q5_K 26.9 / 28.9 / 50.1 -> 22.8 / 24.9 / 42.0, Q6_K 40.8 / 59.7 / 80.6 -> 26.0 / 27.2 / 46.6; 4096 x 14336 at 40 rows 49.2, 56.6, 60.4 -> 27.3, 29.7, 33.0; 4096 x
+// 4096 at 40 rows 21.1, 25.8, 26.9 -> 10.9, 11.9, 12.8; SwiGLU 2 x 14336 x 4096 at 40 rows 53.8, 60.6, 120 -> 41.8, 51.4, 51.4, 2 x 14336 x 1024 Q4_K 20.7 -> 17.2,
+// Q5_K 22.9 -> 20.3 (with the lanes of gate alone gating 20.3 and 24.1); Q6_K 128256 x 4096 at 37 rows 378 -> 158.
 // Every wait is bounded; on a timeout the CTA is marked dead, records a status and frees its tensor memory.
 #include <cuda.h>
 
